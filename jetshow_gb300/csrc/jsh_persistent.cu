@@ -22,16 +22,22 @@
 // rotation.  Intensities are scaled by a per-frequency power of two and
 // lengths are in pc so the FP32 state stays well inside its range.
 //
-// Code size matters as much as arithmetic here: the stages run as a rolled
-// loop over a __constant__ tableau with the stage derivatives in shared
-// memory, so the coefficient code exists once per kernel and the kernel
-// fits the SM instruction caches even when the lanes of a warp are in
-// different phases.
+// A step's coefficients depend on the stage points alone, so they are
+// evaluated before the stages: five independent chains instead of six
+// dependent ones (the last two stages share their point), the stage
+// derivatives in registers and the stages unrolled.  On the 512x1024 conical
+// jet the render went from 2.76 to 2.25 ms, on its 102x333 image (set by the
+// heaviest ray's chain of steps) from 1.29 to 0.99 ms, on a ParabaloidCone
+// image with the Faraday-thick mode from 71 to 40 ms.  The kernels for every
+// field law keep one copy of the coefficient code (a rolled loop over the
+// points, the coefficients in shared memory), so that they fit the SM
+// instruction caches even when the lanes of a warp are in different phases.
 #include <float.h>
 #include <math.h>
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 #include "jsh_batch.cuh"
@@ -92,13 +98,19 @@ __host__ __device__ constexpr float dp_a32(int s, int j) {
 
 // Dormand-Prince nodes c, error weights e = b - b_hat and dense-output
 // weights d in FP32.
+__host__ __device__ constexpr float dp_c32(int s) {
+  return s == 1 ? (float)dp::C2 : s == 2 ? (float)dp::C3 : s == 3 ? (float)dp::C4 : s == 4 ? (float)dp::C5
+       : s >= 5 ? 1.f : 0.f;
+}
+__host__ __device__ constexpr float dp_e32(int j) {
+  return j == 0 ? (float)dp::E1 : j == 2 ? (float)dp::E3 : j == 3 ? (float)dp::E4 : j == 4 ? (float)dp::E5
+       : j == 5 ? (float)dp::E6 : j == 6 ? (float)dp::E7 : 0.f;
+}
 __constant__ float c_C[7] = {0, (float)dp::C2, (float)dp::C3, (float)dp::C4, (float)dp::C5, 1.f, 1.f};
 __constant__ float c_E[7] = {(float)dp::E1, 0, (float)dp::E3, (float)dp::E4, (float)dp::E5, (float)dp::E6,
                              (float)dp::E7};
 __constant__ float c_D[7] = {(float)dp::D1, 0, (float)dp::D3, (float)dp::D4, (float)dp::D5, (float)dp::D6,
                              (float)dp::D7};
-// 5th-order weights b of the first six stages (b_7 = 0)
-__constant__ float c_B[6] = {(float)dp::B1, 0, (float)dp::B3, (float)dp::B4, (float)dp::B5, (float)dp::B6};
 
 // Compensated FP32 pair x = hi + lo, |lo| <= ulp(hi) / 2 (about 48 bits):
 // the step-control state (segment coordinate, remainder, optical depth,
@@ -174,40 +186,31 @@ struct Lane {
   int32_t tri;           // gridded fields on one grid: triangle of the last evaluation (-1: none)
 };
 
-// Stage derivatives of this thread, thread-major: t[s * NK + c] with t =
-// shared + tid * W.  Every access is a compile-time offset from one base
-// register (no per-access address arithmetic), and W = 35 or 7 floats maps
-// a warp's 32 threads onto 32 distinct banks (W odd).  W is the per-thread
-// region of the kernel's buffer, so a one-component view of a 5-component
-// buffer (the single-kernel form's tau lanes) stays inside its own thread.
-template <int NK, int W = 7 * NK>
-struct Stages {
-  float* t;
-  __device__ __forceinline__ float& operator()(int s, int c) const { return t[s * NK + c]; }
+// Stage storage of this thread in shared memory, thread-major: t = shared +
+// tid * stride, every access a fixed offset from one base register, and the
+// odd stride maps a warp's 32 threads onto 32 distinct banks.  It holds the
+// stages' k_I of a Dormand-Prince tau pass (7 words) or, in the kernels
+// built for every field law, the coefficients of an I/IQUV step's stage
+// points (StageWidth<FULL>::kWords).
+template <bool FULL>
+struct StageWidth {
+  static constexpr int NK = FULL ? 5 : 1;        // stage components: the IQUV state and chi, or I only
+  static constexpr int NX = FULL ? 4 : 1;
+  static constexpr int NC = FULL ? 8 : 2;        // coefficients of a stage point
+  static constexpr int kWords = FULL ? 49 : 13;  // six points, odd
 };
+constexpr int kTauWords = 7;
 
-// acc = sum_{j < S} a_Sj K_j with S and j compile-time: the tableau entries
-// are immediate operands and the S*NK shared loads are independent.
-template <int S, int NK, int W>
-__device__ __forceinline__ void combine_stage(const Stages<NK, W>& K, float* acc) {
+// acc = sum_{j < S} a_Sj K_j over the stage derivatives held in registers
+// (S and j compile-time: the tableau entries are immediate operands).
+template <int S, int NK>
+__device__ __forceinline__ void combine_stage(const float (&K)[7][NK], float* acc) {
 #pragma unroll
   for (int c = 0; c < NK; ++c) acc[c] = 0.f;
 #pragma unroll
   for (int j = 0; j < S; ++j) {
 #pragma unroll
-    for (int c = 0; c < NK; ++c) acc[c] = fmaf(dp_a32(S, j), K(j, c), acc[c]);
-  }
-}
-
-template <int NK, int W>
-__device__ __forceinline__ void combine(int s, const Stages<NK, W>& K, float* acc) {
-  switch (s) {
-    case 1: combine_stage<1, NK, W>(K, acc); break;
-    case 2: combine_stage<2, NK, W>(K, acc); break;
-    case 3: combine_stage<3, NK, W>(K, acc); break;
-    case 4: combine_stage<4, NK, W>(K, acc); break;
-    case 5: combine_stage<5, NK, W>(K, acc); break;
-    default: combine_stage<6, NK, W>(K, acc); break;
+    for (int c = 0; c < NK; ++c) acc[c] = fmaf(dp_a32(S, j), K[j][c], acc[c]);
   }
 }
 
@@ -493,21 +496,15 @@ __device__ __noinline__ double crossing_time(double tau_old, double t_old, doubl
   return 0.5 * (t0 + t1);
 }
 
-// Coefficients and Stokes derivatives of the I/IQUV pass (one call site per
-// kernel); `full` = false stops after k_I, eta_I (I-only output).  Returns
-// the magnitude of the terms summed into the derivatives (eta_I + k_I |I|):
-// the scale of their FP32 rounding noise.
-template <bool GENERAL>
-__device__ __forceinline__ float rhs32(const JshRequest& R, const JshFreqConst& F, bool full, F3 p, const float* y,
-                                       float cs, float sn, float* dk, float& kI, uint32_t rk_h, uint32_t rk_f,
-                                       uint32_t rk_e, int* tri, bool ft = false, float* cpl = nullptr) {
-  Coef32 c;
-  coef32_rt<GENERAL>(R, F, p, full ? COEF_FULL : COEF_I, c, rk_h, rk_f, rk_e, tri);
-  kI = c.kI;
+// Stokes derivatives of the I/IQUV pass from the coefficients of the stage's
+// point.  Returns the magnitude of the terms summed into the derivatives
+// (eta_I + k_I |I|): the scale of their FP32 rounding noise.
+template <bool FULL>
+__device__ __forceinline__ float stokes_rhs(const Coef32& c, const float* y, float cs, float sn, float* dk,
+                                            bool ft, float* cpl) {
   const float scale = fabsf(c.eI) + fabsf(c.kI * y[0]);
-  if (!full) {
+  if (!FULL) {
     dk[0] = c.eI - c.kI * y[0];
-    dk[1] = dk[2] = dk[3] = dk[4] = 0.f;
     return scale;
   }
   if (ft) {
@@ -670,14 +667,6 @@ constexpr float kFtAxis = 0.25f;  // largest step / distance from the jet axis
 __device__ __forceinline__ float ft_tolerance(float I, float rtol, float atol) {
   return kFtTol * fmaf(rtol, fabsf(I), atol);
 }
-
-// Stage components of the I/IQUV pass's Dormand-Prince machine: the IQUV
-// state and chi (full Stokes) or I only.
-template <bool FULL>
-struct StageWidth {
-  static constexpr int NK = FULL ? 5 : 1;
-  static constexpr int NX = FULL ? 4 : 1;
-};
 
 // ---------------------------------------------------------------- tau pass
 // The tau pass integrates dtau/dt = k_I along each segment.  Its right-hand
@@ -980,9 +969,9 @@ abort:
 // quadrature panel's error estimate can miss a jump between its nodes).
 // dtau/dt = k_I does not depend on the state, so only the last stage
 // combination (the increment) is formed.
-template <int PASS, bool GENERAL, int W>
-__device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __restrict__ reqs, const Stages<1, W>& K,
-                                               int part, Tally& T) {
+template <int PASS, bool GENERAL>
+__device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __restrict__ reqs, float* K, int part,
+                                               Tally& T) {
   const JshRequest& R = reqs[L.r];
   const JshFreqConst F = R.mix.fc[L.f];
   const F3 dirf = f3(-R.mix.nl[0], -R.mix.nl[1], -R.mix.nl[2]);
@@ -1019,24 +1008,27 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
       L.evals++;
       L.init = true;
     }
-    K(0, 0) = L.k1[0];
-    float inc = 0.f;
+    K[0] = L.k1[0];
+    // k_I does not depend on the state, and the last two stages share their
+    // point (c = 1): five evaluations serve the six stages, unless every
+    // evaluation draws its own random direction
+    const int np = R.model.rnd_kind == JSH_RND_POINTS ? 6 : 5;
 #pragma unroll 1
-    for (int s = 1; s < 7; ++s) {
-      if (s == 6) {
-        float acc[1];
-        combine<1, W>(6, K, acc);
-        inc = h * acc[0];
-      }
+    for (int s = 1; s <= np; ++s) {
       Coef32 c;
       coef32_rt<GENERAL>(R, F, pn + dirf * (c_C[s] * h), COEF_KI, c, L.h, (uint32_t)L.f,
                          L.evals + (uint32_t)(s - 1), &L.tri);
-      K(s, 0) = c.kI;
+      K[s] = c.kI;
     }
+    if (np == 5) K[6] = K[5];
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) acc = fmaf(dp_a32(6, j), K[j], acc);
+    const float inc = h * acc;
     L.evals += 6;
     float a = 0.f;
 #pragma unroll
-    for (int j = 0; j < 7; ++j) a = fmaf(c_E[j], K(j, 0), a);
+    for (int j = 0; j < 7; ++j) a = fmaf(c_E[j], K[j], a);
     const float adt = fabsf(h);
     // no cancellation in dtau/dt = k_I: the plain odeint norm
     const float e = fabsf(h * a) / fmaf(rtol, fmaf(adt, fabsf(L.k1[0]), fabsf(L.tau_seg.hi)), atol);
@@ -1092,8 +1084,8 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
     if (L.tau_seg.hi > R.mix.tau_max_hi || (L.tau_seg.hi == R.mix.tau_max_hi && L.tau_seg.lo >= R.mix.tau_max_lo)) {
       L.status |= JSH_ST_TAU_CROSSED;
       const double t_old = df_val(t_prev);
-      double tc = crossing_time(df_val(tau_prev), t_old, (double)h, h, K(0, 0), K(2, 0), K(3, 0), K(4, 0),
-                                K(5, 0), K(6, 0), inc, R.P.tau_max, R.P.tau_precision);
+      double tc = crossing_time(df_val(tau_prev), t_old, (double)h, h, K[0], K[2], K[3], K[4], K[5], K[6], inc,
+                                R.P.tau_max, R.P.tau_precision);
       if (tc < 0.0) {
         // the reference keeps bisecting; stop at the last bracket's midpoint
         L.status |= JSH_ST_BISECT_LIMIT;
@@ -1109,7 +1101,7 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
       tau_pass_done<PASS>(L, reqs, part, T);
       return;
     }
-    L.k1[0] = K(6, 0);
+    L.k1[0] = K[6];
     return;
   }
 
@@ -1135,11 +1127,10 @@ abort:
 // benchmark family (helical conical B and BK n in the plasma frame, flat
 // flow), a Dormand-Prince attempt otherwise.  The choice belongs to the
 // request, so every build of the kernels gives the same bits.
-template <int PASS, bool GENERAL, int W>
-__device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__ reqs, const Stages<1, W>& K1,
-                                         int part, Tally& T) {
+template <int PASS, bool GENERAL>
+__device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__ reqs, float* K, int part, Tally& T) {
   if (!GENERAL || reqs[L.r].mix.helical_log) tau_panel_step<PASS, GENERAL>(L, reqs, part, T);
-  else tau_dopri_step<PASS, GENERAL, W>(L, reqs, K1, part, T);
+  else tau_dopri_step<PASS, GENERAL>(L, reqs, K, part, T);
 }
 
 // ------------------------------------------------------- I / IQUV pass
@@ -1148,8 +1139,7 @@ __device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__
 // every form (static, single-kernel, split), so the images are bitwise the
 // same.
 template <bool FULL, int PASS, bool GENERAL = true>
-__device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict__ reqs,
-                                          const Stages<StageWidth<FULL>::NK>& K, Tally& T) {
+__device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict__ reqs, float* Q, Tally& T) {
   constexpr int NK = StageWidth<FULL>::NK;
   constexpr int NX = StageWidth<FULL>::NX;
   const JshRequest& R = reqs[L.r];
@@ -1196,19 +1186,20 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     if (FULL) sincosf(L.chi.hi, &s0, &c0);
     const float h = L.dt;
     const bool ft = kFtm && FULL && L.ft;
-    float dk[5], cpl = 0.f;  // cpl: Faraday-thick mode, max(|k_Q|, |k_C|) / |lambda| of the last evaluation
+    float cpl = 0.f;  // Faraday-thick mode: max(|k_Q|, |k_C|) / |lambda| of the last evaluation
+    constexpr int mode = FULL ? COEF_FULL : COEF_I;
     if (!L.init) {
-      L.s1 = rhs32<GENERAL>(R, F, FULL, pn, L.x, c0, s0, dk, L.kI1, L.h, (uint32_t)L.f, L.evals0 + L.evals, &L.tri,
-                            ft, &cpl);
-#pragma unroll
-      for (int c = 0; c < NK; ++c) L.k1[c] = dk[c];
+      Coef32 c;
+      coef32_rt<GENERAL>(R, F, pn, mode, c, L.h, (uint32_t)L.f, L.evals0 + L.evals, &L.tri);
+      L.s1 = stokes_rhs<FULL>(c, L.x, c0, s0, L.k1, ft, &cpl);
+      L.kI1 = c.kI;
       L.evals++;
       L.init = true;
       if (ft) {
         // entry: the transient carried in, d = (q, u) - e^{-i chi} S / lambda,
         // must be small enough that the rotating coupling the mode leaves
         // out of I and V stays within the tolerance
-        const float dq = L.x[1] - dk[1], du = L.x[2] - dk[2];
+        const float dq = L.x[1] - L.k1[1], du = L.x[2] - L.k1[2];
         if (!(cpl * sqrtf(fmaf(dq, dq, du * du)) <= ft_tolerance(L.x[0], rtol, atol))) {
           L.ft = 0;
           L.ft_cool = kFtCooldown;
@@ -1217,15 +1208,48 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
         }
       }
     }
+    // The coefficients depend on the stage's point alone, not on the state,
+    // and the last two stages share their point (c = 1): all five points are
+    // evaluated before the stages, so that their chains of dependent
+    // operations overlap.  The fused build keeps them in registers; the
+    // builds for every field law (one copy of that code) in shared memory,
+    // with a sixth point where every evaluation draws a random direction.
+    Coef32 C[5];
+    const bool six = GENERAL && R.model.rnd_kind == JSH_RND_POINTS;
+    if (GENERAL) {
+      const int np = six ? 6 : 5;
+#pragma unroll 1
+      for (int s = 1; s <= np; ++s) {
+        Coef32 c;
+        coef32_rt<GENERAL>(R, F, pn + dirf * (c_C[s] * h), mode, c, L.h, (uint32_t)L.f,
+                           L.evals0 + L.evals + (uint32_t)(s - 1), &L.tri);
+        float* q = Q + (s - 1) * StageWidth<FULL>::NC;
+        q[0] = c.kI;
+        q[1] = c.eI;
+        if (FULL) {
+          q[2] = c.kQ;
+          q[3] = c.kV;
+          q[4] = c.kF;
+          q[5] = c.kC;
+          q[6] = c.eQ;
+          q[7] = c.eV;
+        }
+      }
+    } else {
 #pragma unroll
-    for (int c = 0; c < NK; ++c) K(0, c) = L.k1[c];
+      for (int s = 1; s <= 5; ++s)
+        coef32_rt<GENERAL>(R, F, pn + dirf * (dp_c32(s) * h), mode, C[s - 1], L.h, (uint32_t)L.f, 0, &L.tri);
+    }
+    float K[7][NK];
+#pragma unroll
+    for (int c = 0; c < NK; ++c) K[0][c] = L.k1[c];
     float inc[NK];
     float smax = L.s1, s7 = 0.f, kI7 = 0.f;
-#pragma unroll 1
-    for (int s = 1; s < 7; ++s) {
+    auto stage = [&](auto S) {
+      constexpr int s = decltype(S)::value;
       float acc[NK];
-      combine<NK>(s, K, acc);
-      float y[4];
+      combine_stage<s, NK>(K, acc);
+      float y[4], dk[5];
 #pragma unroll
       for (int c = 0; c < 4; ++c) y[c] = (c < NX) ? fmaf(h, acc[c < NK ? c : 0], L.x[c]) : 0.f;
       float cs = c0, sn = s0;
@@ -1235,10 +1259,26 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
         cs = c0 * cd - s0 * sd;
         sn = s0 * cd + c0 * sd;
       }
-      const float sc = rhs32<GENERAL>(R, F, FULL, pn + dirf * (c_C[s] * h), y, cs, sn, dk, kI7, L.h, (uint32_t)L.f,
-                                      L.evals0 + L.evals + (uint32_t)(s - 1), &L.tri, ft, &cpl);
+      Coef32 c;
+      if (GENERAL) {
+        const float* q = Q + (s == 6 ? (six ? 5 : 4) : s - 1) * StageWidth<FULL>::NC;
+        c.kI = q[0];
+        c.eI = q[1];
+        if (FULL) {
+          c.kQ = q[2];
+          c.kV = q[3];
+          c.kF = q[4];
+          c.kC = q[5];
+          c.eQ = q[6];
+          c.eV = q[7];
+        }
+      } else {
+        c = C[s == 6 ? 4 : s - 1];
+      }
+      const float sc = stokes_rhs<FULL>(c, y, cs, sn, dk, ft, &cpl);
       smax = fmaxf(smax, sc);
       s7 = sc;
+      kI7 = c.kI;
       if (ft && s < 6) {
         // Faraday-thick mode: the inner stages' (q, u) slots are free (no
         // stage point uses (q, u)); they keep the stage's k_I and its coupling
@@ -1250,12 +1290,18 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
         dk[1] = kI7;
       }
 #pragma unroll
-      for (int c = 0; c < NK; ++c) K(s, c) = dk[c];
+      for (int c = 0; c < NK; ++c) K[s][c] = dk[c];
       if (s == 6) {
 #pragma unroll
         for (int c = 0; c < NK; ++c) inc[c] = h * acc[c];
       }
-    }
+    };
+    stage(std::integral_constant<int, 1>());
+    stage(std::integral_constant<int, 2>());
+    stage(std::integral_constant<int, 3>());
+    stage(std::integral_constant<int, 4>());
+    stage(std::integral_constant<int, 5>());
+    stage(std::integral_constant<int, 6>());
     L.evals += 6;
     // embedded error estimate and odeint's default error checker:
     // max_i |err_i| / (atol + rtol (|x_i| + |dt| |x'_i|))
@@ -1264,7 +1310,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     for (int c = 0; c < NK; ++c) {
       float a = 0.f;
 #pragma unroll
-      for (int j = 0; j < 7; ++j) a = fmaf(c_E[j], K(j, c), a);
+      for (int j = 0; j < 7; ++j) a = fmaf(dp_e32(j), K[j][c], a);
       err[c] = h * a;
     }
     // FP32 resolution floor: an error estimate below the rounding noise of
@@ -1309,16 +1355,16 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
           sn6 = s0 * cd + c0 * sd;
         }
         float cpl_max = cpl;
-        bool ft_ok = fabsf(K(6, NK - 1)) >= kFtRatio * kI7;
+        bool ft_ok = fabsf(K[6][NK - 1]) >= kFtRatio * kI7;
 #pragma unroll
-        for (int j = 1; j < 6; ++j) cpl_max = fmaxf(cpl_max, K(j, 2));
+        for (int j = 1; j < 6; ++j) cpl_max = fmaxf(cpl_max, K[j][2]);
         ft_ok = ft_ok && cpl_max < INFINITY;
         const float ft_tol = ft_tolerance(L.x[0], rtol, atol);
-        const float p0r = c0 * K(0, 1) - s0 * K(0, 2), p0i = s0 * K(0, 1) + c0 * K(0, 2);
-        const float p6r = cs6 * K(6, 1) - sn6 * K(6, 2), p6i = sn6 * K(6, 1) + cs6 * K(6, 2);
+        const float p0r = c0 * K[0][1] - s0 * K[0][2], p0i = s0 * K[0][1] + c0 * K[0][2];
+        const float p6r = cs6 * K[6][1] - sn6 * K[6][2], p6i = sn6 * K[6][1] + cs6 * K[6][2];
         const float dr = p6r - p0r, di = p6i - p0i;
-        const float lam = sqrtf(fmaf(kI7, kI7, K(6, NK - 1) * K(6, NK - 1)));
-        const float dq = L.x[1] - K(0, 1), du = L.x[2] - K(0, 2);
+        const float lam = sqrtf(fmaf(kI7, kI7, K[6][NK - 1] * K[6][NK - 1]));
+        const float dq = L.x[1] - K[0][1], du = L.x[2] - K[0][2];
         if (!ft_ok || !(sqrtf(fmaf(dr, dr, di * di)) <= adt * lam * ft_tol) ||
             !(cpl_max * sqrtf(fmaf(dq, dq, du * du)) <= ft_tol)) {
           L.ft = 0;
@@ -1371,12 +1417,12 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     if (ft) {
       // quasi-static part at the end plus the transient, decayed by the
       // step's optical depth (h sum b_j k_I,j over the stages)
-      float btau = c_B[0] * L.kI1;
+      float btau = dp_a32(6, 0) * L.kI1;
 #pragma unroll
-      for (int j = 1; j < 6; ++j) btau = fmaf(c_B[j], K(j, 1), btau);
+      for (int j = 1; j < 6; ++j) btau = fmaf(dp_a32(6, j), K[j][1], btau);
       const float decay = expf(-h * btau);
-      qn = fmaf(L.x[1] - K(0, 1), decay, K(6, 1));
-      un = fmaf(L.x[2] - K(0, 2), decay, K(6, 2));
+      qn = fmaf(L.x[1] - K[0][1], decay, K[6][1]);
+      un = fmaf(L.x[2] - K[0][2], decay, K[6][2]);
     }
 #pragma unroll
     for (int c = 0; c < NX; ++c) L.x[c] += inc[c];
@@ -1395,7 +1441,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
       }
     }
 #pragma unroll
-    for (int c = 0; c < NK; ++c) L.k1[c] = K(6, c);
+    for (int c = 0; c < NK; ++c) L.k1[c] = K[6][c];
     L.s1 = s7;
     L.kI1 = kI7;
     if (kFtm && FULL && !ft) {
@@ -1426,7 +1472,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
         }
       }
     }
-    return;
+    if (!L.last) return;
   }
 
 segment_done : {
@@ -1453,11 +1499,10 @@ abort:
 
 // One step of an active lane in whichever pass it is.
 template <bool FULL, int PASS, bool GENERAL = true>
-__device__ __forceinline__ void lane_advance(Lane& L, const JshRequest* __restrict__ reqs,
-                                             const Stages<StageWidth<FULL>::NK>& K, Tally& T, int part = 0) {
-  if (PASS == PASS_BOTH && L.phase == PH_TAU)
-    tau_step<PASS, GENERAL, 7 * StageWidth<FULL>::NK>(L, reqs, Stages<1, 7 * StageWidth<FULL>::NK>{K.t}, part, T);
-  else lane_step<FULL, PASS, GENERAL>(L, reqs, K, T);
+__device__ __forceinline__ void lane_advance(Lane& L, const JshRequest* __restrict__ reqs, float* Q, Tally& T,
+                                             int part = 0) {
+  if (PASS == PASS_BOTH && L.phase == PH_TAU) tau_step<PASS, GENERAL>(L, reqs, Q, part, T);
+  else lane_step<FULL, PASS, GENERAL>(L, reqs, Q, T);
 }
 
 // ------------------------------------------------------------- ranking
@@ -1544,7 +1589,7 @@ __global__ void __launch_bounds__(128) transfer_static_mixed_kernel(const JshReq
   extern __shared__ float ksh[];
   batch_prefix(reqs, n_req, base);
   const unsigned long long w = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const Stages<FULL ? 5 : 1> K{ksh + threadIdx.x * (FULL ? 35 : 7)};
+  float* K = ksh + threadIdx.x * StageWidth<FULL>::kWords;
   Tally T = tally_new();
   if (w < base[n_req]) {
     Lane L;
@@ -1567,7 +1612,7 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 3 : 1)
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
   extern __shared__ float ksh[];
   batch_prefix(reqs, n_req, base);
-  const Stages<FULL ? 5 : 1> K{ksh + threadIdx.x * (FULL ? 35 : 7)};
+  float* K = ksh + threadIdx.x * StageWidth<FULL>::kWords;
   const unsigned long long total = base[n_req];
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -1635,7 +1680,7 @@ __global__ void __launch_bounds__(256, GENERAL ? 2 : 3) transfer_tau_kernel(cons
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
   extern __shared__ float ksh[];
   tau_prefix(reqs, n_req, part, base);
-  const Stages<1> K1{ksh + threadIdx.x * 7};
+  float* K1 = ksh + threadIdx.x * kTauWords;
   const unsigned long long total = base[n_req];
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -1736,7 +1781,7 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 3 : 1)
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
   extern __shared__ float ksh[];
   iquv_prefix(reqs, n_req, part, base);
-  const Stages<FULL ? 5 : 1> K{ksh + threadIdx.x * (FULL ? 35 : 7)};
+  float* K = ksh + threadIdx.x * StageWidth<FULL>::kWords;
   const unsigned long long total = base[n_req];
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
@@ -1769,7 +1814,7 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 3 : 1)
 
 template <bool FULL>
 constexpr size_t stage_smem(int block) {
-  return sizeof(float) * 7 * (FULL ? 5 : 1) * (size_t)block;
+  return sizeof(float) * StageWidth<FULL>::kWords * (size_t)block;
 }
 
 // Resident CTAs per SM of the IQUV kernel / the single-kernel form.
@@ -1915,7 +1960,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   // runs panels only, which keep their sums in registers; the general build
   // keeps Dormand-Prince stages in shared memory)
   const int bt = 256;
-  const size_t smem_t = shape.fused ? 0 : stage_smem<false>(bt);
+  const size_t smem_t = shape.fused ? 0 : sizeof(float) * kTauWords * bt;
   void (*tau_k)(const JshRequest*, int, unsigned long long*, int, int) =
       shape.fused ? transfer_tau_kernel<false> : transfer_tau_kernel<true>;
   int per_sm_t = 0;
@@ -1925,6 +1970,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   if ((uint64_t)bl_t * bt > need) bl_t = (unsigned)((need + bt - 1) / bt);
   if (bl_t == 0) bl_t = 1;
   const IquvKernel iquv_k = iquv_kernel(full, shape.compact != 0, shape.fused != 0);
+  const size_t smem_q = shape.fused ? 0 : smem;  // the fused build keeps its stages in registers
   const dim3 gi((unsigned)num_sms, (unsigned)n_req);
   if (!overlap) {
     if (shape.marks) cudaEventRecord(shape.marks[0], stream);
@@ -1934,7 +1980,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
     iquv_prefix_kernel<<<n_req, 32, 0, stream>>>(d_reqs, 0);
     iquv_scatter_kernel<<<gi, 256, 0, stream>>>(d_reqs, 0);
     if (shape.marks) cudaEventRecord(shape.marks[2], stream);
-    iquv_k<<<blocks, bs, smem, stream>>>(d_reqs, n_req, q + 1, rf, 0);
+    iquv_k<<<blocks, bs, smem_q, stream>>>(d_reqs, n_req, q + 1, rf, 0);
     if (shape.marks) cudaEventRecord(shape.marks[3], stream);
     return cudaGetLastError();
   }
@@ -1962,7 +2008,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   e = cudaEventRecord(shape.fork[0], stream);
   if (e != cudaSuccess) return e;
   e = launch_prio(iquv_k, (unsigned)(num_sms * kDeepIquvPerSm), kDeepIquvBlock,
-                  full ? stage_smem<true>(kDeepIquvBlock) : stage_smem<false>(kDeepIquvBlock), stream, prio_hi,
+                  smem_q / bs * kDeepIquvBlock, stream, prio_hi,
                   d_reqs, n_req, q + 1, rf, 0);
   if (e != cudaSuccess) return e;
   e = cudaStreamWaitEvent(shape.side, shape.fork[0], 0);
@@ -1976,7 +2022,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   iquv_prefix_kernel<<<n_req, 32, 0, shape.side>>>(d_reqs, 1);
   iquv_scatter_kernel<<<gi, 256, 0, shape.side>>>(d_reqs, 1);
   if (shape.marks) cudaEventRecord(shape.marks[2], shape.side);
-  iquv_k<<<blocks, bs, smem, shape.side>>>(d_reqs, n_req, q + 3, rf, 1);
+  iquv_k<<<blocks, bs, smem_q, shape.side>>>(d_reqs, n_req, q + 3, rf, 1);
   e = cudaEventRecord(shape.fork[1], shape.side);
   if (e != cudaSuccess) return e;
   e = cudaStreamWaitEvent(stream, shape.fork[1], 0);
