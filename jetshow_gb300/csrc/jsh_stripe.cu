@@ -3,7 +3,7 @@
 // and Image::getStripe (src/Image.cpp:31-41), the tau-only pass along half of
 // the central row that the reference's image-size search runs.
 //
-// One thread per stripe pixel (row n_across / 2, columns n_along / 2 ..
+// One warp per stripe pixel (row n_across / 2, columns n_along / 2 ..
 // n_along - 1), all FP64: the geometry hit, then per intersection a
 // constant-step classical RK4 over the const-step time range [0, L] with
 // dt = L / n (odeint runge_kutta4 through make_const_step_time_range: it
@@ -11,7 +11,12 @@
 // first yielded state with tau >= tau_max, whose tau is kept and whose
 // later intersections are dropped; otherwise the state after the last step.
 // dtau/dt = k_I does not depend on tau, so the two middle stages share one
-// evaluation.  A ray that misses keeps tau = 0.
+// evaluation, and 32 consecutive steps are evaluated at once, a step a lane;
+// their increments are then added in the order of the steps (the sums round
+// as the serial steps do).  A ray that misses keeps tau = 0.  With a thread
+// per pixel the 300 serial evaluations of FP64 set the time: 6.91 ms for the
+// 1 000 pixels of a 2 000-column stripe on 8 CTAs, 0.79 ms with a warp per
+// pixel (0.29 of it the plane's recurrence); 10 000 pixels 8.8 -> 6.6 ms.
 #include <cuda_runtime.h>
 #include <float.h>
 
@@ -27,12 +32,22 @@ using namespace jsh;
 
 namespace {
 
-__global__ void __launch_bounds__(128) stripe_tau_kernel(const JshRequest* __restrict__ req, double nu,
-                                                        double* __restrict__ tau_out) {
+// dtau/dt at path coordinate t.
+__device__ __forceinline__ double tau_rate(const JshModel& m, const Path64& P, double t) {
+  double k[NCOEF];
+  coefficients64<false>(m, P.p0 + P.dir * t, P.nl, P.nu, k);
+  return k[CK_I];
+}
+
+constexpr int kStripeThreads = 128;
+
+__global__ void __launch_bounds__(kStripeThreads) stripe_tau_kernel(const JshRequest* __restrict__ req, double nu,
+                                                                   double* __restrict__ tau_out) {
   const JshRequest& R = *req;
   const JshPlane& pl = R.plane;
   const uint64_t c0 = pl.n_along / 2;
-  const uint64_t col = c0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t col = c0 + ((uint64_t)blockIdx.x * kStripeThreads + threadIdx.x) / 32;
+  const int lane = (int)(threadIdx.x & 31u);
   if (col >= pl.n_along) return;
   Hits h;
   geo_hit(R.model, plane_origin(pl, pl.n_across / 2, col), mk(pl.dx, pl.dy, pl.dz), h);
@@ -47,25 +62,35 @@ __global__ void __launch_bounds__(128) stripe_tau_kernel(const JshRequest* __res
     const double length = sq(ad(ad(ml(dd.x, dd.x), ml(dd.y, dd.y)), ml(dd.z, dd.z)));
     const double dt = length / n;
     const Path64 P{pin, rd, nl, nu};
-    double x = 0.0, t = 0.0, k1, k2, k4, dum = 0.0;
-    int64_t step = 0;
+    double x = 0.0;
     bool found = (x >= tau_max);
     if (dt > 0.0) {
       const double w1 = ml(1.0 / 6.0, dt), w2 = ml(1.0 / 3.0, dt);
-      while (!found && sb(ad(t, dt), length) <= DBL_EPSILON && step <= (int64_t)n + 1) {
-        Rhs64<1, false>::eval(R.model, P, true, t, &dum, &k1);
-        Rhs64<1, false>::eval(R.model, P, true, ad(t, ml(0.5, dt)), &dum, &k2);
-        Rhs64<1, false>::eval(R.model, P, true, ad(t, dt), &dum, &k4);
-        x = ad(ad(ad(ad(x, ml(w1, k1)), ml(w2, k2)), ml(w2, k2)), ml(w1, k4));
-        ++step;
-        t = ml((double)step, dt);
-        found = (x >= tau_max);
+      for (int64_t first = 0; !found && first <= (int64_t)n + 1; first += 32) {
+        const int64_t step = first + lane;
+        const double t = ml((double)step, dt);
+        // the steps of the range are a prefix of the lanes: t grows with the step
+        const bool in = step <= (int64_t)n + 1 && sb(ad(t, dt), length) <= DBL_EPSILON;
+        const int steps = __popc(__ballot_sync(0xffffffffu, in));
+        double a = 0.0, b = 0.0, c = 0.0;
+        if (in) {
+          a = ml(w1, tau_rate(R.model, P, t));
+          b = ml(w2, tau_rate(R.model, P, ad(t, ml(0.5, dt))));
+          c = ml(w1, tau_rate(R.model, P, ad(t, dt)));
+        }
+        __syncwarp();
+        for (int i = 0; i < steps && !found; ++i) {
+          const double bi = __shfl_sync(0xffffffffu, b, i);
+          x = ad(ad(ad(ad(x, __shfl_sync(0xffffffffu, a, i)), bi), bi), __shfl_sync(0xffffffffu, c, i));
+          found = (x >= tau_max);
+        }
+        if (steps < 32) break;
       }
     }
     bg += x;
     if (found) break;
   }
-  tau_out[col - c0] = bg;
+  if (lane == 0) tau_out[col - c0] = bg;
 }
 
 }  // namespace
@@ -105,7 +130,7 @@ extern "C" int jsh_observation_run_stripe(jsh_ctx* ctx, const jsh_model_desc* mo
   const JshRequest* d_req = (const JshRequest*)(base + L.off_req);
   JSH_CUDA_TRY(jsh_launch_plane(d_req, 1, plane->n_along, s));
   if (count > 0) {
-    stripe_tau_kernel<<<(unsigned)((count + 127) / 128), 128, 0, s>>>(d_req, nu_hz, (double*)(base + off_out));
+    stripe_tau_kernel<<<(unsigned)((count * 32 + kStripeThreads - 1) / kStripeThreads), kStripeThreads, 0, s>>>(d_req, nu_hz, (double*)(base + off_out));
     JSH_CUDA_TRY(cudaGetLastError());
     JSH_CUDA_TRY(cudaMemcpyAsync(tau_host, base + off_out, sizeof(double) * count, cudaMemcpyDeviceToHost, s));
   }
