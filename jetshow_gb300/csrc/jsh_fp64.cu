@@ -1,6 +1,6 @@
-// jsh_fp64.cu -- the all-FP64 transfer kernels: one thread per work item
-// (static schedule, the plain GPU drop-in) and item-granular dynamic
-// scheduling from a global queue.
+// jsh_fp64.cu -- the all-FP64 transfer kernels: one group of five lanes per
+// work item (static schedule, the plain GPU drop-in) and item-granular
+// dynamic scheduling from a global queue.
 #include <cuda_runtime.h>
 
 #include "jsh_batch.cuh"
@@ -11,75 +11,78 @@ using namespace jsh;
 
 namespace {
 
-// One thread per (request, hit ray, frequency), all FP64.  Items are laid
-// out frequency-major within a request so adjacent lanes trace adjacent
+constexpr int kThreads64 = 128;
+constexpr int kItemsPerCta = kThreads64 / 32 * kGroupsPerWarp;
+
+// One item by the lanes of a group; lane 0 writes it.  Returns its counters
+// (lane 0) and status.
+__device__ __forceinline__ uint32_t run_item64(const JshRequest& R, unsigned long long local, const Group64& G,
+                                               Ctl64& tot) {
+  const unsigned nhit = *R.n_hit;
+  const int f = (int)(local / nhit);
+  const JshHit& H = R.hits[(unsigned)(local % nhit)];
+  ItemOut o;
+  if (R.P.full) transfer_item64<true>(R.model, R.plane, R.P, H, R.nu[f], f, G, o, tot);
+  else transfer_item64<false>(R.model, R.plane, R.P, H, R.nu[f], f, G, o, tot);
+  if (R.P.flags & JSH_FLAG_COST_MAP) o.l = (double)tot.evals;
+  if (G.sub == 0) write_item(R, f, H.pix, o);
+  return o.status;
+}
+
+// One lane group per (request, hit ray, frequency), all FP64.  Items are laid
+// out frequency-major within a request so adjacent groups trace adjacent
 // pixels (similar path lengths, less divergence).
-__global__ void __launch_bounds__(128) transfer_static64_kernel(const JshRequest* __restrict__ reqs, int n_req) {
+__global__ void __launch_bounds__(kThreads64) transfer_static64_kernel(const JshRequest* __restrict__ reqs, int n_req) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
+  __shared__ double sh[kThreads64 / 32][kGroupsPerWarp * kGroup * NCOEF];
   batch_prefix(reqs, n_req, base);
-  unsigned long long w = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  bool active = w < base[n_req];
+  const Group64 G = group_of(sh[threadIdx.x / 32]);
+  const unsigned long long w =
+      (unsigned long long)blockIdx.x * kItemsPerCta + (threadIdx.x / 32) * kGroupsPerWarp + G.base / kGroup;
+  const bool active = G.mask != 0 && w < base[n_req];
   int r = 0;
   Ctl64 tot{0, 0, 0, 0, 0, 0, 0};
-  ItemOut o;
-  o.status = 0;
+  uint32_t status = 0;
   if (active) {
     r = find_request(base, n_req, w);
-    const JshRequest& R = reqs[r];
-    unsigned long long local = w - base[r];
-    unsigned nhit = *R.n_hit;
-    int f = (int)(local / nhit);
-    unsigned h = (unsigned)(local % nhit);
-    const JshHit& H = R.hits[h];
-    if (R.P.full) transfer_item64<true>(R.model, R.plane, R.P, H, R.nu[f], f, o, tot);
-    else transfer_item64<false>(R.model, R.plane, R.P, H, R.nu[f], f, o, tot);
-    if (R.P.flags & JSH_FLAG_COST_MAP) o.l = (double)tot.evals;
-    write_item(R, f, H.pix, o);
+    status = run_item64(reqs[r], w - base[r], G, tot);
   }
-  add_counters(reqs, r, active, tot.evals, tot.acc, tot.rej, o.status);
+  __syncwarp();
+  add_counters(reqs, r, active && G.sub == 0, tot.evals, tot.acc, tot.rej, status);
 }
 
 // FP64 items with dynamic (queue) scheduling at item granularity.
-__global__ void __launch_bounds__(128) transfer_queue64_kernel(const JshRequest* __restrict__ reqs, int n_req,
-                                                                 unsigned long long* queue) {
+__global__ void __launch_bounds__(kThreads64) transfer_queue64_kernel(const JshRequest* __restrict__ reqs, int n_req,
+                                                                        unsigned long long* queue) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
+  __shared__ double sh[kThreads64 / 32][kGroupsPerWarp * kGroup * NCOEF];
   batch_prefix(reqs, n_req, base);
   const unsigned long long total = base[n_req];
+  const Group64 G = group_of(sh[threadIdx.x / 32]);
+  if (G.mask == 0) return;
   for (;;) {
-    unsigned long long w = atomicAdd(queue, 1ull);
+    unsigned long long w = 0;
+    if (G.sub == 0) w = atomicAdd(queue, 1ull);
+    w = __shfl_sync(G.mask, w, G.base);
     if (w >= total) break;
-    int r = find_request(base, n_req, w);
-    const JshRequest& R = reqs[r];
-    unsigned long long local = w - base[r];
-    unsigned nhit = *R.n_hit;
-    int f = (int)(local / nhit);
-    const JshHit& H = R.hits[(unsigned)(local % nhit)];
+    const int r = find_request(base, n_req, w);
     Ctl64 tot{0, 0, 0, 0, 0, 0, 0};
-    ItemOut o;
-    if (R.P.full) transfer_item64<true>(R.model, R.plane, R.P, H, R.nu[f], f, o, tot);
-    else transfer_item64<false>(R.model, R.plane, R.P, H, R.nu[f], f, o, tot);
-    uint64_t q = (uint64_t)f * R.npix + (uint64_t)H.pix;
-    if (R.tau) R.tau[q] = o.tau;
-    if (R.l) R.l[q] = (R.P.flags & JSH_FLAG_COST_MAP) ? (double)tot.evals : o.l;
-    if (R.I) R.I[q] = o.iquv[0];
-    if (R.Q) R.Q[q] = o.iquv[1];
-    if (R.U) R.U[q] = o.iquv[2];
-    if (R.V) R.V[q] = o.iquv[3];
-    if (R.status) R.status[q] = o.status;
-    atomicAdd(&R.counters[0], (unsigned long long)tot.evals);
-    atomicAdd(&R.counters[1], (unsigned long long)tot.acc);
-    atomicAdd(&R.counters[2], (unsigned long long)tot.rej);
-    atomicOr(&R.counters[3], (unsigned long long)o.status);
+    const uint32_t status = run_item64(reqs[r], w - base[r], G, tot);
+    if (G.sub == 0) {
+      unsigned long long* c = reqs[r].counters;
+      atomicAdd(&c[0], (unsigned long long)tot.evals);
+      atomicAdd(&c[1], (unsigned long long)tot.acc);
+      atomicAdd(&c[2], (unsigned long long)tot.rej);
+      atomicOr(&c[3], (unsigned long long)status);
+    }
   }
 }
-
 
 }  // namespace
 
 cudaError_t jsh_launch_transfer_static64(const JshRequest* d_reqs, int n_req, uint64_t max_items, cudaStream_t stream) {
-  const int bs = 128;
-  uint64_t blocks = (max_items + bs - 1) / bs;
-  transfer_static64_kernel<<<(unsigned)blocks, bs, 0, stream>>>(d_reqs, n_req);
+  const uint64_t blocks = (max_items + kItemsPerCta - 1) / kItemsPerCta;
+  transfer_static64_kernel<<<(unsigned)blocks, kThreads64, 0, stream>>>(d_reqs, n_req);
   return cudaGetLastError();
 }
 
@@ -87,12 +90,12 @@ cudaError_t jsh_launch_transfer_persistent64(const JshRequest* d_reqs, int n_req
                                              const JshLaunchShape& shape, unsigned int* queue, int num_sms,
                                              cudaStream_t stream) {
   int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, transfer_queue64_kernel, 128, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, transfer_queue64_kernel, kThreads64, 0);
   if (per_sm < 1) per_sm = 1;
   unsigned blocks = (unsigned)(num_sms * per_sm);
-  uint64_t need = (max_items + 127) / 128;
+  uint64_t need = (max_items + kItemsPerCta - 1) / kItemsPerCta;
   if (blocks > need) blocks = (unsigned)(need ? need : 1);
-  transfer_queue64_kernel<<<blocks, 128, 0, stream>>>(d_reqs, n_req, (unsigned long long*)queue);
+  transfer_queue64_kernel<<<blocks, kThreads64, 0, stream>>>(d_reqs, n_req, (unsigned long long*)queue);
   return cudaGetLastError();
 }
 

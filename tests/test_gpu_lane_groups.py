@@ -1,16 +1,67 @@
 """The forms that spread one ray over several lanes, at the sizes where their
 maps can go wrong.
 
+* FP64 transfer, five lanes an item, six items a warp, 24 a CTA: item counts
+  around those edges, one and two segments a ray, random directions drawn at
+  every evaluation (a sixth evaluation per step); the static and the queue
+  schedule bitwise the same, and the oracle at the same tolerances within the
+  contract gates.
 * The stripe pass, 32 steps of a pixel at a time: step counts around 32 and a
   stop inside a group of steps, against the oracle to the last bits of pow
   over n steps (1e-10, as the stripe test).
 """
+import math
+
 import numpy as np
 import pytest
 
+from jetshow_gb300 import jet as J
 from jetshow_gb300 import workloads as W
+from helpers import compare_images, flat
 
 pytestmark = pytest.mark.gpu
+
+
+def conical(points=False, half=0.05):
+    jet = W.conical_model(half_angle=half)
+    if points:
+        jet.bfield = J.PointsRandomVectorBField(jet.bfield, 0.3, seed=11)
+    return jet
+
+
+@pytest.mark.parametrize("output", ["I", "full"])
+@pytest.mark.parametrize("along,n_nu,half", [(2, 1, 0.05), (3, 1, 0.05), (4, 2, 0.05), (13, 1, 0.05), (5, 1, 0.15)])
+def test_fp64_groups(ctx, oracle, output, along, n_nu, half):
+    lg = math.log10(0.4 * 1.8443 * J.pc)
+    plane = J.ImagePlane((2, along), lg, lg, 0.1)
+    nu = np.array([8e9, 15.4e9][:n_nu]) * 1.1
+    jet = conical(half=half)
+    kw = dict(W.ACCURATE_KW, output=output)
+    g, st = ctx.render(jet.desc(), plane.desc(), nu, J.make_params(precision="fp64", schedule="static", **kw))
+    q, sq = ctx.render(jet.desc(), plane.desc(), nu, J.make_params(precision="fp64", schedule="persistent", **kw))
+    assert st["n_work_items"] > 0
+    for k in g:
+        assert np.array_equal(g[k], q[k]), k
+    assert (st["rhs_evals"], st["steps_accepted"], st["steps_rejected"]) == (
+        sq["rhs_evals"], sq["steps_accepted"], sq["steps_rejected"])
+    r = oracle.render(jet.desc(), plane.desc(), nu, J.make_params(precision="fp64", schedule="static", **kw))
+    compare_images(flat(g), r, full=output == "full", tau_max=1e4)
+
+
+def test_fp64_group_random_directions(ctx, oracle):
+    """The sixth evaluation of a step has a direction of its own: the image
+    follows the oracle's draws (evaluation by evaluation) and differs from
+    the unperturbed field's."""
+    plane = W.conical_c0(scale=16)[1]
+    nu = np.array([16.94e9])
+    p = J.make_params(precision="fp64", schedule="static", **dict(W.ACCURATE_KW, tau_rtol=1e-3, rtol=1e-3, dt_max=0.0))
+    g, _ = ctx.render(conical(True).desc(), plane.desc(), nu, p)
+    r = oracle.render(conical(True).desc(), plane.desc(), nu, p)
+    assert np.array_equal(g["status"].reshape(1, -1) & 1, r["status"] & 1)
+    hit = (r["status"] & 1) != 0
+    # the draws never converge: only the same directions at the same
+    # evaluations give the same image, up to the last bits of pow
+    np.testing.assert_allclose(g["I"].reshape(1, -1)[hit], r["I"][hit], rtol=1e-6)
 
 
 @pytest.mark.parametrize("n", [1, 31, 32, 33, 100])
