@@ -1,0 +1,30 @@
+// jsh_split.h -- the mixed path's kernels shared between its translation
+// units: ranking and tau kernels (jsh_tau.cu) and the static and
+// single-kernel forms (jsh_forms.cu and, with the Faraday-thick mode,
+// jsh_forms_ft.cu), for the launch sequences of jsh_persistent.cu.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "jsh_request.h"
+
+using TauKernel = void (*)(const JshRequest*, int, unsigned long long*, int, int);
+using StaticKernel = void (*)(const JshRequest*, int);
+using SingleKernel = void (*)(const JshRequest*, int, unsigned long long*, int);
+
+// The tau kernel (fused: built for the log-domain family alone) and its
+// dynamic shared memory.
+TauKernel jsh_tau_kernel(bool fused);
+size_t jsh_tau_smem(bool fused, int block);
+
+// Heaviest-first order of every request's hit rays; deep_key as
+// rank_prefix_kernel.
+void jsh_launch_rank(const JshRequest* d_reqs, int n_req, uint64_t max_hits, int deep_key, cudaStream_t stream);
+
+// Heaviest-first order of the items the tau kernel handed on.
+void jsh_launch_iquv_rank(const JshRequest* d_reqs, int n_req, int num_sms, int part, cudaStream_t stream);
+
+StaticKernel jsh_static_kernel(bool full);
+SingleKernel jsh_single_kernel(bool full, bool compact);
+StaticKernel jsh_static_kernel_ft(bool full);
+SingleKernel jsh_single_kernel_ft(bool full, bool compact);

@@ -1,0 +1,225 @@
+// jsh_tau.cu -- the split form's first half: the heaviest-first ranking of the
+// hit rays, the tau kernels, and the ranking of the items they hand on.  The
+// Faraday-thick mode of the IQUV pass does not reach this code, so both
+// launch sequences (jsh_persistent.cu and its second build) share it.
+#include "jsh_mixed.cuh"
+
+#include "jsh_split.h"
+
+namespace jsh {
+
+namespace {
+
+// ------------------------------------------------------------- ranking
+// Heaviest-first order of the hit rays for the persistent schedule.  A ray's
+// cost grows with its optical depth (up to the optically thick start of the
+// IQUV pass): rays through the core take thousands of steps, rays far out a
+// few hundred.  So each ray's optical depth at the request's first
+// frequency is estimated (4-point Gauss-Legendre over each segment, the FP32
+// coefficients), bucketed by factors of 2 and counting-sorted in descending
+// order; the queue then hands out the heaviest rays first and they run while
+// the bulk fills the GPU, instead of starting late and setting the render's
+// makespan.
+__global__ void __launch_bounds__(256) rank_cost_kernel(const JshRequest* __restrict__ reqs) {
+  __shared__ uint32_t hist[JSH_RANK_BUCKETS];
+  const JshRequest& R = reqs[blockIdx.y];
+  for (int b = threadIdx.x; b < JSH_RANK_BUCKETS; b += blockDim.x) hist[b] = 0;
+  __syncthreads();
+  const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h < *R.n_hit) {
+    const JshHit& H = R.hits[h];
+    const JshFreqConst F = R.mix.fc[0];
+    const float xk[4] = {0.0694318442f, 0.330009478f, 0.669990522f, 0.930568156f};
+    const float wk[4] = {0.173927423f, 0.326072577f, 0.326072577f, 0.173927423f};
+    float tau = 0.f;
+    for (int s = 0; s < H.nseg && s < 2; ++s) {
+      const F3 a = f3((float)(H.seg[s][0] * INV_PC), (float)(H.seg[s][1] * INV_PC), (float)(H.seg[s][2] * INV_PC));
+      const F3 b = f3((float)(H.seg[s][3] * INV_PC), (float)(H.seg[s][4] * INV_PC), (float)(H.seg[s][5] * INV_PC));
+      const F3 d = b - a;
+      float acc = 0.f;
+#pragma unroll 1
+      for (int k = 0; k < 4; ++k) {
+        Coef32 c;
+        coef32_rt(R, F, a + d * xk[k], COEF_KI, c);
+        acc = fmaf(wk[k], c.kI, acc);
+      }
+      tau = fmaf(acc, sqrtf(fdot(d, d)), tau);
+    }
+    int key = 0;
+    if (tau > 0.f && tau < INFINITY) key = min(max((int)floorf(__log2f(tau)) + 40, 1), JSH_RANK_BUCKETS - 1);
+    R.key[h] = (uint8_t)key;
+    atomicAdd(&hist[key], 1u);
+  }
+  __syncthreads();
+  for (int b = threadIdx.x; b < JSH_RANK_BUCKETS; b += blockDim.x)
+    if (hist[b]) atomicAdd(&R.buckets[b], hist[b]);
+}
+
+// Start of each bucket in descending bucket order (one thread per request),
+// and the size of the deep prefix: the rays of buckets >= deep_key (every
+// ray for deep_key <= 0).
+__global__ void rank_prefix_kernel(const JshRequest* __restrict__ reqs, int deep_key) {
+  const JshRequest& R = reqs[blockIdx.x];
+  if (threadIdx.x != 0) return;
+  uint32_t run = 0, deep = 0;
+  for (int b = JSH_RANK_BUCKETS - 1; b >= 0; --b) {
+    R.buckets[JSH_RANK_BUCKETS + b] = run;
+    run += R.buckets[b];
+    if (b == deep_key) deep = run;
+  }
+  R.buckets[JSH_RANK_DEEP] = deep_key > 0 ? deep : run;
+}
+
+// order[position] = hit index; the lanes of a warp with the same bucket take
+// consecutive positions with one atomic.
+__global__ void __launch_bounds__(256) rank_scatter_kernel(const JshRequest* __restrict__ reqs) {
+  const JshRequest& R = reqs[blockIdx.y];
+  const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h >= *R.n_hit) return;
+  const int key = R.key[h];
+  const unsigned peers = __match_any_sync(__activemask(), key);
+  const int leader = __ffs(peers) - 1;
+  const unsigned lane = threadIdx.x & 31u;
+  uint32_t base = 0;
+  if ((int)lane == leader) base = atomicAdd(&R.buckets[JSH_RANK_BUCKETS + key], (uint32_t)__popc(peers));
+  base = __shfl_sync(peers, base, leader);
+  R.order[base + __popc(peers & ((1u << lane) - 1u))] = h;
+}
+
+// ------------------------------------------------------------ split form
+// The persistent schedule's default form runs the passes in two kernels:
+// every item's tau pass first (one stage component, k_I only: a short
+// right-hand side, few registers, many resident warps, and no warp whose
+// lanes mix tau and IQUV code), then the I/IQUV pass of the items that need
+// one, ranked by the optical depth it integrates through.
+
+// Work items of part `part` of the ranked rays over the batch (exclusive
+// prefix in shared memory): part 0 the deep prefix (every ray when the
+// passes are not overlapped), part 1 the rays after it.
+__device__ __forceinline__ void tau_prefix(const JshRequest* __restrict__ reqs, int n_req, int part,
+                                           unsigned long long* base) {
+  if (threadIdx.x == 0) {
+    unsigned long long acc = 0;
+    for (int r = 0; r < n_req; ++r) {
+      base[r] = acc;
+      const uint32_t deep = reqs[r].buckets[JSH_RANK_DEEP];
+      const uint32_t rays = part ? *reqs[r].n_hit - deep : deep;
+      acc += (unsigned long long)rays * (unsigned long long)reqs[r].n_nu;
+    }
+    base[n_req] = acc;
+  }
+  __syncthreads();
+}
+
+// Tau kernel: persistent CTAs, lanes refilled from the ranked queue (the
+// same order as the single-kernel form), each item's tau pass to its end,
+// over the rays of part `part`.
+// GENERAL = false: the build for batches of the fused benchmark family
+// alone (80 registers, 24 resident warps per SM, against 128 and 16).
+template <bool GENERAL>
+__global__ void __launch_bounds__(256, GENERAL ? 2 : 3) transfer_tau_kernel(const JshRequest* __restrict__ reqs,
+                                                                          int n_req, unsigned long long* queue,
+                                                                          int refill, int part) {
+  __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
+  extern __shared__ float ksh[];
+  tau_prefix(reqs, n_req, part, base);
+  float* K1 = ksh + threadIdx.x * kTauWords;
+  const unsigned long long total = base[n_req];
+  const unsigned lane = threadIdx.x & 31u;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  Lane L;
+  L.phase = PH_IDLE;
+  Tally T = tally_new();
+  bool exhausted = false;
+  for (;;) {
+    unsigned idle = __ballot_sync(0xffffffffu, L.phase == PH_IDLE);
+    int nidle = __popc(idle);
+    if (!exhausted && (nidle >= refill || nidle == 32) && nidle > 0) {
+      unsigned long long b = 0;
+      if (lane == 0) b = atomicAdd(queue, (unsigned long long)nidle);
+      b = __shfl_sync(0xffffffffu, b, 0);
+      if (b + (unsigned long long)nidle >= total) exhausted = true;
+      if (L.phase == PH_IDLE) {
+        unsigned long long w = b + (unsigned long long)__popc(idle & lt_mask);
+        if (w < total) lane_start(L, reqs, base, n_req, w, true, part);
+      }
+    }
+    unsigned active = __ballot_sync(0xffffffffu, L.phase != PH_IDLE);
+    if (active == 0) {
+      if (exhausted) break;
+      continue;
+    }
+    if (L.phase != PH_IDLE) tau_step<PASS_TAU, GENERAL>(L, reqs, K1, part, T);
+  }
+  tally_flush(T, reqs);
+}
+
+// Cost histogram of part `part`'s emitted items of request blockIdx.y
+// (grid-stride).
+__global__ void __launch_bounds__(256) iquv_hist_kernel(const JshRequest* __restrict__ reqs, int part) {
+  __shared__ uint32_t hist[JSH_RANK_BUCKETS];
+  const JshRequest& R = reqs[blockIdx.y];
+  for (int b = threadIdx.x; b < JSH_RANK_BUCKETS; b += blockDim.x) hist[b] = 0;
+  __syncthreads();
+  const uint32_t n = R.iq_count[part], o = iq_first(R, part);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    atomicAdd(&hist[R.iq_items[o + i].key], 1u);
+  __syncthreads();
+  uint32_t* bk = R.iq_buckets + 2 * JSH_RANK_BUCKETS * part;
+  for (int b = threadIdx.x; b < JSH_RANK_BUCKETS; b += blockDim.x)
+    if (hist[b]) atomicAdd(&bk[b], hist[b]);
+}
+
+// Start of each cost bucket in descending order (one thread per request).
+__global__ void iquv_prefix_kernel(const JshRequest* __restrict__ reqs, int part) {
+  const JshRequest& R = reqs[blockIdx.x];
+  if (threadIdx.x != 0) return;
+  uint32_t* bk = R.iq_buckets + 2 * JSH_RANK_BUCKETS * part;
+  uint32_t run = 0;
+  for (int b = JSH_RANK_BUCKETS - 1; b >= 0; --b) {
+    bk[JSH_RANK_BUCKETS + b] = run;
+    run += bk[b];
+  }
+}
+
+// iq_order[first + position] = emitted item (absolute slot); lanes with the
+// same bucket take consecutive positions with one atomic.
+__global__ void __launch_bounds__(256) iquv_scatter_kernel(const JshRequest* __restrict__ reqs, int part) {
+  const JshRequest& R = reqs[blockIdx.y];
+  const uint32_t n = R.iq_count[part], o = iq_first(R, part);
+  uint32_t* bk = R.iq_buckets + 2 * JSH_RANK_BUCKETS * part;
+  const unsigned lane = threadIdx.x & 31u;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const int key = R.iq_items[o + i].key;
+    const unsigned peers = __match_any_sync(__activemask(), key);
+    const int leader = __ffs(peers) - 1;
+    uint32_t b = 0;
+    if ((int)lane == leader) b = atomicAdd(&bk[JSH_RANK_BUCKETS + key], (uint32_t)__popc(peers));
+    b = __shfl_sync(peers, b, leader);
+    R.iq_order[o + b + __popc(peers & ((1u << lane) - 1u))] = o + i;
+  }
+}
+
+}  // namespace
+
+}  // namespace jsh
+
+using namespace jsh;
+
+TauKernel jsh_tau_kernel(bool fused) { return fused ? transfer_tau_kernel<false> : transfer_tau_kernel<true>; }
+
+size_t jsh_tau_smem(bool fused, int block) { return fused ? 0 : sizeof(float) * kTauWords * (size_t)block; }
+
+void jsh_launch_rank(const JshRequest* d_reqs, int n_req, uint64_t max_hits, int deep_key, cudaStream_t stream) {
+  const dim3 g((unsigned)((max_hits + 255) / 256), (unsigned)n_req);
+  rank_cost_kernel<<<g, 256, 0, stream>>>(d_reqs);
+  rank_prefix_kernel<<<n_req, 32, 0, stream>>>(d_reqs, deep_key);
+  rank_scatter_kernel<<<g, 256, 0, stream>>>(d_reqs);
+}
+
+void jsh_launch_iquv_rank(const JshRequest* d_reqs, int n_req, int num_sms, int part, cudaStream_t stream) {
+  const dim3 g((unsigned)num_sms, (unsigned)n_req);
+  iquv_hist_kernel<<<g, 256, 0, stream>>>(d_reqs, part);
+  iquv_prefix_kernel<<<n_req, 32, 0, stream>>>(d_reqs, part);
+  iquv_scatter_kernel<<<g, 256, 0, stream>>>(d_reqs, part);
+}
