@@ -68,29 +68,88 @@ __device__ __forceinline__ bool grid_tri32(const JshGrid& G, int t, float px, fl
   return false;
 }
 
-// Point location of (px, py).  `hint` (may be null): the triangle of the
-// lane's previous evaluation, tried first -- consecutive evaluation points
-// along a ray mostly fall in the same triangle, and the bucket search costs
-// a chain of dependent loads per candidate (bucket, list, triangle,
-// vertices); the found triangle is stored back.  The hint restarts with
-// each item, so an item's lookups do not depend on the lane that runs it.
-__device__ inline GridW grid_locate32(const JshGrid& G, float px, float py, int* hint = nullptr) {
-  GridW g;
-  g.ok = false;
-  if (G.n_tri == 0) return g;
-  if (hint && *hint >= 0 && grid_tri32(G, *hint, px, py, g)) return g;
+// The first triangle of (px, py)'s bucket that holds the point, or -1.
+__device__ __forceinline__ int grid_search32(const JshGrid& G, float px, float py, GridW& g) {
   const float fx = (px - G.x0f) * G.inv_hf, fy = (py - G.y0f) * G.inv_hf;
-  if (!(fx >= 0.f && fy >= 0.f)) return g;
+  if (!(fx >= 0.f && fy >= 0.f)) return -1;
   const int i = min((int)fx, G.nbx - 1), j = min((int)fy, G.nby - 1);
   const int b = j * G.nbx + i;
   const int q1 = G.bstart[b + 1];
   for (int q = G.bstart[b]; q < q1; ++q) {
     const int t = G.bitems[q];
-    if (grid_tri32(G, t, px, py, g)) {
-      if (hint) *hint = t;
-      return g;
-    }
+    if (grid_tri32(G, t, px, py, g)) return t;
   }
+  return -1;
+}
+__device__ inline GridW grid_locate32(const JshGrid& G, float px, float py) {
+  GridW g;
+  g.ok = false;
+  if (G.n_tri > 0) grid_search32(G, px, py, g);
+  return g;
+}
+
+// The lanes that run one item together: one, or a group of kGroupLanes.
+struct LaneGroup {
+  unsigned mask;     // the group's lanes (0: this lane belongs to none)
+  int base, sub, n;  // its first lane, this lane's place in it, its size
+  __device__ __forceinline__ void sync() const {
+    if (n > 1) __syncwarp(mask);
+  }
+};
+constexpr int kGroupLanes = 5;
+constexpr int kWarpGroups = 6;  // per warp, the last two lanes idle
+__device__ __forceinline__ LaneGroup lane_group() {
+  const int lane = (int)(threadIdx.x & 31u), g = lane / kGroupLanes;
+  return LaneGroup{g < kWarpGroups ? 0x1fu << (kGroupLanes * g) : 0u, kGroupLanes * g, lane - kGroupLanes * g,
+                   kGroupLanes};
+}
+__device__ __forceinline__ LaneGroup single_lane() {
+  const int lane = (int)(threadIdx.x & 31u);
+  return LaneGroup{1u << lane, lane, 0, 1};
+}
+
+// Point location with a hint: the triangle of the lane's previous evaluation is
+// tried first -- consecutive evaluation points along a ray mostly fall in the
+// same triangle, and the bucket search costs a chain of dependent loads per
+// candidate (bucket, list, triangle, vertices) -- and the found triangle is
+// stored back.  The hint restarts with each item, so an item's lookups do not
+// depend on the lane that runs it.  A group locates its points at once, lane k
+// the k-th point.  A point near an edge belongs to whichever
+// of the two triangles is tried first, so the answers must be those of the
+// serial order, in which point k tries the triangle of point k - 1 before its
+// bucket: every lane first tries the step's hint and, failing that, its
+// bucket; then the points take their turn with the triangle before them,
+// which most often is one of the two already tried.
+static __device__ __noinline__ GridW grid_locate32_group(const JshGrid& G, float px, float py, int* hint, LaneGroup L) {
+  GridW g, own;
+  g.ok = own.ok = false;
+  if (G.n_tri == 0) return g;
+  const int t0 = *hint;
+  const bool in0 = t0 >= 0 && grid_tri32(G, t0, px, py, g);
+  int found = in0 ? -1 : grid_search32(G, px, py, own);
+  if (L.n == 1) {
+    if (found >= 0) *hint = found;
+    return in0 ? g : own;
+  }
+  bool searched = !in0;
+  int t = t0;
+#pragma unroll 1
+  for (int k = 0; k < L.n; ++k) {
+    int mine = t;
+    if (L.sub == k && !(t == t0 && in0)) {
+      g.ok = false;
+      if (t != t0 && !(searched && found == t) && grid_tri32(G, t, px, py, g)) {
+        // inside the triangle of the point before
+      } else {
+        if (!searched) found = grid_search32(G, px, py, own);
+        searched = true;
+        g = own;
+        if (found >= 0) mine = found;
+      }
+    }
+    t = __shfl_sync(L.mask, mine, L.base + k);
+  }
+  *hint = t;
   return g;
 }
 __device__ __forceinline__ float grid_val32(const JshGrid& G, const GridW& g, int field, float nan_value) {
@@ -455,7 +514,7 @@ __device__ __forceinline__ void coef32_helical_log(const JshMixed& X, const JshF
 template <bool GENERAL = true>
 __device__ __forceinline__ void coef32_rt(const JshRequest& R, const JshFreqConst& F, F3 p, int mode, Coef32& c,
                                           uint32_t rk_h = 0, uint32_t rk_f = 0, uint32_t rk_e = 0,
-                                          int* tri_hint = nullptr) {
+                                          int* tri_hint = nullptr, const LaneGroup group = LaneGroup{0u, 0, 0, 1}) {
   const JshModel& m = R.model;
   const JshMixed& X = R.mix;
   if (!GENERAL || X.helical_log) {
@@ -493,7 +552,10 @@ __device__ __forceinline__ void coef32_rt(const JshRequest& R, const JshFreqCons
   } else if (X.sim_shared) {
     // every field from one grid (the simulation workload): one point location
     // for Gamma, n, B_p and B_phi
-    const GridW g = grid_locate32(m.grids[0], p.z, sqrtf(p.x * p.x + p.y * p.y), tri_hint);
+    const float rc = sqrtf(p.x * p.x + p.y * p.y);
+    int hint = tri_hint ? *tri_hint : -1;  // its address escapes, the lane's state must not
+    const GridW g = grid_locate32_group(m.grids[0], p.z, rc, &hint, group);
+    if (tri_hint) *tri_hint = hint;
     gamma = grid_val32(m.grids[0], g, m.f_v, 1.0f);
     vdir = f3(0, 0, 1);
     kinematics32(gamma, vdir, f3(X.nl[0], X.nl[1], X.nl[2]), D, nlp, beta);

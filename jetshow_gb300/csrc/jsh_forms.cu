@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(128) transfer_static_mixed_kernel(const JshReq
   extern __shared__ float ksh[];
   batch_prefix(reqs, n_req, base);
   const unsigned long long w = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  float* K = ksh + threadIdx.x * StageWidth<FULL>::kWords;
+  float* K = ksh + threadIdx.x * form_words<FULL>();
   Tally T = tally_new();
   if (w < base[n_req]) {
     Lane L;
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 3 : 1)
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
   extern __shared__ float ksh[];
   batch_prefix(reqs, n_req, base);
-  float* K = ksh + threadIdx.x * StageWidth<FULL>::kWords;
+  float* K = ksh + threadIdx.x * form_words<FULL>();
   const unsigned long long total = base[n_req];
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;

@@ -197,7 +197,17 @@ struct StageWidth {
   static constexpr int NC = FULL ? 8 : 2;        // coefficients of a stage point
   static constexpr int kWords = FULL ? 49 : 13;  // six points, odd
 };
-constexpr int kTauWords = 7;
+constexpr int kTauWords = 17;  // the 15 nodes of a panel, odd
+
+// Lanes that run one item: one, or a group of kGroupLanes.  A group's lanes
+// hold the same state and take the same branches; each evaluates one stage
+// point of a Dormand-Prince step (or every fifth node of a panel) and the
+// results are exchanged, so a step costs one evaluation's latency instead of
+// five.  Lane 0 writes the outputs.  The fused build has a copy of the step
+// for each (NG = 1, 5); the builds for every field law (NG = 0: the group's
+// size is LaneGroup::n) evaluate the points in a rolled loop, one copy of that
+// larger code, and exchange through the stage storage of the group (or lane).
+constexpr int kGroupWords = 52;  // fused I/IQUV step: six points of two float4, the groups spread over the banks
 
 // acc = sum_{j < S} a_Sj K_j over the stage derivatives held in registers
 // (S and j compile-time: the tableau entries are immediate operands).
@@ -401,11 +411,12 @@ __device__ __noinline__ void write_finished(const JshRequest* __restrict__ reqs,
   if (R.status) R.status[q] = status;
 }
 
-__device__ __forceinline__ void lane_finish(Lane& L, const JshRequest* __restrict__ reqs, Tally& T) {
+__device__ __forceinline__ void lane_finish(Lane& L, const JshRequest* __restrict__ reqs, Tally& T, bool lead) {
+  L.phase = PH_IDLE;
+  if (!lead) return;
   write_finished(reqs, L.r, L.f, L.h, L.tau_bg, L.thick, L.chi.hi, L.chi.lo, L.x[0], L.x[1], L.x[2], L.x[3],
                  L.status, L.evals);
   tally_add(T, reqs, L.r, L.evals, L.acc, L.rej, L.status);
-  L.phase = PH_IDLE;
 }
 
 // Split form, IQUV kernel: the item's Stokes planes and final status (its
@@ -548,11 +559,12 @@ __device__ __forceinline__ float stokes_rhs(const Coef32& c, const float* y, flo
 // definite: |k_Q|, |k_V| < k_I).  chi = 0 there, so the rotating frame is the
 // lab frame.  The state is in the request's scaled intensity units, like the
 // coefficients.  (ox, oy, oz): the start point [cm].
+template <bool GENERAL>
 __device__ __noinline__ float4 equilibrium_state(const JshRequest* __restrict__ reqs, int r, int f, double ox,
                                                 double oy, double oz) {
   const JshRequest& R = reqs[r];
   Coef32 c;
-  coef32_rt(R, R.mix.fc[f], f3((float)(ox * INV_PC), (float)(oy * INV_PC), (float)(oz * INV_PC)), COEF_FULL, c);
+  coef32_rt<GENERAL>(R, R.mix.fc[f], f3((float)(ox * INV_PC), (float)(oy * INV_PC), (float)(oz * INV_PC)), COEF_FULL, c);
   double A[4][5] = {{c.kI, c.kQ, 0.0, c.kV, c.eI},
                     {c.kQ, c.kI, c.kF, 0.0, c.eQ},
                     {0.0, -c.kF, c.kI, c.kC, 0.0},
@@ -580,11 +592,12 @@ __device__ __noinline__ float4 equilibrium_state(const JshRequest* __restrict__ 
   return make_float4((float)x[0], (float)x[1], (float)x[2], (float)x[3]);
 }
 
-__device__ __forceinline__ void lane_finish_iquv(Lane& L, const JshRequest* __restrict__ reqs, Tally& T) {
+__device__ __forceinline__ void lane_finish_iquv(Lane& L, const JshRequest* __restrict__ reqs, Tally& T, bool lead) {
+  L.phase = PH_IDLE;
+  if (!lead) return;
   write_finished_iquv(reqs, L.r, L.f, L.h, L.chi.hi, L.chi.lo, L.x[0], L.x[1], L.x[2], L.x[3], L.status, L.evals0,
                       L.evals);
   tally_add(T, reqs, L.r, L.evals, L.acc, L.rej, L.status);
-  L.phase = PH_IDLE;
 }
 
 // First item slot of part `part`'s emitted items in iq_items / iq_order.
@@ -595,6 +608,7 @@ __device__ __forceinline__ uint32_t iq_first(const JshRequest& R, int part) {
 // Split form, IQUV kernel: start work item w (heaviest-first over the
 // batch's emitted items) where the tau kernel left it -- the I/IQUV pass's
 // first segment, start point and state (zero, or the local equilibrium).
+template <bool GENERAL>
 __device__ __forceinline__ void lane_start_iquv(Lane& L, const JshRequest* __restrict__ reqs,
                                                 const unsigned long long* base, int n_req, unsigned long long w,
                                                 int part) {
@@ -624,7 +638,7 @@ __device__ __forceinline__ void lane_start_iquv(Lane& L, const JshRequest* __res
   if (eq) {
     const int s = L.seg;
     const double tc = L.t_first * JSH_PC;
-    const float4 xe = equilibrium_state(reqs, L.r, L.f, H.seg[s][0] + R.plane.rx * tc, H.seg[s][1] + R.plane.ry * tc,
+    const float4 xe = equilibrium_state<GENERAL>(reqs, L.r, L.f, H.seg[s][0] + R.plane.rx * tc, H.seg[s][1] + R.plane.ry * tc,
                                         H.seg[s][2] + R.plane.rz * tc);
     L.x[0] = xe.x;
     L.x[1] = xe.y;
@@ -722,11 +736,12 @@ constexpr int kCrossIters = 48;
 
 // The end of an item's tau pass: finish it (tau <= tau_min), hand it to the
 // IQUV kernel (PASS_TAU) or start its I/IQUV pass in the same lane.
-template <int PASS>
-__device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restrict__ reqs, int part, Tally& T) {
+template <int PASS, bool GENERAL>
+__device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restrict__ reqs, int part, Tally& T,
+                                              bool lead) {
   const JshRequest& R = reqs[L.r];
   if (!(L.tau_bg > R.P.tau_min)) {
-    lane_finish(L, reqs, T);
+    lane_finish(L, reqs, T, lead);
     return;
   }
   L.status |= JSH_ST_IQUV;
@@ -739,9 +754,10 @@ __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restr
     else L.first_seg = -1;
   }
   if (PASS == PASS_TAU) {
+    L.phase = PH_IDLE;
+    if (!lead) return;
     emit_iquv(reqs, part, L.r, L.f, L.h, L.tau_bg, L.thick, L.t_first, L.first_seg, L.nseg, eq, L.status, L.evals);
     tally_add(T, reqs, L.r, L.evals, L.acc, L.rej, 0u);
-    L.phase = PH_IDLE;
     return;
   }
   L.seg = L.first_seg >= 0 ? L.first_seg : L.nseg - 1;
@@ -752,7 +768,7 @@ __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restr
   if (eq) {
     const int s = L.seg;
     const double tc = L.t_first * JSH_PC;
-    const float4 xe = equilibrium_state(reqs, L.r, L.f, H.seg[s][0] + R.plane.rx * tc, H.seg[s][1] + R.plane.ry * tc,
+    const float4 xe = equilibrium_state<GENERAL>(reqs, L.r, L.f, H.seg[s][0] + R.plane.rx * tc, H.seg[s][1] + R.plane.ry * tc,
                                         H.seg[s][2] + R.plane.rz * tc);
     L.x[0] = xe.x;
     L.x[1] = xe.y;
@@ -766,8 +782,9 @@ __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restr
 // While the lane bisects a tau_max crossing (L.init set; the tau pass has
 // no other use for it), the panel [t, t + w] with w the midpoint of the
 // bracket [k1[0], k1[1]] is evaluated instead.
-template <int PASS, bool GENERAL>
-__device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __restrict__ reqs, int part, Tally& T) {
+template <int PASS, bool GENERAL, int NG>
+__device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __restrict__ reqs, float* Ksh, int part,
+                                               Tally& T, const LaneGroup& grp) {
   const JshRequest& R = reqs[L.r];
   const JshFreqConst F = R.mix.fc[L.f];
   const bool bis = L.init;
@@ -809,13 +826,47 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
     const float h = bis ? 0.5f * (L.k1[0] + L.k1[1]) : L.dt;
     const F3 pn = f3(L.bx, L.by, L.bz);
     float K = 0.f, G = 0.f, A = 0.f;
+    if (NG == 1) {
 #pragma unroll 1
-    for (int i = 0; i < 15; ++i) {
-      Coef32 c;
-      coef32_rt<GENERAL>(R, F, pn + dir * (c_gk_t[i] * h), COEF_KI, c, L.h, (uint32_t)L.f, L.evals + (uint32_t)i);
-      K = fmaf(c_gk_wk[i], c.kI, K);
-      G = fmaf(c_gk_wg[i], c.kI, G);
-      A = fmaf(c_gk_wd[i], fabsf(c.kI), A);
+      for (int i = 0; i < 15; ++i) {
+        Coef32 c;
+        coef32_rt<GENERAL>(R, F, pn + dir * (c_gk_t[i] * h), COEF_KI, c, L.h, (uint32_t)L.f, L.evals + (uint32_t)i);
+        K = fmaf(c_gk_wk[i], c.kI, K);
+        G = fmaf(c_gk_wg[i], c.kI, G);
+        A = fmaf(c_gk_wd[i], fabsf(c.kI), A);
+      }
+    } else if (NG > 1) {
+      // three nodes a lane, then the sums in the nodes' order
+      float k3[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        Coef32 c;
+        coef32_rt<GENERAL>(R, F, pn + dir * (c_gk_t[kGroupLanes * j + grp.sub] * h), COEF_KI, c);
+        k3[j] = c.kI;
+      }
+#pragma unroll
+      for (int i = 0; i < 15; ++i) {
+        const float kI = __shfl_sync(grp.mask, k3[i / kGroupLanes], grp.base + i % kGroupLanes);
+        K = fmaf(c_gk_wk[i], kI, K);
+        G = fmaf(c_gk_wg[i], kI, G);
+        A = fmaf(c_gk_wd[i], fabsf(kI), A);
+      }
+    } else {
+      grp.sync();  // the panel before has read its nodes
+#pragma unroll 1
+      for (int i = grp.sub; i < 15; i += grp.n) {
+        Coef32 c;
+        coef32_rt<GENERAL>(R, F, pn + dir * (c_gk_t[i] * h), COEF_KI, c);
+        Ksh[i] = c.kI;
+      }
+      grp.sync();
+#pragma unroll 1
+      for (int i = 0; i < 15; ++i) {
+        const float kI = Ksh[i];
+        K = fmaf(c_gk_wk[i], kI, K);
+        G = fmaf(c_gk_wg[i], kI, G);
+        A = fmaf(c_gk_wd[i], fabsf(kI), A);
+      }
     }
     L.evals += 15;
     K *= h;
@@ -845,7 +896,7 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
       L.nseg = L.seg + 1;
       L.tau_bg += df_val(L.tau_seg);
       L.thick += L.length_cm;
-      tau_pass_done<PASS>(L, reqs, part, T);
+      tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
       return;
     }
     // error test: |K - G| against the tolerance of the running depth, never
@@ -908,7 +959,7 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
         L.nseg = L.seg + 1;
         L.tau_bg += df_val(L.tau_seg);
         L.thick += L.length_cm;
-        tau_pass_done<PASS>(L, reqs, part, T);
+        tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
         return;
       }
     }
@@ -950,7 +1001,7 @@ segment_done : {
     begin_tau_segment(L, R, R.hits[L.h]);
     return;
   }
-  tau_pass_done<PASS>(L, reqs, part, T);
+  tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
   return;
 }
 
@@ -958,7 +1009,7 @@ abort:
   L.init = false;
   L.tau_bg += df_val(L.tau_seg);
   L.thick += L.length_cm;
-  lane_finish(L, reqs, T);
+  lane_finish(L, reqs, T, (grp.sub == 0));
 }
 
 // One Dormand-Prince attempt of an active lane's tau pass (the reference's
@@ -969,7 +1020,7 @@ abort:
 // combination (the increment) is formed.
 template <int PASS, bool GENERAL>
 __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __restrict__ reqs, float* K, int part,
-                                               Tally& T) {
+                                               Tally& T, const LaneGroup& grp) {
   const JshRequest& R = reqs[L.r];
   const JshFreqConst F = R.mix.fc[L.f];
   const F3 dirf = f3(-R.mix.nl[0], -R.mix.nl[1], -R.mix.nl[2]);
@@ -1006,19 +1057,22 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
       L.evals++;
       L.init = true;
     }
-    K[0] = L.k1[0];
     // k_I does not depend on the state, and the last two stages share their
     // point (c = 1): five evaluations serve the six stages, unless every
     // evaluation draws its own random direction
+    grp.sync();  // the step before has read its stages
+    if (grp.sub == 0) K[0] = L.k1[0];
     const int np = R.model.rnd_kind == JSH_RND_POINTS ? 6 : 5;
 #pragma unroll 1
-    for (int s = 1; s <= np; ++s) {
+    for (int s = grp.sub + 1; s <= np; s += grp.n) {
       Coef32 c;
+      // the sixth point is the group's first lane's alone
       coef32_rt<GENERAL>(R, F, pn + dirf * (c_C[s] * h), COEF_KI, c, L.h, (uint32_t)L.f,
-                         L.evals + (uint32_t)(s - 1), &L.tri);
+                         L.evals + (uint32_t)(s - 1), &L.tri, s <= 5 ? grp : single_lane());
       K[s] = c.kI;
+      if (s == 5 && np == 5) K[6] = c.kI;
     }
-    if (np == 5) K[6] = K[5];
+    grp.sync();
     float acc = 0.f;
 #pragma unroll
     for (int j = 0; j < 6; ++j) acc = fmaf(dp_a32(6, j), K[j], acc);
@@ -1096,7 +1150,7 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
       L.nseg = L.seg + 1;
       L.tau_bg += df_val(L.tau_seg);
       L.thick += L.length_cm;
-      tau_pass_done<PASS>(L, reqs, part, T);
+      tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
       return;
     }
     L.k1[0] = K[6];
@@ -1111,24 +1165,63 @@ segment_done : {
     begin_tau_segment(L, R, R.hits[L.h]);
     return;
   }
-  tau_pass_done<PASS>(L, reqs, part, T);
+  tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
   return;
 }
 
 abort:
   L.tau_bg += df_val(L.tau_seg);
   L.thick += L.length_cm;
-  lane_finish(L, reqs, T);
+  lane_finish(L, reqs, T, (grp.sub == 0));
 }
 
 // One step of an active lane's tau pass: a quadrature panel for the smooth
 // benchmark family (helical conical B and BK n in the plasma frame, flat
 // flow), a Dormand-Prince attempt otherwise.  The choice belongs to the
 // request, so every build of the kernels gives the same bits.
-template <int PASS, bool GENERAL>
-__device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__ reqs, float* K, int part, Tally& T) {
-  if (!GENERAL || reqs[L.r].mix.helical_log) tau_panel_step<PASS, GENERAL>(L, reqs, part, T);
-  else tau_dopri_step<PASS, GENERAL>(L, reqs, K, part, T);
+template <int PASS, bool GENERAL, int NG>
+__device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__ reqs, float* K, int part, Tally& T,
+                                         const LaneGroup& grp) {
+  if (!GENERAL || reqs[L.r].mix.helical_log) tau_panel_step<PASS, GENERAL, NG>(L, reqs, K, part, T, grp);
+  else tau_dopri_step<PASS, GENERAL>(L, reqs, K, part, T, grp);
+}
+
+// A stage point's coefficients in shared memory: words, or two float4 (NG > 1).
+template <bool FULL, int NG>
+__device__ __forceinline__ void put_coefficients(float* q, const Coef32& c) {
+  if (NG > 1 && FULL) {
+    reinterpret_cast<float4*>(q)[0] = make_float4(c.kI, c.eI, c.kQ, c.kV);
+    reinterpret_cast<float4*>(q)[1] = make_float4(c.kF, c.kC, c.eQ, c.eV);
+    return;
+  }
+  q[0] = c.kI;
+  q[1] = c.eI;
+  if (FULL) {
+    q[2] = c.kQ;
+    q[3] = c.kV;
+    q[4] = c.kF;
+    q[5] = c.kC;
+    q[6] = c.eQ;
+    q[7] = c.eV;
+  }
+}
+template <bool FULL, int NG>
+__device__ __forceinline__ void get_coefficients(const float* q, Coef32& c) {
+  if (NG > 1 && FULL) {
+    const float4 a = reinterpret_cast<const float4*>(q)[0], b = reinterpret_cast<const float4*>(q)[1];
+    c = Coef32{a.x, a.z, a.w, b.x, b.y, a.y, b.z, b.w};
+    return;
+  }
+  c.kI = q[0];
+  c.eI = q[1];
+  if (FULL) {
+    c.kQ = q[2];
+    c.kV = q[3];
+    c.kF = q[4];
+    c.kC = q[5];
+    c.eQ = q[6];
+    c.eV = q[7];
+  }
 }
 
 // ------------------------------------------------------- I / IQUV pass
@@ -1136,8 +1229,9 @@ __device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__
 // its I/IQUV pass, towards the observer.  The arithmetic is the same in
 // every form (static, single-kernel, split), so the images are bitwise the
 // same.
-template <bool FULL, int PASS, bool GENERAL = true>
-__device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict__ reqs, float* Q, Tally& T) {
+template <bool FULL, int PASS, bool GENERAL, int NG>
+__device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict__ reqs, float* Q, Tally& T,
+                                          const LaneGroup& grp) {
   constexpr int NK = StageWidth<FULL>::NK;
   constexpr int NX = StageWidth<FULL>::NX;
   const JshRequest& R = reqs[L.r];
@@ -1213,30 +1307,24 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     // builds for every field law (one copy of that code) in shared memory,
     // with a sixth point where every evaluation draws a random direction.
     Coef32 C[5];
+    constexpr int kPoint = NG > 1 ? 8 : StageWidth<FULL>::NC;  // words of a point (a fused group's: two float4)
     const bool six = GENERAL && R.model.rnd_kind == JSH_RND_POINTS;
-    if (GENERAL) {
-      const int np = six ? 6 : 5;
-#pragma unroll 1
-      for (int s = 1; s <= np; ++s) {
-        Coef32 c;
-        coef32_rt<GENERAL>(R, F, pn + dirf * (c_C[s] * h), mode, c, L.h, (uint32_t)L.f,
-                           L.evals0 + L.evals + (uint32_t)(s - 1), &L.tri);
-        float* q = Q + (s - 1) * StageWidth<FULL>::NC;
-        q[0] = c.kI;
-        q[1] = c.eI;
-        if (FULL) {
-          q[2] = c.kQ;
-          q[3] = c.kV;
-          q[4] = c.kF;
-          q[5] = c.kC;
-          q[6] = c.eQ;
-          q[7] = c.eV;
-        }
-      }
-    } else {
+    if (NG == 1) {
 #pragma unroll
       for (int s = 1; s <= 5; ++s)
-        coef32_rt<GENERAL>(R, F, pn + dirf * (dp_c32(s) * h), mode, C[s - 1], L.h, (uint32_t)L.f, 0, &L.tri);
+        coef32_rt<GENERAL>(R, F, pn + dirf * (dp_c32(s) * h), mode, C[s - 1]);
+    } else {
+      grp.sync();  // the step before has read its coefficients
+      const int np = six ? 6 : 5;
+#pragma unroll 1
+      for (int s = grp.sub + 1; s <= (NG > 1 ? 5 : np); s += NG > 1 ? NG : grp.n) {
+        Coef32 c;
+        // a sixth point is the group's first lane's alone
+        coef32_rt<GENERAL>(R, F, pn + dirf * (c_C[s] * h), mode, c, L.h, (uint32_t)L.f,
+                           L.evals0 + L.evals + (uint32_t)(s - 1), &L.tri, s <= 5 ? grp : single_lane());
+        put_coefficients<FULL, NG>(Q + (s - 1) * kPoint, c);
+      }
+      grp.sync();
     }
     float K[7][NK];
 #pragma unroll
@@ -1258,21 +1346,8 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
         sn = s0 * cd + c0 * sd;
       }
       Coef32 c;
-      if (GENERAL) {
-        const float* q = Q + (s == 6 ? (six ? 5 : 4) : s - 1) * StageWidth<FULL>::NC;
-        c.kI = q[0];
-        c.eI = q[1];
-        if (FULL) {
-          c.kQ = q[2];
-          c.kV = q[3];
-          c.kF = q[4];
-          c.kC = q[5];
-          c.eQ = q[6];
-          c.eV = q[7];
-        }
-      } else {
-        c = C[s == 6 ? 4 : s - 1];
-      }
+      if (NG != 1) get_coefficients<FULL, NG>(Q + (s == 6 ? (six ? 5 : 4) : s - 1) * kPoint, c);
+      else c = C[s == 6 ? 4 : s - 1];
       const float sc = stokes_rhs<FULL>(c, y, cs, sn, dk, ft, &cpl);
       smax = fmaxf(smax, sc);
       s7 = sc;
@@ -1480,32 +1555,86 @@ segment_done : {
     return;
   }
   if (PASS == PASS_IQUV) {
-    lane_finish_iquv(L, reqs, T);
+    lane_finish_iquv(L, reqs, T, (grp.sub == 0));
     return;
   }
-  lane_finish(L, reqs, T);
+  lane_finish(L, reqs, T, (grp.sub == 0));
   return;
 }
 
 abort:
   if (PASS == PASS_IQUV) {
-    lane_finish_iquv(L, reqs, T);
+    lane_finish_iquv(L, reqs, T, (grp.sub == 0));
     return;
   }
-  lane_finish(L, reqs, T);
+  lane_finish(L, reqs, T, (grp.sub == 0));
 }
 
-// One step of an active lane in whichever pass it is.
-template <bool FULL, int PASS, bool GENERAL = true>
-__device__ __forceinline__ void lane_advance(Lane& L, const JshRequest* __restrict__ reqs, float* Q, Tally& T,
-                                             int part = 0) {
-  if (PASS == PASS_BOTH && L.phase == PH_TAU) tau_step<PASS, GENERAL>(L, reqs, Q, part, T);
-  else lane_step<FULL, PASS, GENERAL>(L, reqs, Q, T);
+// One step of an active lane in whichever pass it is (one lane per item).
+template <bool FULL, int PASS>
+__device__ __forceinline__ void lane_advance(Lane& L, const JshRequest* __restrict__ reqs, float* Q, Tally& T) {
+  const LaneGroup one = single_lane();
+  if (PASS == PASS_BOTH && L.phase == PH_TAU) tau_step<PASS, true, 0>(L, reqs, Q, 0, T, one);
+  else lane_step<FULL, PASS, true, 0>(L, reqs, Q, T, one);
 }
 
+// A persistent warp's work: every idle lane (or group of lanes) takes the next
+// item of the queue once at least `refill` lanes of the warp idle, `start(w)`
+// begins item w on this lane, `step()` advances an active one.
+template <typename Start, typename Step>
+__device__ __forceinline__ void run_queue(Lane& L, unsigned long long* queue, unsigned long long total, int refill,
+                                          const LaneGroup& grp, Start start, Step step) {
+  const bool member = grp.mask != 0;
+  const unsigned before = (1u << (grp.base & 31)) - 1u;
+  const int slots = grp.n == 1 ? 32 : kWarpGroups;
+  bool exhausted = false;
+  for (;;) {
+    const unsigned idle = __ballot_sync(0xffffffffu, member && L.phase == PH_IDLE && grp.sub == 0);
+    const int nidle = __popc(idle);
+    if (!exhausted && (nidle * grp.n >= refill || nidle == slots) && nidle > 0) {
+      unsigned long long b = 0;
+      if ((threadIdx.x & 31u) == 0) b = atomicAdd(queue, (unsigned long long)nidle);
+      b = __shfl_sync(0xffffffffu, b, 0);
+      if (b + (unsigned long long)nidle >= total) exhausted = true;
+      if (member && L.phase == PH_IDLE) {
+        const unsigned long long w = b + (unsigned long long)__popc(idle & before);
+        if (w < total) start(w);
+      }
+    }
+    const unsigned active = __ballot_sync(0xffffffffu, L.phase != PH_IDLE);
+    if (active == 0) {
+      if (exhausted) break;
+      continue;
+    }
+    if (L.phase != PH_IDLE) step();
+  }
+}
+
+// Place of this lane's group among the CTA's groups (the last one for a lane
+// that belongs to none).
+__device__ __forceinline__ int group_slot(const LaneGroup& grp) {
+  return (int)(threadIdx.x / 32) * kWarpGroups + min(grp.base / kGroupLanes, kWarpGroups - 1);
+}
+
+// Whether a launch of `total` items runs them on groups of lanes: up to
+// `slots_factor` items for each group the grid holds.
+__device__ __forceinline__ bool on_groups(unsigned long long total, int slots_factor) {
+  return total <= (unsigned long long)slots_factor * gridDim.x * (blockDim.x / 32) * kWarpGroups;
+}
+
+// Words of stage storage of a lane that runs both passes.
 template <bool FULL>
-constexpr size_t stage_smem(int block) {
-  return sizeof(float) * StageWidth<FULL>::kWords * (size_t)block;
+__device__ __host__ constexpr int form_words() {
+  return StageWidth<FULL>::kWords > kTauWords ? StageWidth<FULL>::kWords : kTauWords;
+}
+
+// Dynamic shared memory of a CTA: the lanes' stage storage (none in the fused
+// IQUV build: `lanes` false), or that of its groups.
+template <bool FULL>
+constexpr size_t stage_smem(int block, bool lanes = true) {
+  const size_t one = lanes ? sizeof(float) * form_words<FULL>() * (size_t)block : 0;
+  const size_t groups = sizeof(float) * kGroupWords * kWarpGroups * (size_t)(block / 32);
+  return one > groups ? one : groups;
 }
 
 }  // namespace

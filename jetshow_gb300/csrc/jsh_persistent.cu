@@ -42,43 +42,58 @@ __device__ __forceinline__ void iquv_prefix(const JshRequest* __restrict__ reqs,
   __syncthreads();
 }
 
-// IQUV kernel: persistent CTAs over the ranked emitted items (COMPACT: the
-// register-capped build, as for the single-kernel form).
-template <bool FULL, bool COMPACT, bool GENERAL>
-__global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 3 : 1)
+// IQUV kernels: persistent CTAs over the ranked emitted items.
+//
+// The build for the fused benchmark family alone (COMPACT: at most 128 threads
+// and 128 registers, 16 resident warps per SM).  Up to kIquvGroups* items per
+// group of the grid they run on groups of lanes: fewer evaluations one after
+// another in each step (full Stokes: 8 092 items 86 -> 74 us, 79 782 items 891
+// -> 707 us, above about 100 000 items a lane each is faster: 129 394 items 428
+// against 471 us on groups; Stokes I alone: 2 022 items 55 -> 45 us, 32 350
+// items 80 against 90 us).
+constexpr int kIquvGroupsFull = 9, kIquvGroupsI = 1;
+template <bool FULL, bool COMPACT>
+__global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 4 : 1)
     transfer_iquv_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
                          int part) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
-  extern __shared__ float ksh[];
+  extern __shared__ __align__(16) float ksh[];
   iquv_prefix(reqs, n_req, part, base);
-  float* K = ksh + threadIdx.x * StageWidth<FULL>::kWords;
-  const unsigned long long total = base[n_req];
-  const unsigned lane = threadIdx.x & 31u;
-  const unsigned lt_mask = (1u << lane) - 1u;
   Lane L;
   L.phase = PH_IDLE;
   Tally T = tally_new();
-  bool exhausted = false;
-  for (;;) {
-    unsigned idle = __ballot_sync(0xffffffffu, L.phase == PH_IDLE);
-    int nidle = __popc(idle);
-    if (!exhausted && (nidle >= refill || nidle == 32) && nidle > 0) {
-      unsigned long long b = 0;
-      if (lane == 0) b = atomicAdd(queue, (unsigned long long)nidle);
-      b = __shfl_sync(0xffffffffu, b, 0);
-      if (b + (unsigned long long)nidle >= total) exhausted = true;
-      if (L.phase == PH_IDLE) {
-        unsigned long long w = b + (unsigned long long)__popc(idle & lt_mask);
-        if (w < total) lane_start_iquv(L, reqs, base, n_req, w, part);
-      }
-    }
-    unsigned active = __ballot_sync(0xffffffffu, L.phase != PH_IDLE);
-    if (active == 0) {
-      if (exhausted) break;
-      continue;
-    }
-    if (L.phase != PH_IDLE) lane_step<FULL, PASS_IQUV, GENERAL>(L, reqs, K, T);
+  const unsigned long long total = base[n_req];
+  auto start = [&](unsigned long long w) { lane_start_iquv<false>(L, reqs, base, n_req, w, part); };
+  if (on_groups(total, FULL ? (COMPACT ? kIquvGroupsFull * 3 / 4 : kIquvGroupsFull) : kIquvGroupsI)) {
+    const LaneGroup grp = lane_group();
+    float* Q = ksh + group_slot(grp) * kGroupWords;
+    run_queue(L, queue, total, refill, grp, start,
+              [&] { lane_step<FULL, PASS_IQUV, false, kGroupLanes>(L, reqs, Q, T, grp); });
+  } else {
+    const LaneGroup one = single_lane();
+    run_queue(L, queue, total, refill, one, start,
+              [&] { lane_step<FULL, PASS_IQUV, false, 1>(L, reqs, nullptr, T, one); });
   }
+  tally_flush(T, reqs);
+}
+
+// The build for every field law, with a lane or a group of lanes per item.
+template <bool FULL, bool COMPACT, bool GROUPS>
+__global__ void __launch_bounds__(COMPACT || GROUPS ? 128 : 256, COMPACT || GROUPS ? 3 : 1)
+    transfer_iquv_general_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
+                                 int part) {
+  __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
+  extern __shared__ __align__(16) float ksh[];
+  iquv_prefix(reqs, n_req, part, base);
+  Lane L;
+  L.phase = PH_IDLE;
+  Tally T = tally_new();
+  const LaneGroup grp = GROUPS ? lane_group() : single_lane();
+  float* Q = ksh + (GROUPS ? group_slot(grp) : (int)threadIdx.x) * StageWidth<FULL>::kWords;
+  run_queue(
+      L, queue, base[n_req], refill, grp,
+      [&](unsigned long long w) { lane_start_iquv<true>(L, reqs, base, n_req, w, part); },
+      [&] { lane_step<FULL, PASS_IQUV, true, 0>(L, reqs, Q, T, grp); });
   tally_flush(T, reqs);
 }
 
@@ -91,11 +106,11 @@ int occupancy_mixed(bool split, bool full, int block_size, bool compact) {
   if (split) {
     // the general build bounds both (it holds at least the fused one's registers)
     if (compact) {
-      if (full) JSH_OCC((transfer_iquv_kernel<true, true, true>));
-      else JSH_OCC((transfer_iquv_kernel<false, true, true>));
+      if (full) JSH_OCC((transfer_iquv_general_kernel<true, true, false>));
+      else JSH_OCC((transfer_iquv_general_kernel<false, true, false>));
     } else {
-      if (full) JSH_OCC((transfer_iquv_kernel<true, false, true>));
-      else JSH_OCC((transfer_iquv_kernel<false, false, true>));
+      if (full) JSH_OCC((transfer_iquv_general_kernel<true, false, false>));
+      else JSH_OCC((transfer_iquv_general_kernel<false, false, false>));
     }
   } else {
     JSH_OCC(JSH_SINGLE_KERNEL(full, compact));
@@ -147,14 +162,24 @@ cudaError_t launch_prio(void (*kernel)(KArgs...), unsigned grid, unsigned block,
 
 // IQUV kernel instantiation of a launch.
 using IquvKernel = void (*)(const JshRequest*, int, unsigned long long*, int, int);
-IquvKernel iquv_kernel(bool full, bool compact, bool fused) {
+IquvKernel iquv_kernel(bool full, bool compact, bool fused, bool groups) {
   if (fused) {
-    if (compact) return full ? transfer_iquv_kernel<true, true, false> : transfer_iquv_kernel<false, true, false>;
-    return full ? transfer_iquv_kernel<true, false, false> : transfer_iquv_kernel<false, false, false>;
+    if (compact) return full ? transfer_iquv_kernel<true, true> : transfer_iquv_kernel<false, true>;
+    return full ? transfer_iquv_kernel<true, false> : transfer_iquv_kernel<false, false>;
   }
-  if (compact) return full ? transfer_iquv_kernel<true, true, true> : transfer_iquv_kernel<false, true, true>;
-  return full ? transfer_iquv_kernel<true, false, true> : transfer_iquv_kernel<false, false, true>;
+  if (groups) return full ? transfer_iquv_general_kernel<true, false, true> : transfer_iquv_general_kernel<false, false, true>;
+  if (compact)
+    return full ? transfer_iquv_general_kernel<true, true, false> : transfer_iquv_general_kernel<false, true, false>;
+  return full ? transfer_iquv_general_kernel<true, false, false> : transfer_iquv_general_kernel<false, false, false>;
 }
+
+// Work items up to which the kernels for every law put each on a group of
+// lanes, per SM (the host knows the pixels, not the hits: an upper bound).
+// At 29 092 items of a radial field the tau kernel took 287 us on lanes and
+// 217 on groups, the IQUV kernel 686 and 365; 33 640 items of a gridded jet
+// 65.3 and 37.0 ms, 31.7 and 25.2 ms; at 134 556 of them 108 and 134 ms, 95
+// and 90 ms, at 415 968 items of a radial field 1.6 and 4.0 ms, 1.6 and 2.7.
+constexpr uint64_t kGroupItemsPerSm = 432;
 
 // CTAs of the deep chain's IQUV kernel per SM (64 threads each) when the
 // passes overlap: room for the deep prefix's longest items from the start,
@@ -199,24 +224,39 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   // tau kernel: 256 threads, every CTA it can keep resident (the fused build
   // runs panels only, which keep their sums in registers; the general build
   // keeps Dormand-Prince stages in shared memory)
-  const int bt = 256;
-  const size_t smem_t = jsh_tau_smem(shape.fused != 0, bt);
-  const TauKernel tau_k = jsh_tau_kernel(shape.fused != 0);
+  const bool groups = !shape.fused && need <= kGroupItemsPerSm * (uint64_t)num_sms;
+  const TauLaunch tau = jsh_tau_kernel(shape.fused != 0, groups);
+  const TauKernel tau_k = tau.kernel;
+  const int bt = tau.block;
+  const size_t smem_t = tau.smem;
   int per_sm_t = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_t, tau_k, bt, smem_t);
   if (per_sm_t < 1) per_sm_t = 1;
   unsigned bl_t = (unsigned)(num_sms * per_sm_t);
-  if ((uint64_t)bl_t * bt > need) bl_t = (unsigned)((need + bt - 1) / bt);
-  if (bl_t == 0) bl_t = 1;
-  const IquvKernel iquv_k = iquv_kernel(full, shape.compact != 0, shape.fused != 0);
-  const size_t smem_q = shape.fused ? 0 : smem;  // the fused build keeps its stages in registers
+  // a CTA holds fewer items on groups of lanes than on single ones: enough
+  // CTAs for the former
+  auto enough = [&](unsigned grid, int block) {
+    const unsigned per_cta = (unsigned)(block / 32 * kWarpGroups);
+    return (unsigned)std::min<uint64_t>(grid, (need + per_cta - 1) / per_cta);
+  };
+  bl_t = enough(bl_t, bt);
+  const IquvKernel iquv_k = iquv_kernel(full, shape.compact != 0, shape.fused != 0, groups);
+  // the fused build keeps a single lane's stages in registers
+  auto smem_of = [&](int block) {
+    return full ? stage_smem<true>(block, !shape.fused) : stage_smem<false>(block, !shape.fused);
+  };
+  if (groups && bs > 128) bs = 128;
+  const size_t smem_q = smem_of(bs);
+  int per_sm_q = shape.ctas_per_sm;
+  if (per_sm_q <= 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_q, iquv_k, bs, smem_q);
+  const unsigned blocks_q = enough((unsigned)(num_sms * std::max(per_sm_q, 1)), bs);
   if (!overlap) {
     if (shape.marks) cudaEventRecord(shape.marks[0], stream);
     tau_k<<<bl_t, bt, smem_t, stream>>>(d_reqs, n_req, q, rf, 0);
     if (shape.marks) cudaEventRecord(shape.marks[1], stream);
     jsh_launch_iquv_rank(d_reqs, n_req, num_sms, 0, stream);
     if (shape.marks) cudaEventRecord(shape.marks[2], stream);
-    iquv_k<<<blocks, bs, smem_q, stream>>>(d_reqs, n_req, q + 1, rf, 0);
+    iquv_k<<<blocks_q, bs, smem_q, stream>>>(d_reqs, n_req, q + 1, rf, 0);
     if (shape.marks) cudaEventRecord(shape.marks[3], stream);
     return cudaGetLastError();
   }
@@ -242,19 +282,18 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   e = cudaEventRecord(shape.fork[0], stream);
   if (e != cudaSuccess) return e;
   e = launch_prio(iquv_k, (unsigned)(num_sms * kDeepIquvPerSm), kDeepIquvBlock,
-                  smem_q / bs * kDeepIquvBlock, stream, prio_hi,
+                  smem_of(kDeepIquvBlock), stream, prio_hi,
                   d_reqs, n_req, q + 1, rf, 0);
   if (e != cudaSuccess) return e;
   e = cudaStreamWaitEvent(shape.side, shape.fork[0], 0);
   if (e != cudaSuccess) return e;
   unsigned bl_t2 = (unsigned)(num_sms * per_sm_t2);
-  if ((uint64_t)bl_t2 * bt > need) bl_t2 = (unsigned)((need + bt - 1) / bt);
-  if (bl_t2 == 0) bl_t2 = 1;
+  bl_t2 = enough(bl_t2, bt);
   tau_k<<<bl_t2, bt, smem_t, shape.side>>>(d_reqs, n_req, q + 2, rf, 1);
   if (shape.marks) cudaEventRecord(shape.marks[1], shape.side);
   jsh_launch_iquv_rank(d_reqs, n_req, num_sms, 1, shape.side);
   if (shape.marks) cudaEventRecord(shape.marks[2], shape.side);
-  iquv_k<<<blocks, bs, smem_q, shape.side>>>(d_reqs, n_req, q + 3, rf, 1);
+  iquv_k<<<blocks_q, bs, smem_q, shape.side>>>(d_reqs, n_req, q + 3, rf, 1);
   e = cudaEventRecord(shape.fork[1], shape.side);
   if (e != cudaSuccess) return e;
   e = cudaStreamWaitEvent(stream, shape.fork[1], 0);

@@ -12,10 +12,15 @@ using TauKernel = void (*)(const JshRequest*, int, unsigned long long*, int, int
 using StaticKernel = void (*)(const JshRequest*, int);
 using SingleKernel = void (*)(const JshRequest*, int, unsigned long long*, int);
 
-// The tau kernel (fused: built for the log-domain family alone) and its
+// The tau kernel (fused: built for the log-domain family alone; otherwise for
+// every law, with a lane or a group of lanes per item), its threads and its
 // dynamic shared memory.
-TauKernel jsh_tau_kernel(bool fused);
-size_t jsh_tau_smem(bool fused, int block);
+struct TauLaunch {
+  TauKernel kernel;
+  int block;
+  size_t smem;
+};
+TauLaunch jsh_tau_kernel(bool fused, bool groups);
 
 // Heaviest-first order of every request's hit rays; deep_key as
 // rank_prefix_kernel.

@@ -111,46 +111,58 @@ __device__ __forceinline__ void tau_prefix(const JshRequest* __restrict__ reqs, 
   __syncthreads();
 }
 
-// Tau kernel: persistent CTAs, lanes refilled from the ranked queue (the
-// same order as the single-kernel form), each item's tau pass to its end,
-// over the rays of part `part`.
-// GENERAL = false: the build for batches of the fused benchmark family
-// alone (80 registers, 24 resident warps per SM, against 128 and 16).
-template <bool GENERAL>
-__global__ void __launch_bounds__(256, GENERAL ? 2 : 3) transfer_tau_kernel(const JshRequest* __restrict__ reqs,
-                                                                          int n_req, unsigned long long* queue,
-                                                                          int refill, int part) {
+// Tau kernels: persistent CTAs, lanes (or groups of lanes) refilled from the
+// ranked queue (the same order as the single-kernel form), each item's tau
+// pass to its end, over the rays of part `part`.
+//
+// The build for batches of the fused benchmark family alone (80 registers, 24
+// resident warps per SM).  Up to kTauGroupsFused items per group of the grid
+// (88 000 on 152 SMs) they run on groups: a panel is three evaluations' time
+// instead of fifteen, which counts while rays are few (2 022 items 129 -> 50
+// us, 32 350 items 160 -> 80 us, 79 782 items 174 -> 165 us); above, a lane
+// each does less work per panel (129 394 items 201 us against 227 us on
+// groups, 705 176 items 555 against 1 155 us).
+constexpr int kTauGroupsFused = 4;
+__global__ void __launch_bounds__(256, 3)
+    transfer_tau_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
+                        int part) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
-  extern __shared__ float ksh[];
   tau_prefix(reqs, n_req, part, base);
-  float* K1 = ksh + threadIdx.x * kTauWords;
-  const unsigned long long total = base[n_req];
-  const unsigned lane = threadIdx.x & 31u;
-  const unsigned lt_mask = (1u << lane) - 1u;
   Lane L;
   L.phase = PH_IDLE;
   Tally T = tally_new();
-  bool exhausted = false;
-  for (;;) {
-    unsigned idle = __ballot_sync(0xffffffffu, L.phase == PH_IDLE);
-    int nidle = __popc(idle);
-    if (!exhausted && (nidle >= refill || nidle == 32) && nidle > 0) {
-      unsigned long long b = 0;
-      if (lane == 0) b = atomicAdd(queue, (unsigned long long)nidle);
-      b = __shfl_sync(0xffffffffu, b, 0);
-      if (b + (unsigned long long)nidle >= total) exhausted = true;
-      if (L.phase == PH_IDLE) {
-        unsigned long long w = b + (unsigned long long)__popc(idle & lt_mask);
-        if (w < total) lane_start(L, reqs, base, n_req, w, true, part);
-      }
-    }
-    unsigned active = __ballot_sync(0xffffffffu, L.phase != PH_IDLE);
-    if (active == 0) {
-      if (exhausted) break;
-      continue;
-    }
-    if (L.phase != PH_IDLE) tau_step<PASS_TAU, GENERAL>(L, reqs, K1, part, T);
+  const unsigned long long total = base[n_req];
+  auto start = [&](unsigned long long w) { lane_start(L, reqs, base, n_req, w, true, part); };
+  if (on_groups(total, kTauGroupsFused)) {
+    const LaneGroup grp = lane_group();
+    run_queue(L, queue, total, refill, grp, start,
+              [&] { tau_step<PASS_TAU, false, kGroupLanes>(L, reqs, nullptr, part, T, grp); });
+  } else {
+    const LaneGroup one = single_lane();
+    run_queue(L, queue, total, refill, one, start,
+              [&] { tau_step<PASS_TAU, false, 1>(L, reqs, nullptr, part, T, one); });
   }
+  tally_flush(T, reqs);
+}
+
+// The build for every field law, with a lane per item (128 registers, 16
+// resident warps per SM) or a group per item (168, 12).
+template <bool GROUPS>
+__global__ void __launch_bounds__(128, GROUPS ? 3 : 4)
+    transfer_tau_general_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
+                                int part) {
+  __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
+  extern __shared__ float ksh[];
+  tau_prefix(reqs, n_req, part, base);
+  Lane L;
+  L.phase = PH_IDLE;
+  Tally T = tally_new();
+  const LaneGroup grp = GROUPS ? lane_group() : single_lane();
+  float* K = ksh + (GROUPS ? group_slot(grp) : (int)threadIdx.x) * kTauWords;
+  run_queue(
+      L, queue, base[n_req], refill, grp,
+      [&](unsigned long long w) { lane_start(L, reqs, base, n_req, w, true, part); },
+      [&] { tau_step<PASS_TAU, true, 0>(L, reqs, K, part, T, grp); });
   tally_flush(T, reqs);
 }
 
@@ -206,9 +218,11 @@ __global__ void __launch_bounds__(256) iquv_scatter_kernel(const JshRequest* __r
 
 using namespace jsh;
 
-TauKernel jsh_tau_kernel(bool fused) { return fused ? transfer_tau_kernel<false> : transfer_tau_kernel<true>; }
-
-size_t jsh_tau_smem(bool fused, int block) { return fused ? 0 : sizeof(float) * kTauWords * (size_t)block; }
+TauLaunch jsh_tau_kernel(bool fused, bool groups) {
+  if (fused) return TauLaunch{transfer_tau_kernel, 256, 0};
+  return TauLaunch{groups ? transfer_tau_general_kernel<true> : transfer_tau_general_kernel<false>, 128,
+                   sizeof(float) * kTauWords * (groups ? 128 / 32 * kWarpGroups : 128)};
+}
 
 void jsh_launch_rank(const JshRequest* d_reqs, int n_req, uint64_t max_hits, int deep_key, cudaStream_t stream) {
   const dim3 g((unsigned)((max_hits + 255) / 256), (unsigned)n_req);

@@ -6,6 +6,11 @@ maps can go wrong.
   every evaluation (a sixth evaluation per step); the static and the queue
   schedule bitwise the same, and the oracle at the same tolerances within the
   contract gates.
+* Mixed precision, an item on one lane (static schedule) or on a group of five
+  (persistent schedule, up to a number of items): every plane and counter
+  bitwise the same, for the fused family and the general build, with a random
+  direction per evaluation, and on a gridded field, whose point location
+  tries the triangle of the point before.
 * The stripe pass, 32 steps of a pixel at a time: step counts around 32 and a
   stop inside a group of steps, against the oracle to the last bits of pow
   over n steps (1e-10, as the stripe test).
@@ -15,6 +20,7 @@ import math
 import numpy as np
 import pytest
 
+from jetshow_gb300 import _capi as A
 from jetshow_gb300 import jet as J
 from jetshow_gb300 import workloads as W
 from helpers import compare_images, flat
@@ -72,3 +78,44 @@ def test_stripe_step_groups(ctx, oracle, n, tau_max):
     r = oracle.stripe(jet.desc(), plane.desc(), nu[0], n=n, tau_max=tau_max)
     assert np.array_equal(g == 0, r == 0) and (g > 0).any()
     np.testing.assert_allclose(g, r, rtol=1e-10, atol=0)
+
+
+@pytest.fixture(scope="module")
+def grid_id(ctx):
+    from jetshow_gb300.runtime import triangulate
+    xy, vals = W.simulation_grid_c3(n_points=20_000)
+    return ctx.grid_upload(xy, vals, triangulate(xy))
+
+
+def mixed_jet(kind, grid_id):
+    jet = conical(points=kind == "points")
+    if kind == "sheath":
+        jet.vfield = J.SheathFlatVField(10.0, 3.0, 0.5 * J.pc)
+    elif kind == "tangled":
+        jet.bfield = J.RandomScalarBFieldZ(0.1, 1.0)
+    elif kind == "grid":
+        jet.vfield, jet.nfield = J.SimulationVField(grid_id, 3), J.SimulationNField(grid_id, 2, True)
+        jet.bfield = J.SimulationBField(grid_id, 0, 1, True)
+    return jet
+
+
+@pytest.mark.parametrize("output", ["I", "full"])
+@pytest.mark.parametrize("kind", ["fused", "general", "sheath", "tangled", "points", "grid"])
+@pytest.mark.parametrize("shape,n_nu", [((2, 2), 1), ((2, 7), 1), ((6, 13), 3), ((64, 66), 1)])
+def test_mixed_groups_match_lanes(ctx, grid_id, output, kind, shape, n_nu):
+    mas = (0.01 if kind == "grid" else 6.4) / shape[1]
+    lg = math.log10(mas * 1.8443 * J.pc)
+    plane = J.ImagePlane(shape, lg, lg, 0.1)
+    nu = np.array([8e9, 15.4e9, 22e9][:n_nu]) * 1.1
+    kw = dict(W.ACCURATE_KW, output=output)
+    if kind == "points":  # the draws never converge: the step limits must
+        kw.update(tau_rtol=1e-3, rtol=1e-3)
+    flags = A.FLAG_GENERAL_KERNELS if kind == "general" else 0
+    jet = mixed_jet(kind, grid_id).desc()
+    a, sa = ctx.render(jet, plane.desc(), nu, J.make_params(precision="mixed", schedule="static", **kw))
+    b, sb = ctx.render(jet, plane.desc(), nu, J.make_params(precision="mixed", schedule="persistent", flags=flags, **kw))
+    assert sa["n_work_items"] > 0
+    for k in a:
+        assert np.array_equal(a[k], b[k], equal_nan=True), k
+    for k in ("rhs_evals", "steps_accepted", "steps_rejected", "status_or"):
+        assert sa[k] == sb[k], k
