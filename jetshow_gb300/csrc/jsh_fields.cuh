@@ -1,7 +1,8 @@
 // jsh_fields.cuh -- FP64 field laws, Lorentz kinematics and synchrotron
-// transfer coefficients on the device, written as the reference writes them
-// (src/VField.cpp:25-274, src/BField.cpp:35-224, src/NField.cpp:5-60,
-// src/utils.cpp:8-173, src/Jet.cpp:15-46, :218-237), plus the gridded-field
+// transfer coefficients on the device: the laws as the reference writes them
+// (src/VField.cpp:25-274, src/BField.cpp:35-224, src/NField.cpp:5-60), the
+// coefficients (src/utils.cpp:8-173, src/Jet.cpp:15-46, :218-237) with the
+// constants of a frequency folded (Freq64), plus the gridded-field
 // lookup (src/SimulationInterpolater.cpp:43-102) on a uniform bucket grid.
 // This is the all-FP64 "plain" form; the mixed-precision form lives in
 // jsh_fields_mixed.cuh.
@@ -294,81 +295,119 @@ __device__ inline D3 brandom64(const JshModel& m, D3 b, D3 p, uint32_t k0, uint3
 // ------------------------------------------------------- coefficients
 enum { CK_I = 0, CK_Q, CK_V, CK_F, CK_C, CE_I, CE_Q, CE_V, NCOEF };
 
-// Lab-frame coefficients at p for LOS n_los (towards the observer):
-// k = k'/D and eta = eta' D D with k', eta' evaluated on the plasma-frame
-// B', n', nu' = nu/D and n_los'.  kU = etaU = hQ = 0 (src/utils.cpp:67-69,
-// :101-103, :136-138) and are not stored.  FULL = false computes kI, etaI.
-// (rk0, rk1, rk2): key of a per-evaluation random direction (pixel,
-// frequency, evaluation index), used by JSH_RND_POINTS only.
-template <bool FULL>
-__device__ inline void coefficients64(const JshModel& m, D3 p, D3 nl, double nu, double* k, uint32_t rk0 = 0,
-                                      uint32_t rk1 = 0, uint32_t rk2 = 0) {
-  D3 v = vfield(m, p);
-  D3 beta = v / JSH_C;
-  double gamma = sqrt(1. / (1. - dot(beta, beta)));
-  double D = 1. / (gamma * (1. - dot(beta, nl)));
-  double n = nfield(m, p);
-  double n_prime = m.n_plasma ? n : n / gamma;
-  double nu_prime = nu / D;
-  double s = m.s;
-  double np = sqrt(n_prime * JSH_Q_E * JSH_Q_E / (JSH_PI * JSH_M_E));
+// Constants of one frequency: with b_perp = |n'_los x B'|, w = b_perp D,
+// q = (nu_B sin theta)' / nu' = q1 w and B_par = B'.n'_los, the reference's
+// k'/D and eta' D^2 (src/utils.cpp:39-143, src/Jet.cpp:15-46, :218-237) are
+//   k_I = ki n' w q^(s/2)                eta_I = ei n' w D q^((s-1)/2)
+//   k_V = -kv n' B_par D q^((s+1)/2)     eta_V = -ev n' B_par D^2 q^(s/2)
+//   k_F = kf n' B_par D                  k_C   = -kc n' w^2 (a (b - q^((s-2)/2)) + f_thermal)
+//   k_Q = q_k k_I                        eta_Q = q_e eta_I:
+// every division, and the square root of the plasma frequency that the
+// formulas square again, is out of the evaluation, and the four powers of q
+// follow from one.  GB300's FP64 pipe is the transfer's bound: this form took
+// the 64x96 conical jet from 4.8 to 3.0 ms, get_i_image of 60x90 pixels from
+// 1.05 to 0.80 ms and 1 000 stripe pixels from 0.79 to 0.66 ms, with the same
+// distance from 64-bit references that do not use either form.
+struct Freq64 {
+  double q1, ki, ei, kv, ev, kf, kc;
+};
+__device__ __forceinline__ Freq64 freq64(const JshModel& m, double nu) {
+  const double cb = JSH_Q_E / (2. * JSH_PI * JSH_M_E * JSH_C);  // nu_B per gauss
+  const double cp = JSH_Q_E * JSH_Q_E / (JSH_PI * JSH_M_E);     // nu_p^2 per cm^-3
+  const double k = JSH_PI * cp * cb / (JSH_C * nu * nu), e = JSH_PI * cp * cb * JSH_M_E / JSH_C;
+  const double rk = m.b_scalar ? m.rnd_k : 1.0, re = m.b_scalar ? m.rnd_e : 1.0;
+  return Freq64{cb / nu,    k * (m.fk_i * rk), e * (m.fe_i * re), k * m.fk_v, e * m.fe_v,
+                2. * k * (m.kfr_factor + m.thermal_fraction), k * (cb / nu)};
+}
+
+// Kinematics at a point (src/utils.cpp:147-162): beta, gamma, the Doppler
+// factor and the aberrated line of sight.
+struct Frame64 {
+  D3 beta, nlp;
+  double gamma, D;
+};
+__device__ __forceinline__ Frame64 frame64(const JshModel& m, D3 p, D3 nl) {
+  Frame64 f;
+  f.beta = vfield(m, p) / JSH_C;
+  f.gamma = sqrt(1. / (1. - dot(f.beta, f.beta)));
+  f.D = 1. / (f.gamma * (1. - dot(f.beta, nl)));
+  f.nlp = nl * f.D - f.beta * ((f.D + 1.) * (f.gamma / (f.gamma + 1.)));
+  return f;
+}
+
+// The powers of q the coefficients need, from q^(s/2); each by itself where a
+// quotient would leave the range (q = 0 and NaN included).
+struct Powers64 {
+  double p, m1, p1, m2;  // exponents s/2, (s-1)/2, (s+1)/2, (s-2)/2
+};
+template <int MODE>
+__device__ __forceinline__ Powers64 powers64(double q, double s) {
+  Powers64 P;
+  P.p = pow(q, 0.5 * s);
+  P.m1 = P.p1 = P.m2 = 0.0;
+  if (MODE == 0) return P;
+  if (q > 1e-140 && q < 1e140 && P.p > 1e-140 && P.p < 1e140) {
+    const double r = sqrt(q);
+    P.m1 = P.p / r;
+    if (MODE == 2) {
+      P.p1 = P.p * r;
+      P.m2 = P.p / q;
+    }
+  } else {
+    P.m1 = pow(q, (s - 1.) / 2.);
+    if (MODE == 2) {
+      P.p1 = pow(q, (s + 1.) / 2.);
+      P.m2 = pow(q, (s - 2.) / 2.);
+    }
+  }
+  return P;
+}
+
+// Lab-frame coefficients at p for LOS nl (towards the observer).  kU = etaU =
+// hQ = 0 (src/utils.cpp:67-69, :101-103, :136-138) and are not stored.  MODE:
+// 0 k_I alone, 1 k_I and eta_I, 2 all.  `flat`: the kinematics of a constant
+// flat flow, the same at every point.  (rk0, rk1, rk2): key of a
+// per-evaluation random direction (pixel, frequency, evaluation index), used
+// by JSH_RND_POINTS only.
+template <int MODE>
+__device__ inline void coefficients64(const JshModel& m, const Freq64& F, const Frame64& flat, D3 p, D3 nl, double* k,
+                                      uint32_t rk0 = 0, uint32_t rk1 = 0, uint32_t rk2 = 0) {
+  Frame64 f = flat;
+  if (m.v_kind != JSH_V_CONST_FLAT) f = frame64(m, p, nl);
+  const double n = nfield(m, p);
+  const double np = m.n_plasma ? n : n / f.gamma;
   if (m.b_scalar) {
-    double b = bscalar(m, p);
-    double nb = JSH_Q_E * b / (2. * JSH_PI * JSH_M_E * JSH_C);
-    double k0 = JSH_PI * np * np * nb / (JSH_C * nu_prime * nu_prime);
-    double ki = k0 * pow(nb / nu_prime, s / 2.) * (m.fk_i * m.rnd_k);
-    double e0 = JSH_PI * np * np * nb * JSH_M_E / JSH_C;
-    double ei = e0 * pow(nb / nu_prime, (s - 1.) / 2.) * (m.fe_i * m.rnd_e);
-    k[CK_I] = ki / D;
-    k[CE_I] = ei * D * D;
-    if (FULL) {
+    const double w = bscalar(m, p) * f.D;
+    const Powers64 P = powers64<MODE == 2 ? 1 : MODE>(F.q1 * w, m.s);
+    k[CK_I] = F.ki * np * w * P.p;
+    if (MODE > 0) k[CE_I] = F.ei * np * w * f.D * P.m1;
+    if (MODE == 2) {
       k[CK_Q] = k[CK_V] = k[CK_F] = k[CK_C] = 0.0;
       k[CE_Q] = k[CE_V] = 0.0;
     }
     return;
   }
-  D3 bl = bvector(m, p);
-  if (m.rnd_kind != JSH_RND_NONE) bl = brandom64(m, bl, p, rk0, rk1, rk2);
-  D3 b;
-  if (m.b_plasma) {
-    b = bl;
-  } else {
-    double s1 = gamma / ((1. + gamma) * (JSH_C * JSH_C));
-    double vb = dot(v, bl);
-    b = bl / gamma + d3(s1 * v.x * vb, s1 * v.y * vb, s1 * v.z * vb);
+  D3 b = bvector(m, p);
+  if (m.rnd_kind != JSH_RND_NONE) b = brandom64(m, b, p, rk0, rk1, rk2);
+  if (!m.b_plasma) {
+    // B' = B / Gamma + Gamma / (1 + Gamma) beta (beta . B)
+    b = b / f.gamma + f.beta * (f.gamma / (1. + f.gamma) * dot(f.beta, b));
   }
-  double df = D;
-  D3 nlp = nl * df - beta * ((df + 1.) * (gamma / (gamma + 1.)));
-  double nb = JSH_Q_E * norm(cross(nlp, b)) / (2. * JSH_PI * JSH_M_E * JSH_C);
-  double k0 = JSH_PI * np * np * nb / (JSH_C * nu_prime * nu_prime);
-  double ki = k0 * pow(nb / nu_prime, s / 2.) * m.fk_i;
-  double e0 = JSH_PI * np * np * nb * JSH_M_E / JSH_C;
-  double ei = e0 * pow(nb / nu_prime, (s - 1.) / 2.) * m.fe_i;
-  k[CK_I] = ki / D;
-  k[CE_I] = ei * D * D;
-  if (!FULL) return;
-  double bn = norm(b);
-  double cos_theta = dot(b, nlp) / bn;
-  double nbv = JSH_Q_E * bn / (2. * JSH_PI * JSH_M_E * JSH_C);
-  double k0v = JSH_PI * np * np * nbv / (JSH_C * nu_prime * nu_prime);
-  double kv = -k0v * cos_theta * pow(nb / nu_prime, (s + 1.) / 2.) * m.fk_v;
-  double kfc = 2. * JSH_PI * np * np * nbv * cos_theta / (JSH_C * nu_prime * nu_prime);
-  double kcc = -JSH_PI * np * np * nb * nb / (JSH_C * nu_prime * nu_prime * nu_prime);
-  double kf = m.kfr_factor * kfc;
-  double kc = m.kcr_a * (m.kcr_b - pow(nb / nu_prime, (s - 2.) / 2.)) * kcc;
-  if (m.thermal_fraction != 0.0) {
-    double npt = sqrt(m.thermal_fraction * n_prime * JSH_Q_E * JSH_Q_E / (JSH_PI * JSH_M_E));
-    kf = kf + 2. * JSH_PI * npt * npt * nbv * cos_theta / (JSH_C * nu_prime * nu_prime);
-    kc = kc + -JSH_PI * npt * npt * nb * nb / (JSH_C * nu_prime * nu_prime * nu_prime);
-  }
-  double e0v = JSH_PI * np * np * nbv * JSH_M_E / JSH_C;
-  double ev = -e0v * cos_theta * pow(nb / nu_prime, s / 2.) * m.fe_v;
-  k[CK_Q] = (m.kq_ratio * ki) / D;
-  k[CK_V] = kv / D;
-  k[CK_F] = kf / D;
-  k[CK_C] = kc / D;
-  k[CE_Q] = (m.eq_ratio * ei) * D * D;
-  k[CE_V] = ev * D * D;
+  const double w = norm(cross(f.nlp, b)) * f.D;
+  const Powers64 P = powers64<MODE>(F.q1 * w, m.s);
+  k[CK_I] = F.ki * np * w * P.p;
+  if (MODE == 0) return;
+  k[CE_I] = F.ei * np * w * f.D * P.m1;
+  if (MODE == 1) return;
+  // B = 0: the reference's cos(theta) = B.n'/|B| is 0/0
+  const double bpar = dot(b, b) == 0.0 ? NAN : dot(b, f.nlp);
+  const double c = np * bpar * f.D;
+  k[CK_Q] = m.kq_ratio * k[CK_I];
+  k[CE_Q] = m.eq_ratio * k[CE_I];
+  k[CK_V] = -F.kv * c * P.p1;
+  k[CE_V] = -F.ev * c * f.D * P.p;
+  k[CK_F] = F.kf * c;
+  k[CK_C] = -F.kc * np * (w * w) * (m.kcr_a * (m.kcr_b - P.m2) + m.thermal_fraction);
 }
 
 }  // namespace jsh

@@ -35,7 +35,7 @@ namespace {
 // dtau/dt at path coordinate t.
 __device__ __forceinline__ double tau_rate(const JshModel& m, const Path64& P, double t) {
   double k[NCOEF];
-  coefficients64<false>(m, P.p0 + P.dir * t, P.nl, P.nu, k);
+  P.at<0>(m, t, k, 0);
   return k[CK_I];
 }
 
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kStripeThreads) stripe_tau_kernel(const JshReq
     const D3 dd = d3(h.s[s].out.x, h.s[s].out.y, h.s[s].out.z) - pin;
     const double length = sq(ad(ad(ml(dd.x, dd.x), ml(dd.y, dd.y)), ml(dd.z, dd.z)));
     const double dt = length / n;
-    const Path64 P{pin, rd, nl, nu};
+    const Path64 P = path64(R.model, pin, rd, nl, nu);
     double x = 0.0;
     bool found = (x >= tau_max);
     if (dt > 0.0) {

@@ -67,9 +67,21 @@ __device__ __forceinline__ constexpr double dp_a(int s, int j) {
 // Path point(t) = p0 + t * dir; nl = LOS towards the observer.
 struct Path64 {
   D3 p0, dir, nl;
-  double nu;
+  Freq64 F;
+  Frame64 flat;       // kinematics of a constant flat flow
   uint32_t rk0, rk1;  // random-direction key of the item: pixel, frequency
+  // coefficients at path coordinate t for the item's evaluation `ev`
+  template <int MODE>
+  __device__ __forceinline__ void at(const JshModel& m, double t, double* k, uint32_t ev) const {
+    coefficients64<MODE>(m, F, flat, p0 + dir * t, nl, k, rk0, rk1, ev);
+  }
 };
+__device__ __forceinline__ Path64 path64(const JshModel& m, D3 p0, D3 dir, D3 nl, double nu, uint32_t rk0 = 0,
+                                         uint32_t rk1 = 0) {
+  Path64 P{p0, dir, nl, freq64(m, nu), Frame64{}, rk0, rk1};
+  if (m.v_kind == JSH_V_CONST_FLAT) P.flat = frame64(m, p0, nl);
+  return P;
+}
 
 struct Ctl64 {
   double atol, rtol, max_dt;
@@ -138,11 +150,11 @@ struct ItemOut {
 
 // The coefficients at point t + c dt of this lane's stage (lane k: stage
 // k + 2), keyed as the (k + 1)-th of the step's evaluations.
-template <bool FULL>
+template <int MODE>
 __device__ __forceinline__ void stage_coefficients(const JshModel& m, const Path64& P, const Group64& G, double t,
                                                    double dt, uint32_t ev, double* k) {
   const double c = G.sub == 0 ? dp::C2 : G.sub == 1 ? dp::C3 : G.sub == 2 ? dp::C4 : G.sub == 3 ? dp::C5 : 1.0;
-  coefficients64<FULL>(m, P.p0 + P.dir * (t + c * dt), P.nl, P.nu, k, P.rk0, P.rk1, ev + (uint32_t)G.sub);
+  P.at<MODE>(m, t + c * dt, k, ev + (uint32_t)G.sub);
 }
 
 // Tau pass of one segment (src/Observation.cpp:150-211): dense-output
@@ -159,7 +171,7 @@ __device__ __forceinline__ uint32_t tau_segment64(const JshModel& m, const Path6
   {
     double c[NCOEF];
     if (!(length - t > DBL_EPSILON)) return 0;
-    coefficients64<false>(m, P.p0, P.nl, P.nu, c, P.rk0, P.rk1, ev++);
+    P.at<0>(m, 0.0, c, ev++);
     C.evals++;
     k[0] = c[CK_I];
   }
@@ -176,12 +188,12 @@ __device__ __forceinline__ uint32_t tau_segment64(const JshModel& m, const Path6
       continue;
     }
     double c[NCOEF];
-    stage_coefficients<false>(m, P, G, t, dt, ev, c);
+    stage_coefficients<0>(m, P, G, t, dt, ev, c);
 #pragma unroll
     for (int s = 1; s < 6; ++s) k[s] = from_lane(G, c[CK_I], s - 1);
     k[6] = k[5];
     if (m.rnd_kind == JSH_RND_POINTS) {  // every evaluation draws its own direction: a sixth one
-      coefficients64<false>(m, P.p0 + P.dir * (t + dt), P.nl, P.nu, c, P.rk0, P.rk1, ev + 5);
+      P.at<0>(m, t + dt, c, ev + 5);
       k[6] = c[CK_I];
     }
     ev += 6;
@@ -247,7 +259,7 @@ __device__ __forceinline__ uint32_t iquv_segment64(const JshModel& m, const Path
   {
     if (!(length - t > DBL_EPSILON)) return 0;
     double c[NCOEF];
-    coefficients64<FULL>(m, P.p0, P.nl, P.nu, c, P.rk0, P.rk1, ev++);
+    P.at<FULL ? 2 : 1>(m, 0.0, c, ev++);
     C.evals++;
     if (FULL) {
       __syncwarp(G.mask);
@@ -267,9 +279,9 @@ __device__ __forceinline__ uint32_t iquv_segment64(const JshModel& m, const Path
     }
     if (nsteps++ >= C.max_steps) return JSH_ST_STEP_LIMIT;
     double c[NCOEF], c6[NCOEF];
-    stage_coefficients<FULL>(m, P, G, t, dt, ev, c);
+    stage_coefficients<FULL ? 2 : 1>(m, P, G, t, dt, ev, c);
     const bool six = m.rnd_kind == JSH_RND_POINTS;
-    if (six) coefficients64<FULL>(m, P.p0 + P.dir * (t + dt), P.nl, P.nu, c6, P.rk0, P.rk1, ev + 5);
+    if (six) P.at<FULL ? 2 : 1>(m, t + dt, c6, ev + 5);
     ev += 6;
     C.evals += 6;
     if (FULL) {
@@ -361,7 +373,7 @@ __device__ void transfer_item64(const JshModel& m, const JshPlane& pl, const Jsh
     D3 pout = d3(hit.seg[sidx][3], hit.seg[sidx][4], hit.seg[sidx][5]);
     D3 dd = pout - pin;
     double length = sqrt((dd.x * dd.x + dd.y * dd.y) + dd.z * dd.z);
-    Path64 P{pin, rd, nl, nu, (uint32_t)hit.pix, (uint32_t)f};
+    const Path64 P = path64(m, pin, rd, nl, nu, (uint32_t)hit.pix, (uint32_t)f);
     Ctl64 C{Pp.tau_atol, Pp.tau_rtol, Pp.dt_max, max_steps, 0, 0, 0};
     double x = 0.0, k[7], x_old = 0.0, dt_used = 0.0, t_old = 0.0;
     const uint32_t fail =
@@ -417,7 +429,7 @@ __device__ void transfer_item64(const JshModel& m, const JshPlane& pl, const Jsh
     double length = sqrt((dd.x * dd.x + dd.y * dd.y) + dd.z * dd.z);
     double auto_n = Pp.n;
     if (background_tau > 0.1) auto_n = steps_schedule(background_tau, Pp.n, 10 * Pp.n);
-    Path64 P{pout, nl, nl, nu, (uint32_t)hit.pix, (uint32_t)f};
+    const Path64 P = path64(m, pout, nl, nl, nu, (uint32_t)hit.pix, (uint32_t)f);
     Ctl64 C{Pp.atol, Pp.rtol, 0.0, max_steps, 0, 0, 0};
     const uint32_t fail = iquv_segment64<FULL>(m, P, G, C, length, length / auto_n, ev, st);
     tot.evals += C.evals;
