@@ -49,20 +49,16 @@ struct GridW {
   bool ok;
 };
 // Barycentric weights of (px, py) in triangle t; true when inside (the
-// -1e-6 tolerance of the bucket search).
+// -1e-6 tolerance of the bucket search).  The triangle's record holds what
+// depends on it alone.
 __device__ __forceinline__ bool grid_tri32(const JshGrid& G, int t, float px, float py, GridW& g) {
-  const int v0 = G.tri[3 * t], v1 = G.tri[3 * t + 1], v2 = G.tri[3 * t + 2];
-  const float2 a = *reinterpret_cast<const float2*>(G.xyf + 2 * v0);
-  const float2 bb = *reinterpret_cast<const float2*>(G.xyf + 2 * v1);
-  const float2 c = *reinterpret_cast<const float2*>(G.xyf + 2 * v2);
-  const float area = (bb.x - a.x) * (c.y - a.y) - (bb.y - a.y) * (c.x - a.x);
-  if (area == 0.f) return false;
-  const float ia = 1.f / area;
-  const float w0 = ((bb.x - px) * (c.y - py) - (bb.y - py) * (c.x - px)) * ia;
-  const float w1 = ((px - a.x) * (c.y - a.y) - (py - a.y) * (c.x - a.x)) * ia;
+  const float4* r = reinterpret_cast<const float4*>(G.rec) + 3 * (int64_t)t;
+  const float4 ab = r[0], ce = r[1], iv = r[2];
+  const float w0 = ((ab.z - px) * (ce.y - py) - (ab.w - py) * (ce.x - px)) * iv.x;
+  const float w1 = ((px - ab.x) * ce.w - (py - ab.y) * ce.z) * iv.x;
   const float w2 = 1.f - w0 - w1;
   if (w0 >= -1e-6f && w1 >= -1e-6f && w2 >= -1e-6f) {
-    g = GridW{v0, v1, v2, w0, w1, w2, true};
+    g = GridW{__float_as_int(iv.y), __float_as_int(iv.z), __float_as_int(iv.w), w0, w1, w2, true};
     return true;
   }
   return false;
@@ -120,7 +116,7 @@ __device__ __forceinline__ LaneGroup single_lane() {
 // bucket: every lane first tries the step's hint and, failing that, its
 // bucket; then the points take their turn with the triangle before them,
 // which most often is one of the two already tried.
-static __device__ __noinline__ GridW grid_locate32_group(const JshGrid& G, float px, float py, int* hint, LaneGroup L) {
+__device__ __forceinline__ GridW grid_locate32_group(const JshGrid& G, float px, float py, int* hint, LaneGroup L) {
   GridW g, own;
   g.ok = own.ok = false;
   if (G.n_tri == 0) return g;
@@ -154,14 +150,28 @@ static __device__ __noinline__ GridW grid_locate32_group(const JshGrid& G, float
 }
 __device__ __forceinline__ float grid_val32(const JshGrid& G, const GridW& g, int field, float nan_value) {
   if (!g.ok) return nan_value;
-  const int64_t nf = G.n_fields;
-  const float v = g.w0 * G.val[g.v0 * nf + field] + g.w1 * G.val[g.v1 * nf + field] +
-                  g.w2 * G.val[g.v2 * nf + field];
+  const uint32_t nf = (uint32_t)G.n_fields;  // n and n_fields are bounded: 2^30 points x 64 fields
+  const float v = g.w0 * G.val[(uint64_t)g.v0 * nf + field] + g.w1 * G.val[(uint64_t)g.v1 * nf + field] +
+                  g.w2 * G.val[(uint64_t)g.v2 * nf + field];
   return isnan(v) ? nan_value : v;
 }
-// (z, r) in pc: one field of a gridded field
-__device__ inline float sim32(const JshGrid& G, int field, F3 p, float nan_value) {
+// (z, r) in pc: one field of a gridded field.  The gridded laws (and the other
+// long ones) are calls: inlined at every law that may use them they set the
+// registers and the code size of the kernels for every other law too.  With
+// the calls and the triangle records a simulation grid at 256^2 went from
+// 36.0 + 26.2 ms (tau, IQUV kernel) to 25.0 + 17.5, 512^2 from 114 + 96 to 76
+// + 55; 415 968 items of a radial field from 1.53 + 1.78 to 1.36 + 1.08.
+static __device__ __noinline__ float sim32(const JshGrid& G, int field, F3 p, float nan_value) {
   return grid_val32(G, grid_locate32(G, p.z, sqrtf(p.x * p.x + p.y * p.y)), field, nan_value);
+}
+
+// The simulation workload's four fields from their one grid: Gamma, n, B_p and
+// B_phi at (z, rc) by one point location.
+static __device__ __noinline__ float4 sim_shared32(const JshModel& m, float z, float rc, int* hint, LaneGroup group) {
+  const JshGrid& G = m.grids[0];
+  const GridW g = grid_locate32_group(G, z, rc, hint, group);
+  return make_float4(grid_val32(G, g, m.f_v, 1.0f), grid_val32(G, g, m.f_n, 0.f), grid_val32(G, g, m.fb_p, 0.f),
+                     grid_val32(G, g, m.fb_phi, 0.f));
 }
 
 // ---------------------------------------------------------------- V
@@ -170,7 +180,7 @@ struct Vel {
   F3 dir;  // unit
 };
 
-__device__ __forceinline__ F3 parabolic_dir(float Rz0_pc, F3 p) {
+static __device__ __noinline__ F3 parabolic_dir(float Rz0_pc, F3 p) {
   float r = hypotf(p.x, p.y);
   if (r == 0.f) return f3(0.f, 0.f, 1.f);
   float R = sqrtf(Rz0_pc * Rz0_pc * p.z);
@@ -396,7 +406,7 @@ __device__ inline int cells_nearest32(const JshCells& C, F3 p) {
 // RandomVectorBField::bf (src/BField.cpp:154-161) in FP32: B + fraction |B| n
 // with the nearest cell's direction or the per-evaluation draw of the key
 // (pixel of hit h, frequency f, evaluation index e).
-__device__ inline F3 brandom32(const JshRequest& R, F3 B, F3 p, uint32_t h, uint32_t f, uint32_t e) {
+static __device__ __noinline__ F3 brandom32(const JshRequest& R, F3 B, F3 p, uint32_t h, uint32_t f, uint32_t e) {
   const JshModel& m = R.model;
   F3 n;
   if (m.rnd_kind == JSH_RND_CELLS) {
@@ -552,19 +562,16 @@ __device__ __forceinline__ void coef32_rt(const JshRequest& R, const JshFreqCons
   } else if (X.sim_shared) {
     // every field from one grid (the simulation workload): one point location
     // for Gamma, n, B_p and B_phi
-    const float rc = sqrtf(p.x * p.x + p.y * p.y);
     int hint = tri_hint ? *tri_hint : -1;  // its address escapes, the lane's state must not
-    const GridW g = grid_locate32_group(m.grids[0], p.z, rc, &hint, group);
+    const float4 v = sim_shared32(m, p.z, sqrtf(p.x * p.x + p.y * p.y), &hint, group);
     if (tri_hint) *tri_hint = hint;
-    gamma = grid_val32(m.grids[0], g, m.f_v, 1.0f);
+    gamma = v.x;
     vdir = f3(0, 0, 1);
     kinematics32(gamma, vdir, f3(X.nl[0], X.nl[1], X.nl[2]), D, nlp, beta);
-    const float n = grid_val32(m.grids[0], g, m.f_n, 0.f);
-    np_ = m.n_plasma ? n : n / gamma;
+    np_ = m.n_plasma ? v.y : v.y / gamma;
     float s, cph;
     sincos_atan(p.y / p.x, s, cph);
-    const float bp = grid_val32(m.grids[0], g, m.fb_p, 0.f);
-    const float bphi = grid_val32(m.grids[0], g, m.fb_phi, 0.f);
+    const float bp = v.z, bphi = v.w;
     B = f3(-s * bphi, cph * bphi, bp);
   } else {
     if (X.v_const) {

@@ -422,8 +422,20 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
   for (int64_t t = 0; t < n_tri; ++t)
     for (int32_t j = box[4 * t + 2]; j <= box[4 * t + 3]; ++j)
       for (int32_t i = box[4 * t]; i <= box[4 * t + 1]; ++i) items[fill[(size_t)j * nbx + i]++] = (int32_t)t;
-  std::vector<float> xyf((size_t)2 * n);
-  for (int64_t i = 0; i < 2 * n; ++i) xyf[i] = (float)xy[i];
+  // triangle records: the FP32 operations here round as the device's would
+  std::vector<float> rec((size_t)12 * n_tri);
+  for (int64_t t = 0; t < n_tri; ++t) {
+    float* r = &rec[(size_t)12 * t];
+    for (int k = 0; k < 3; ++k) {
+      r[2 * k] = (float)xy[2 * (int64_t)tri[3 * t + k]];
+      r[2 * k + 1] = (float)xy[2 * (int64_t)tri[3 * t + k] + 1];
+    }
+    r[6] = r[4] - r[0];
+    r[7] = r[5] - r[1];
+    const float area = (r[2] - r[0]) * r[7] - (r[3] - r[1]) * r[6];
+    r[8] = area == 0.f ? NAN : 1.f / area;
+    memcpy(r + 9, tri + 3 * t, 3 * sizeof(int32_t));
+  }
 
   std::lock_guard<std::mutex> lk(ctx->mu);
   int id = -1;
@@ -434,7 +446,7 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
     return JSH_ERR_INVALID;
   }
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-  const size_t o_xy = 0, o_xyf = o_xy + al(sizeof(double) * 2 * n), o_val = o_xyf + al(sizeof(float) * 2 * n),
+  const size_t o_xy = 0, o_rec = o_xy + al(sizeof(double) * 2 * n), o_val = o_rec + al(sizeof(float) * rec.size()),
                o_tri = o_val + al(sizeof(float) * (size_t)n * n_fields), o_bs = o_tri + al(sizeof(int32_t) * 3 * n_tri),
                o_bi = o_bs + al(sizeof(int32_t) * (nbk + 1)), total = o_bi + al(sizeof(int32_t) * items.size());
   JSH_CUDA_TRY(cudaSetDevice(ctx->device));
@@ -443,7 +455,7 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
   if (st) return st;
   char* base = (char*)mem;
   cudaError_t e = cudaMemcpy(base + o_xy, xy, sizeof(double) * 2 * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(base + o_xyf, xyf.data(), sizeof(float) * 2 * n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(base + o_rec, rec.data(), sizeof(float) * rec.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(base + o_val, values, sizeof(float) * (size_t)n * n_fields, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(base + o_tri, tri, sizeof(int32_t) * 3 * n_tri, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(base + o_bs, bstart.data(), sizeof(int32_t) * (nbk + 1), cudaMemcpyHostToDevice);
@@ -459,7 +471,7 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
   S.bytes = total;
   JshGrid& G = S.view;
   G.xy = (const double*)(base + o_xy);
-  G.xyf = (const float*)(base + o_xyf);
+  G.rec = (const float*)(base + o_rec);
   G.val = (const float*)(base + o_val);
   G.tri = (const int32_t*)(base + o_tri);
   G.bstart = (const int32_t*)(base + o_bs);

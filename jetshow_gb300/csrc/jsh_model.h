@@ -31,7 +31,10 @@ struct JshCone {
 
 struct JshGrid {         // device view of an uploaded triangulated (z, r) grid
   const double* xy;      // [n][2] (z, r) in pc
-  const float* xyf;      // [n][2] the same in FP32 (mixed-precision lookups)
+  // [n_tri][12] mixed-precision lookups, a triangle in three float4: FP32
+  // vertices a, b, c, the edge c - a, 1 / (twice its area) (NaN for a
+  // degenerate one), and its vertex ids as integer bits
+  const float* rec;
   const float* val;      // [n][n_fields]
   const int32_t* tri;    // [n_tri][3]
   const int32_t* bstart; // [nbx*nby + 1] bucket -> triangle list offsets
