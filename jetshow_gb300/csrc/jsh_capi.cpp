@@ -94,6 +94,8 @@ void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int3
   o = align_up(o + sizeof(JshIquvItem) * npix * (uint64_t)n_nu);
   L->off_iq_order = o;
   o = align_up(o + sizeof(uint32_t) * npix * (uint64_t)n_nu);
+  L->off_seg32 = o;
+  o = align_up(o + sizeof(JshSeg32) * JSH_MAX_SEG * npix);
   L->own_outputs = own_outputs;
   for (int k = 0; k < 7; ++k) {
     L->off_out[k] = o;
@@ -111,6 +113,7 @@ void jsh_bind_request(JshRequest* req, char* base, const JshRequestLayout& L, bo
   req->plane.along_center = (double*)(base + L.off_along_center);
   req->plane.across_pos = (double*)(base + L.off_across);
   req->hits = (JshHit*)(base + L.off_hits);
+  req->seg32 = (JshSeg32*)(base + L.off_seg32);
   req->buckets = (uint32_t*)(base + L.off_buckets);
   req->order = (uint32_t*)(base + L.off_order);
   req->key = (uint8_t*)(base + L.off_key);

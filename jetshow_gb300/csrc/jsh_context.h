@@ -47,7 +47,7 @@ struct JshHullSlot {
 struct JshRequestLayout {
   size_t off_req, off_counters, off_nhit, off_queue, off_buckets, off_iq_count, off_iq_buckets, off_nu, off_fc,
       off_along_size, off_along_center, off_across, off_hits, off_order, off_key, off_iq_items, off_iq_order,
-      off_out[7];
+      off_seg32, off_out[7];
   size_t total;
   bool own_outputs;
 };

@@ -167,10 +167,10 @@ struct Lane {
                          // stage points are b + c h d in FP32 (error u |b|)
   DF length, t;          // segment length and coordinate [pc]
   float dt;              // [pc]
-  double length_cm;
   DF tau_seg;            // optical depth of the current tau segment
   float thick_left;      // tau_thick - (depth of the finished segments)
-  double tau_bg, thick;
+  float first_div;       // I/IQUV pass: divisor of a segment's first step
+  double tau_bg, thick;  // tau pass: depth and length of the finished segments
   double t_first;        // [pc] IQUV start on first_seg: tau_max crossing or optically thick point
   DF chi;                // Faraday rotation angle, kept reduced to [-pi, pi]
   float x[4];
@@ -207,7 +207,12 @@ constexpr int kTauWords = 17;  // the 15 nodes of a panel, odd
 // for each (NG = 1, 5); the builds for every field law (NG = 0: the group's
 // size is LaneGroup::n) evaluate the points in a rolled loop, one copy of that
 // larger code, and exchange through the stage storage of the group (or lane).
-constexpr int kGroupWords = 52;  // fused I/IQUV step: six points of two float4, the groups spread over the banks
+// fused I/IQUV step: five points of two float4 (three with the Faraday-thick
+// mode), the groups spread over the banks
+#ifndef JSH_FARADAY_THICK_BUILD
+#define JSH_FARADAY_THICK_BUILD 0
+#endif
+constexpr int kGroupWords = JSH_FARADAY_THICK_BUILD ? 76 : 52;
 
 // acc = sum_{j < S} a_Sj K_j over the stage derivatives held in registers
 // (S and j compile-time: the tableau entries are immediate operands).
@@ -241,14 +246,12 @@ __device__ __forceinline__ float first_step_divisor(double tau_bg, int n) {
   return ceilf(fmaf(k * l, l, (float)n));
 }
 
-__device__ __forceinline__ void set_segment(Lane& L, double ox, double oy, double oz, double length_cm) {
-  L.length_cm = length_cm;
-  const double len = length_cm * INV_PC;
-  L.length = df_of(len);
+__device__ __forceinline__ void start_segment(Lane& L, DF px, DF py, DF pz, DF len) {
+  L.length = len;
   L.t = DF{0.f, 0.f};
-  L.p0x = df_of(ox * INV_PC);
-  L.p0y = df_of(oy * INV_PC);
-  L.p0z = df_of(oz * INV_PC);
+  L.p0x = px;
+  L.p0y = py;
+  L.p0z = pz;
   L.bx = L.p0x.hi;
   L.by = L.p0y.hi;
   L.bz = L.p0z.hi;
@@ -258,12 +261,24 @@ __device__ __forceinline__ void set_segment(Lane& L, double ox, double oy, doubl
   L.fails = 0;
 }
 
-__device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R, const JshHit& H) {
-  int s = L.seg;
-  set_segment(L, H.seg[s][0], H.seg[s][1], H.seg[s][2], seg_len_cm(H, s, H.seg[s][3], H.seg[s][4], H.seg[s][5]));
+// Total optical depth of the lane's tau pass, which is in its last segment.
+__device__ __forceinline__ double tau_total(const Lane& L) {
+  return L.seg == 0 ? df_val(L.tau_seg) : L.tau_bg + df_val(L.tau_seg);
+}
+
+__device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R) {
+  const JshSeg32& S = R.seg32[(uint64_t)L.h * JSH_MAX_SEG + L.seg];
+  start_segment(L, DF{S.in[0], S.in[1]}, DF{S.in[2], S.in[3]}, DF{S.in[4], S.in[5]}, DF{S.len[0], S.len[1]});
   const float len = L.length.hi + L.length.lo;
+  if (L.seg == 0) {
+    L.thick = S.len_cm;
+    L.thick_left = R.mix.tau_eq_f;
+  } else {
+    L.tau_bg = df_val(L.tau_seg);  // two segments at most: that of segment 0
+    L.thick += S.len_cm;
+    L.thick_left = (float)(R.mix.tau_eq - L.tau_bg);
+  }
   L.tau_seg = DF{0.f, 0.f};
-  L.thick_left = (float)(R.mix.tau_eq - L.tau_bg);
   if (!R.mix.helical_log) {
     // the Dormand-Prince tau pass: the reference's first step L / n
     L.dt = len / (float)R.P.n;
@@ -294,18 +309,22 @@ __device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R, 
   }
 }
 
-__device__ __forceinline__ void begin_iquv_segment(Lane& L, const JshRequest& R, const JshHit& H) {
-  int s = L.seg;
-  double ox = H.seg[s][3], oy = H.seg[s][4], oz = H.seg[s][5];
+__device__ __forceinline__ void begin_iquv_segment(Lane& L, const JshRequest& R) {
+  const int s = L.seg;
   if (s == L.first_seg) {
+    // inside the segment, t_first from its near end
     L.first_seg = -1;
-    double tc = L.t_first * JSH_PC;
-    ox = H.seg[s][0] + R.plane.rx * tc;
-    oy = H.seg[s][1] + R.plane.ry * tc;
-    oz = H.seg[s][2] + R.plane.rz * tc;
+    const JshHit& H = R.hits[L.h];
+    const double tc = L.t_first * JSH_PC;
+    const double ox = H.seg[s][0] + R.plane.rx * tc, oy = H.seg[s][1] + R.plane.ry * tc,
+                 oz = H.seg[s][2] + R.plane.rz * tc;
+    start_segment(L, df_of(ox * INV_PC), df_of(oy * INV_PC), df_of(oz * INV_PC),
+                  df_of(seg_len_cm(H, s, ox, oy, oz) * INV_PC));
+  } else {
+    const JshSeg32& S = R.seg32[(uint64_t)L.h * JSH_MAX_SEG + s];
+    start_segment(L, DF{S.out[0], S.out[1]}, DF{S.out[2], S.out[3]}, DF{S.out[4], S.out[5]}, DF{S.len[0], S.len[1]});
   }
-  set_segment(L, ox, oy, oz, seg_len_cm(H, s, ox, oy, oz));
-  L.dt = (L.length.hi + L.length.lo) / first_step_divisor(L.tau_bg, R.P.n);
+  L.dt = (L.length.hi + L.length.lo) / L.first_div;
   L.ft = 0;  // (Q, U) enters a segment as it left the last one, not quasi-static
   L.ft_cool = 0;
   L.ft_back = 0;
@@ -347,7 +366,7 @@ __device__ __forceinline__ void lane_start(Lane& L, const JshRequest* __restrict
   L.ft = 0;
   L.ft_cool = 0;
   L.evals0 = 0;
-  begin_tau_segment(L, R, H);
+  begin_tau_segment(L, R);
 }
 
 // Per-lane totals of a request's counters (right-hand-side evaluations,
@@ -440,27 +459,35 @@ __device__ __noinline__ void write_finished_iquv(const JshRequest* __restrict__ 
   if (R.status) R.status[q] = status;
 }
 
-// Optical depth the I/IQUV pass of an item integrates through (its cost
-// grows with it), bucketed by half octaves; everything below 0.5 in bucket 1.
-__device__ __forceinline__ uint8_t iquv_cost_key(double tau_bg, bool eq, bool first, const JshMixed& X) {
-  double d = eq ? X.tau_eq : (first ? fmin(tau_bg, X.tau_thick) : tau_bg);
-  if (!(d > 0.5)) return 1;
-  const int k = (int)floorf(2.f * __log2f((float)d)) + 3;
+// Optical depth the I/IQUV pass of an item integrates through, bucketed by
+// half octaves from 2^-19 up.  The pass's cost grows with it, also where the
+// ray is thin (its Faraday depth grows with the optical depth: on a
+// ParabaloidCone image the mean cost falls from 8 700 evaluations at depth 1
+// to 430 at 2^-11), so the order puts the longest items first and items of one
+// length into one warp.
+__device__ __forceinline__ uint8_t iquv_cost_key(float tau, bool eq, bool first, const JshMixed& X) {
+  float d = first ? fminf(tau, (float)X.tau_thick) : tau;
+  // from the equilibrium at tau_eq the pass is the shorter the deeper the ray
+  // (512x1024 conical jet: 1 450 evaluations at depth 50, 820 at 240, 425 at
+  // 10^4, as rays of depth 30, 10 and 2)
+  if (eq) d = (float)X.tau_eq * sqrtf((float)X.eq_min / tau);
+  if (!(d > 0.f)) return 1;
+  const int k = (int)floorf(2.f * __log2f(d)) + 40;
   return (uint8_t)min(max(k, 1), JSH_RANK_BUCKETS - 1);
 }
 
 // Split form, tau kernel: hand an item whose I/IQUV pass is still to run to
-// the IQUV kernel.  Writes the item's tau and l planes and its tau-pass
+// the IQUV kernel.  Writes the item's l plane (and its tau plane, unless the
+// depth is left a pair for the ranking kernel to convert) and its tau-pass
 // counters, appends its record to the request's list of its part (one
 // atomic per request among the lanes that emit together).
 __device__ __noinline__ void emit_iquv(const JshRequest* __restrict__ reqs, int part, int r, int f, uint32_t h,
-                                       double tau_bg,
-                                       double thick, double t_first, int first_seg, int nseg, bool eq,
-                                       uint32_t status, uint32_t evals) {
+                                       bool pair, DF tau, double tau_bg, double thick, double t_first, int first_seg,
+                                       int nseg, bool eq, uint32_t status, uint32_t evals) {
   const JshRequest& R = reqs[r];
   const JshHit& H = R.hits[h];
   uint64_t q = (uint64_t)f * R.npix + (uint64_t)H.pix;
-  if (R.tau) R.tau[q] = tau_bg;
+  if (R.tau && !pair) R.tau[q] = tau_bg;
   if (R.l) R.l[q] = (R.P.flags & JSH_FLAG_COST_MAP) ? (double)evals : thick;
   const unsigned mask = __activemask();
   const unsigned peers = __match_any_sync(mask, r);
@@ -473,11 +500,16 @@ __device__ __noinline__ void emit_iquv(const JshRequest* __restrict__ reqs, int 
   JshIquvItem it;
   it.h = h;
   it.f = (uint16_t)f;
-  it.key = iquv_cost_key(tau_bg, eq, first_seg >= 0, R.mix);
-  it.flags = (uint8_t)((nseg & 3) | (eq ? 4 : 0) | ((first_seg + 1) << 3));
+  it.key = iquv_cost_key(pair ? tau.hi : (float)tau_bg, eq, first_seg >= 0, R.mix);
+  it.flags = (uint8_t)((nseg & 3) | (eq ? 4 : 0) | ((first_seg + 1) << 3) | (pair ? 32 : 0));
   it.status = status;
   it.evals = evals;
-  it.tau_bg = tau_bg;
+  if (pair) {
+    it.tau_pair[0] = tau.hi;
+    it.tau_pair[1] = tau.lo;
+  } else {
+    it.tau_bg = tau_bg;
+  }
   it.t_first = t_first;
   R.iq_items[slot] = it;
 }
@@ -508,9 +540,21 @@ __device__ __noinline__ double crossing_time(double tau_old, double t_old, doubl
 // Stokes derivatives of the I/IQUV pass from the coefficients of the stage's
 // point.  Returns the magnitude of the terms summed into the derivatives
 // (eta_I + k_I |I|): the scale of their FP32 rounding noise.
+//
+// FtPoint: what the Faraday-thick mode needs of a stage point besides the
+// coefficients, 1 / |lambda|^2 and max(|k_Q|, |k_C|) / |lambda| (lambda = k_I -
+// i k_F): it does not depend on the state either.
+struct FtPoint {
+  float il, cpl;
+};
+__device__ __forceinline__ FtPoint ft_point(const Coef32& c) {
+  const float il = 1.f / fmaf(c.kI, c.kI, c.kF * c.kF);
+  return FtPoint{il, fmaxf(fabsf(c.kQ), fabsf(c.kC)) * sqrtf(il)};
+}
+
 template <bool FULL>
-__device__ __forceinline__ float stokes_rhs(const Coef32& c, const float* y, float cs, float sn, float* dk,
-                                            bool ft, float* cpl) {
+__device__ __forceinline__ float stokes_rhs(const Coef32& c, const FtPoint& q, const float* y, float cs, float sn,
+                                            float* dk, bool ft, float* cpl) {
   const float scale = fabsf(c.eI) + fabsf(c.kI * y[0]);
   if (!FULL) {
     dk[0] = c.eI - c.kI * y[0];
@@ -526,14 +570,13 @@ __device__ __forceinline__ float stokes_rhs(const Coef32& c, const float* y, flo
     // share rotates at k_F and integrates to at most ~cpl |d|.  dk[1], dk[2]
     // carry the rotating-frame value e^{-i chi} S / lambda itself.
     const float sre = c.eQ - c.kQ * y[0], sim = -c.kC * y[3];
-    const float il = 1.f / fmaf(c.kI, c.kI, c.kF * c.kF);
-    const float pre = fmaf(sre, c.kI, -sim * c.kF) * il, pim = fmaf(sre, c.kF, sim * c.kI) * il;
+    const float pre = fmaf(sre, c.kI, -sim * c.kF) * q.il, pim = fmaf(sre, c.kF, sim * c.kI) * q.il;
     dk[0] = c.eI - c.kI * y[0] - c.kQ * pre - c.kV * y[3];
     dk[1] = fmaf(cs, pre, sn * pim);
     dk[2] = fmaf(-sn, pre, cs * pim);
     dk[3] = c.eV - c.kI * y[3] - c.kV * y[0] + c.kC * pim;
     dk[4] = c.kF;
-    *cpl = fmaxf(fabsf(c.kQ), fabsf(c.kC)) * sqrtf(il);
+    *cpl = q.cpl;
     return scale;
   }
   float Qlab = cs * y[1] - sn * y[2];
@@ -622,8 +665,7 @@ __device__ __forceinline__ void lane_start_iquv(Lane& L, const JshRequest* __res
   L.nseg = (int8_t)(it.flags & 3);
   L.first_seg = (int8_t)((it.flags >> 3) & 3) - 1;
   const bool eq = (it.flags & 4) != 0;
-  L.tau_bg = it.tau_bg;
-  L.thick = 0.0;
+  L.first_div = it.first_div;
   L.t_first = it.t_first;
   L.chi = DF{0.f, 0.f};
   L.x[0] = L.x[1] = L.x[2] = L.x[3] = 0.f;
@@ -645,7 +687,7 @@ __device__ __forceinline__ void lane_start_iquv(Lane& L, const JshRequest* __res
     L.x[2] = xe.z;
     L.x[3] = xe.w;
   }
-  begin_iquv_segment(L, R, H);
+  begin_iquv_segment(L, R);
 }
 
 // FP32 unit roundoff; the Stokes error norm's noise floor is
@@ -740,9 +782,14 @@ template <int PASS, bool GENERAL>
 __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restrict__ reqs, int part, Tally& T,
                                               bool lead) {
   const JshRequest& R = reqs[L.r];
-  if (!(L.tau_bg > R.P.tau_min)) {
-    lane_finish(L, reqs, T, lead);
-    return;
+  // a depth of one segment surely above tau_min stays a pair (no FP64 here)
+  const bool pair = PASS == PASS_TAU && L.seg == 0 && L.tau_seg.hi > R.mix.tau_min_f;
+  if (!pair) {
+    L.tau_bg = tau_total(L);
+    if (!(L.tau_bg > R.P.tau_min)) {
+      lane_finish(L, reqs, T, lead);
+      return;
+    }
   }
   L.status |= JSH_ST_IQUV;
   L.phase = PH_IQUV;
@@ -750,16 +797,18 @@ __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restr
   if (L.first_seg >= 0 && R.mix.eq_start) {
     // the equilibrium start needs depth behind tau_eq: rays shallower than
     // eq_min are integrated whole from their far end
-    if (L.tau_bg >= R.mix.eq_min || (L.status & JSH_ST_TAU_CROSSED)) eq = true;
+    if ((pair ? df_val(L.tau_seg) : L.tau_bg) >= R.mix.eq_min || (L.status & JSH_ST_TAU_CROSSED)) eq = true;
     else L.first_seg = -1;
   }
   if (PASS == PASS_TAU) {
     L.phase = PH_IDLE;
     if (!lead) return;
-    emit_iquv(reqs, part, L.r, L.f, L.h, L.tau_bg, L.thick, L.t_first, L.first_seg, L.nseg, eq, L.status, L.evals);
+    emit_iquv(reqs, part, L.r, L.f, L.h, pair, L.tau_seg, L.tau_bg, L.thick, L.t_first, L.first_seg, L.nseg, eq,
+              L.status, L.evals);
     tally_add(T, reqs, L.r, L.evals, L.acc, L.rej, 0u);
     return;
   }
+  L.first_div = first_step_divisor(L.tau_bg, R.P.n);
   L.seg = L.first_seg >= 0 ? L.first_seg : L.nseg - 1;
   L.tri = -1;  // as the IQUV kernel's fresh lanes
   L.ft = 0;
@@ -775,7 +824,7 @@ __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restr
     L.x[2] = xe.z;
     L.x[3] = xe.w;
   }
-  begin_iquv_segment(L, R, H);
+  begin_iquv_segment(L, R);
 }
 
 // One panel of an active lane's tau pass (or a segment / pass transition).
@@ -894,8 +943,6 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
       L.first_seg = L.seg;
       L.t_first = df_val(L.t) + (double)h;
       L.nseg = L.seg + 1;
-      L.tau_bg += df_val(L.tau_seg);
-      L.thick += L.length_cm;
       tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
       return;
     }
@@ -957,8 +1004,6 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
         }
         L.tau_seg = tn;
         L.nseg = L.seg + 1;
-        L.tau_bg += df_val(L.tau_seg);
-        L.thick += L.length_cm;
         tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
         return;
       }
@@ -994,11 +1039,9 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
   }
 
 segment_done : {
-  L.tau_bg += df_val(L.tau_seg);
-  L.thick += L.length_cm;
   if (L.seg + 1 < L.nseg) {
     L.seg++;
-    begin_tau_segment(L, R, R.hits[L.h]);
+    begin_tau_segment(L, R);
     return;
   }
   tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
@@ -1007,8 +1050,7 @@ segment_done : {
 
 abort:
   L.init = false;
-  L.tau_bg += df_val(L.tau_seg);
-  L.thick += L.length_cm;
+  L.tau_bg = tau_total(L);
   lane_finish(L, reqs, T, (grp.sub == 0));
 }
 
@@ -1148,8 +1190,6 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
         L.t_first = tc;
       }
       L.nseg = L.seg + 1;
-      L.tau_bg += df_val(L.tau_seg);
-      L.thick += L.length_cm;
       tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
       return;
     }
@@ -1158,11 +1198,9 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
   }
 
 segment_done : {
-  L.tau_bg += df_val(L.tau_seg);
-  L.thick += L.length_cm;
   if (L.seg + 1 < L.nseg) {
     L.seg++;
-    begin_tau_segment(L, R, R.hits[L.h]);
+    begin_tau_segment(L, R);
     return;
   }
   tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
@@ -1170,8 +1208,7 @@ segment_done : {
 }
 
 abort:
-  L.tau_bg += df_val(L.tau_seg);
-  L.thick += L.length_cm;
+  L.tau_bg = tau_total(L);
   lane_finish(L, reqs, T, (grp.sub == 0));
 }
 
@@ -1283,7 +1320,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     if (!L.init) {
       Coef32 c;
       coef32_rt<GENERAL>(R, F, pn, mode, c, L.h, (uint32_t)L.f, L.evals0 + L.evals, &L.tri);
-      L.s1 = stokes_rhs<FULL>(c, L.x, c0, s0, L.k1, ft, &cpl);
+      L.s1 = stokes_rhs<FULL>(c, ft ? ft_point(c) : FtPoint{}, L.x, c0, s0, L.k1, ft, &cpl);
       L.kI1 = c.kI;
       L.evals++;
       L.init = true;
@@ -1307,7 +1344,9 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     // builds for every field law (one copy of that code) in shared memory,
     // with a sixth point where every evaluation draws a random direction.
     Coef32 C[5];
-    constexpr int kPoint = NG > 1 ? 8 : StageWidth<FULL>::NC;  // words of a point (a fused group's: two float4)
+    // words of a point (a fused group's: two float4, three with the
+    // Faraday-thick mode)
+    constexpr int kPoint = NG > 1 ? (kFtm ? 12 : 8) : StageWidth<FULL>::NC;
     const bool six = GENERAL && R.model.rnd_kind == JSH_RND_POINTS;
     if (NG == 1) {
 #pragma unroll
@@ -1323,6 +1362,11 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
         coef32_rt<GENERAL>(R, F, pn + dirf * (c_C[s] * h), mode, c, L.h, (uint32_t)L.f,
                            L.evals0 + L.evals + (uint32_t)(s - 1), &L.tri, s <= 5 ? grp : single_lane());
         put_coefficients<FULL, NG>(Q + (s - 1) * kPoint, c);
+        if (NG > 1 && kFtm && FULL && ft) {
+          const FtPoint q = ft_point(c);
+          Q[(s - 1) * kPoint + 8] = q.il;
+          Q[(s - 1) * kPoint + 9] = q.cpl;
+        }
       }
       grp.sync();
     }
@@ -1346,9 +1390,13 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
         sn = s0 * cd + c0 * sd;
       }
       Coef32 c;
-      if (NG != 1) get_coefficients<FULL, NG>(Q + (s == 6 ? (six ? 5 : 4) : s - 1) * kPoint, c);
+      const float* q = Q + (s == 6 ? (six ? 5 : 4) : s - 1) * kPoint;
+      if (NG != 1) get_coefficients<FULL, NG>(q, c);
       else c = C[s == 6 ? 4 : s - 1];
-      const float sc = stokes_rhs<FULL>(c, y, cs, sn, dk, ft, &cpl);
+      FtPoint cq{};
+      if (ft && NG > 1) cq = FtPoint{q[8], q[9]};
+      else if (ft) cq = ft_point(c);
+      const float sc = stokes_rhs<FULL>(c, cq, y, cs, sn, dk, ft, &cpl);
       smax = fmaxf(smax, sc);
       s7 = sc;
       kI7 = c.kI;
@@ -1551,7 +1599,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
 segment_done : {
   if (L.seg > 0) {
     L.seg--;
-    begin_iquv_segment(L, R, R.hits[L.h]);
+    begin_iquv_segment(L, R);
     return;
   }
   if (PASS == PASS_IQUV) {
@@ -1581,12 +1629,24 @@ __device__ __forceinline__ void lane_advance(Lane& L, const JshRequest* __restri
 // A persistent warp's work: every idle lane (or group of lanes) takes the next
 // item of the queue once at least `refill` lanes of the warp idle, `start(w)`
 // begins item w on this lane, `step()` advances an active one.
+//
+// Groups begin without the queue, the k-th group of every warp with the k-th
+// stretch of the order, so that the longest items are in different warps: a
+// warp that is left with one item runs its steps faster than one with six.
+// (Single lanes take consecutive items: items of one length end together.)
 template <typename Start, typename Step>
 __device__ __forceinline__ void run_queue(Lane& L, unsigned long long* queue, unsigned long long total, int refill,
                                           const LaneGroup& grp, Start start, Step step) {
   const bool member = grp.mask != 0;
   const unsigned before = (1u << (grp.base & 31)) - 1u;
   const int slots = grp.n == 1 ? 32 : kWarpGroups;
+  unsigned long long dealt = 0;
+  if (grp.n > 1) {
+    const unsigned warps = gridDim.x * (blockDim.x / 32), warp = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    const unsigned long long w = (unsigned long long)(grp.base / kGroupLanes) * warps + warp;
+    if (member && w < total) start(w);
+    dealt = (unsigned long long)kWarpGroups * warps;
+  }
   bool exhausted = false;
   for (;;) {
     const unsigned idle = __ballot_sync(0xffffffffu, member && L.phase == PH_IDLE && grp.sub == 0);
@@ -1595,6 +1655,7 @@ __device__ __forceinline__ void run_queue(Lane& L, unsigned long long* queue, un
       unsigned long long b = 0;
       if ((threadIdx.x & 31u) == 0) b = atomicAdd(queue, (unsigned long long)nidle);
       b = __shfl_sync(0xffffffffu, b, 0);
+      b += dealt;
       if (b + (unsigned long long)nidle >= total) exhausted = true;
       if (member && L.phase == PH_IDLE) {
         const unsigned long long w = b + (unsigned long long)__popc(idle & before);

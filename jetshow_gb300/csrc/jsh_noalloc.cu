@@ -34,7 +34,10 @@
 
 #include "jsh_context.h"
 
-#define JSH_NOALLOC_SCRATCH_BYTES (8u << 20)
+// A request's state may take 8 MiB besides its segments in FP32.
+#define JSH_NOALLOC_STATE_BYTES (8u << 20)
+#define JSH_NOALLOC_SCRATCH_BYTES \
+  (JSH_NOALLOC_STATE_BYTES + JSH_NOALLOC_MAX_PIXELS * JSH_MAX_SEG * sizeof(JshSeg32))
 #define JSH_NOALLOC_MAX_DEVICES 64
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[JSH_NOALLOC_SCRATCH_BYTES];
@@ -151,9 +154,10 @@ extern "C" int jsh_observation_run_noalloc(const jsh_model_desc* model, const js
   if (st) return st;
   JshRequestLayout L;
   jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, false, &L);
-  if (L.total > JSH_NOALLOC_SCRATCH_BYTES) {
-    jsh_set_error("request needs %zu scratch bytes, more than the %u of the no-alloc array", L.total,
-                  JSH_NOALLOC_SCRATCH_BYTES);
+  const size_t state = L.total - (L.off_out[0] - L.off_seg32);
+  if (state > JSH_NOALLOC_STATE_BYTES) {
+    jsh_set_error("request needs %zu scratch bytes, more than the %u of the no-alloc array", state,
+                  JSH_NOALLOC_STATE_BYTES);
     return JSH_ERR_INVALID;
   }
   jsh_bind_request(&in.req, base, L, false);

@@ -53,7 +53,7 @@ __device__ __forceinline__ void iquv_prefix(const JshRequest* __restrict__ reqs,
 // items 80 against 90 us).
 constexpr int kIquvGroupsFull = 9, kIquvGroupsI = 1;
 template <bool FULL, bool COMPACT>
-__global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 4 : 1)
+__global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? (kFtm ? 3 : 4) : 1)
     transfer_iquv_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
                          int part) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
@@ -64,13 +64,12 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 4 : 1)
   Tally T = tally_new();
   const unsigned long long total = base[n_req];
   auto start = [&](unsigned long long w) { lane_start_iquv<false>(L, reqs, base, n_req, w, part); };
+  const LaneGroup grp = lane_group(), one = single_lane();
+  float* Q = ksh + group_slot(grp) * kGroupWords;
+  auto group_step = [&] { lane_step<FULL, PASS_IQUV, false, kGroupLanes>(L, reqs, Q, T, grp); };
   if (on_groups(total, FULL ? (COMPACT ? kIquvGroupsFull * 3 / 4 : kIquvGroupsFull) : kIquvGroupsI)) {
-    const LaneGroup grp = lane_group();
-    float* Q = ksh + group_slot(grp) * kGroupWords;
-    run_queue(L, queue, total, refill, grp, start,
-              [&] { lane_step<FULL, PASS_IQUV, false, kGroupLanes>(L, reqs, Q, T, grp); });
+    run_queue(L, queue, total, refill, grp, start, group_step);
   } else {
-    const LaneGroup one = single_lane();
     run_queue(L, queue, total, refill, one, start,
               [&] { lane_step<FULL, PASS_IQUV, false, 1>(L, reqs, nullptr, T, one); });
   }
@@ -327,6 +326,7 @@ int jsh_prepare_mixed(JshRequest* req, const double* nu_host, JshFreqConst* fc) 
   X.pk = (float)((s + 2.) / 2.);
   X.dt_max_pc = req->P.dt_max / JSH_PC;
   X.dt_max_f = (float)X.dt_max_pc;
+  X.tau_min_f = nextafterf((float)(std::max(req->P.tau_min, 0.0) * (1.0 + 1e-6)), INFINITY);
   {
     const double d[3] = {req->plane.dx, req->plane.dy, req->plane.dz};
     for (int k = 0; k < 3; ++k) {
@@ -379,6 +379,7 @@ int jsh_prepare_mixed(JshRequest* req, const double* nu_host, JshFreqConst* fc) 
     // the gradients of the source function, attenuated by exp(-(1 - p) 30)
     X.eq_start = (req->P.full && X.tau_thick < INFINITY && kTauEq < X.tau_thick) ? 1 : 0;
     X.tau_eq = X.eq_start ? kTauEq : X.tau_thick;
+    X.tau_eq_f = (float)X.tau_eq;
     X.eq_min = X.eq_start ? std::min(kTauEqMin, X.tau_thick) : X.tau_thick;
   }
   if (m.v_kind == JSH_V_CONST_FLAT) {

@@ -14,6 +14,17 @@ struct JshHit {           // one intersecting pixel (Intersection list)
   double seg[JSH_MAX_SEG][6];  // {point_in xyz, point_out xyz}
 };
 
+// One segment of a hit for the mixed path, in pc: both end points and the
+// length as compensated FP32 pairs (hi, lo), and the length in cm.  The hit
+// kernel computes them in FP64 once per ray, with every lane of its warps:
+// in the transfer kernels, where a few lanes at a time start an item, each
+// FP64 instruction holds the sub-partition's pipe for all of them.
+struct alignas(16) JshSeg32 {
+  float in[6], out[6];  // x hi, x lo, y hi, ...
+  float len[2];
+  double len_cm;
+};
+
 // Cost buckets of the heaviest-first ranking (factors of 2 in optical depth).
 #define JSH_RANK_BUCKETS 64
 // Words of a request's ranking state: bucket counts, bucket cursors, then
@@ -27,16 +38,24 @@ struct JshHit {           // one intersecting pixel (Intersection list)
 
 // Persistent mixed schedule, split form: one work item whose tau pass has
 // finished and whose I/IQUV pass is still to run, as the tau kernel hands it
-// to the IQUV kernel (32 bytes).  The tau and l planes of the item are
-// written already; the IQUV kernel writes I, Q, U, V and the final status.
+// to the IQUV kernel (32 bytes).  The tau kernel writes the item's l plane, it
+// or the ranking the tau plane, the IQUV kernel I, Q, U, V and the final status.
 struct JshIquvItem {
   uint32_t h;          // hit index
   uint16_t f;          // frequency index
   uint8_t key;         // IQUV cost bucket (heaviest-first order)
-  uint8_t flags;       // bits 0-1: nseg; bit 2: equilibrium start; bits 3-4: first_seg + 1
+  uint8_t flags;       // bits 0-1: nseg; bit 2: equilibrium start; bits 3-4: first_seg + 1;
+                       // bit 5: the depth is a pair and not yet in the tau plane
   uint32_t status;     // status bits of the tau pass (JSH_ST_IQUV set)
   uint32_t evals;      // right-hand-side evaluations of the tau pass (cost map)
-  double tau_bg;       // total optical depth of the tau pass
+  // total optical depth of the tau pass, as an FP64 value or (flags bit 5) a
+  // compensated FP32 pair; the ranking kernel replaces it by the divisor of
+  // the I/IQUV pass's first steps
+  union {
+    double tau_bg;
+    float tau_pair[2];
+    float first_div;
+  };
   double t_first;      // [pc] IQUV start on first_seg (tau_max crossing or optically thick point)
 };
 
@@ -88,6 +107,8 @@ struct JshMixed {
   float sin_pitch, cos_pitch, tan_pitch, b_bessel0, b_bessel1;
   float tau_atol, tau_rtol, rtol;  // FP32 copies of the step-control tolerances
   float dt_max_f;                  // dt_max_pc in FP32
+  float tau_eq_f;                  // tau_eq in FP32
+  float tau_min_f;                 // an FP32 depth above this is above tau_min
   float dhi[3], dlo[3];            // ray direction as compensated FP32 pairs
   float tau_max_hi, tau_max_lo;    // tau_max as a compensated FP32 pair
   const JshFreqConst* fc;  // device [n_nu]
@@ -99,6 +120,7 @@ struct JshRequest {
   JshPlane plane;
   JshParamsDev P;
   JshHit* hits;           // device [npix] (first n_hit valid)
+  JshSeg32* seg32;        // device [npix][JSH_MAX_SEG], mixed precision: the hits' segments
   // persistent mixed schedule: hit rays ranked by estimated cost, heaviest
   // first (order[rank] = hit index), their cost buckets and the ranking
   // state [JSH_RANK_WORDS] (zeroed with the counters)

@@ -33,8 +33,8 @@ __global__ void __launch_bounds__(256) rank_cost_kernel(const JshRequest* __rest
     const float wk[4] = {0.173927423f, 0.326072577f, 0.326072577f, 0.173927423f};
     float tau = 0.f;
     for (int s = 0; s < H.nseg && s < 2; ++s) {
-      const F3 a = f3((float)(H.seg[s][0] * INV_PC), (float)(H.seg[s][1] * INV_PC), (float)(H.seg[s][2] * INV_PC));
-      const F3 b = f3((float)(H.seg[s][3] * INV_PC), (float)(H.seg[s][4] * INV_PC), (float)(H.seg[s][5] * INV_PC));
+      const JshSeg32& S = R.seg32[(uint64_t)h * JSH_MAX_SEG + s];
+      const F3 a = f3(S.in[0], S.in[2], S.in[4]), b = f3(S.out[0], S.out[2], S.out[4]);
       const F3 d = b - a;
       float acc = 0.f;
 #pragma unroll 1
@@ -167,15 +167,24 @@ __global__ void __launch_bounds__(128, GROUPS ? 3 : 4)
 }
 
 // Cost histogram of part `part`'s emitted items of request blockIdx.y
-// (grid-stride).
+// (grid-stride), and the items' FP64 work, a full warp of them at a time: the
+// tau plane where the depth is still a pair, the first-step divisor.
 __global__ void __launch_bounds__(256) iquv_hist_kernel(const JshRequest* __restrict__ reqs, int part) {
   __shared__ uint32_t hist[JSH_RANK_BUCKETS];
   const JshRequest& R = reqs[blockIdx.y];
   for (int b = threadIdx.x; b < JSH_RANK_BUCKETS; b += blockDim.x) hist[b] = 0;
   __syncthreads();
   const uint32_t n = R.iq_count[part], o = iq_first(R, part);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    atomicAdd(&hist[R.iq_items[o + i].key], 1u);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    JshIquvItem& it = R.iq_items[o + i];
+    atomicAdd(&hist[it.key], 1u);
+    double tau = it.tau_bg;
+    if (it.flags & 32) {
+      tau = df_val(DF{it.tau_pair[0], it.tau_pair[1]});
+      if (R.tau) R.tau[(uint64_t)it.f * R.npix + (uint64_t)R.hits[it.h].pix] = tau;
+    }
+    it.first_div = first_step_divisor(tau, R.P.n);
+  }
   __syncthreads();
   uint32_t* bk = R.iq_buckets + 2 * JSH_RANK_BUCKETS * part;
   for (int b = threadIdx.x; b < JSH_RANK_BUCKETS; b += blockDim.x)
