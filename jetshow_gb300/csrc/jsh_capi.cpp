@@ -383,6 +383,7 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   JshLaunchShape shape = jsh_effective_shape(ctx, params);
   shape.fused = (req.mix.helical_log && !(params->flags & JSH_FLAG_GENERAL_KERNELS)) ? 1 : 0;
   shape.marks = nullptr;
+  shape.mix = &req.mix;
   const bool overlap = jsh_overlap_passes(params, shape, npix * (uint64_t)n_nu);
   if (overlap && shape.overlap_key <= 0) shape.overlap_key = JSH_OVERLAP_KEY;
   shape.side = overlap ? ctx->side : nullptr;

@@ -467,6 +467,21 @@ __device__ __forceinline__ void coef32_tail(const JshFreqConst& F, const JshMixe
 // force on it.
 enum CoefMode { COEF_KI = 0, COEF_I = 1, COEF_FULL = 2 };
 
+// log2 and exp2 without the scaling that subnormal operands and results need
+// (three instructions each): |p|^2 in pc^2 and |n' x u|^2 are 0 or far above
+// 2^-126 (u and n' have components of order 1, rounded to 2^-24), and so are
+// the densities, fields and coefficients in their units.
+__device__ __forceinline__ float lg2(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // The benchmark family in the plasma frame (ConstFlat V, helical conical B,
 // BK n) in the log domain: with l = log2|p|, u the helical unit direction
 // and w = |n' x B| D = b |n' x u| D,
@@ -479,7 +494,7 @@ enum CoefMode { COEF_KI = 0, COEF_I = 1, COEF_FULL = 2 };
 // + (a_C c2 / a_k) k_I, B_par = b (u . n').
 __device__ __forceinline__ void coef32_helical_log(const JshMixed& X, const JshFreqConst& F, F3 p, int mode,
                                                    Coef32& c) {
-  const float l = 0.5f * __log2f(fdot(p, p));
+  const float l = 0.5f * lg2(fdot(p, p));
   const float rc2 = p.x * p.x + p.y * p.y;
   float px = 0.f, py = 0.f;
   if (rc2 > 0.f) {
@@ -495,17 +510,17 @@ __device__ __forceinline__ void coef32_helical_log(const JshMixed& X, const JshF
   const F3 u = f3(st * px, st * py, X.b_sign * X.cos_pitch);
   const F3 nlp = f3(X.nlp[0], X.nlp[1], X.nlp[2]);
   const F3 cr = fcross(nlp, u);
-  const float lw = fmaf(-X.bq[1], l, X.l2_b0D) + 0.5f * __log2f(fdot(cr, cr));
+  const float lw = fmaf(-X.bq[1], l, X.l2_b0D) + 0.5f * lg2(fdot(cr, cr));
   // n' and w^pk as two exp2 of arguments of ~20 each rather than one of ~50:
   // exp2f's relative error is ~ulp(argument), so the split keeps k_I's
   // rounding at the level of the product form
-  const float n_ = exp2f(fmaf(-X.nq[1], l, X.l2_n0));
-  c.kI = (F.ak * n_) * exp2f(X.pk * lw);
+  const float n_ = ex2(fmaf(-X.nq[1], l, X.l2_n0));
+  c.kI = (F.ak * n_) * ex2(X.pk * lw);
   if (mode == COEF_KI) return;
-  c.eI = (F.ae * X.D * n_) * exp2f(X.pk_h * lw);
+  c.eI = (F.ae * X.D * n_) * ex2(X.pk_h * lw);
   if (mode == COEF_I) return;
-  const float bpar = exp2f(fmaf(-X.bq[1], l, X.l2_b0)) * fdot(u, nlp);
-  const float w = exp2f(lw);
+  const float bpar = ex2(fmaf(-X.bq[1], l, X.l2_b0)) * fdot(u, nlp);
+  const float w = ex2(lw);
   const float D = X.D;
   c.kQ = X.kq * c.kI;
   c.eQ = X.eq * c.eI;
@@ -515,6 +530,8 @@ __device__ __forceinline__ void coef32_helical_log(const JshMixed& X, const JshF
   c.kC = fmaf(F.r_kc, c.kI, -F.ac * F.c1 * n_ * (w * w));
 }
 
+// X is R.mix, or the same record in the kernel's parameters (a launch on one
+// request: the constants are then operands of the instructions, not loads).
 // (rk_h, rk_f, rk_e): hit index, frequency and evaluation index of the
 // per-evaluation random direction (JSH_RND_POINTS only); tri_hint: the
 // lane's point-location hint for fields on one shared grid (may be null).
@@ -522,11 +539,10 @@ __device__ __forceinline__ void coef32_helical_log(const JshMixed& X, const JshF
 // kernels launched only on requests whose mix.helical_log is set (the same
 // arithmetic as the general build takes for them).
 template <bool GENERAL = true>
-__device__ __forceinline__ void coef32_rt(const JshRequest& R, const JshFreqConst& F, F3 p, int mode, Coef32& c,
+__device__ __forceinline__ void coef32_rt(const JshRequest& R, const JshMixed& X, const JshFreqConst& F, F3 p, int mode, Coef32& c,
                                           uint32_t rk_h = 0, uint32_t rk_f = 0, uint32_t rk_e = 0,
                                           int* tri_hint = nullptr, const LaneGroup group = LaneGroup{0u, 0, 0, 1}) {
   const JshModel& m = R.model;
-  const JshMixed& X = R.mix;
   if (!GENERAL || X.helical_log) {
     coef32_helical_log(X, F, p, mode, c);
     return;

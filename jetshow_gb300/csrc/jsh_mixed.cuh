@@ -266,20 +266,20 @@ __device__ __forceinline__ double tau_total(const Lane& L) {
   return L.seg == 0 ? df_val(L.tau_seg) : L.tau_bg + df_val(L.tau_seg);
 }
 
-__device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R) {
+__device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R, const JshMixed& X) {
   const JshSeg32& S = R.seg32[(uint64_t)L.h * JSH_MAX_SEG + L.seg];
   start_segment(L, DF{S.in[0], S.in[1]}, DF{S.in[2], S.in[3]}, DF{S.in[4], S.in[5]}, DF{S.len[0], S.len[1]});
   const float len = L.length.hi + L.length.lo;
   if (L.seg == 0) {
     L.thick = S.len_cm;
-    L.thick_left = R.mix.tau_eq_f;
+    L.thick_left = X.tau_eq_f;
   } else {
     L.tau_bg = df_val(L.tau_seg);  // two segments at most: that of segment 0
     L.thick += S.len_cm;
-    L.thick_left = (float)(R.mix.tau_eq - L.tau_bg);
+    L.thick_left = (float)(X.tau_eq - L.tau_bg);
   }
   L.tau_seg = DF{0.f, 0.f};
-  if (!R.mix.helical_log) {
+  if (!X.helical_log) {
     // the Dormand-Prince tau pass: the reference's first step L / n
     L.dt = len / (float)R.P.n;
     return;
@@ -292,7 +292,7 @@ __device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R) 
   // nodes of the first panels resolve (L.k1[2], [pc] along it; L.k1[3] the
   // approach distance, at least 1e-6 of the segment).  FP32 is enough: it
   // only places panels.
-  const float ux = R.mix.dhi[0], uy = R.mix.dhi[1];
+  const float ux = X.dhi[0], uy = X.dhi[1];
   const float uu = fmaf(ux, ux, uy * uy);
   L.k1[2] = INFINITY;
   L.k1[3] = 1e-6f * len;
@@ -336,7 +336,7 @@ __device__ __forceinline__ void begin_iquv_segment(Lane& L, const JshRequest& R)
 // the deep prefix of overlapped passes) starts after the deep prefix.
 __device__ __forceinline__ void lane_start(Lane& L, const JshRequest* __restrict__ reqs,
                                            const unsigned long long* base, int n_req, unsigned long long w,
-                                           bool ranked, int part = 0) {
+                                           bool ranked, int part = 0, const JshMixed* one = nullptr) {
   int r = find_request(base, n_req, w);
   const JshRequest& R = reqs[r];
   unsigned long long local = w - base[r];
@@ -366,7 +366,7 @@ __device__ __forceinline__ void lane_start(Lane& L, const JshRequest* __restrict
   L.ft = 0;
   L.ft_cool = 0;
   L.evals0 = 0;
-  begin_tau_segment(L, R);
+  begin_tau_segment(L, R, one ? *one : R.mix);
 }
 
 // Per-lane totals of a request's counters (right-hand-side evaluations,
@@ -607,7 +607,7 @@ __device__ __noinline__ float4 equilibrium_state(const JshRequest* __restrict__ 
                                                 double oy, double oz) {
   const JshRequest& R = reqs[r];
   Coef32 c;
-  coef32_rt<GENERAL>(R, R.mix.fc[f], f3((float)(ox * INV_PC), (float)(oy * INV_PC), (float)(oz * INV_PC)), COEF_FULL, c);
+  coef32_rt<GENERAL>(R, R.mix, R.mix.fc[f], f3((float)(ox * INV_PC), (float)(oy * INV_PC), (float)(oz * INV_PC)), COEF_FULL, c);
   double A[4][5] = {{c.kI, c.kQ, 0.0, c.kV, c.eI},
                     {c.kQ, c.kI, c.kF, 0.0, c.eQ},
                     {0.0, -c.kF, c.kI, c.kC, 0.0},
@@ -779,11 +779,11 @@ constexpr int kCrossIters = 48;
 // The end of an item's tau pass: finish it (tau <= tau_min), hand it to the
 // IQUV kernel (PASS_TAU) or start its I/IQUV pass in the same lane.
 template <int PASS, bool GENERAL>
-__device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restrict__ reqs, int part, Tally& T,
-                                              bool lead) {
+__device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restrict__ reqs, const JshMixed& X,
+                                              int part, Tally& T, bool lead) {
   const JshRequest& R = reqs[L.r];
   // a depth of one segment surely above tau_min stays a pair (no FP64 here)
-  const bool pair = PASS == PASS_TAU && L.seg == 0 && L.tau_seg.hi > R.mix.tau_min_f;
+  const bool pair = PASS == PASS_TAU && L.seg == 0 && L.tau_seg.hi > X.tau_min_f;
   if (!pair) {
     L.tau_bg = tau_total(L);
     if (!(L.tau_bg > R.P.tau_min)) {
@@ -794,10 +794,10 @@ __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restr
   L.status |= JSH_ST_IQUV;
   L.phase = PH_IQUV;
   bool eq = false;
-  if (L.first_seg >= 0 && R.mix.eq_start) {
+  if (L.first_seg >= 0 && X.eq_start) {
     // the equilibrium start needs depth behind tau_eq: rays shallower than
     // eq_min are integrated whole from their far end
-    if ((pair ? df_val(L.tau_seg) : L.tau_bg) >= R.mix.eq_min || (L.status & JSH_ST_TAU_CROSSED)) eq = true;
+    if ((pair ? df_val(L.tau_seg) : L.tau_bg) >= X.eq_min || (L.status & JSH_ST_TAU_CROSSED)) eq = true;
     else L.first_seg = -1;
   }
   if (PASS == PASS_TAU) {
@@ -832,19 +832,19 @@ __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restr
 // no other use for it), the panel [t, t + w] with w the midpoint of the
 // bracket [k1[0], k1[1]] is evaluated instead.
 template <int PASS, bool GENERAL, int NG>
-__device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __restrict__ reqs, float* Ksh, int part,
-                                               Tally& T, const LaneGroup& grp) {
+__device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __restrict__ reqs, const JshMixed& X,
+                                               float* Ksh, int part, Tally& T, const LaneGroup& grp) {
   const JshRequest& R = reqs[L.r];
-  const JshFreqConst F = R.mix.fc[L.f];
+  const JshFreqConst F = X.fc[L.f];
   const bool bis = L.init;
   // integration direction: +d (away from the observer)
-  const F3 dir = f3(-R.mix.nl[0], -R.mix.nl[1], -R.mix.nl[2]);
+  const F3 dir = f3(-X.nl[0], -X.nl[1], -X.nl[2]);
   bool at_bp = false;
   if (!bis) {
     const DF rem = df_sub(L.length, L.t);
     const float remf = rem.hi + rem.lo;
     if (!(remf > 0.f)) goto segment_done;
-    if (R.mix.dt_max_f != 0.f && L.dt > R.mix.dt_max_f) L.dt = R.mix.dt_max_f;
+    if (X.dt_max_f != 0.f && L.dt > X.dt_max_f) L.dt = X.dt_max_f;
     if (L.k1[2] < INFINITY) {
       // the segment's closest approach to the jet axis lies ahead: panels
       // close in on it by factors of 4 down to the approach distance and
@@ -879,7 +879,7 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
 #pragma unroll 1
       for (int i = 0; i < 15; ++i) {
         Coef32 c;
-        coef32_rt<GENERAL>(R, F, pn + dir * (c_gk_t[i] * h), COEF_KI, c, L.h, (uint32_t)L.f, L.evals + (uint32_t)i);
+        coef32_rt<GENERAL>(R, X, F, pn + dir * (c_gk_t[i] * h), COEF_KI, c, L.h, (uint32_t)L.f, L.evals + (uint32_t)i);
         K = fmaf(c_gk_wk[i], c.kI, K);
         G = fmaf(c_gk_wg[i], c.kI, G);
         A = fmaf(c_gk_wd[i], fabsf(c.kI), A);
@@ -890,7 +890,7 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         Coef32 c;
-        coef32_rt<GENERAL>(R, F, pn + dir * (c_gk_t[kGroupLanes * j + grp.sub] * h), COEF_KI, c);
+        coef32_rt<GENERAL>(R, X, F, pn + dir * (c_gk_t[kGroupLanes * j + grp.sub] * h), COEF_KI, c);
         k3[j] = c.kI;
       }
 #pragma unroll
@@ -905,7 +905,7 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
 #pragma unroll 1
       for (int i = grp.sub; i < 15; i += grp.n) {
         Coef32 c;
-        coef32_rt<GENERAL>(R, F, pn + dir * (c_gk_t[i] * h), COEF_KI, c);
+        coef32_rt<GENERAL>(R, X, F, pn + dir * (c_gk_t[i] * h), COEF_KI, c);
         Ksh[i] = c.kI;
       }
       grp.sync();
@@ -943,13 +943,13 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
       L.first_seg = L.seg;
       L.t_first = df_val(L.t) + (double)h;
       L.nseg = L.seg + 1;
-      tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
+      tau_pass_done<PASS, GENERAL>(L, reqs, X, part, T, (grp.sub == 0));
       return;
     }
     // error test: |K - G| against the tolerance of the running depth, never
     // below the FP32 noise floor of the estimate
     const float err = fabsf(K - G);
-    const float tol = fmaf(R.mix.tau_rtol, fabsf(L.tau_seg.hi) + fabsf(K), R.mix.tau_atol) + kPanelNoise * h * A;
+    const float tol = fmaf(X.tau_rtol, fabsf(L.tau_seg.hi) + fabsf(K), X.tau_atol) + kPanelNoise * h * A;
     const float r = err > 0.f ? tol / err : 1e30f;
     if (!(r >= 1.f)) {
       L.dt = h * fminf(fmaxf(0.9f * __powf(r, 1.0f / 15.0f), 0.2f), 0.9f);
@@ -980,9 +980,9 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
     // pass starts at the crossing point, bisected for inside the panel
     {
       const DF tn = df_add(L.tau_seg, K);
-      if (tn.hi > R.mix.tau_max_hi || (tn.hi == R.mix.tau_max_hi && tn.lo >= R.mix.tau_max_lo)) {
-        if (tn.hi > 1.25f * R.mix.tau_max_hi) {
-          L.dt = h * fmaxf((1.1f * R.mix.tau_max_hi - L.tau_seg.hi) / K, 0.01f);
+      if (tn.hi > X.tau_max_hi || (tn.hi == X.tau_max_hi && tn.lo >= X.tau_max_lo)) {
+        if (tn.hi > 1.25f * X.tau_max_hi) {
+          L.dt = h * fmaxf((1.1f * X.tau_max_hi - L.tau_seg.hi) / K, 0.01f);
           L.last = false;
           L.rej++;
           if (++L.fails >= dp::FAIL_LIMIT) {
@@ -1004,7 +1004,7 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
         }
         L.tau_seg = tn;
         L.nseg = L.seg + 1;
-        tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
+        tau_pass_done<PASS, GENERAL>(L, reqs, X, part, T, (grp.sub == 0));
         return;
       }
     }
@@ -1016,9 +1016,9 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
       goto abort;
     }
     L.t = t_new;
-    L.bx = df_axpy_round(t_new, DF{R.mix.dhi[0], R.mix.dlo[0]}, L.p0x);
-    L.by = df_axpy_round(t_new, DF{R.mix.dhi[1], R.mix.dlo[1]}, L.p0y);
-    L.bz = df_axpy_round(t_new, DF{R.mix.dhi[2], R.mix.dlo[2]}, L.p0z);
+    L.bx = df_axpy_round(t_new, DF{X.dhi[0], X.dlo[0]}, L.p0x);
+    L.by = df_axpy_round(t_new, DF{X.dhi[1], X.dlo[1]}, L.p0y);
+    L.bz = df_axpy_round(t_new, DF{X.dhi[2], X.dlo[2]}, L.p0z);
     L.fails = 0;
     L.acc++;
     L.dt = h * fminf(fmaxf(0.9f * __powf(fminf(r, 1e15f), 1.0f / 15.0f), 1.f), 4.f);
@@ -1041,10 +1041,10 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
 segment_done : {
   if (L.seg + 1 < L.nseg) {
     L.seg++;
-    begin_tau_segment(L, R);
+    begin_tau_segment(L, R, X);
     return;
   }
-  tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
+  tau_pass_done<PASS, GENERAL>(L, reqs, X, part, T, (grp.sub == 0));
   return;
 }
 
@@ -1061,14 +1061,14 @@ abort:
 // dtau/dt = k_I does not depend on the state, so only the last stage
 // combination (the increment) is formed.
 template <int PASS, bool GENERAL>
-__device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __restrict__ reqs, float* K, int part,
-                                               Tally& T, const LaneGroup& grp) {
+__device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __restrict__ reqs, const JshMixed& X,
+                                               float* K, int part, Tally& T, const LaneGroup& grp) {
   const JshRequest& R = reqs[L.r];
-  const JshFreqConst F = R.mix.fc[L.f];
-  const F3 dirf = f3(-R.mix.nl[0], -R.mix.nl[1], -R.mix.nl[2]);
-  const float max_dt = R.mix.dt_max_f;
-  const float atol = R.mix.tau_atol;
-  const float rtol = R.mix.tau_rtol;
+  const JshFreqConst F = X.fc[L.f];
+  const F3 dirf = f3(-X.nl[0], -X.nl[1], -X.nl[2]);
+  const float max_dt = X.dt_max_f;
+  const float atol = X.tau_atol;
+  const float rtol = X.tau_rtol;
   {
     const DF rem = df_sub(L.length, L.t);
     const float remf = rem.hi + rem.lo;
@@ -1094,7 +1094,7 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
     const float h = L.dt;
     if (!L.init) {
       Coef32 c;
-      coef32_rt<GENERAL>(R, F, pn, COEF_KI, c, L.h, (uint32_t)L.f, L.evals, &L.tri);
+      coef32_rt<GENERAL>(R, X, F, pn, COEF_KI, c, L.h, (uint32_t)L.f, L.evals, &L.tri);
       L.k1[0] = c.kI;
       L.evals++;
       L.init = true;
@@ -1109,7 +1109,7 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
     for (int s = grp.sub + 1; s <= np; s += grp.n) {
       Coef32 c;
       // the sixth point is the group's first lane's alone
-      coef32_rt<GENERAL>(R, F, pn + dirf * (c_C[s] * h), COEF_KI, c, L.h, (uint32_t)L.f,
+      coef32_rt<GENERAL>(R, X, F, pn + dirf * (c_C[s] * h), COEF_KI, c, L.h, (uint32_t)L.f,
                          L.evals + (uint32_t)(s - 1), &L.tri, s <= 5 ? grp : single_lane());
       K[s] = c.kI;
       if (s == 5 && np == 5) K[6] = c.kI;
@@ -1159,9 +1159,9 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
       goto abort;
     }
     L.t = t_new;
-    L.bx = df_axpy_round(t_new, DF{R.mix.dhi[0], R.mix.dlo[0]}, L.p0x);
-    L.by = df_axpy_round(t_new, DF{R.mix.dhi[1], R.mix.dlo[1]}, L.p0y);
-    L.bz = df_axpy_round(t_new, DF{R.mix.dhi[2], R.mix.dlo[2]}, L.p0z);
+    L.bx = df_axpy_round(t_new, DF{X.dhi[0], X.dlo[0]}, L.p0x);
+    L.by = df_axpy_round(t_new, DF{X.dhi[1], X.dlo[1]}, L.p0y);
+    L.bz = df_axpy_round(t_new, DF{X.dhi[2], X.dlo[2]}, L.p0z);
     L.fails = 0;
     L.acc++;
     if (e < 0.5f) {
@@ -1175,7 +1175,7 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
       L.first_seg = L.seg;
       L.t_first = df_val(t_new);
     }
-    if (L.tau_seg.hi > R.mix.tau_max_hi || (L.tau_seg.hi == R.mix.tau_max_hi && L.tau_seg.lo >= R.mix.tau_max_lo)) {
+    if (L.tau_seg.hi > X.tau_max_hi || (L.tau_seg.hi == X.tau_max_hi && L.tau_seg.lo >= X.tau_max_lo)) {
       L.status |= JSH_ST_TAU_CROSSED;
       const double t_old = df_val(t_prev);
       double tc = crossing_time(df_val(tau_prev), t_old, (double)h, h, K[0], K[2], K[3], K[4], K[5], K[6], inc,
@@ -1190,7 +1190,7 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
         L.t_first = tc;
       }
       L.nseg = L.seg + 1;
-      tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
+      tau_pass_done<PASS, GENERAL>(L, reqs, X, part, T, (grp.sub == 0));
       return;
     }
     L.k1[0] = K[6];
@@ -1200,10 +1200,10 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
 segment_done : {
   if (L.seg + 1 < L.nseg) {
     L.seg++;
-    begin_tau_segment(L, R);
+    begin_tau_segment(L, R, X);
     return;
   }
-  tau_pass_done<PASS, GENERAL>(L, reqs, part, T, (grp.sub == 0));
+  tau_pass_done<PASS, GENERAL>(L, reqs, X, part, T, (grp.sub == 0));
   return;
 }
 
@@ -1217,10 +1217,10 @@ abort:
 // flow), a Dormand-Prince attempt otherwise.  The choice belongs to the
 // request, so every build of the kernels gives the same bits.
 template <int PASS, bool GENERAL, int NG>
-__device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__ reqs, float* K, int part, Tally& T,
-                                         const LaneGroup& grp) {
-  if (!GENERAL || reqs[L.r].mix.helical_log) tau_panel_step<PASS, GENERAL, NG>(L, reqs, K, part, T, grp);
-  else tau_dopri_step<PASS, GENERAL>(L, reqs, K, part, T, grp);
+__device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__ reqs, const JshMixed& X, float* K,
+                                         int part, Tally& T, const LaneGroup& grp) {
+  if (!GENERAL || X.helical_log) tau_panel_step<PASS, GENERAL, NG>(L, reqs, X, K, part, T, grp);
+  else tau_dopri_step<PASS, GENERAL>(L, reqs, X, K, part, T, grp);
 }
 
 // A stage point's coefficients in shared memory: words, or two float4 (NG > 1).
@@ -1267,16 +1267,16 @@ __device__ __forceinline__ void get_coefficients(const float* q, Coef32& c) {
 // every form (static, single-kernel, split), so the images are bitwise the
 // same.
 template <bool FULL, int PASS, bool GENERAL, int NG>
-__device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict__ reqs, float* Q, Tally& T,
-                                          const LaneGroup& grp) {
+__device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict__ reqs, const JshMixed& X, float* Q,
+                                          Tally& T, const LaneGroup& grp) {
   constexpr int NK = StageWidth<FULL>::NK;
   constexpr int NX = StageWidth<FULL>::NX;
   const JshRequest& R = reqs[L.r];
-  const JshFreqConst F = R.mix.fc[L.f];
-  const F3 dirf = f3(R.mix.nl[0], R.mix.nl[1], R.mix.nl[2]);
+  const JshFreqConst F = X.fc[L.f];
+  const F3 dirf = f3(X.nl[0], X.nl[1], X.nl[2]);
   // error-norm tolerances in FP32 (the norm needs a few digits; t and dt stay FP64)
   const float atol = F.atol;
-  const float rtol = R.mix.rtol;
+  const float rtol = X.rtol;
 
   if (kFtm && FULL && L.ft) {
     // Faraday-thick mode: its steps follow I and V only, so nothing else
@@ -1319,7 +1319,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     constexpr int mode = FULL ? COEF_FULL : COEF_I;
     if (!L.init) {
       Coef32 c;
-      coef32_rt<GENERAL>(R, F, pn, mode, c, L.h, (uint32_t)L.f, L.evals0 + L.evals, &L.tri);
+      coef32_rt<GENERAL>(R, X, F, pn, mode, c, L.h, (uint32_t)L.f, L.evals0 + L.evals, &L.tri);
       L.s1 = stokes_rhs<FULL>(c, ft ? ft_point(c) : FtPoint{}, L.x, c0, s0, L.k1, ft, &cpl);
       L.kI1 = c.kI;
       L.evals++;
@@ -1351,7 +1351,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     if (NG == 1) {
 #pragma unroll
       for (int s = 1; s <= 5; ++s)
-        coef32_rt<GENERAL>(R, F, pn + dirf * (dp_c32(s) * h), mode, C[s - 1]);
+        coef32_rt<GENERAL>(R, X, F, pn + dirf * (dp_c32(s) * h), mode, C[s - 1]);
     } else {
       grp.sync();  // the step before has read its coefficients
       const int np = six ? 6 : 5;
@@ -1359,7 +1359,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
       for (int s = grp.sub + 1; s <= (NG > 1 ? 5 : np); s += NG > 1 ? NG : grp.n) {
         Coef32 c;
         // a sixth point is the group's first lane's alone
-        coef32_rt<GENERAL>(R, F, pn + dirf * (c_C[s] * h), mode, c, L.h, (uint32_t)L.f,
+        coef32_rt<GENERAL>(R, X, F, pn + dirf * (c_C[s] * h), mode, c, L.h, (uint32_t)L.f,
                            L.evals0 + L.evals + (uint32_t)(s - 1), &L.tri, s <= 5 ? grp : single_lane());
         put_coefficients<FULL, NG>(Q + (s - 1) * kPoint, c);
         if (NG > 1 && kFtm && FULL && ft) {
@@ -1525,9 +1525,9 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
       goto abort;
     }
     L.t = t_new;
-    L.bx = df_axpy_round(t_new, DF{-R.mix.dhi[0], -R.mix.dlo[0]}, L.p0x);
-    L.by = df_axpy_round(t_new, DF{-R.mix.dhi[1], -R.mix.dlo[1]}, L.p0y);
-    L.bz = df_axpy_round(t_new, DF{-R.mix.dhi[2], -R.mix.dlo[2]}, L.p0z);
+    L.bx = df_axpy_round(t_new, DF{-X.dhi[0], -X.dlo[0]}, L.p0x);
+    L.by = df_axpy_round(t_new, DF{-X.dhi[1], -X.dlo[1]}, L.p0y);
+    L.bz = df_axpy_round(t_new, DF{-X.dhi[2], -X.dlo[2]}, L.p0z);
     L.fails = 0;
     L.acc++;
     if (e < 0.5f) {
@@ -1622,8 +1622,9 @@ abort:
 template <bool FULL, int PASS>
 __device__ __forceinline__ void lane_advance(Lane& L, const JshRequest* __restrict__ reqs, float* Q, Tally& T) {
   const LaneGroup one = single_lane();
-  if (PASS == PASS_BOTH && L.phase == PH_TAU) tau_step<PASS, true, 0>(L, reqs, Q, 0, T, one);
-  else lane_step<FULL, PASS, true, 0>(L, reqs, Q, T, one);
+  const JshMixed& X = reqs[L.r].mix;
+  if (PASS == PASS_BOTH && L.phase == PH_TAU) tau_step<PASS, true, 0>(L, reqs, X, Q, 0, T, one);
+  else lane_step<FULL, PASS, true, 0>(L, reqs, X, Q, T, one);
 }
 
 // A persistent warp's work: every idle lane (or group of lanes) takes the next

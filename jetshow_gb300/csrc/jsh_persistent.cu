@@ -66,12 +66,12 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? (kFtm ? 3 : 4) 
   auto start = [&](unsigned long long w) { lane_start_iquv<false>(L, reqs, base, n_req, w, part); };
   const LaneGroup grp = lane_group(), one = single_lane();
   float* Q = ksh + group_slot(grp) * kGroupWords;
-  auto group_step = [&] { lane_step<FULL, PASS_IQUV, false, kGroupLanes>(L, reqs, Q, T, grp); };
+  auto group_step = [&] { lane_step<FULL, PASS_IQUV, false, kGroupLanes>(L, reqs, reqs[L.r].mix, Q, T, grp); };
   if (on_groups(total, FULL ? (COMPACT ? kIquvGroupsFull * 3 / 4 : kIquvGroupsFull) : kIquvGroupsI)) {
     run_queue(L, queue, total, refill, grp, start, group_step);
   } else {
     run_queue(L, queue, total, refill, one, start,
-              [&] { lane_step<FULL, PASS_IQUV, false, 1>(L, reqs, nullptr, T, one); });
+              [&] { lane_step<FULL, PASS_IQUV, false, 1>(L, reqs, reqs[L.r].mix, nullptr, T, one); });
   }
   tally_flush(T, reqs);
 }
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(COMPACT || GROUPS ? 128 : 256, COMPACT || GROU
   run_queue(
       L, queue, base[n_req], refill, grp,
       [&](unsigned long long w) { lane_start_iquv<true>(L, reqs, base, n_req, w, part); },
-      [&] { lane_step<FULL, PASS_IQUV, true, 0>(L, reqs, Q, T, grp); });
+      [&] { lane_step<FULL, PASS_IQUV, true, 0>(L, reqs, reqs[L.r].mix, Q, T, grp); });
   tally_flush(T, reqs);
 }
 
@@ -160,7 +160,6 @@ cudaError_t launch_prio(void (*kernel)(KArgs...), unsigned grid, unsigned block,
 }
 
 // IQUV kernel instantiation of a launch.
-using IquvKernel = void (*)(const JshRequest*, int, unsigned long long*, int, int);
 IquvKernel iquv_kernel(bool full, bool compact, bool fused, bool groups) {
   if (fused) {
     if (compact) return full ? transfer_iquv_kernel<true, true> : transfer_iquv_kernel<false, true>;
@@ -224,7 +223,9 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   // runs panels only, which keep their sums in registers; the general build
   // keeps Dormand-Prince stages in shared memory)
   const bool groups = !shape.fused && need <= kGroupItemsPerSm * (uint64_t)num_sms;
-  const TauLaunch tau = jsh_tau_kernel(shape.fused != 0, groups);
+  const bool one = shape.mix != nullptr && n_req == 1;
+  const JshMixed mix = one ? *shape.mix : JshMixed{};
+  const TauLaunch tau = jsh_tau_kernel(shape.fused != 0, groups, one);
   const TauKernel tau_k = tau.kernel;
   const int bt = tau.block;
   const size_t smem_t = tau.smem;
@@ -251,7 +252,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   const unsigned blocks_q = enough((unsigned)(num_sms * std::max(per_sm_q, 1)), bs);
   if (!overlap) {
     if (shape.marks) cudaEventRecord(shape.marks[0], stream);
-    tau_k<<<bl_t, bt, smem_t, stream>>>(d_reqs, n_req, q, rf, 0);
+    tau_k<<<bl_t, bt, smem_t, stream>>>(d_reqs, n_req, q, rf, 0, mix);
     if (shape.marks) cudaEventRecord(shape.marks[1], stream);
     jsh_launch_iquv_rank(d_reqs, n_req, num_sms, 0, stream);
     if (shape.marks) cudaEventRecord(shape.marks[2], stream);
@@ -275,7 +276,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   int per_sm_t2 = (65536 - deep_warps * wr_iquv) / ((bt / 32) * wr_tau);
   per_sm_t2 = std::min(std::max(per_sm_t2, 1), per_sm_t);
   if (shape.marks) cudaEventRecord(shape.marks[0], stream);
-  cudaError_t e = launch_prio(tau_k, bl_t, bt, smem_t, stream, prio_hi, d_reqs, n_req, q, rf, 0);
+  cudaError_t e = launch_prio(tau_k, bl_t, bt, smem_t, stream, prio_hi, d_reqs, n_req, q, rf, 0, mix);
   if (e != cudaSuccess) return e;
   jsh_launch_iquv_rank(d_reqs, n_req, num_sms, 0, stream);
   e = cudaEventRecord(shape.fork[0], stream);
@@ -288,7 +289,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   if (e != cudaSuccess) return e;
   unsigned bl_t2 = (unsigned)(num_sms * per_sm_t2);
   bl_t2 = enough(bl_t2, bt);
-  tau_k<<<bl_t2, bt, smem_t, shape.side>>>(d_reqs, n_req, q + 2, rf, 1);
+  tau_k<<<bl_t2, bt, smem_t, shape.side>>>(d_reqs, n_req, q + 2, rf, 1, mix);
   if (shape.marks) cudaEventRecord(shape.marks[1], shape.side);
   jsh_launch_iquv_rank(d_reqs, n_req, num_sms, 1, shape.side);
   if (shape.marks) cudaEventRecord(shape.marks[2], shape.side);

@@ -8,19 +8,22 @@
 
 #include "jsh_request.h"
 
-using TauKernel = void (*)(const JshRequest*, int, unsigned long long*, int, int);
+// (requests, their number, queue, refill threshold, part); the tau kernel takes
+// the constants of a single request besides.
+using TauKernel = void (*)(const JshRequest*, int, unsigned long long*, int, int, const JshMixed);
+using IquvKernel = void (*)(const JshRequest*, int, unsigned long long*, int, int);
 using StaticKernel = void (*)(const JshRequest*, int);
 using SingleKernel = void (*)(const JshRequest*, int, unsigned long long*, int);
 
 // The tau kernel (fused: built for the log-domain family alone; otherwise for
-// every law, with a lane or a group of lanes per item), its threads and its
-// dynamic shared memory.
+// every law, with a lane or a group of lanes per item; one: for a launch on a
+// single request), its threads and its dynamic shared memory.
 struct TauLaunch {
   TauKernel kernel;
   int block;
   size_t smem;
 };
-TauLaunch jsh_tau_kernel(bool fused, bool groups);
+TauLaunch jsh_tau_kernel(bool fused, bool groups, bool one);
 
 // Heaviest-first order of every request's hit rays; deep_key as
 // rank_prefix_kernel.

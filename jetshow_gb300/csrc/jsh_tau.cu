@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(256) rank_cost_kernel(const JshRequest* __rest
 #pragma unroll 1
       for (int k = 0; k < 4; ++k) {
         Coef32 c;
-        coef32_rt(R, F, a + d * xk[k], COEF_KI, c);
+        coef32_rt(R, R.mix, F, a + d * xk[k], COEF_KI, c);
         acc = fmaf(wk[k], c.kI, acc);
       }
       tau = fmaf(acc, sqrtf(fdot(d, d)), tau);
@@ -122,25 +122,35 @@ __device__ __forceinline__ void tau_prefix(const JshRequest* __restrict__ reqs, 
 // us, 32 350 items 160 -> 80 us, 79 782 items 174 -> 165 us); above, a lane
 // each does less work per panel (129 394 items 201 us against 227 us on
 // groups, 705 176 items 555 against 1 155 us).
+//
+// ONE: a launch on a single request, whose constants (`mix`) are the kernel's
+// parameters and so operands of its instructions; otherwise each lane loads
+// them from its request's record, again for every node at 80 registers (a
+// batch cannot do else).  512x1024 x 4: 522 -> 430 us.  The IQUV kernel, whose
+// step is more code than the instruction caches hold, loses by it (1.39 -> 1.56
+// ms): constants and instructions share a cache.
 constexpr int kTauGroupsFused = 4;
+template <bool ONE>
 __global__ void __launch_bounds__(256, 3)
     transfer_tau_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
-                        int part) {
+                        int part, const __grid_constant__ JshMixed mix) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
   tau_prefix(reqs, n_req, part, base);
   Lane L;
   L.phase = PH_IDLE;
   Tally T = tally_new();
   const unsigned long long total = base[n_req];
-  auto start = [&](unsigned long long w) { lane_start(L, reqs, base, n_req, w, true, part); };
+  auto start = [&](unsigned long long w) {
+    lane_start(L, reqs, base, n_req, w, true, part, ONE ? &mix : nullptr);
+  };
   if (on_groups(total, kTauGroupsFused)) {
     const LaneGroup grp = lane_group();
     run_queue(L, queue, total, refill, grp, start,
-              [&] { tau_step<PASS_TAU, false, kGroupLanes>(L, reqs, nullptr, part, T, grp); });
+              [&] { tau_step<PASS_TAU, false, kGroupLanes>(L, reqs, ONE ? mix : reqs[L.r].mix, nullptr, part, T, grp); });
   } else {
     const LaneGroup one = single_lane();
     run_queue(L, queue, total, refill, one, start,
-              [&] { tau_step<PASS_TAU, false, 1>(L, reqs, nullptr, part, T, one); });
+              [&] { tau_step<PASS_TAU, false, 1>(L, reqs, ONE ? mix : reqs[L.r].mix, nullptr, part, T, one); });
   }
   tally_flush(T, reqs);
 }
@@ -150,7 +160,7 @@ __global__ void __launch_bounds__(256, 3)
 template <bool GROUPS>
 __global__ void __launch_bounds__(128, GROUPS ? 3 : 4)
     transfer_tau_general_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
-                                int part) {
+                                int part, const __grid_constant__ JshMixed) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
   extern __shared__ float ksh[];
   tau_prefix(reqs, n_req, part, base);
@@ -162,7 +172,7 @@ __global__ void __launch_bounds__(128, GROUPS ? 3 : 4)
   run_queue(
       L, queue, base[n_req], refill, grp,
       [&](unsigned long long w) { lane_start(L, reqs, base, n_req, w, true, part); },
-      [&] { tau_step<PASS_TAU, true, 0>(L, reqs, K, part, T, grp); });
+      [&] { tau_step<PASS_TAU, true, 0>(L, reqs, reqs[L.r].mix, K, part, T, grp); });
   tally_flush(T, reqs);
 }
 
@@ -227,8 +237,8 @@ __global__ void __launch_bounds__(256) iquv_scatter_kernel(const JshRequest* __r
 
 using namespace jsh;
 
-TauLaunch jsh_tau_kernel(bool fused, bool groups) {
-  if (fused) return TauLaunch{transfer_tau_kernel, 256, 0};
+TauLaunch jsh_tau_kernel(bool fused, bool groups, bool one) {
+  if (fused) return TauLaunch{one ? transfer_tau_kernel<true> : transfer_tau_kernel<false>, 256, 0};
   return TauLaunch{groups ? transfer_tau_general_kernel<true> : transfer_tau_general_kernel<false>, 128,
                    sizeof(float) * kTauWords * (groups ? 128 / 32 * kWarpGroups : 128)};
 }
