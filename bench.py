@@ -581,7 +581,8 @@ def main():
             e2e_ms.append((t1 - t0) * 1e3)
     e2e_value = job_rate(st.n_work_items, world, max_over_ranks(float(np.mean(e2e_ms)), world))
     d2h = sum(v.numel() * v.element_size() for v in host.values())
-    h2d = int(ctx.lib.jsh_request_h2d_bytes(nu_c.size, A.PREC_MIXED))
+    # the request's record, frequencies and constants, and its plane's two along tables
+    h2d = int(ctx.lib.jsh_request_h2d_bytes(nu_c.size, A.PREC_MIXED)) + 16 * int(pdesc.n_along)
 
     # ---- roofline of the dominant kernel: the split form's tau kernel or
     # IQUV kernel, each timed live with CUDA events on the launching stream

@@ -596,7 +596,8 @@ int jsh_last_kernel_ms(jsh_ctx* ctx, double* tau_ms, double* iquv_rank_ms, doubl
 /* Host-to-device bytes that one jsh_observation_run or
  * jsh_observation_run_device call copies: the compiled request record, the
  * n_nu frequencies and, for JSH_PREC_MIXED, their FP32 coefficient
- * constants.  The descriptors themselves are read on the host.  No device
+ * constants; the two tables of the plane's columns (16 bytes a column, up to
+ * 16384 columns) come on top.  The descriptors themselves are read on the host.  No device
  * work; no reference counterpart. */
 uint64_t jsh_request_h2d_bytes(int32_t n_nu, int32_t precision);
 

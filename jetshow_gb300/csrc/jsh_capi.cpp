@@ -62,6 +62,14 @@ void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int3
   size_t o = 0;
   L->off_req = o;
   o = align_up(o + sizeof(JshRequest));
+  L->off_nu = o;
+  o = align_up(o + sizeof(double) * n_nu);
+  L->off_fc = o;
+  o = align_up(o + sizeof(JshFreqConst) * n_nu);
+  L->off_along_size = o;
+  o = align_up(o + sizeof(double) * n_along);
+  L->off_along_center = o;
+  o = align_up(o + sizeof(double) * n_along);
   L->off_counters = o;
   o = align_up(o + 8 * sizeof(unsigned long long));
   L->off_nhit = o;
@@ -74,14 +82,6 @@ void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int3
   o = align_up(o + 2 * sizeof(uint32_t));
   L->off_iq_buckets = o;
   o = align_up(o + sizeof(uint32_t) * JSH_IQ_WORDS);
-  L->off_nu = o;
-  o = align_up(o + sizeof(double) * n_nu);
-  L->off_fc = o;
-  o = align_up(o + sizeof(JshFreqConst) * n_nu);
-  L->off_along_size = o;
-  o = align_up(o + sizeof(double) * n_along);
-  L->off_along_center = o;
-  o = align_up(o + sizeof(double) * n_along);
   L->off_across = o;
   o = align_up(o + sizeof(double) * (n_across / 2) * n_along);
   L->off_hits = o;
@@ -278,8 +278,6 @@ extern "C" int jsh_ctx_create(int device, uint64_t hbm_budget_bytes, jsh_ctx** o
       cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->fork[0], cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->fork[1], cudaEventDisableTiming) != cudaSuccess ||
-      cudaMallocHost((void**)&c->h_req, sizeof(JshRequest)) != cudaSuccess ||
-      cudaMallocHost((void**)&c->h_fc, 4096 * sizeof(JshFreqConst)) != cudaSuccess ||
       cudaMallocHost((void**)&c->h_counters, 8 * sizeof(unsigned long long)) != cudaSuccess) {
     jsh_set_error("context creation failed: %s", cudaGetErrorString(cudaGetLastError()));
     jsh_ctx_destroy(c);
@@ -302,8 +300,10 @@ extern "C" void jsh_ctx_destroy(jsh_ctx* c) {
     if (h.used) jsh_free_device(c, h.mem, h.bytes);
   for (auto& h : c->cells)
     if (h.used) jsh_free_device(c, h.mem, h.bytes);
-  if (c->h_req) cudaFreeHost(c->h_req);
-  if (c->h_fc) cudaFreeHost(c->h_fc);
+  for (auto& g : c->stages) {
+    if (g.host) cudaFreeHost(g.host);
+    if (g.copied) cudaEventDestroy(g.copied);
+  }
   if (c->h_counters) cudaFreeHost(c->h_counters);
   if (c->ev_start) cudaEventDestroy(c->ev_start);
   if (c->ev_stop) cudaEventDestroy(c->ev_stop);
@@ -332,6 +332,48 @@ int ensure_workspace(jsh_ctx* ctx, size_t need) {
   if (st) return st;
   ctx->ws = p;
   ctx->ws_cap = cap;
+  return JSH_OK;
+}
+
+int jsh_next_stage(jsh_ctx* ctx, const JshRequestLayout& L, JshStage** out) {
+  JshStage& g = ctx->stages[ctx->next_stage];
+  ctx->next_stage = (ctx->next_stage + 1) % JSH_STAGES;
+  if (!g.copied) JSH_CUDA_TRY(cudaEventCreateWithFlags(&g.copied, cudaEventDisableTiming));
+  else JSH_CUDA_TRY(cudaEventSynchronize(g.copied));
+  // without tables where the device makes them
+  const size_t tables = L.off_counters - L.off_along_size;
+  const size_t need = L.off_along_size - L.off_req + std::min<size_t>(tables, 2 * sizeof(double) * JSH_HOST_TABLE_COLUMNS + 512);
+  if (need > g.cap) {
+    if (g.host) cudaFreeHost(g.host);
+    g.host = nullptr;
+    g.cap = 0;
+    const size_t cap = std::max(need, (size_t)65536);
+    JSH_CUDA_TRY(cudaMallocHost((void**)&g.host, cap));
+    g.cap = cap;
+  }
+  *out = &g;
+  return JSH_OK;
+}
+
+int jsh_upload_request(JshStage* g, JshRequest* req, const JshRequestLayout& L, char* base, const double* nu,
+                       cudaStream_t stream) {
+  const uint64_t n_along = req->plane.n_along;
+  req->plane.host_tables = n_along <= JSH_HOST_TABLE_COLUMNS ? 1 : 0;
+  char* h = g->host - L.off_req;  // the stage mirrors the layout from off_req
+  memcpy(h + L.off_req, req, sizeof(JshRequest));
+  if (nu) memcpy(h + L.off_nu, nu, sizeof(double) * req->n_nu);
+  size_t end = L.off_along_size;
+  if (req->plane.host_tables) {
+    jsh_plane_tables(&req->plane, (double*)(h + L.off_along_size), (double*)(h + L.off_along_center));
+    end = L.off_along_center + sizeof(double) * n_along;
+  }
+  JSH_CUDA_TRY(cudaMemcpyAsync(base + L.off_req, g->host, end - L.off_req, cudaMemcpyHostToDevice, stream));
+  JSH_CUDA_TRY(cudaEventRecord(g->copied, stream));
+  const size_t zero = L.off_across - L.off_counters;
+  if (req->plane.host_tables) JSH_CUDA_TRY(jsh_launch_clear(base + L.off_counters, zero, stream));
+  else JSH_CUDA_TRY(cudaMemsetAsync(base + L.off_counters, 0, zero, stream));
+  JSH_CUDA_TRY(jsh_launch_plane((const JshRequest*)(base + L.off_req), 1, n_along, stream,
+                                req->plane.host_tables != 0));
   return JSH_OK;
 }
 
@@ -365,20 +407,16 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   }
   // the previous user of the workspace (possibly on another stream) must finish
   JSH_CUDA_TRY(cudaStreamWaitEvent(stream, ctx->ws_ready, 0));
-  // the pinned staging buffers are reused: wait for their previous copies
-  JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
+  JshStage* stage = nullptr;
+  st = jsh_next_stage(ctx, L, &stage);
+  if (st) return st;
   if (params->precision == JSH_PREC_MIXED) {
-    st = jsh_prepare_mixed(&req, nu_hz, ctx->h_fc);
+    st = jsh_prepare_mixed(&req, nu_hz, (JshFreqConst*)(stage->host + (L.off_fc - L.off_req)));
     if (st) return st;
-    JSH_CUDA_TRY(cudaMemcpyAsync(base + L.off_fc, ctx->h_fc, sizeof(JshFreqConst) * n_nu, cudaMemcpyHostToDevice,
-                                 stream));
   }
-  *ctx->h_req = req;
-  JSH_CUDA_TRY(cudaMemcpyAsync(base + L.off_req, ctx->h_req, sizeof(JshRequest), cudaMemcpyHostToDevice, stream));
-  JSH_CUDA_TRY(cudaMemcpyAsync(base + L.off_nu, nu_hz, sizeof(double) * n_nu, cudaMemcpyHostToDevice, stream));
-  JSH_CUDA_TRY(cudaMemsetAsync(base + L.off_counters, 0, L.off_nu - L.off_counters, stream));
+  st = jsh_upload_request(stage, &req, L, base, nu_hz, stream);
+  if (st) return st;
   const JshRequest* d_req = (const JshRequest*)(base + L.off_req);
-  JSH_CUDA_TRY(jsh_launch_plane(d_req, 1, plane->n_along, stream));
   JSH_CUDA_TRY(jsh_launch_hit(d_req, 1, npix, stream));
   JshLaunchShape shape = jsh_effective_shape(ctx, params);
   shape.fused = (req.mix.helical_log && !(params->flags & JSH_FLAG_GENERAL_KERNELS)) ? 1 : 0;
@@ -402,7 +440,7 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
                                    ctx->num_sms, stream));
   JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, stream));
   ctx->last_pending = true;
-  // plane (2), hit, transfer; the persistent mixed schedule adds 3 ranking
+  // counters and plane (2), hit, transfer; the persistent mixed schedule adds 3 ranking
   // kernels, and its split form the tau kernel and 3 IQUV ranking kernels
   // (twice over when the passes overlap)
   ctx->last_kernels = jsh_kernels_per_request(params->precision, params->schedule, shape.single != 0, overlap);
@@ -512,31 +550,37 @@ extern "C" int jsh_plane_rays(jsh_ctx* ctx, const jsh_plane_desc* plane, double*
     return JSH_ERR_INVALID;
   }
   std::lock_guard<std::mutex> lk(ctx->mu);
-  JSH_CUDA_TRY(cudaSetDevice(ctx->device));
   JshRequest req;
   memset(&req, 0, sizeof(req));
   int st = jsh_compile_plane(plane, &req.plane);
   if (st) return st;
-  uint64_t npix = plane->n_across * plane->n_along;
-  JshRequestLayout L;
-  jsh_request_layout(0, plane->n_along, plane->n_across, 1, false, &L);
-  size_t off_o = L.total, off_s = align_up(off_o + sizeof(double) * 3 * npix);
-  size_t total = align_up(off_s + sizeof(double) * npix);
-  st = ensure_workspace(ctx, total);
-  if (st) return st;
-  JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
-  char* base = (char*)ctx->ws;
-  jsh_bind_request(&req, base, L, false);
-  *ctx->h_req = req;
-  cudaStream_t s = ctx->stream;
-  JSH_CUDA_TRY(cudaMemcpyAsync(base + L.off_req, ctx->h_req, sizeof(JshRequest), cudaMemcpyHostToDevice, s));
-  JSH_CUDA_TRY(jsh_launch_plane((const JshRequest*)(base + L.off_req), 1, plane->n_along, s));
-  JSH_CUDA_TRY(jsh_launch_plane_rays(req.plane, (double*)(base + off_o), (double*)(base + off_s), s));
-  if (origins) JSH_CUDA_TRY(cudaMemcpyAsync(origins, base + off_o, sizeof(double) * 3 * npix, cudaMemcpyDeviceToHost, s));
-  if (pixel_sizes)
-    JSH_CUDA_TRY(cudaMemcpyAsync(pixel_sizes, base + off_s, sizeof(double) * npix, cudaMemcpyDeviceToHost, s));
-  JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, s));
-  JSH_CUDA_TRY(cudaStreamSynchronize(s));
+  const uint64_t npix = plane->n_across * plane->n_along;
+  if (pixel_sizes) {  // every row has the along sizes
+    jsh_plane_tables(&req.plane, pixel_sizes, nullptr);
+    for (uint64_t i = 1; i < plane->n_across; ++i)
+      memcpy(pixel_sizes + i * plane->n_along, pixel_sizes, sizeof(double) * plane->n_along);
+  }
+  if (origins) {
+    JSH_CUDA_TRY(cudaSetDevice(ctx->device));
+    JshRequestLayout L;
+    jsh_request_layout(0, plane->n_along, plane->n_across, 1, false, &L);
+    const size_t off_o = L.total;
+    st = ensure_workspace(ctx, align_up(off_o + sizeof(double) * 3 * npix));
+    if (st) return st;
+    JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
+    char* base = (char*)ctx->ws;
+    jsh_bind_request(&req, base, L, false);
+    cudaStream_t s = ctx->stream;
+    JshStage* stage = nullptr;
+    st = jsh_next_stage(ctx, L, &stage);
+    if (st) return st;
+    st = jsh_upload_request(stage, &req, L, base, nullptr, s);
+    if (st) return st;
+    JSH_CUDA_TRY(jsh_launch_plane_rays(req.plane, (double*)(base + off_o), nullptr, s));
+    JSH_CUDA_TRY(cudaMemcpyAsync(origins, base + off_o, sizeof(double) * 3 * npix, cudaMemcpyDeviceToHost, s));
+    JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, s));
+    JSH_CUDA_TRY(cudaStreamSynchronize(s));
+  }
   if (direction) {
     direction[0] = req.plane.dx;
     direction[1] = req.plane.dy;
@@ -571,12 +615,13 @@ extern "C" int jsh_trace_plane(jsh_ctx* ctx, const jsh_model_desc* model, const 
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
   char* base = (char*)ctx->ws;
   jsh_bind_request(&req, base, L, false);
-  *ctx->h_req = req;
   cudaStream_t s = ctx->stream;
-  JSH_CUDA_TRY(cudaMemcpyAsync(base + L.off_req, ctx->h_req, sizeof(JshRequest), cudaMemcpyHostToDevice, s));
-  JSH_CUDA_TRY(cudaMemsetAsync(base + L.off_nhit, 0, sizeof(uint32_t), s));
+  JshStage* stage = nullptr;
+  st = jsh_next_stage(ctx, L, &stage);
+  if (st) return st;
+  st = jsh_upload_request(stage, &req, L, base, nullptr, s);
+  if (st) return st;
   const JshRequest* d_req = (const JshRequest*)(base + L.off_req);
-  JSH_CUDA_TRY(jsh_launch_plane(d_req, 1, plane->n_along, s));
   JSH_CUDA_TRY(jsh_launch_hit(d_req, 1, npix, s));
   uint32_t nhit = 0;
   JSH_CUDA_TRY(cudaMemcpyAsync(&nhit, base + L.off_nhit, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

@@ -45,12 +45,26 @@ struct JshHullSlot {
 
 // Layout of one request's device memory inside an arena allocation.
 struct JshRequestLayout {
-  size_t off_req, off_counters, off_nhit, off_queue, off_buckets, off_iq_count, off_iq_buckets, off_nu, off_fc,
-      off_along_size, off_along_center, off_across, off_hits, off_order, off_key, off_iq_items, off_iq_order,
+  // [off_req, off_counters) comes from the host, [off_counters, off_across) starts at zero
+  size_t off_req, off_nu, off_fc, off_along_size, off_along_center, off_counters, off_nhit, off_queue, off_buckets,
+      off_iq_count, off_iq_buckets, off_across, off_hits, off_order, off_key, off_iq_items, off_iq_order,
       off_seg32, off_out[7];
   size_t total;
   bool own_outputs;
 };
+
+// Pinned staging of a request's upload: one of a few used in turn, so that a
+// render can be enqueued while earlier ones still run; the host waits only
+// for the copy that last used the stage.
+#define JSH_STAGES 4
+struct JshStage {
+  char* host = nullptr;
+  size_t cap = 0;
+  cudaEvent_t copied = nullptr;
+};
+// Columns up to which the host computes a request's along tables and uploads
+// them (16 bytes each); above, the device's serial kernel does.
+#define JSH_HOST_TABLE_COLUMNS 16384
 
 struct jsh_ctx {
   int device = 0;
@@ -68,8 +82,8 @@ struct jsh_ctx {
   std::atomic<uint64_t> used{0};
   void* ws = nullptr;  // workspace of the blocking / device entry points
   size_t ws_cap = 0;
-  JshRequest* h_req = nullptr;               // pinned staging of one request
-  JshFreqConst* h_fc = nullptr;              // pinned staging of its frequency constants [4096]
+  JshStage stages[JSH_STAGES];               // pinned staging of requests, in turn
+  int next_stage = 0;
   unsigned long long* h_counters = nullptr;  // pinned [8]
   JshGridSlot grids[JSH_MAX_GRIDS];
   JshHullSlot hulls[JSH_MAX_HULLS];
@@ -107,6 +121,13 @@ int jsh_kernels_per_request(int precision, int schedule, bool single, bool overl
 // them; large requests on the mixed persistent schedule only, never with
 // JSH_FLAG_SERIAL_PASSES or the single-kernel form).
 bool jsh_overlap_passes(const jsh_params* params, const JshLaunchShape& shape, uint64_t items);
+// The next stage, free and large enough for the upload of layout L.
+int jsh_next_stage(jsh_ctx* ctx, const JshRequestLayout& L, JshStage** out);
+// Upload `req` with its frequencies (may be null), the constants the caller
+// has put at (off_fc - off_req) of the stage and the along tables, clear its
+// counters, and run ray generation, all on `stream`.
+int jsh_upload_request(JshStage* stage, JshRequest* req, const JshRequestLayout& L, char* base, const double* nu,
+                       cudaStream_t stream);
 // Grow the context workspace to `need` bytes (waits for its previous user).
 int ensure_workspace(jsh_ctx* ctx, size_t need);
 // Enqueue one request on `stream` in the context workspace; dev_out NULL

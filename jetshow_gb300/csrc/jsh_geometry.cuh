@@ -56,9 +56,10 @@ struct Hits {
 // plane_origin for the layout of the across table.
 __device__ __forceinline__ V3 plane_origin(const JshPlane& p, uint64_t i, uint64_t j) {
   uint64_t nh = p.n_across / 2;
+  const double half = ml(0.5, p.along_size[j]);
   double across;
-  if (i < nh) across = p.across_pos[(nh - i - 1) * p.n_along + j];
-  else across = -p.across_pos[(i - nh) * p.n_along + j];
+  if (i < nh) across = sb(p.across_pos[(nh - i - 1) * p.n_along + j], half);
+  else across = -sb(p.across_pos[(i - nh) * p.n_along + j], half);
   return mk(ml(1., 0.0), ml(1., across), ml(p.inv_sin, p.along_center[j]));
 }
 

@@ -323,6 +323,16 @@ int jsh_compile_plane(const jsh_plane_desc* d, JshPlane* p) {
   return JSH_OK;
 }
 
+void jsh_plane_tables(const JshPlane* p, double* size, double* center) {
+  double cur = p->real_start, acc = 0.0;
+  for (uint64_t j = 0; j < p->n_along; ++j) {
+    acc = j == 0 ? cur : acc + cur;
+    if (size) size[j] = cur;
+    if (center) center[j] = acc - 0.5 * cur;
+    cur *= p->real_base;
+  }
+}
+
 // ------------------------------------------------------------- cosmology
 // comoving_transfer_distance2 + mas_to_pc (src/utils.cpp:186-208, :373-378):
 // dX/dz = ((Om + (1+z) g_nu)(1+z)^3 + OV)^-1/2 integrated from 0 to z by an

@@ -10,17 +10,18 @@ using namespace jsh;
 
 namespace {
 
-constexpr int kPlaneThreads = 128;
+constexpr int kPlaneThreads = 32;  // a warp a sub-partition: the across chain holds its FP64 pipe
 constexpr int kHitThreads = 256;
 
 // ---------------------------------------------------------------- plane
 // pyLogspace by repeated multiplication and the running partial sum are
-// sequential recurrences (include/logspace.h:9-33, src/Image.cpp:70-75): one
-// thread per request walks them so every value rounds as in the reference.
-// Only the two recurrences run here (one FP64 multiply and one add per
-// column: an FP64 instruction holds the SM sub-partition's FP64 pipe for
-// ~64 cycles on GB300, so the sequential thread is set by their count); the
-// running sum goes to along_center and plane_across_kernel turns it into
+// sequential recurrences (include/logspace.h:9-33, src/Image.cpp:70-75).  A
+// request that the host uploads brings its along tables (jsh_plane_tables: a
+// few ns a column there); for the records of a batch that is built on the
+// device one thread per request walks the recurrences, so every value rounds
+// as in the reference (an FP64 instruction holds the SM sub-partition's FP64
+// pipe for ~64 cycles: 107 ns a column).  Only the two recurrences run here;
+// the running sum goes to along_center and plane_across_kernel turns it into
 // the centre, acc - size / 2 (the halving is exact, one rounding as before).
 __global__ void plane_along_kernel(const JshRequest* __restrict__ reqs) {
   if (threadIdx.x != 0) return;
@@ -38,23 +39,28 @@ __global__ void plane_along_kernel(const JshRequest* __restrict__ reqs) {
   }
 }
 
-// Column j of the across table: partial sums of n_across/2 copies of the
-// column's pixel size, minus half a size (src/Image.cpp:110-126); and the
-// column's centre along the plane, its running size sum minus half its size
-// (src/Image.cpp:70-75).
+// Zeroes a request's counters.
+__global__ void clear_kernel(uint4* __restrict__ p, unsigned n) {
+  for (unsigned i = threadIdx.x; i < n; i += blockDim.x) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// Column j of the across table: partial sums of 1 .. n_across/2 copies of the
+// column's pixel size (src/Image.cpp:110-126; plane_origin takes half a size
+// off, so that the chain here is one FP64 addition per row: 512x1024 27 -> 15
+// us); and the column's centre along the plane where the along kernel left
+// its running size sum (src/Image.cpp:70-75).
 __global__ void plane_across_kernel(const JshRequest* __restrict__ reqs) {
   const JshPlane& p = reqs[blockIdx.y].plane;
   uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= p.n_along) return;
-  p.along_center[j] = sb(p.along_center[j], ml(0.5, p.along_size[j]));
+  const double s = p.along_size[j];
+  if (!p.host_tables) p.along_center[j] = sb(p.along_center[j], ml(0.5, s));
   uint64_t nh = p.n_across / 2, na = p.n_along;
   double* __restrict__ pos = p.across_pos;
-  double s = ml(p.along_size[j], 1.0);
-  double half = ml(0.5, s);
   double a = 0.0;
   for (uint64_t k = 0; k < nh; ++k) {
     a = (k == 0) ? s : ad(a, s);
-    pos[k * na + j] = sb(a, half);
+    pos[k * na + j] = a;
   }
 }
 
@@ -292,13 +298,21 @@ cudaError_t jsh_launch_transfer_mixed_ft(const JshRequest* d_reqs, int n_req, in
                                          uint64_t max_items, uint64_t max_hits, const JshLaunchShape& shape,
                                          unsigned int* queue, int num_sms, cudaStream_t stream);
 
-cudaError_t jsh_launch_plane(const JshRequest* d_reqs, int n_req, uint64_t max_along, cudaStream_t stream) {
+cudaError_t jsh_launch_plane(const JshRequest* d_reqs, int n_req, uint64_t max_along, cudaStream_t stream,
+                             bool host_tables) {
   if (n_req <= 0) return cudaSuccess;
-  plane_along_kernel<<<n_req, 32, 0, stream>>>(d_reqs);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  if (!host_tables) {
+    plane_along_kernel<<<n_req, 32, 0, stream>>>(d_reqs);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
   dim3 g((unsigned)((max_along + kPlaneThreads - 1) / kPlaneThreads), (unsigned)n_req);
   plane_across_kernel<<<g, kPlaneThreads, 0, stream>>>(d_reqs);
+  return cudaGetLastError();
+}
+
+cudaError_t jsh_launch_clear(void* p, size_t bytes, cudaStream_t stream) {
+  clear_kernel<<<1, 256, 0, stream>>>((uint4*)p, (unsigned)(bytes / sizeof(uint4)));
   return cudaGetLastError();
 }
 

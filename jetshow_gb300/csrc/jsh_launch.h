@@ -45,10 +45,14 @@ struct JshLaunchShape {
   int faraday_thick;
 };
 
-// Ray generation: along sizes and centres (sequential recurrence of
-// pyLogspace / partial_sum), then the across-centre table.  max_along is
-// the largest n_along of the batch.
-cudaError_t jsh_launch_plane(const JshRequest* d_reqs, int n_req, uint64_t max_along, cudaStream_t stream);
+// Ray generation: along sizes and centres (the sequential recurrences of
+// pyLogspace / partial_sum, unless every request came with them: host_tables),
+// then the across table.  max_along is the largest n_along of the batch.
+cudaError_t jsh_launch_plane(const JshRequest* d_reqs, int n_req, uint64_t max_along, cudaStream_t stream,
+                             bool host_tables = false);
+
+// Zero `bytes` (a multiple of 16, 16-byte aligned) at p.
+cudaError_t jsh_launch_clear(void* p, size_t bytes, cudaStream_t stream);
 
 // Hit every pixel's ray against the request's geometry, append the hit rays
 // to req.hits (count in *req.n_hit, zeroed beforehand), write the outputs of

@@ -120,7 +120,8 @@ struct JshPlane {
   double rx, ry, rz;             // direction normalised once more (Ray re-built at tau_max)
   double* along_size;            // device [n_along]
   double* along_center;          // device [n_along]
-  double* across_pos;            // device [n_across/2][n_along]
+  double* across_pos;            // device [n_across/2][n_along]: sums of k + 1 sizes
+  int32_t host_tables, pad_;     // the along tables came with the request
 };
 
 #ifdef __cplusplus
@@ -130,5 +131,10 @@ extern "C++" {
 int jsh_compile_model(const jsh_model_desc* d, JshModel* m);
 int jsh_compile_plane(const jsh_plane_desc* d, JshPlane* p);
 void jsh_set_error(const char* fmt, ...);
+// The along tables of a compiled plane [n_along]: pyLogspace's sizes by
+// repeated multiplication and the centres, running sum minus half a size
+// (include/logspace.h:9-33, src/Image.cpp:70-75), rounded step by step as the
+// device's plane kernels round them.
+void jsh_plane_tables(const JshPlane* p, double* size, double* center);
 }
 #endif

@@ -11,9 +11,9 @@
 // first yielded state with tau >= tau_max, whose tau is kept and whose
 // later intersections are dropped; otherwise the state after the last step.
 // dtau/dt = k_I does not depend on tau, so the two middle stages share one
-// evaluation, and 32 consecutive steps are evaluated at once, a step a lane;
-// their increments are then added in the order of the steps (the sums round
-// as the serial steps do).  A ray that misses keeps tau = 0.  With a thread
+// evaluation, and the three evaluations of 32 consecutive steps are spread over
+// the lanes; their increments are then added in the order of the steps (the
+// sums round as the serial steps do).  A ray that misses keeps tau = 0.  With a thread
 // per pixel the 300 serial evaluations of FP64 set the time: 6.91 ms for the
 // 1 000 pixels of a 2 000-column stripe on 8 CTAs, 0.79 ms with a warp per
 // pixel (0.29 of it the plane's recurrence); 10 000 pixels 8.8 -> 6.6 ms.
@@ -43,6 +43,8 @@ constexpr int kStripeThreads = 128;
 
 __global__ void __launch_bounds__(kStripeThreads) stripe_tau_kernel(const JshRequest* __restrict__ req, double nu,
                                                                    double* __restrict__ tau_out) {
+  __shared__ double increments[kStripeThreads / 32][96];
+  double* inc = increments[threadIdx.x / 32];
   const JshRequest& R = *req;
   const JshPlane& pl = R.plane;
   const uint64_t c0 = pl.n_along / 2;
@@ -72,16 +74,18 @@ __global__ void __launch_bounds__(kStripeThreads) stripe_tau_kernel(const JshReq
         // the steps of the range are a prefix of the lanes: t grows with the step
         const bool in = step <= (int64_t)n + 1 && sb(ad(t, dt), length) <= DBL_EPSILON;
         const int steps = __popc(__ballot_sync(0xffffffffu, in));
-        double a = 0.0, b = 0.0, c = 0.0;
-        if (in) {
-          a = ml(w1, tau_rate(R.model, P, t));
-          b = ml(w2, tau_rate(R.model, P, ad(t, ml(0.5, dt))));
-          c = ml(w1, tau_rate(R.model, P, ad(t, dt)));
+        // evaluation e of the 3 * steps: stage e % 3 of step e / 3
+        __syncwarp();
+        for (int e = lane; e < 3 * steps; e += 32) {
+          const int k = e / 3, stage = e - 3 * k;
+          const double tk = ml((double)(first + k), dt);
+          const double te = stage == 0 ? tk : stage == 1 ? ad(tk, ml(0.5, dt)) : ad(tk, dt);
+          inc[e] = ml(stage == 1 ? w2 : w1, tau_rate(R.model, P, te));
         }
         __syncwarp();
         for (int i = 0; i < steps && !found; ++i) {
-          const double bi = __shfl_sync(0xffffffffu, b, i);
-          x = ad(ad(ad(ad(x, __shfl_sync(0xffffffffu, a, i)), bi), bi), __shfl_sync(0xffffffffu, c, i));
+          const double bi = inc[3 * i + 1];
+          x = ad(ad(ad(ad(x, inc[3 * i]), bi), bi), inc[3 * i + 2]);
           found = (x >= tau_max);
         }
         if (steps < 32) break;
@@ -124,11 +128,13 @@ extern "C" int jsh_observation_run_stripe(jsh_ctx* ctx, const jsh_model_desc* mo
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
   char* base = (char*)ctx->ws;
   jsh_bind_request(&req, base, L, false);
-  *ctx->h_req = req;
   cudaStream_t s = ctx->stream;
-  JSH_CUDA_TRY(cudaMemcpyAsync(base + L.off_req, ctx->h_req, sizeof(JshRequest), cudaMemcpyHostToDevice, s));
+  JshStage* stage = nullptr;
+  st = jsh_next_stage(ctx, L, &stage);
+  if (st) return st;
+  st = jsh_upload_request(stage, &req, L, base, nullptr, s);
+  if (st) return st;
   const JshRequest* d_req = (const JshRequest*)(base + L.off_req);
-  JSH_CUDA_TRY(jsh_launch_plane(d_req, 1, plane->n_along, s));
   if (count > 0) {
     stripe_tau_kernel<<<(unsigned)((count * 32 + kStripeThreads - 1) / kStripeThreads), kStripeThreads, 0, s>>>(d_req, nu_hz, (double*)(base + off_out));
     JSH_CUDA_TRY(cudaGetLastError());

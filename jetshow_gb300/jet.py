@@ -461,8 +461,7 @@ class ImagePlane:
         return o, d
 
     def getPixelSizes(self, ctx=None):
-        _, _, s = (ctx or default_context()).plane_rays(self.desc())
-        return s.reshape(self.image_size)
+        return (ctx or default_context()).plane_sizes(self.desc()).reshape(self.image_size)
 
 
 class Observation:

@@ -127,6 +127,12 @@ class Context:
         check(self.lib, self.lib.jsh_plane_rays(self.handle, C.byref(plane), A.dptr(o), A.dptr(d), A.dptr(s)))
         return o, d, s
 
+    def plane_sizes(self, plane: A.PlaneDesc):
+        """Pixel sizes [n_across * n_along] of a plane (computed on the host)."""
+        s = np.zeros(int(plane.n_across * plane.n_along))
+        check(self.lib, self.lib.jsh_plane_rays(self.handle, C.byref(plane), None, None, A.dptr(s)))
+        return s
+
     def trace_plane(self, model: A.ModelDesc, plane: A.PlaneDesc):
         n = int(plane.n_across * plane.n_along)
         nseg = np.zeros(n, np.int32); seg = np.zeros((n, 2, 2, 3)); st = np.zeros(n, np.uint32)
