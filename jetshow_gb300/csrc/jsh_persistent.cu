@@ -254,7 +254,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
     if (shape.marks) cudaEventRecord(shape.marks[0], stream);
     tau_k<<<bl_t, bt, smem_t, stream>>>(d_reqs, n_req, q, rf, 0, mix);
     if (shape.marks) cudaEventRecord(shape.marks[1], stream);
-    jsh_launch_iquv_rank(d_reqs, n_req, num_sms, 0, stream);
+    jsh_launch_iquv_rank(d_reqs, n_req, max_items, num_sms, 0, stream);
     if (shape.marks) cudaEventRecord(shape.marks[2], stream);
     iquv_k<<<blocks_q, bs, smem_q, stream>>>(d_reqs, n_req, q + 1, rf, 0);
     if (shape.marks) cudaEventRecord(shape.marks[3], stream);
@@ -278,7 +278,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   if (shape.marks) cudaEventRecord(shape.marks[0], stream);
   cudaError_t e = launch_prio(tau_k, bl_t, bt, smem_t, stream, prio_hi, d_reqs, n_req, q, rf, 0, mix);
   if (e != cudaSuccess) return e;
-  jsh_launch_iquv_rank(d_reqs, n_req, num_sms, 0, stream);
+  jsh_launch_iquv_rank(d_reqs, n_req, max_items, num_sms, 0, stream);
   e = cudaEventRecord(shape.fork[0], stream);
   if (e != cudaSuccess) return e;
   e = launch_prio(iquv_k, (unsigned)(num_sms * kDeepIquvPerSm), kDeepIquvBlock,
@@ -291,7 +291,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   bl_t2 = enough(bl_t2, bt);
   tau_k<<<bl_t2, bt, smem_t, shape.side>>>(d_reqs, n_req, q + 2, rf, 1, mix);
   if (shape.marks) cudaEventRecord(shape.marks[1], shape.side);
-  jsh_launch_iquv_rank(d_reqs, n_req, num_sms, 1, shape.side);
+  jsh_launch_iquv_rank(d_reqs, n_req, max_items, num_sms, 1, shape.side);
   if (shape.marks) cudaEventRecord(shape.marks[2], shape.side);
   iquv_k<<<blocks_q, bs, smem_q, shape.side>>>(d_reqs, n_req, q + 3, rf, 1);
   e = cudaEventRecord(shape.fork[1], shape.side);

@@ -29,8 +29,10 @@ TauLaunch jsh_tau_kernel(bool fused, bool groups, bool one);
 // rank_prefix_kernel.
 void jsh_launch_rank(const JshRequest* d_reqs, int n_req, uint64_t max_hits, int deep_key, cudaStream_t stream);
 
-// Heaviest-first order of the items the tau kernel handed on.
-void jsh_launch_iquv_rank(const JshRequest* d_reqs, int n_req, int num_sms, int part, cudaStream_t stream);
+// Heaviest-first order of the items the tau kernel handed on (max_items: the
+// batch's bound, the same for each of its requests).
+void jsh_launch_iquv_rank(const JshRequest* d_reqs, int n_req, uint64_t max_items, int num_sms, int part,
+                          cudaStream_t stream);
 
 StaticKernel jsh_static_kernel(bool full);
 SingleKernel jsh_single_kernel(bool full, bool compact);
