@@ -177,6 +177,7 @@ int jsh_prepare_request(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_pla
   if (st) return st;
   st = jsh_compile_plane(plane, &req->plane);
   if (st) return st;
+  jsh_prepare_hit(req);
   const jsh_params& P = *params;
   if (P.n < 1 || !(P.tau_max > 0) || !std::isfinite(P.tau_max) || !(P.tau_precision > 0) || !(P.atol >= 0) ||
       !(P.rtol >= 0) || !(P.tau_atol >= 0) || !(P.tau_rtol >= 0) || (P.atol == 0 && P.rtol == 0) ||
@@ -605,6 +606,7 @@ extern "C" int jsh_trace_plane(jsh_ctx* ctx, const jsh_model_desc* model, const 
   if (st) return st;
   st = jsh_compile_plane(plane, &req.plane);
   if (st) return st;
+  jsh_prepare_hit(&req);
   uint64_t npix = plane->n_across * plane->n_along;
   req.npix = npix;
   req.n_nu = 0;  // the hit kernel writes no output planes

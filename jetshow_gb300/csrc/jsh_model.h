@@ -29,6 +29,12 @@ struct JshCone {
   double big_scale;
 };
 
+struct JshConeRay {        // cone_hit's terms that depend on the ray's direction alone
+  double M[3][3];          // d d^T - cos^2 I
+  double u[3];             // r M
+  double c2, cos_ray;      // r M r, r . d
+};
+
 struct JshGrid {         // device view of an uploaded triangulated (z, r) grid
   const double* xy;      // [n][2] (z, r) in pc
   // [n_tri][12] mixed-precision lookups, a triangle in three float4: FP32

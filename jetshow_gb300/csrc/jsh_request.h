@@ -118,6 +118,7 @@ struct JshRequest {
   JshModel model;
   JshMixed mix;
   JshPlane plane;
+  JshConeRay cone_ray;    // of the plane's rays (jsh_prepare_hit)
   JshParamsDev P;
   JshHit* hits;           // device [npix] (first n_hit valid)
   JshSeg32* seg32;        // device [npix][JSH_MAX_SEG], mixed precision: the hits' segments

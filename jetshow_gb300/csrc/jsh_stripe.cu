@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kStripeThreads) stripe_tau_kernel(const JshReq
   const int lane = (int)(threadIdx.x & 31u);
   if (col >= pl.n_along) return;
   Hits h;
-  geo_hit(R.model, plane_origin(pl, pl.n_across / 2, col), mk(pl.dx, pl.dy, pl.dz), h);
+  geo_hit(R.model, R.cone_ray, plane_origin(pl, pl.n_across / 2, col), mk(pl.dx, pl.dy, pl.dz), h);
   const D3 rd = d3(pl.dx, pl.dy, pl.dz);
   const D3 nl = rd * -1.;
   const int n = R.P.n;
