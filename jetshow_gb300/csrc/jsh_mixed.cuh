@@ -1629,26 +1629,27 @@ __device__ __forceinline__ void lane_advance(Lane& L, const JshRequest* __restri
 
 // A persistent warp's work: every idle lane (or group of lanes) takes the next
 // item of the queue once at least `refill` lanes of the warp idle, `start(w)`
-// begins item w on this lane, `step()` advances an active one.
+// begins item w on this lane, `step()` advances an active one.  Returns once
+// the queue is empty and at most `leave` of the warp's items are unfinished.
 //
-// Groups begin without the queue, the k-th group of every warp with the k-th
-// stretch of the order, so that the longest items are in different warps: a
-// warp that is left with one item runs its steps faster than one with six.
-// (Single lanes take consecutive items: items of one length end together.)
+// `deal`: the warps begin without the queue, the k-th lane or group of every
+// warp with the k-th stretch of the order, so that the longest items are in
+// different warps.  `drained`: there is nothing left to begin.
 template <typename Start, typename Step>
 __device__ __forceinline__ void run_queue(Lane& L, unsigned long long* queue, unsigned long long total, int refill,
-                                          const LaneGroup& grp, Start start, Step step) {
+                                          const LaneGroup& grp, bool deal, bool drained, int leave, Start start,
+                                          Step step) {
   const bool member = grp.mask != 0;
   const unsigned before = (1u << (grp.base & 31)) - 1u;
   const int slots = grp.n == 1 ? 32 : kWarpGroups;
   unsigned long long dealt = 0;
-  if (grp.n > 1) {
+  if (deal) {
     const unsigned warps = gridDim.x * (blockDim.x / 32), warp = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    const unsigned long long w = (unsigned long long)(grp.base / kGroupLanes) * warps + warp;
+    const unsigned long long w = (unsigned long long)(grp.base / grp.n) * warps + warp;
     if (member && w < total) start(w);
-    dealt = (unsigned long long)kWarpGroups * warps;
+    dealt = (unsigned long long)slots * warps;
   }
-  bool exhausted = false;
+  bool exhausted = drained;
   for (;;) {
     const unsigned idle = __ballot_sync(0xffffffffu, member && L.phase == PH_IDLE && grp.sub == 0);
     const int nidle = __popc(idle);
@@ -1664,12 +1665,42 @@ __device__ __forceinline__ void run_queue(Lane& L, unsigned long long* queue, un
       }
     }
     const unsigned active = __ballot_sync(0xffffffffu, L.phase != PH_IDLE);
-    if (active == 0) {
-      if (exhausted) break;
-      continue;
-    }
+    if (exhausted && (active == 0 || __popc(active) <= leave)) break;
     if (L.phase != PH_IDLE) step();
   }
+}
+
+// Hand the warp's unfinished items of single lanes (kWarpGroups at most) to
+// its groups: the k-th to the k-th group, whose lanes then hold its state.
+// An item in its I/IQUV pass only, on a field that is not gridded.
+__device__ __forceinline__ void spread_items(Lane& L, const LaneGroup& grp) {
+  const unsigned active = __ballot_sync(0xffffffffu, L.phase != PH_IDLE);
+  const int k = grp.base / kGroupLanes;
+  const bool has = grp.mask != 0 && k < __popc(active);
+  const int src = has ? (int)__fns(active, 0, k + 1) : 0;
+  auto from = [&](auto& v) { v = __shfl_sync(0xffffffffu, v, src); };
+  auto from_df = [&](DF& v) { from(v.hi), from(v.lo); };
+  auto from_byte = [&](auto& v) {
+    int i = (int)v;
+    from(i);
+    v = (std::remove_reference_t<decltype(v)>)i;
+  };
+  from(L.r), from(L.f), from(L.h);
+  from_byte(L.phase), from_byte(L.seg), from_byte(L.first_seg), from_byte(L.init);
+  from_byte(L.ft), from_byte(L.ft_cool), from_byte(L.ft_back);
+  from_df(L.p0x), from_df(L.p0y), from_df(L.p0z);
+  from(L.bx), from(L.by), from(L.bz);
+  from_df(L.length), from_df(L.t);
+  from(L.dt), from(L.first_div), from(L.t_first);
+  from_df(L.chi);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) from(L.x[c]);
+#pragma unroll
+  for (int c = 0; c < 5; ++c) from(L.k1[c]);
+  from(L.s1), from(L.kI1);
+  from(L.nsteps), from(L.fails), from(L.status);
+  from(L.evals), from(L.acc), from(L.rej), from(L.evals0);
+  if (!has) L.phase = PH_IDLE;
 }
 
 // Place of this lane's group among the CTA's groups (the last one for a lane

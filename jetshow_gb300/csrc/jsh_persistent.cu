@@ -45,13 +45,23 @@ __device__ __forceinline__ void iquv_prefix(const JshRequest* __restrict__ reqs,
 // IQUV kernels: persistent CTAs over the ranked emitted items.
 //
 // The build for the fused benchmark family alone (COMPACT: at most 128 threads
-// and 128 registers, 16 resident warps per SM).  Up to kIquvGroups* items per
-// group of the grid they run on groups of lanes: fewer evaluations one after
-// another in each step (full Stokes: 8 092 items 86 -> 74 us, 79 782 items 891
-// -> 707 us, above about 100 000 items a lane each is faster: 129 394 items 428
-// against 471 us on groups; Stokes I alone: 2 022 items 55 -> 45 us, 32 350
-// items 80 against 90 us).
-constexpr int kIquvGroupsFull = 9, kIquvGroupsI = 1;
+// and 128 registers, 16 resident warps per SM).  With many items they run on a
+// lane each, dealt so that the longest are in different warps, and once the
+// queue is empty a warp's last six are handed to its groups of lanes, which
+// take a step in under half the time: the longest items decide when the launch
+// ends (the longest of 517 856 Faraday-thick items has 21 000 evaluations: 11.8
+// -> 9.1 ms; 129 468 of them 11.2 -> 6.6 ms; 129 394 items of a conical jet 430
+// -> 345 us, 517 550 1.10 -> 0.91 ms; 705 176 of a longer-tailed image 1.42 ms
+// before and after, bound by the step's instructions).  Without the dealing the
+// longest are one warp's and the 517 856 items take 12.8 ms; handing over the
+// last three only, 11.8.
+//
+// Up to kIquvGroups* items per group of the grid they run on groups from the
+// start: 8 092 items 86 us on lanes, 74 on groups.  Above, lanes have the
+// better throughput: 32 350 items 221 against 236 us, 79 782 items 639 against
+// 713; in the Faraday-thick build 32 368 items 5.5 against 5.2 ms, 50 572 items
+// 6.15 against 6.23; Stokes I alone 2 022 items 43 us on either.
+constexpr int kIquvGroupsFull = kFtm ? 4 : 2, kIquvGroupsI = 1;
 template <bool FULL, bool COMPACT>
 __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? (kFtm ? 3 : 4) : 1)
     transfer_iquv_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
@@ -67,12 +77,13 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? (kFtm ? 3 : 4) 
   const LaneGroup grp = lane_group(), one = single_lane();
   float* Q = ksh + group_slot(grp) * kGroupWords;
   auto group_step = [&] { lane_step<FULL, PASS_IQUV, false, kGroupLanes>(L, reqs, reqs[L.r].mix, Q, T, grp); };
-  if (on_groups(total, FULL ? (COMPACT ? kIquvGroupsFull * 3 / 4 : kIquvGroupsFull) : kIquvGroupsI)) {
-    run_queue(L, queue, total, refill, grp, start, group_step);
-  } else {
-    run_queue(L, queue, total, refill, one, start,
+  const bool lanes = !on_groups(total, FULL ? kIquvGroupsFull : kIquvGroupsI);
+  if (lanes) {
+    run_queue(L, queue, total, refill, one, true, false, kWarpGroups, start,
               [&] { lane_step<FULL, PASS_IQUV, false, 1>(L, reqs, reqs[L.r].mix, nullptr, T, one); });
+    spread_items(L, grp);
   }
+  run_queue(L, queue, total, refill, grp, !lanes, lanes, 0, start, group_step);
   tally_flush(T, reqs);
 }
 
@@ -90,7 +101,7 @@ __global__ void __launch_bounds__(COMPACT || GROUPS ? 128 : 256, COMPACT || GROU
   const LaneGroup grp = GROUPS ? lane_group() : single_lane();
   float* Q = ksh + (GROUPS ? group_slot(grp) : (int)threadIdx.x) * StageWidth<FULL>::kWords;
   run_queue(
-      L, queue, base[n_req], refill, grp,
+      L, queue, base[n_req], refill, grp, GROUPS, false, 0,
       [&](unsigned long long w) { lane_start_iquv<true>(L, reqs, base, n_req, w, part); },
       [&] { lane_step<FULL, PASS_IQUV, true, 0>(L, reqs, reqs[L.r].mix, Q, T, grp); });
   tally_flush(T, reqs);

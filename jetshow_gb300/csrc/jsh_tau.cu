@@ -147,11 +147,11 @@ __global__ void __launch_bounds__(256, 3)
   };
   if (on_groups(total, kTauGroupsFused)) {
     const LaneGroup grp = lane_group();
-    run_queue(L, queue, total, refill, grp, start,
+    run_queue(L, queue, total, refill, grp, true, false, 0, start,
               [&] { tau_step<PASS_TAU, false, kGroupLanes>(L, reqs, ONE ? mix : reqs[L.r].mix, nullptr, part, T, grp); });
   } else {
     const LaneGroup one = single_lane();
-    run_queue(L, queue, total, refill, one, start,
+    run_queue(L, queue, total, refill, one, false, false, 0, start,
               [&] { tau_step<PASS_TAU, false, 1>(L, reqs, ONE ? mix : reqs[L.r].mix, nullptr, part, T, one); });
   }
   tally_flush(T, reqs);
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(128, GROUPS ? 3 : 4)
   const LaneGroup grp = GROUPS ? lane_group() : single_lane();
   float* K = ksh + (GROUPS ? group_slot(grp) : (int)threadIdx.x) * kTauWords;
   run_queue(
-      L, queue, base[n_req], refill, grp,
+      L, queue, base[n_req], refill, grp, GROUPS, false, 0,
       [&](unsigned long long w) { lane_start(L, reqs, base, n_req, w, true, part); },
       [&] { tau_step<PASS_TAU, true, 0>(L, reqs, reqs[L.r].mix, K, part, T, grp); });
   tally_flush(T, reqs);

@@ -119,3 +119,24 @@ def test_mixed_groups_match_lanes(ctx, grid_id, output, kind, shape, n_nu):
         assert np.array_equal(a[k], b[k], equal_nan=True), k
     for k in ("rhs_evals", "steps_accepted", "steps_rejected", "status_or"):
         assert sa[k] == sb[k], k
+
+
+@pytest.mark.parametrize("output", ["I", "full"])
+@pytest.mark.parametrize("flags", [0, A.FLAG_FARADAY_THICK])
+@pytest.mark.parametrize("shape,refill", [((80, 120), 1), ((80, 120), 0), ((128, 140), 32)])
+def test_mixed_lanes_handed_to_groups(ctx, output, flags, shape, refill):
+    """More items than the grid's groups take (one warp an SM): they begin on
+    single lanes and the last of each warp end on its groups, bitwise as on
+    one lane throughout."""
+    lg = math.log10(6.4 / shape[1] * 1.8443 * J.pc)
+    plane = J.ImagePlane(shape, lg, lg, 0.1)
+    jet, nu = conical().desc(), np.array([8e9 * 1.1])
+    kw = dict(W.ACCURATE_KW, output=output, flags=flags)
+    a, sa = ctx.render(jet, plane.desc(), nu, J.make_params(precision="mixed", schedule="static", **kw))
+    b, sb = ctx.render(jet, plane.desc(), nu, J.make_params(precision="mixed", schedule="persistent", block_size=32,
+                                                           ctas_per_sm=1, refill_threshold=refill, **kw))
+    assert sa["n_work_items"] > 4 * 6 * 152
+    for k in a:
+        assert np.array_equal(a[k], b[k], equal_nan=True), k
+    for k in ("rhs_evals", "steps_accepted", "steps_rejected", "status_or"):
+        assert sa[k] == sb[k], k
