@@ -49,10 +49,11 @@ __device__ inline double grid_value(const JshGrid& G, int field, double px, doub
   if (i >= G.nbx) i = G.nbx - 1;
   if (j >= G.nby) j = G.nby - 1;
   if (i < 0 || j < 0) return nan_value;
-  int b = j * G.nbx + i;
-  int q0 = G.bstart[b], q1 = G.bstart[b + 1];
-  for (int q = q0; q < q1; ++q) {
-    int t = G.bitems[q];
+  const int32_t* head = G.bhead + 8 * ((int64_t)j * G.nbx + i);
+  for (int q = 0;; ++q) {
+    if (q == 7 && head[7] < 0) break;
+    const int t = q < 7 ? head[q] : G.bmore[head[7] + (q - 7)];
+    if (t < 0) break;
     int v0 = G.tri[3 * t], v1 = G.tri[3 * t + 1], v2 = G.tri[3 * t + 2];
     double ax = G.xy[2 * v0], ay = G.xy[2 * v0 + 1];
     double bx = G.xy[2 * v1], by = G.xy[2 * v1 + 1];
@@ -63,9 +64,9 @@ __device__ inline double grid_value(const JshGrid& G, int field, double px, doub
     double w1 = __ddiv_rn(orient2_rn(ax, ay, px, py, cx, cy), area);
     double w2 = __ddiv_rn(orient2_rn(ax, ay, bx, by, px, py), area);
     if (w0 < 0 || w1 < 0 || w2 < 0) continue;
-    double val = __dadd_rn(__dadd_rn(__dmul_rn(w0, (double)G.val[(int64_t)v0 * G.n_fields + field]),
-                                     __dmul_rn(w1, (double)G.val[(int64_t)v1 * G.n_fields + field])),
-                           __dmul_rn(w2, (double)G.val[(int64_t)v2 * G.n_fields + field]));
+    double val = __dadd_rn(__dadd_rn(__dmul_rn(w0, (double)G.val[(int64_t)v0 * G.stride + field]),
+                                     __dmul_rn(w1, (double)G.val[(int64_t)v1 * G.stride + field])),
+                           __dmul_rn(w2, (double)G.val[(int64_t)v2 * G.stride + field]));
     if (isnan(val)) return nan_value;
     return val;
   }

@@ -48,12 +48,18 @@ struct GridW {
   float w0, w1, w2;
   bool ok;
 };
-// Barycentric weights of (px, py) in triangle t; true when inside (the
-// -1e-6 tolerance of the bucket search).  The triangle's record holds what
-// depends on it alone.
-__device__ __forceinline__ bool grid_tri32(const JshGrid& G, int t, float px, float py, GridW& g) {
+// A triangle's record, which holds what depends on it alone.
+struct GridTri {
+  float4 ab, ce, iv;
+};
+__device__ __forceinline__ GridTri grid_tri_load(const JshGrid& G, int t) {
   const float4* r = reinterpret_cast<const float4*>(G.rec) + 3 * (int64_t)t;
-  const float4 ab = r[0], ce = r[1], iv = r[2];
+  return GridTri{r[0], r[1], r[2]};
+}
+// Barycentric weights of (px, py) in a triangle; true when inside (the -1e-6
+// tolerance of the bucket search).
+__device__ __forceinline__ bool grid_tri_in(const GridTri& T, float px, float py, GridW& g) {
+  const float4 &ab = T.ab, &ce = T.ce, &iv = T.iv;
   const float w0 = ((ab.z - px) * (ce.y - py) - (ab.w - py) * (ce.x - px)) * iv.x;
   const float w1 = ((px - ab.x) * ce.w - (py - ab.y) * ce.z) * iv.x;
   const float w2 = 1.f - w0 - w1;
@@ -63,24 +69,48 @@ __device__ __forceinline__ bool grid_tri32(const JshGrid& G, int t, float px, fl
   }
   return false;
 }
+__device__ __forceinline__ bool grid_tri32(const JshGrid& G, int t, float px, float py, GridW& g) {
+  return grid_tri_in(grid_tri_load(G, t), px, py, g);
+}
 
-// The first triangle of (px, py)'s bucket that holds the point, or -1.
-__device__ __forceinline__ int grid_search32(const JshGrid& G, float px, float py, GridW& g) {
+// The bucket of (px, py), first id -1 outside the grid's rectangle.
+struct GridBucket {
+  int4 h0, h1;
+};
+__device__ __forceinline__ GridBucket grid_bucket32(const JshGrid& G, float px, float py) {
   const float fx = (px - G.x0f) * G.inv_hf, fy = (py - G.y0f) * G.inv_hf;
-  if (!(fx >= 0.f && fy >= 0.f)) return -1;
+  if (!(fx >= 0.f && fy >= 0.f)) return GridBucket{make_int4(-1, -1, -1, -1), make_int4(-1, -1, -1, -1)};
   const int i = min((int)fx, G.nbx - 1), j = min((int)fy, G.nby - 1);
-  const int b = j * G.nbx + i;
-  const int q1 = G.bstart[b + 1];
-  for (int q = G.bstart[b]; q < q1; ++q) {
-    const int t = G.bitems[q];
+  const int4* h = reinterpret_cast<const int4*>(G.bhead) + 2 * ((int64_t)j * G.nbx + i);
+  return GridBucket{h[0], h[1]};
+}
+// The first triangle of the bucket that holds the point, or -1: two records in
+// flight at a time.
+__device__ __forceinline__ int grid_search32(const JshGrid& G, GridBucket B, float px, float py, GridW& g) {
+  const int off = B.h1.w;
+  B.h1.w = -1;
+#pragma unroll 1
+  for (;;) {
+    const int t0 = B.h0.x, t1 = B.h0.y;
+    if (t0 < 0) return -1;
+    const GridTri T0 = grid_tri_load(G, t0), T1 = grid_tri_load(G, t1 < 0 ? t0 : t1);
+    if (grid_tri_in(T0, px, py, g)) return t0;
+    if (t1 < 0) break;
+    if (grid_tri_in(T1, px, py, g)) return t1;
+    B.h0 = make_int4(B.h0.z, B.h0.w, B.h1.x, B.h1.y);
+    B.h1 = make_int4(B.h1.z, B.h1.w, -1, -1);
+  }
+  if (off < 0) return -1;
+  for (int q = off;; ++q) {
+    const int t = G.bmore[q];
+    if (t < 0) return -1;
     if (grid_tri32(G, t, px, py, g)) return t;
   }
-  return -1;
 }
 __device__ inline GridW grid_locate32(const JshGrid& G, float px, float py) {
   GridW g;
   g.ok = false;
-  if (G.n_tri > 0) grid_search32(G, px, py, g);
+  if (G.n_tri > 0) grid_search32(G, grid_bucket32(G, px, py), px, py, g);
   return g;
 }
 
@@ -105,26 +135,41 @@ __device__ __forceinline__ LaneGroup single_lane() {
 }
 
 // Point location with a hint: the triangle of the lane's previous evaluation is
-// tried first -- consecutive evaluation points along a ray mostly fall in the
-// same triangle, and the bucket search costs a chain of dependent loads per
-// candidate (bucket, list, triangle, vertices) -- and the found triangle is
-// stored back.  The hint restarts with each item, so an item's lookups do not
-// depend on the lane that runs it.  A group locates its points at once, lane k
-// the k-th point.  A point near an edge belongs to whichever
-// of the two triangles is tried first, so the answers must be those of the
-// serial order, in which point k tries the triangle of point k - 1 before its
-// bucket: every lane first tries the step's hint and, failing that, its
-// bucket; then the points take their turn with the triangle before them,
-// which most often is one of the two already tried.
+// tried first (its bucket's loads under way meanwhile) -- consecutive
+// evaluation points along a ray often fall in the same triangle -- and the
+// found triangle is stored back.  The hint restarts with each item, so an
+// item's lookups do not depend on the lane that runs it.
+//
+// A group locates its points at once, lane k the k-th point.  A point near an
+// edge belongs to whichever of the two triangles is tried first, so the
+// answers must be those of the serial order, in which point k tries the
+// triangle of point k - 1 before its bucket.  Every lane tries the step's hint
+// and, failing that, its bucket, and then the triangle that the lane before it
+// has come to.  Where no lane is inside that one (and none that is inside the
+// hint follows one that has left it) each lane's own answer is the serial
+// one; otherwise the points take their turn.
 __device__ __forceinline__ GridW grid_locate32_group(const JshGrid& G, float px, float py, int* hint, LaneGroup L) {
   GridW g, own;
   g.ok = own.ok = false;
   if (G.n_tri == 0) return g;
   const int t0 = *hint;
+  const GridBucket B = grid_bucket32(G, px, py);
   const bool in0 = t0 >= 0 && grid_tri32(G, t0, px, py, g);
-  int found = in0 ? -1 : grid_search32(G, px, py, own);
+  int found = in0 ? -1 : grid_search32(G, B, px, py, own);
   if (L.n == 1) {
     if (found >= 0) *hint = found;
+    return in0 ? g : own;
+  }
+  const int mine0 = in0 ? t0 : found;
+  int prev = __shfl_sync(L.mask, mine0, L.sub > 0 ? L.base + L.sub - 1 : L.base);
+  if (L.sub == 0) prev = t0;
+  bool settled = in0 ? prev == t0 : found >= 0 && (prev == t0 || prev == found);
+  if (!settled && !in0 && found >= 0 && prev >= 0) {
+    GridW other;
+    settled = !grid_tri32(G, prev, px, py, other);
+  }
+  if (__all_sync(L.mask, settled)) {
+    *hint = __shfl_sync(L.mask, mine0, L.base + L.n - 1);
     return in0 ? g : own;
   }
   bool searched = !in0;
@@ -137,7 +182,7 @@ __device__ __forceinline__ GridW grid_locate32_group(const JshGrid& G, float px,
       if (t != t0 && !(searched && found == t) && grid_tri32(G, t, px, py, g)) {
         // inside the triangle of the point before
       } else {
-        if (!searched) found = grid_search32(G, px, py, own);
+        if (!searched) found = grid_search32(G, B, px, py, own);
         searched = true;
         g = own;
         if (found >= 0) mine = found;
@@ -150,7 +195,7 @@ __device__ __forceinline__ GridW grid_locate32_group(const JshGrid& G, float px,
 }
 __device__ __forceinline__ float grid_val32(const JshGrid& G, const GridW& g, int field, float nan_value) {
   if (!g.ok) return nan_value;
-  const uint32_t nf = (uint32_t)G.n_fields;  // n and n_fields are bounded: 2^30 points x 64 fields
+  const uint32_t nf = (uint32_t)G.stride;  // n and stride are bounded: 2^30 points x 64 fields
   const float v = g.w0 * G.val[(uint64_t)g.v0 * nf + field] + g.w1 * G.val[(uint64_t)g.v1 * nf + field] +
                   g.w2 * G.val[(uint64_t)g.v2 * nf + field];
   return isnan(v) ? nan_value : v;
@@ -160,7 +205,7 @@ __device__ __forceinline__ float grid_val32(const JshGrid& G, const GridW& g, in
 // registers and the code size of the kernels for every other law too.  With
 // the calls and the triangle records a simulation grid at 256^2 went from
 // 36.0 + 26.2 ms (tau, IQUV kernel) to 25.0 + 17.5, 512^2 from 114 + 96 to 76
-// + 55; 415 968 items of a radial field from 1.53 + 1.78 to 1.36 + 1.08.
+// + 55 (by later lookups 48 + 44); 415 968 items of a radial field from 1.53 + 1.78 to 1.36 + 1.08.
 static __device__ __noinline__ float sim32(const JshGrid& G, int field, F3 p, float nan_value) {
   return grid_val32(G, grid_locate32(G, p.z, sqrtf(p.x * p.x + p.y * p.y)), field, nan_value);
 }
@@ -170,8 +215,21 @@ static __device__ __noinline__ float sim32(const JshGrid& G, int field, F3 p, fl
 static __device__ __noinline__ float4 sim_shared32(const JshModel& m, float z, float rc, int* hint, LaneGroup group) {
   const JshGrid& G = m.grids[0];
   const GridW g = grid_locate32_group(G, z, rc, hint, group);
-  return make_float4(grid_val32(G, g, m.f_v, 1.0f), grid_val32(G, g, m.f_n, 0.f), grid_val32(G, g, m.fb_p, 0.f),
-                     grid_val32(G, g, m.fb_phi, 0.f));
+  const int q = m.f_v >> 2;
+  if (!g.ok || (m.f_n >> 2) != q || (m.fb_p >> 2) != q || (m.fb_phi >> 2) != q)
+    return make_float4(grid_val32(G, g, m.f_v, 1.0f), grid_val32(G, g, m.f_n, 0.f), grid_val32(G, g, m.fb_p, 0.f),
+                       grid_val32(G, g, m.fb_phi, 0.f));
+  // all four in one float4 of a point's row: 3 loads for 12, of as many sectors
+  const float4* val = reinterpret_cast<const float4*>(G.val) + q;
+  const uint32_t row = (uint32_t)G.stride >> 2;
+  const float4 a = val[(uint64_t)g.v0 * row], b = val[(uint64_t)g.v1 * row], c = val[(uint64_t)g.v2 * row];
+  const float4 v = make_float4(g.w0 * a.x + g.w1 * b.x + g.w2 * c.x, g.w0 * a.y + g.w1 * b.y + g.w2 * c.y,
+                               g.w0 * a.z + g.w1 * b.z + g.w2 * c.z, g.w0 * a.w + g.w1 * b.w + g.w2 * c.w);
+  auto field = [&](int f, float nan_value) {
+    const float x = (f & 2) ? ((f & 1) ? v.w : v.z) : ((f & 1) ? v.y : v.x);
+    return isnan(x) ? nan_value : x;
+  };
+  return make_float4(field(m.f_v, 1.0f), field(m.f_n, 0.f), field(m.fb_p, 0.f), field(m.fb_phi, 0.f));
 }
 
 // ---------------------------------------------------------------- V

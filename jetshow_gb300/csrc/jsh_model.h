@@ -41,12 +41,14 @@ struct JshGrid {         // device view of an uploaded triangulated (z, r) grid
   // vertices a, b, c, the edge c - a, 1 / (twice its area) (NaN for a
   // degenerate one), and its vertex ids as integer bits
   const float* rec;
-  const float* val;      // [n][n_fields]
+  const float* val;      // [n][stride], stride = n_fields rounded up to float4
   const int32_t* tri;    // [n_tri][3]
-  const int32_t* bstart; // [nbx*nby + 1] bucket -> triangle list offsets
-  const int32_t* bitems; // triangle ids
+  // [nbx*nby][8] a bucket's triangles in ascending order: the first 7 ids (-1:
+  // none) and where the others begin in bmore (-1: none; they end with a -1)
+  const int32_t* bhead;
+  const int32_t* bmore;
   int64_t n, n_tri;
-  int32_t n_fields, nbx, nby, pad_;
+  int32_t n_fields, nbx, nby, stride;
   double x0, y0, h;      // bucket grid origin and (square) cell size
   float x0f, y0f, inv_hf;
 };
