@@ -207,12 +207,18 @@ constexpr int kTauWords = 17;  // the 15 nodes of a panel, odd
 // for each (NG = 1, 5); the builds for every field law (NG = 0: the group's
 // size is LaneGroup::n) evaluate the points in a rolled loop, one copy of that
 // larger code, and exchange through the stage storage of the group (or lane).
-// fused I/IQUV step: five points of two float4 (three with the Faraday-thick
-// mode), the groups spread over the banks
+// The I/IQUV kernels' files are compiled twice: as is, and by the _ft.cu files with
+// JSH_FARADAY_THICK_BUILD 1 for requests that ask for the Faraday-thick mode
+// (JSH_FLAG_FARADAY_THICK).  The mode's bookkeeping in the step costs the
+// other requests ~18 % of the IQUV kernel even where it never engages, so
+// the default kernels are built without it.
 #ifndef JSH_FARADAY_THICK_BUILD
 #define JSH_FARADAY_THICK_BUILD 0
 #endif
-constexpr int kGroupWords = JSH_FARADAY_THICK_BUILD ? 76 : 52;
+constexpr bool kFtm = JSH_FARADAY_THICK_BUILD != 0;
+// fused I/IQUV step: five points of two float4 (three with the Faraday-thick
+// mode), the groups spread over the banks
+constexpr int kGroupWords = kFtm ? 76 : 52;
 
 // acc = sum_{j < S} a_Sj K_j over the stage derivatives held in registers
 // (S and j compile-time: the tableau entries are immediate operands).
@@ -560,7 +566,7 @@ __device__ __forceinline__ float stokes_rhs(const Coef32& c, const FtPoint& q, c
     dk[0] = c.eI - c.kI * y[0];
     return scale;
   }
-  if (ft) {
+  if (kFtm) {
     // Faraday-thick mode: the lab-frame polarisation Pi = Q + iU obeys
     // Pi' = -lambda Pi + S, lambda = k_I - i k_F, S = (eta_Q - k_Q I) - i k_C V.
     // Where |lambda| is far above the rate at which S / lambda changes, Pi is
@@ -568,15 +574,19 @@ __device__ __forceinline__ float stokes_rhs(const Coef32& c, const FtPoint& q, c
     // only decays (d' = -k_I d, up to the adiabatic lag); I and V see the
     // quasi-static part through k_Q Re Pi and k_C Im Pi, the transient's
     // share rotates at k_F and integrates to at most ~cpl |d|.  dk[1], dk[2]
-    // carry the rotating-frame value e^{-i chi} S / lambda itself.
-    const float sre = c.eQ - c.kQ * y[0], sim = -c.kC * y[3];
-    const float pre = fmaf(sre, c.kI, -sim * c.kF) * q.il, pim = fmaf(sre, c.kF, sim * c.kI) * q.il;
-    dk[0] = c.eI - c.kI * y[0] - c.kQ * pre - c.kV * y[3];
-    dk[1] = fmaf(cs, pre, sn * pim);
-    dk[2] = fmaf(-sn, pre, cs * pim);
-    dk[3] = c.eV - c.kI * y[3] - c.kV * y[0] + c.kC * pim;
+    // carry the rotating-frame value e^{-i chi} S / lambda itself.  Both modes
+    // are formed and selected: a warp mostly has lanes in each, and its six
+    // stages stay free of branches (with the points' FtPoint formed together:
+    // 3.57 G evaluations 56.0 -> 52.6 ms, 24.5 M on groups 5.50 -> 5.06).
+    const float sQ = c.eQ - c.kQ * y[0], sU = -c.kC * y[3];
+    const float pre = fmaf(sQ, c.kI, -sU * c.kF) * q.il, pim = fmaf(sQ, c.kF, sU * c.kI) * q.il;
+    const float Ql = ft ? pre : cs * y[1] - sn * y[2], Ul = ft ? pim : sn * y[1] + cs * y[2];
+    dk[0] = c.eI - c.kI * y[0] - c.kQ * Ql - c.kV * y[3];
+    dk[1] = ft ? fmaf(cs, pre, sn * pim) : -c.kI * y[1] + cs * sQ + sn * sU;
+    dk[2] = ft ? fmaf(-sn, pre, cs * pim) : -c.kI * y[2] - sn * sQ + cs * sU;
+    dk[3] = c.eV - c.kI * y[3] - c.kV * y[0] + c.kC * Ul;
     dk[4] = c.kF;
-    *cpl = q.cpl;
+    if (ft) *cpl = q.cpl;
     return scale;
   }
   float Qlab = cs * y[1] - sn * y[2];
@@ -695,15 +705,6 @@ __device__ __forceinline__ void lane_start_iquv(Lane& L, const JshRequest* __res
 // a Stokes component is about 0.3 u h scale (four terms of magnitude
 // <= scale per derivative, weighted by |e_j| <= 0.05).
 constexpr float kNoise = 5.9604645e-8f;
-// This file is compiled twice: as is, and by jsh_persistent_ft.cu with
-// JSH_FARADAY_THICK_BUILD 1 for requests that ask for the Faraday-thick mode
-// (JSH_FLAG_FARADAY_THICK).  The mode's bookkeeping in the step costs the
-// other requests ~18 % of the IQUV kernel even where it never engages, so
-// the default kernels are built without it.
-#ifndef JSH_FARADAY_THICK_BUILD
-#define JSH_FARADAY_THICK_BUILD 0
-#endif
-constexpr bool kFtm = JSH_FARADAY_THICK_BUILD != 0;
 // Faraday-thick mode of the IQUV pass: entry where
 // |k_F| >= kFtRatio k_I; the quasi-static part's lag and the transient's
 // left-out coupling must stay within kFtTol (atol + rtol I); after a refused
@@ -1344,6 +1345,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     // builds for every field law (one copy of that code) in shared memory,
     // with a sixth point where every evaluation draws a random direction.
     Coef32 C[5];
+    FtPoint P[5] = {};
     // words of a point (a fused group's: two float4, three with the
     // Faraday-thick mode)
     constexpr int kPoint = NG > 1 ? (kFtm ? 12 : 8) : StageWidth<FULL>::NC;
@@ -1352,6 +1354,10 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
 #pragma unroll
       for (int s = 1; s <= 5; ++s)
         coef32_rt<GENERAL>(R, X, F, pn + dirf * (dp_c32(s) * h), mode, C[s - 1]);
+      if (ft) {
+#pragma unroll
+        for (int s = 0; s < 5; ++s) P[s] = ft_point(C[s]);
+      }
     } else {
       grp.sync();  // the step before has read its coefficients
       const int np = six ? 6 : 5;
@@ -1394,7 +1400,8 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
       if (NG != 1) get_coefficients<FULL, NG>(q, c);
       else c = C[s == 6 ? 4 : s - 1];
       FtPoint cq{};
-      if (ft && NG > 1) cq = FtPoint{q[8], q[9]};
+      if (NG == 1) cq = P[s == 6 ? 4 : s - 1];
+      else if (ft && NG > 1) cq = FtPoint{q[8], q[9]};
       else if (ft) cq = ft_point(c);
       const float sc = stokes_rhs<FULL>(c, cq, y, cs, sn, dk, ft, &cpl);
       smax = fmaxf(smax, sc);
