@@ -1635,7 +1635,8 @@ __device__ __forceinline__ void lane_advance(Lane& L, const JshRequest* __restri
 }
 
 // A persistent warp's work: every idle lane (or group of lanes) takes the next
-// item of the queue once at least `refill` lanes of the warp idle, `start(w)`
+// item of the queue once at least `refill` lanes of the warp idle (with groups
+// the two that belong to none among them), `start(w)`
 // begins item w on this lane, `step()` advances an active one.  Returns once
 // the queue is empty and at most `leave` of the warp's items are unfinished.
 //
@@ -1660,7 +1661,7 @@ __device__ __forceinline__ void run_queue(Lane& L, unsigned long long* queue, un
   for (;;) {
     const unsigned idle = __ballot_sync(0xffffffffu, member && L.phase == PH_IDLE && grp.sub == 0);
     const int nidle = __popc(idle);
-    if (!exhausted && (nidle * grp.n >= refill || nidle == slots) && nidle > 0) {
+    if (!exhausted && (32 - (slots - nidle) * grp.n >= refill || nidle == slots) && nidle > 0) {
       unsigned long long b = 0;
       if ((threadIdx.x & 31u) == 0) b = atomicAdd(queue, (unsigned long long)nidle);
       b = __shfl_sync(0xffffffffu, b, 0);
