@@ -219,6 +219,8 @@ constexpr bool kFtm = JSH_FARADAY_THICK_BUILD != 0;
 // fused I/IQUV step: five points of two float4 (three with the Faraday-thick
 // mode), the groups spread over the banks
 constexpr int kGroupWords = kFtm ? 76 : 52;
+// the same of a lane: five points of two float4, the lanes over the banks
+constexpr int kLaneWords = 44;
 
 // acc = sum_{j < S} a_Sj K_j over the stage derivatives held in registers
 // (S and j compile-time: the tableau entries are immediate operands).
@@ -1227,7 +1229,7 @@ __device__ __forceinline__ void tau_step(Lane& L, const JshRequest* __restrict__
 // A stage point's coefficients in shared memory: words, or two float4 (NG > 1).
 template <bool FULL, int NG>
 __device__ __forceinline__ void put_coefficients(float* q, const Coef32& c) {
-  if (NG > 1 && FULL) {
+  if (NG >= 1 && FULL) {
     reinterpret_cast<float4*>(q)[0] = make_float4(c.kI, c.eI, c.kQ, c.kV);
     reinterpret_cast<float4*>(q)[1] = make_float4(c.kF, c.kC, c.eQ, c.eV);
     return;
@@ -1245,7 +1247,7 @@ __device__ __forceinline__ void put_coefficients(float* q, const Coef32& c) {
 }
 template <bool FULL, int NG>
 __device__ __forceinline__ void get_coefficients(const float* q, Coef32& c) {
-  if (NG > 1 && FULL) {
+  if (NG >= 1 && FULL) {
     const float4 a = reinterpret_cast<const float4*>(q)[0], b = reinterpret_cast<const float4*>(q)[1];
     c = Coef32{a.x, a.z, a.w, b.x, b.y, a.y, b.z, b.w};
     return;
@@ -1318,9 +1320,9 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
     const bool ft = kFtm && FULL && L.ft;
     float cpl = 0.f;  // Faraday-thick mode: max(|k_Q|, |k_C|) / |lambda| of the last evaluation
     constexpr int mode = FULL ? COEF_FULL : COEF_I;
-    if (!L.init) {
-      Coef32 c;
-      coef32_rt<GENERAL>(R, X, F, pn, mode, c, L.h, (uint32_t)L.f, L.evals0 + L.evals, &L.tri);
+    // first derivative from the coefficients at the step's start; false: the
+    // Faraday-thick mode was refused there
+    auto first = [&](const Coef32& c) {
       L.s1 = stokes_rhs<FULL>(c, ft ? ft_point(c) : FtPoint{}, L.x, c0, s0, L.k1, ft, &cpl);
       L.kI1 = c.kI;
       L.evals++;
@@ -1334,30 +1336,56 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
           L.ft = 0;
           L.ft_cool = kFtCooldown;
           L.init = false;
-          return;
+          return false;
         }
       }
+      return true;
+    };
+    constexpr bool kLoop = NG == 1 && FULL;  // the start's evaluation is in the points' loop
+    if (!kLoop && !L.init) {
+      Coef32 c;
+      coef32_rt<GENERAL>(R, X, F, pn, mode, c, L.h, (uint32_t)L.f, L.evals0 + L.evals, &L.tri);
+      if (!first(c)) return;
     }
     // The coefficients depend on the stage's point alone, not on the state,
     // and the last two stages share their point (c = 1): all five points are
     // evaluated before the stages, so that their chains of dependent
-    // operations overlap.  The fused build keeps them in registers; the
-    // builds for every field law (one copy of that code) in shared memory,
-    // with a sixth point where every evaluation draws a random direction.
+    // operations overlap.  The fused build of Stokes I keeps them in registers;
+    // the others in shared memory, with one copy of the coefficients' code, and
+    // a sixth point where every evaluation draws a random direction.
     Coef32 C[5];
     FtPoint P[5] = {};
     // words of a point (a fused group's: two float4, three with the
     // Faraday-thick mode)
     constexpr int kPoint = NG > 1 ? (kFtm ? 12 : 8) : StageWidth<FULL>::NC;
     const bool six = GENERAL && R.model.rnd_kind == JSH_RND_POINTS;
-    if (NG == 1) {
+    if (kLoop) {
+      // one copy of the coefficients' code (six copies were more than the
+      // instruction caches hold: the warps waited for instructions a third of
+      // the time) and 128 registers instead of 149: 517 550 items 897 -> 850 us,
+      // 705 176 1.39 -> 1.37 ms, Faraday-thick 3.57 G evaluations 55.6 -> 51.2 ms.
+      // Stokes I alone is faster unrolled (530 against 590 us).
+      bool in_mode = true;
+#pragma unroll 1
+      for (int s = L.init ? 1 : 0; s <= 5; ++s) {
+        Coef32 c;
+        coef32_rt<GENERAL>(R, X, F, pn + dirf * (c_C[s] * h), mode, c);
+        if (s == 0) in_mode = first(c);
+        else put_coefficients<FULL, NG>(Q + (s - 1) * kPoint, c);
+      }
+      if (!in_mode) return;
+      if (ft) {
+#pragma unroll
+        for (int s = 0; s < 5; ++s) {
+          Coef32 c;
+          get_coefficients<FULL, NG>(Q + s * kPoint, c);
+          P[s] = ft_point(c);
+        }
+      }
+    } else if (NG == 1) {
 #pragma unroll
       for (int s = 1; s <= 5; ++s)
         coef32_rt<GENERAL>(R, X, F, pn + dirf * (dp_c32(s) * h), mode, C[s - 1]);
-      if (ft) {
-#pragma unroll
-        for (int s = 0; s < 5; ++s) P[s] = ft_point(C[s]);
-      }
     } else {
       grp.sync();  // the step before has read its coefficients
       const int np = six ? 6 : 5;
@@ -1397,7 +1425,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
       }
       Coef32 c;
       const float* q = Q + (s == 6 ? (six ? 5 : 4) : s - 1) * kPoint;
-      if (NG != 1) get_coefficients<FULL, NG>(q, c);
+      if (NG != 1 || kLoop) get_coefficients<FULL, NG>(q, c);
       else c = C[s == 6 ? 4 : s - 1];
       FtPoint cq{};
       if (NG == 1) cq = P[s == 6 ? 4 : s - 1];
@@ -1682,6 +1710,7 @@ __device__ __forceinline__ void run_queue(Lane& L, unsigned long long* queue, un
 // its groups: the k-th to the k-th group, whose lanes then hold its state.
 // An item in its I/IQUV pass only, on a field that is not gridded.
 __device__ __forceinline__ void spread_items(Lane& L, const LaneGroup& grp) {
+  __syncwarp();  // the lanes have read their stage storage
   const unsigned active = __ballot_sync(0xffffffffu, L.phase != PH_IDLE);
   const int k = grp.base / kGroupLanes;
   const bool has = grp.mask != 0 && k < __popc(active);
@@ -1729,11 +1758,11 @@ __device__ __host__ constexpr int form_words() {
   return StageWidth<FULL>::kWords > kTauWords ? StageWidth<FULL>::kWords : kTauWords;
 }
 
-// Dynamic shared memory of a CTA: the lanes' stage storage (none in the fused
-// IQUV build: `lanes` false), or that of its groups.
+// Dynamic shared memory of a CTA: the lanes' stage storage (`lanes` false, the
+// fused IQUV build: kLaneWords of them, none for Stokes I), or that of its groups.
 template <bool FULL>
 constexpr size_t stage_smem(int block, bool lanes = true) {
-  const size_t one = lanes ? sizeof(float) * form_words<FULL>() * (size_t)block : 0;
+  const size_t one = sizeof(float) * (size_t)block * (lanes ? form_words<FULL>() : FULL ? kLaneWords : 0);
   const size_t groups = sizeof(float) * kGroupWords * kWarpGroups * (size_t)(block / 32);
   return one > groups ? one : groups;
 }

@@ -61,6 +61,7 @@ __device__ __forceinline__ void iquv_prefix(const JshRequest* __restrict__ reqs,
 // better throughput: 32 350 items 221 against 236 us, 79 782 items 639 against
 // 713; in the Faraday-thick build 32 368 items 5.5 against 5.2 ms, 50 572 items
 // 6.15 against 6.23; Stokes I alone 2 022 items 43 us on either.
+static_assert(kWarpGroups * kGroupWords <= 32 * kLaneWords, "a warp's groups fit its lanes' storage");
 constexpr int kIquvGroupsFull = kFtm ? 4 : 2, kIquvGroupsI = 1;
 template <bool FULL, bool COMPACT>
 __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? (kFtm ? 3 : 4) : 1)
@@ -75,12 +76,14 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? (kFtm ? 3 : 4) 
   const unsigned long long total = base[n_req];
   auto start = [&](unsigned long long w) { lane_start_iquv<false>(L, reqs, base, n_req, w, part); };
   const LaneGroup grp = lane_group(), one = single_lane();
-  float* Q = ksh + group_slot(grp) * kGroupWords;
+  // a warp's lanes and groups share its part of the storage (full Stokes)
+  float* W = ksh + threadIdx.x / 32 * 32 * kLaneWords;
+  float* Q = FULL ? W + min(grp.base / kGroupLanes, kWarpGroups - 1) * kGroupWords : ksh + group_slot(grp) * kGroupWords;
   auto group_step = [&] { lane_step<FULL, PASS_IQUV, false, kGroupLanes>(L, reqs, reqs[L.r].mix, Q, T, grp); };
   const bool lanes = !on_groups(total, FULL ? kIquvGroupsFull : kIquvGroupsI);
   if (lanes) {
     run_queue(L, queue, total, refill, one, true, false, kWarpGroups, start,
-              [&] { lane_step<FULL, PASS_IQUV, false, 1>(L, reqs, reqs[L.r].mix, nullptr, T, one); });
+              [&] { lane_step<FULL, PASS_IQUV, false, 1>(L, reqs, reqs[L.r].mix, W + (threadIdx.x & 31u) * kLaneWords, T, one); });
     spread_items(L, grp);
   }
   run_queue(L, queue, total, refill, grp, !lanes, lanes, 0, start, group_step);
@@ -252,7 +255,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   };
   bl_t = enough(bl_t, bt);
   const IquvKernel iquv_k = iquv_kernel(full, shape.compact != 0, shape.fused != 0, groups);
-  // the fused build keeps a single lane's stages in registers
+  // the fused build: a lane keeps its five points (full Stokes) or nothing there
   auto smem_of = [&](int block) {
     return full ? stage_smem<true>(block, !shape.fused) : stage_smem<false>(block, !shape.fused);
   };
