@@ -23,15 +23,15 @@
 // lengths are in pc so the FP32 state stays well inside its range.
 //
 // A step's coefficients depend on the stage points alone, so they are
-// evaluated before the stages: five independent chains instead of six
-// dependent ones (the last two stages share their point), the stage
-// derivatives in registers and the stages unrolled.  On the 512x1024 conical
-// jet the render went from 2.76 to 2.25 ms, on its 102x333 image (set by the
-// heaviest ray's chain of steps) from 1.29 to 0.99 ms, on a ParabaloidCone
-// image with the Faraday-thick mode from 71 to 40 ms.  The kernels for every
-// field law keep one copy of the coefficient code (a rolled loop over the
-// points, the coefficients in shared memory), so that they fit the SM
-// instruction caches even when the lanes of a warp are in different phases.
+// evaluated before the stages: five instead of six (the last two stages share
+// their point), the stage derivatives in registers and the stages unrolled.
+// On the 512x1024 conical jet the render went from 2.76 to 2.25 ms by that, on
+// its 102x333 image (set by the heaviest ray's chain of steps) from 1.29 to
+// 0.99 ms, on a ParabaloidCone image with the Faraday-thick mode from 71 to 40
+// ms.  There is one copy of the coefficient code in a step (a rolled loop over
+// the points, the coefficients in shared memory), so that it fits the SM
+// instruction caches even when the lanes of a warp are in different phases;
+// Stokes I alone, a shorter step, holds its points unrolled in registers.
 #pragma once
 
 #include <float.h>
@@ -204,9 +204,9 @@ constexpr int kTauWords = 17;  // the 15 nodes of a panel, odd
 // point of a Dormand-Prince step (or every fifth node of a panel) and the
 // results are exchanged, so a step costs one evaluation's latency instead of
 // five.  Lane 0 writes the outputs.  The fused build has a copy of the step
-// for each (NG = 1, 5); the builds for every field law (NG = 0: the group's
-// size is LaneGroup::n) evaluate the points in a rolled loop, one copy of that
-// larger code, and exchange through the stage storage of the group (or lane).
+// for each (NG = 1, 5), the builds for every field law one (NG = 0: the group's
+// size is LaneGroup::n).
+
 // The I/IQUV kernels' files are compiled twice: as is, and by the _ft.cu files with
 // JSH_FARADAY_THICK_BUILD 1 for requests that ask for the Faraday-thick mode
 // (JSH_FLAG_FARADAY_THICK).  The mode's bookkeeping in the step costs the

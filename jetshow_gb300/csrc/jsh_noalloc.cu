@@ -20,7 +20,7 @@
 //
 // The array is sized for at most JSH_NOALLOC_MAX_PIXELS pixels,
 // JSH_NOALLOC_MAX_ALONG columns and JSH_NOALLOC_MAX_NU frequencies; every
-// GPU that loads the library holds it (8 MiB) until the process exits.  All
+// GPU that loads the library holds it (16 MiB) until the process exits.  All
 // calls share it and it keeps the last call's contents, so calls whose work
 // overlaps on the GPU (different streams, or another host thread) race.  The
 // first call on a device looks up the array's device address

@@ -44,8 +44,9 @@ __device__ __forceinline__ void iquv_prefix(const JshRequest* __restrict__ reqs,
 
 // IQUV kernels: persistent CTAs over the ranked emitted items.
 //
-// The build for the fused benchmark family alone (COMPACT: at most 128 threads
-// and 128 registers, 16 resident warps per SM).  With many items they run on a
+// The build for the fused benchmark family alone (128 registers, 16 resident
+// warps per SM; with the Faraday-thick mode 142 and 12; COMPACT caps the former
+// for CTAs of at most 128 threads).  With many items they run on a
 // lane each, dealt so that the longest are in different warps, and once the
 // queue is empty a warp's last six are handed to its groups of lanes, which
 // take a step in under half the time: the longest items decide when the launch
@@ -190,7 +191,8 @@ IquvKernel iquv_kernel(bool full, bool compact, bool fused, bool groups) {
 // At 29 092 items of a radial field the tau kernel took 287 us on lanes and
 // 217 on groups, the IQUV kernel 686 and 365; 33 640 items of a gridded jet
 // 65.3 and 37.0 ms, 31.7 and 25.2 ms; at 134 556 of them 108 and 134 ms, 95
-// and 90 ms, at 415 968 items of a radial field 1.6 and 4.0 ms, 1.6 and 2.7.
+// and 90 ms (since then the lookups got faster: 19 + 15 ms at 33 640 items on
+// groups, 48 + 44 ms at 134 556 on lanes), at 415 968 items of a radial field 1.6 and 4.0 ms, 1.6 and 2.7.
 constexpr uint64_t kGroupItemsPerSm = 432;
 
 // CTAs of the deep chain's IQUV kernel per SM (64 threads each) when the
