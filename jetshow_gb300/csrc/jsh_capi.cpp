@@ -57,8 +57,8 @@ void jsh_free_device(jsh_ctx* ctx, void* p, size_t bytes) {
   ctx->used.fetch_sub(bytes);
 }
 
-void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int32_t n_nu, bool own_outputs,
-                        JshRequestLayout* L) {
+void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int32_t n_nu, int precision,
+                        bool own_outputs, JshRequestLayout* L) {
   size_t o = 0;
   L->off_req = o;
   o = align_up(o + sizeof(JshRequest));
@@ -95,7 +95,7 @@ void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int3
   L->off_iq_order = o;
   o = align_up(o + sizeof(uint32_t) * npix * (uint64_t)n_nu);
   L->off_seg32 = o;
-  o = align_up(o + sizeof(JshSeg32) * JSH_MAX_SEG * npix);
+  if (precision == JSH_PREC_MIXED) o = align_up(o + sizeof(JshSeg32) * JSH_MAX_SEG * npix);
   L->own_outputs = own_outputs;
   for (int k = 0; k < 7; ++k) {
     L->off_out[k] = o;
@@ -113,7 +113,7 @@ void jsh_bind_request(JshRequest* req, char* base, const JshRequestLayout& L, bo
   req->plane.along_center = (double*)(base + L.off_along_center);
   req->plane.across_pos = (double*)(base + L.off_across);
   req->hits = (JshHit*)(base + L.off_hits);
-  req->seg32 = (JshSeg32*)(base + L.off_seg32);
+  req->seg32 = L.off_seg32 < L.off_out[0] ? (JshSeg32*)(base + L.off_seg32) : nullptr;
   req->buckets = (uint32_t*)(base + L.off_buckets);
   req->order = (uint32_t*)(base + L.off_order);
   req->key = (uint8_t*)(base + L.off_key);
@@ -392,7 +392,7 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   int st = jsh_prepare_request(ctx, model, plane, params, n_nu, &req, &npix);
   if (st) return st;
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, dev_out == nullptr, &L);
+  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, params->precision, dev_out == nullptr, &L);
   st = ensure_workspace(ctx, L.total);
   if (st) return st;
   char* base = (char*)ctx->ws;
@@ -564,7 +564,7 @@ extern "C" int jsh_plane_rays(jsh_ctx* ctx, const jsh_plane_desc* plane, double*
   if (origins) {
     JSH_CUDA_TRY(cudaSetDevice(ctx->device));
     JshRequestLayout L;
-    jsh_request_layout(0, plane->n_along, plane->n_across, 1, false, &L);
+    jsh_request_layout(0, plane->n_along, plane->n_across, 1, JSH_PREC_FP64, false, &L);
     const size_t off_o = L.total;
     st = ensure_workspace(ctx, align_up(off_o + sizeof(double) * 3 * npix));
     if (st) return st;
@@ -611,7 +611,7 @@ extern "C" int jsh_trace_plane(jsh_ctx* ctx, const jsh_model_desc* model, const 
   req.npix = npix;
   req.n_nu = 0;  // the hit kernel writes no output planes
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, 1, false, &L);
+  jsh_request_layout(npix, plane->n_along, plane->n_across, 1, JSH_PREC_FP64, false, &L);
   st = ensure_workspace(ctx, L.total);
   if (st) return st;
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));

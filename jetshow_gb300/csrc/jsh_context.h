@@ -105,8 +105,9 @@ struct jsh_ctx {
 // Helpers shared by the C-ABI translation units.
 int jsh_prepare_request(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_desc* plane,
                         const jsh_params* params, int32_t n_nu, JshRequest* req, uint64_t* npix);
-void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int32_t n_nu, bool own_outputs,
-                        JshRequestLayout* L);
+// (only mixed requests have the segments in FP32, 128 bytes a pixel)
+void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int32_t n_nu, int precision,
+                        bool own_outputs, JshRequestLayout* L);
 void jsh_bind_request(JshRequest* req, char* base, const JshRequestLayout& L, bool own_outputs);
 int jsh_alloc_device(jsh_ctx* ctx, size_t bytes, void** p);
 // Mixed-precision constants of a prepared request: fills req->mix (except

@@ -153,7 +153,7 @@ extern "C" int jsh_observation_run_noalloc(const jsh_model_desc* model, const js
   st = jsh_prepare_request(nullptr, model, plane, params, n_nu, &in.req, &np);
   if (st) return st;
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, false, &L);
+  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, params->precision, false, &L);
   const size_t state = L.total - (L.off_out[0] - L.off_seg32);
   if (state > JSH_NOALLOC_STATE_BYTES) {
     jsh_set_error("request needs %zu scratch bytes, more than the %u of the no-alloc array", state,

@@ -186,7 +186,8 @@ int prepare_request(jsh_server* S, Request* q) {
   int st = jsh_prepare_request(S->ctx, &q->model, &q->plane, &q->params, (int32_t)q->nu.size(), &q->rec, &npix);
   if (st) return st;
   q->npix = npix;
-  jsh_request_layout(npix, q->plane.n_along, q->plane.n_across, (int32_t)q->nu.size(), true, &q->L);
+  jsh_request_layout(npix, q->plane.n_along, q->plane.n_across, (int32_t)q->nu.size(), q->params.precision, true,
+                     &q->L);
   // the record, counters, n_hit, queue, nu and fc live in the slot's control
   // block; the arena block holds the tables, the hit list and the outputs
   q->arena_bytes = q->L.total - q->L.off_along_size;

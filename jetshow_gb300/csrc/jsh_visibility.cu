@@ -272,7 +272,7 @@ extern "C" int jsh_observation_visibilities(jsh_ctx* ctx, const jsh_model_desc* 
   const int rows_pad = (n_across + kRows - 1) / kRows * kRows;
   // the render's own layout, then the visibility buffers behind it
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, true, &L);
+  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, params->precision, true, &L);
   const size_t o_w = up256(L.total);
   const size_t o_col = up256(o_w + sizeof(float) * (size_t)n_nu * n_along * rows_pad);
   const size_t o_y = up256(o_col + sizeof(double) * n_along);

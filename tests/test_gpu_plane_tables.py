@@ -2,10 +2,13 @@
 columns and walked by the device's serial kernel above: origins and sizes bit
 for bit the oracle's on both sides of the line, and a ring of uploads longer
 than its stages keeps every render's own plane."""
+import math
+
 import numpy as np
 import pytest
 
 from jetshow_gb300 import jet as J
+from jetshow_gb300 import runtime as R
 from jetshow_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +40,21 @@ def test_uploads_in_turn(ctx):
     for k, plane in enumerate(planes):
         ref, _ = ctx.render(jet, plane.desc(), np.array([8e9 + 1e9 * k]), params)
         assert np.array_equal(outs[k].cpu().numpy(), ref["I"]) and ref["I"].max() > 0
+
+
+def test_fp64_request_fits_its_budget(ctx):
+    """The FP64 path has no FP32 segments: a 128x128 request takes about 205
+    bytes a pixel of a context's budget, and not the 128 more of a mixed one."""
+    jet = W.conical_model()
+    lg = math.log10(0.4 * 1.8443 * J.pc)
+    plane = J.ImagePlane((128, 128), lg, lg, 0.1)
+    nu = np.array([15.4e9])
+    kw = dict(W.ACCURATE_KW, output="I", precision="fp64")
+    small = R.Context(0, hbm_budget_bytes=5 << 20)
+    try:
+        g, _ = small.render(jet.desc(), plane.desc(), nu, J.make_params(**kw))
+    finally:
+        small.close()
+    w, _ = ctx.render(jet.desc(), plane.desc(), nu, J.make_params(**kw))
+    for k in w:
+        assert np.array_equal(g[k], w[k]), k
