@@ -18,7 +18,7 @@ struct JshLaunchShape {
   int block_size;        // threads per CTA of the transfer kernel
   int ctas_per_sm;       // persistent schedule: CTAs per SM (0: occupancy max)
   int refill_threshold;  // persistent schedule: refill when >= this many lanes idle
-  int compact;           // mixed persistent schedule: the 168-register build (<= 128 threads)
+  int compact;           // mixed persistent schedule: the register-capped build (<= 128 threads)
   int single;            // mixed persistent schedule: tau and IQUV passes in one kernel (else split)
   int fused;             // split form: every request of the batch is of the fused benchmark
                          // family (mix.helical_log): launch the kernels built for it alone
