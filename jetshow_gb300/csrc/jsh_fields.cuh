@@ -317,8 +317,18 @@ __device__ __forceinline__ Freq64 freq64(const JshModel& m, double nu) {
   const double cp = JSH_Q_E * JSH_Q_E / (JSH_PI * JSH_M_E);     // nu_p^2 per cm^-3
   const double k = JSH_PI * cp * cb / (JSH_C * nu * nu), e = JSH_PI * cp * cb * JSH_M_E / JSH_C;
   const double rk = m.b_scalar ? m.rnd_k : 1.0, re = m.b_scalar ? m.rnd_e : 1.0;
+  // a negative thermal density has no plasma frequency, as in density64
+  const double th = m.thermal_fraction < 0.0 ? NAN : m.thermal_fraction;
   return Freq64{cb / nu,    k * (m.fk_i * rk), e * (m.fe_i * re), k * m.fk_v, e * m.fe_v,
-                2. * k * (m.kfr_factor + m.thermal_fraction), k * (cb / nu)};
+                2. * k * (m.kfr_factor + th), k * (cb / nu)};
+}
+
+// n' as the coefficients' factor: NaN where it is negative, as the plasma
+// frequency sqrt(n' q^2 / (pi m)) that the formulas square is (the pass then
+// stops with JSH_ST_NAN).  The sign is read from the upper word: an FP64
+// comparison would hold the pipe for ~64 cycles.
+__device__ __forceinline__ double density64(double np) {
+  return __double2hiint(np) < 0 && np != 0.0 ? NAN : np;
 }
 
 // Kinematics at a point (src/utils.cpp:147-162): beta, gamma, the Doppler
@@ -376,7 +386,7 @@ __device__ inline void coefficients64(const JshModel& m, const Freq64& F, const 
   Frame64 f = flat;
   if (m.v_kind != JSH_V_CONST_FLAT) f = frame64(m, p, nl);
   const double n = nfield(m, p);
-  const double np = m.n_plasma ? n : n / f.gamma;
+  const double np = density64(m.n_plasma ? n : n / f.gamma);
   if (m.b_scalar) {
     const double w = bscalar(m, p) * f.D;
     const Powers64 P = powers64<MODE == 2 ? 1 : MODE>(F.q1 * w, m.s);
