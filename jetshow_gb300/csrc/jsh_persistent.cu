@@ -111,26 +111,40 @@ __global__ void __launch_bounds__(COMPACT || GROUPS ? 128 : 256, COMPACT || GROU
   tally_flush(T, reqs);
 }
 
+// Lets `kernel` take `smem` bytes of stage storage.  A launch gets 48 KB unasked,
+// static storage included, and a full-Stokes lane of the every-law and
+// single-kernel builds keeps 196 bytes: 256 threads take 50 176.  Where it has
+// to be asked for, always the same bytes are, the largest CTA's: launches of
+// several threads do not lower each other's limit.
+template <typename K>
+cudaError_t allow_storage(K kernel, size_t smem) {
+  constexpr size_t kUnasked = (48u << 10) - 1024;
+  if (smem <= kUnasked) return cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem<true>(256));
+}
+
+template <typename K>
+int occupancy(K kernel, int block, size_t smem) {
+  int n = 0;
+  if (allow_storage(kernel, smem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block, smem) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 // Resident CTAs per SM of the IQUV kernel / the single-kernel form.
 int occupancy_mixed(bool split, bool full, int block_size, bool compact) {
-  int n = 0;
   if (compact && block_size > 128) return 0;
   const size_t sm = full ? stage_smem<true>(block_size) : stage_smem<false>(block_size);
-#define JSH_OCC(kernel) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, block_size, sm)
-  if (split) {
-    // the general build bounds both (it holds at least the fused one's registers)
-    if (compact) {
-      if (full) JSH_OCC((transfer_iquv_general_kernel<true, true, false>));
-      else JSH_OCC((transfer_iquv_general_kernel<false, true, false>));
-    } else {
-      if (full) JSH_OCC((transfer_iquv_general_kernel<true, false, false>));
-      else JSH_OCC((transfer_iquv_general_kernel<false, false, false>));
-    }
-  } else {
-    JSH_OCC(JSH_SINGLE_KERNEL(full, compact));
-  }
-#undef JSH_OCC
-  return n;
+  if (!split) return occupancy(JSH_SINGLE_KERNEL(full, compact), block_size, sm);
+  // the general build bounds both (it holds at least the fused one's registers)
+  if (compact)
+    return full ? occupancy(transfer_iquv_general_kernel<true, true, false>, block_size, sm)
+                : occupancy(transfer_iquv_general_kernel<false, true, false>, block_size, sm);
+  return full ? occupancy(transfer_iquv_general_kernel<true, false, false>, block_size, sm)
+              : occupancy(transfer_iquv_general_kernel<false, false, false>, block_size, sm);
 }
 
 }  // namespace
@@ -230,6 +244,8 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   if (blocks == 0) blocks = 1;
   const size_t smem = full ? stage_smem<true>(bs) : stage_smem<false>(bs);
   if (!split) {
+    const cudaError_t e = allow_storage(JSH_SINGLE_KERNEL(full, shape.compact != 0), smem);
+    if (e != cudaSuccess) return e;
     if (shape.marks) cudaEventRecord(shape.marks[2], stream);
     JSH_SINGLE_KERNEL(full, shape.compact != 0)<<<blocks, bs, smem, stream>>>(d_reqs, n_req, q, rf);
     if (shape.marks) cudaEventRecord(shape.marks[3], stream);
@@ -263,6 +279,8 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   };
   if (groups && bs > 128) bs = 128;
   const size_t smem_q = smem_of(bs);
+  cudaError_t e = allow_storage(iquv_k, smem_q);
+  if (e != cudaSuccess) return e;
   int per_sm_q = shape.ctas_per_sm;
   if (per_sm_q <= 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_q, iquv_k, bs, smem_q);
   const unsigned blocks_q = enough((unsigned)(num_sms * std::max(per_sm_q, 1)), bs);
@@ -292,7 +310,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   int per_sm_t2 = (65536 - deep_warps * wr_iquv) / ((bt / 32) * wr_tau);
   per_sm_t2 = std::min(std::max(per_sm_t2, 1), per_sm_t);
   if (shape.marks) cudaEventRecord(shape.marks[0], stream);
-  cudaError_t e = launch_prio(tau_k, bl_t, bt, smem_t, stream, prio_hi, d_reqs, n_req, q, rf, 0, mix);
+  e = launch_prio(tau_k, bl_t, bt, smem_t, stream, prio_hi, d_reqs, n_req, q, rf, 0, mix);
   if (e != cudaSuccess) return e;
   jsh_launch_iquv_rank(d_reqs, n_req, max_items, num_sms, 0, stream);
   e = cudaEventRecord(shape.fork[0], stream);
