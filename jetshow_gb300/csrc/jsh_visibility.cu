@@ -39,6 +39,7 @@ namespace {
 constexpr int kVisThreads = 128;  // visibilities per CTA
 constexpr int kColTileMax = 8;    // image columns staged in shared memory at a time (at most)
 constexpr int kMaxAcross = 16384;  // rows of one staged column: 64 KB of shared memory
+constexpr int kTileBytes = 96 * 1024;  // shared memory of the staged columns (at most)
 constexpr int kRows = 32;         // rows per inner block
 
 struct Cf {
@@ -317,10 +318,11 @@ extern "C" int jsh_observation_visibilities(jsh_ctx* ctx, const jsh_model_desc* 
     vis_columns_kernel<<<(unsigned)((n_along + 255) / 256), 256, 0, s>>>(asz, acn, n_along, vis->rad_per_cm,
                                                                           (double*)(base + o_col),
                                                                           (double*)(base + o_y));
-    const int col_tile = std::max(1, std::min(kColTileMax, (int)((96 * 1024) / (sizeof(float) * rows_pad))));
+    const int col_tile = std::max(1, std::min(kColTileMax, (int)(kTileBytes / (sizeof(float) * rows_pad))));
     const size_t smem = sizeof(float) * col_tile * rows_pad;
-    if (smem > 48 * 1024)
-      JSH_CUDA_TRY(cudaFuncSetAttribute(vis_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // 48 KB unasked hold the kernel's static arrays too
+    if (smem > 47 * 1024)
+      JSH_CUDA_TRY(cudaFuncSetAttribute(vis_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileBytes));
     vis_sum_kernel<<<dim3(gx, (unsigned)n_split, (unsigned)n_nu), kVisThreads, smem, s>>>(
         (const float*)(base + o_w), (const double*)(base + o_col), (const double*)(base + o_y),
         (const double*)(base + o_uvr), n_uv, n_along, rows_pad, 0.5 * (double)(n_across - 1), cols, col_tile,
