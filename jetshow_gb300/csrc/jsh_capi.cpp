@@ -411,6 +411,7 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   JshStage* stage = nullptr;
   st = jsh_next_stage(ctx, L, &stage);
   if (st) return st;
+  JshWorkspaceUse use(ctx, stream);
   if (params->precision == JSH_PREC_MIXED) {
     st = jsh_prepare_mixed(&req, nu_hz, (JshFreqConst*)(stage->host + (L.off_fc - L.off_req)));
     if (st) return st;
@@ -439,7 +440,7 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   JSH_CUDA_TRY(jsh_launch_transfer(d_req, 1, params->precision, params->schedule, params->output == JSH_OUT_FULL,
                                    npix * (uint64_t)n_nu, npix, shape, (unsigned int*)(base + L.off_queue),
                                    ctx->num_sms, stream));
-  JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, stream));
+  JSH_CUDA_TRY(use.end());
   ctx->last_pending = true;
   // counters and plane (2), hit, transfer; the persistent mixed schedule adds 3 ranking
   // kernels, and its split form the tau kernel and 3 IQUV ranking kernels
@@ -499,6 +500,7 @@ extern "C" int jsh_observation_run(jsh_ctx* ctx, const jsh_model_desc* model, co
   if (st) return st;
   JSH_CUDA_TRY(cudaEventRecord(ctx->ev_stop, ctx->stream));
   if (host_out) {
+    JshWorkspaceUse use(ctx, ctx->stream);
     char* base = (char*)ctx->ws;
     double* planes[6] = {host_out->tau, host_out->l, host_out->I, host_out->Q, host_out->U, host_out->V};
     size_t nb = sizeof(double) * npix * (uint64_t)n_nu;
@@ -507,7 +509,7 @@ extern "C" int jsh_observation_run(jsh_ctx* ctx, const jsh_model_desc* model, co
     if (host_out->status)
       JSH_CUDA_TRY(cudaMemcpyAsync(host_out->status, base + L.off_out[6], sizeof(uint32_t) * npix * (uint64_t)n_nu,
                                    cudaMemcpyDeviceToHost, ctx->stream));
-    JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, ctx->stream));
+    JSH_CUDA_TRY(use.end());
   }
   JSH_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   jsh_stats s{};
@@ -575,11 +577,12 @@ extern "C" int jsh_plane_rays(jsh_ctx* ctx, const jsh_plane_desc* plane, double*
     JshStage* stage = nullptr;
     st = jsh_next_stage(ctx, L, &stage);
     if (st) return st;
+    JshWorkspaceUse use(ctx, s);
     st = jsh_upload_request(stage, &req, L, base, nullptr, s);
     if (st) return st;
     JSH_CUDA_TRY(jsh_launch_plane_rays(req.plane, (double*)(base + off_o), nullptr, s));
     JSH_CUDA_TRY(cudaMemcpyAsync(origins, base + off_o, sizeof(double) * 3 * npix, cudaMemcpyDeviceToHost, s));
-    JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, s));
+    JSH_CUDA_TRY(use.end());
     JSH_CUDA_TRY(cudaStreamSynchronize(s));
   }
   if (direction) {
@@ -621,6 +624,7 @@ extern "C" int jsh_trace_plane(jsh_ctx* ctx, const jsh_model_desc* model, const 
   JshStage* stage = nullptr;
   st = jsh_next_stage(ctx, L, &stage);
   if (st) return st;
+  JshWorkspaceUse use(ctx, s);
   st = jsh_upload_request(stage, &req, L, base, nullptr, s);
   if (st) return st;
   const JshRequest* d_req = (const JshRequest*)(base + L.off_req);
@@ -630,7 +634,7 @@ extern "C" int jsh_trace_plane(jsh_ctx* ctx, const jsh_model_desc* model, const 
   JSH_CUDA_TRY(cudaStreamSynchronize(s));
   std::vector<JshHit> hits(nhit);
   if (nhit) JSH_CUDA_TRY(cudaMemcpy(hits.data(), base + L.off_hits, sizeof(JshHit) * nhit, cudaMemcpyDeviceToHost));
-  JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, s));
+  JSH_CUDA_TRY(use.end());
   if (n_seg) memset(n_seg, 0, sizeof(int32_t) * npix);
   if (seg) memset(seg, 0, sizeof(double) * 12 * npix);
   if (status) memset(status, 0, sizeof(uint32_t) * npix);
@@ -665,6 +669,7 @@ extern "C" int jsh_hit_rays(jsh_ctx* ctx, const jsh_model_desc* model, const dou
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
   char* b = (char*)ctx->ws;
   cudaStream_t s = ctx->stream;
+  JshWorkspaceUse use(ctx, s);
   JSH_CUDA_TRY(cudaMemcpyAsync(b + o_orig, origins, 24 * n, cudaMemcpyHostToDevice, s));
   JSH_CUDA_TRY(cudaMemcpyAsync(b + o_dir, directions, 24 * n, cudaMemcpyHostToDevice, s));
   JSH_CUDA_TRY(jsh_launch_hit_rays(m, (double*)(b + o_orig), (double*)(b + o_dir), n, (int32_t*)(b + o_nseg),
@@ -672,7 +677,7 @@ extern "C" int jsh_hit_rays(jsh_ctx* ctx, const jsh_model_desc* model, const dou
   if (n_seg) JSH_CUDA_TRY(cudaMemcpyAsync(n_seg, b + o_nseg, 4 * n, cudaMemcpyDeviceToHost, s));
   if (seg) JSH_CUDA_TRY(cudaMemcpyAsync(seg, b + o_seg, 96 * n, cudaMemcpyDeviceToHost, s));
   if (status) JSH_CUDA_TRY(cudaMemcpyAsync(status, b + o_st, 4 * n, cudaMemcpyDeviceToHost, s));
-  JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, s));
+  JSH_CUDA_TRY(use.end());
   JSH_CUDA_TRY(cudaStreamSynchronize(s));
   return JSH_OK;
 }

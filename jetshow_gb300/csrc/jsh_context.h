@@ -102,6 +102,33 @@ struct jsh_ctx {
   int last_kernels = 0;
 };
 
+// A call's use of the context workspace, from its first enqueued work on.  It
+// ends, whether the call succeeds or not, in a ws_ready behind all that the call
+// has enqueued on `stream` and on the side stream of overlapped passes: the
+// next user, perhaps on another stream, waits for that event alone.
+class JshWorkspaceUse {
+ public:
+  JshWorkspaceUse(jsh_ctx* ctx, cudaStream_t stream) : ctx_(ctx), stream_(stream) {}
+  JshWorkspaceUse(const JshWorkspaceUse&) = delete;
+  JshWorkspaceUse& operator=(const JshWorkspaceUse&) = delete;
+  ~JshWorkspaceUse() {
+    if (!open_) return;
+    if (cudaEventRecord(ctx_->fork[1], ctx_->side) == cudaSuccess) cudaStreamWaitEvent(stream_, ctx_->fork[1], 0);
+    cudaEventRecord(ctx_->ws_ready, stream_);
+    cudaGetLastError();
+  }
+  // the regular end: the side stream has joined
+  cudaError_t end() {
+    open_ = false;
+    return cudaEventRecord(ctx_->ws_ready, stream_);
+  }
+
+ private:
+  jsh_ctx* ctx_;
+  cudaStream_t stream_;
+  bool open_ = true;
+};
+
 // Helpers shared by the C-ABI translation units.
 int jsh_prepare_request(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_desc* plane,
                         const jsh_params* params, int32_t n_nu, JshRequest* req, uint64_t* npix);

@@ -132,6 +132,7 @@ extern "C" int jsh_observation_run_stripe(jsh_ctx* ctx, const jsh_model_desc* mo
   JshStage* stage = nullptr;
   st = jsh_next_stage(ctx, L, &stage);
   if (st) return st;
+  JshWorkspaceUse use(ctx, s);
   st = jsh_upload_request(stage, &req, L, base, nullptr, s);
   if (st) return st;
   const JshRequest* d_req = (const JshRequest*)(base + L.off_req);
@@ -140,7 +141,7 @@ extern "C" int jsh_observation_run_stripe(jsh_ctx* ctx, const jsh_model_desc* mo
     JSH_CUDA_TRY(cudaGetLastError());
     JSH_CUDA_TRY(cudaMemcpyAsync(tau_host, base + off_out, sizeof(double) * count, cudaMemcpyDeviceToHost, s));
   }
-  JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, s));
+  JSH_CUDA_TRY(use.end());
   JSH_CUDA_TRY(cudaStreamSynchronize(s));
   return JSH_OK;
 }

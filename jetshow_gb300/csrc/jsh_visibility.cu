@@ -301,6 +301,7 @@ extern "C" int jsh_observation_visibilities(jsh_ctx* ctx, const jsh_model_desc* 
   uint64_t np2 = 0;
   st = enqueue_single(ctx, model, plane, nu_hz, n_nu, params, s, nullptr, &L2, &np2);
   if (st) return st;
+  JshWorkspaceUse use(ctx, s);
   char* base = (char*)ctx->ws;
   if (n_uv > 0) {
     const int64_t nv = (int64_t)n_nu * n_uv;
@@ -336,7 +337,7 @@ extern "C" int jsh_observation_visibilities(jsh_ctx* ctx, const jsh_model_desc* 
   if (n_uv > 0)
     JSH_CUDA_TRY(cudaMemcpyAsync(vis_out, base + o_out, sizeof(double) * 2 * (size_t)n_nu * n_uv,
                                  cudaMemcpyDeviceToHost, s));
-  JSH_CUDA_TRY(cudaEventRecord(ctx->ws_ready, s));
+  JSH_CUDA_TRY(use.end());
   JSH_CUDA_TRY(cudaStreamSynchronize(s));
   jsh_stats S{};
   st = collect_stats(ctx, &S);
