@@ -324,6 +324,8 @@ int ensure_workspace(jsh_ctx* ctx, size_t need) {
   if (need <= ctx->ws_cap) return JSH_OK;
   // the previous work on the workspace must be done before it is freed
   cudaEventSynchronize(ctx->ws_ready);
+  int kept = keep_stats(ctx);
+  if (kept) return kept;
   if (ctx->ws) jsh_free_device(ctx, ctx->ws, ctx->ws_cap);
   ctx->ws = nullptr;
   ctx->ws_cap = 0;
@@ -481,7 +483,10 @@ int collect_stats(jsh_ctx* ctx, jsh_stats* s) {
   return JSH_OK;
 }
 
-
+int keep_stats(jsh_ctx* ctx) {
+  jsh_stats s;
+  return collect_stats(ctx, &s);
+}
 
 extern "C" int jsh_observation_run(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_desc* plane,
                                    const double* nu_hz, int32_t n_nu, const jsh_params* params, jsh_image* host_out,
@@ -565,6 +570,8 @@ extern "C" int jsh_plane_rays(jsh_ctx* ctx, const jsh_plane_desc* plane, double*
   }
   if (origins) {
     JSH_CUDA_TRY(cudaSetDevice(ctx->device));
+    st = keep_stats(ctx);
+    if (st) return st;
     JshRequestLayout L;
     jsh_request_layout(0, plane->n_along, plane->n_across, 1, JSH_PREC_FP64, false, &L);
     const size_t off_o = L.total;
@@ -615,6 +622,8 @@ extern "C" int jsh_trace_plane(jsh_ctx* ctx, const jsh_model_desc* model, const 
   req.n_nu = 0;  // the hit kernel writes no output planes
   JshRequestLayout L;
   jsh_request_layout(npix, plane->n_along, plane->n_across, 1, JSH_PREC_FP64, false, &L);
+  st = keep_stats(ctx);
+  if (st) return st;
   st = ensure_workspace(ctx, L.total);
   if (st) return st;
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
@@ -664,6 +673,8 @@ extern "C" int jsh_hit_rays(jsh_ctx* ctx, const jsh_model_desc* model, const dou
   if (st) return st;
   size_t o_orig = 0, o_dir = align_up(24 * n), o_nseg = align_up(o_dir + 24 * n), o_seg = align_up(o_nseg + 4 * n),
          o_st = align_up(o_seg + 96 * n), total = align_up(o_st + 4 * n);
+  st = keep_stats(ctx);
+  if (st) return st;
   st = ensure_workspace(ctx, total);
   if (st) return st;
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));

@@ -177,4 +177,7 @@ int jsh_resolve_hull(jsh_ctx* ctx, JshModel* model);
 int jsh_resolve_cells(jsh_ctx* ctx, JshModel* model);
 // Counters of the last enqueued request (synchronises with it).
 int collect_stats(jsh_ctx* ctx, jsh_stats* s);
+// Read the last render's statistics from the workspace before another use of
+// it overwrites them.
+int keep_stats(jsh_ctx* ctx);
 void jsh_set_error(const char* fmt, ...);

@@ -123,6 +123,8 @@ extern "C" int jsh_observation_run_stripe(jsh_ctx* ctx, const jsh_model_desc* mo
   JshRequestLayout L;
   jsh_request_layout(npix, plane->n_along, plane->n_across, 1, JSH_PREC_FP64, false, &L);
   const size_t off_out = (L.total + 255) / 256 * 256;
+  st = keep_stats(ctx);
+  if (st) return st;
   st = ensure_workspace(ctx, off_out + sizeof(double) * count);
   if (st) return st;
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));

@@ -175,11 +175,41 @@ void error_path() {
   }
 }
 
+// The statistics of the last render are its own, whatever has used the
+// workspace since.
+void statistics() {
+  jsh_ctx* c = nullptr;
+  check(jsh_ctx_create(0, 0, &c) == JSH_OK, "context");
+  const jsh_model_desc m = model();
+  const jsh_params P = mixed();
+  const double nu[3] = {1e10, 2e10, 3e10};
+  static double rays[3 * 64 * 96], dir[3 * 64 * 96], seg[12 * 64 * 96];
+  for (int k = 0; k < 3 * 64 * 96; ++k) rays[k] = dir[k] = 1.0;
+  jsh_image img;
+  memset(&img, 0, sizeof(img));
+  jsh_stats want, got;
+  for (int other = 0; other < 4; ++other) {
+    const jsh_plane_desc p = plane(16, 24), q = plane(64, 96);
+    check(jsh_observation_run_device(c, &m, &p, nu, 3, &P, (void*)c->stream, &img) == JSH_OK, "render");
+    if (other == 0) {
+      check(jsh_last_stats(c, &want) == JSH_OK && want.rhs_evals == 100 && want.n_work_items == 15, "its statistics");
+    } else {
+      int st = JSH_OK;
+      if (other == 1) st = jsh_plane_rays(c, &q, rays, dir, nullptr);
+      if (other == 2) st = jsh_trace_plane(c, &m, &q, nullptr, seg, nullptr);
+      if (other == 3) st = jsh_hit_rays(c, &m, rays, dir, 64 * 96, nullptr, seg, nullptr);
+      check(st == JSH_OK && jsh_last_stats(c, &got) == JSH_OK && !memcmp(&want, &got, sizeof(got)), "the same after");
+    }
+  }
+  jsh_ctx_destroy(c);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   if (!strcmp(what, "error")) error_path();
+  else if (!strcmp(what, "statistics")) statistics();
   else return 2;
   return failed;
 }

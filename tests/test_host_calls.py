@@ -1,5 +1,6 @@
 """The C entry points on a fake CUDA runtime (tests/cpp/fake_runtime.cpp), on the
-CPU: what a failed call leaves behind, without a failing GPU."""
+CPU: what a failed call leaves behind, without a failing GPU, and what the calls that
+share the workspace leave of the last render."""
 import os
 import subprocess
 
@@ -27,3 +28,7 @@ def run(exe, scenario):
 
 def test_failed_launch_keeps_the_workspace_in_use(fake):
     run(fake, "error")
+
+
+def test_last_stats_survive_other_calls(fake):
+    run(fake, "statistics")
