@@ -57,19 +57,9 @@ void jsh_free_device(jsh_ctx* ctx, void* p, size_t bytes) {
   ctx->used.fetch_sub(bytes);
 }
 
-void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int32_t n_nu, int precision,
+void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int32_t n_nu, bool seg32,
                         bool own_outputs, JshRequestLayout* L) {
   size_t o = 0;
-  L->off_req = o;
-  o = align_up(o + sizeof(JshRequest));
-  L->off_nu = o;
-  o = align_up(o + sizeof(double) * n_nu);
-  L->off_fc = o;
-  o = align_up(o + sizeof(JshFreqConst) * n_nu);
-  L->off_along_size = o;
-  o = align_up(o + sizeof(double) * n_along);
-  L->off_along_center = o;
-  o = align_up(o + sizeof(double) * n_along);
   L->off_counters = o;
   o = align_up(o + 8 * sizeof(unsigned long long));
   L->off_nhit = o;
@@ -82,6 +72,16 @@ void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int3
   o = align_up(o + 2 * sizeof(uint32_t));
   L->off_iq_buckets = o;
   o = align_up(o + sizeof(uint32_t) * JSH_IQ_WORDS);
+  L->off_req = o;
+  o = align_up(o + sizeof(JshRequest));
+  L->off_nu = o;
+  o = align_up(o + sizeof(double) * n_nu);
+  L->off_fc = o;
+  o = align_up(o + sizeof(JshFreqConst) * n_nu);
+  L->off_along_size = o;
+  o = align_up(o + sizeof(double) * n_along);
+  L->off_along_center = o;
+  o = align_up(o + sizeof(double) * n_along);
   L->off_across = o;
   o = align_up(o + sizeof(double) * (n_across / 2) * n_along);
   L->off_hits = o;
@@ -95,7 +95,7 @@ void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int3
   L->off_iq_order = o;
   o = align_up(o + sizeof(uint32_t) * npix * (uint64_t)n_nu);
   L->off_seg32 = o;
-  if (precision == JSH_PREC_MIXED) o = align_up(o + sizeof(JshSeg32) * JSH_MAX_SEG * npix);
+  if (seg32) o = align_up(o + sizeof(JshSeg32) * JSH_MAX_SEG * npix);
   L->own_outputs = own_outputs;
   for (int k = 0; k < 7; ++k) {
     L->off_out[k] = o;
@@ -320,6 +320,10 @@ extern "C" void jsh_ctx_destroy(jsh_ctx* c) {
 
 // context-workspace helpers, shared with the autotuner (jsh_autotune.cpp)
 
+bool workspace_fits(const jsh_ctx* ctx, size_t need) {
+  return need <= ctx->ws_cap || (need < ctx->ws_refused && ctx->used.load() - ctx->ws_cap + need <= ctx->budget);
+}
+
 int ensure_workspace(jsh_ctx* ctx, size_t need) {
   if (need <= ctx->ws_cap) return JSH_OK;
   // the previous work on the workspace must be done before it is freed
@@ -332,7 +336,10 @@ int ensure_workspace(jsh_ctx* ctx, size_t need) {
   size_t cap = std::max(need, (size_t)(1u << 20));
   void* p = nullptr;
   int st = jsh_alloc_device(ctx, cap, &p);
-  if (st) return st;
+  if (st) {
+    ctx->ws_refused = std::min(ctx->ws_refused, cap);
+    return st;
+  }
   ctx->ws = p;
   ctx->ws_cap = cap;
   return JSH_OK;
@@ -344,7 +351,7 @@ int jsh_next_stage(jsh_ctx* ctx, const JshRequestLayout& L, JshStage** out) {
   if (!g.copied) JSH_CUDA_TRY(cudaEventCreateWithFlags(&g.copied, cudaEventDisableTiming));
   else JSH_CUDA_TRY(cudaEventSynchronize(g.copied));
   // without tables where the device makes them
-  const size_t tables = L.off_counters - L.off_along_size;
+  const size_t tables = L.off_across - L.off_along_size;
   const size_t need = L.off_along_size - L.off_req + std::min<size_t>(tables, 2 * sizeof(double) * JSH_HOST_TABLE_COLUMNS + 512);
   if (need > g.cap) {
     if (g.host) cudaFreeHost(g.host);
@@ -372,7 +379,7 @@ int jsh_upload_request(JshStage* g, JshRequest* req, const JshRequestLayout& L, 
   }
   JSH_CUDA_TRY(cudaMemcpyAsync(base + L.off_req, g->host, end - L.off_req, cudaMemcpyHostToDevice, stream));
   JSH_CUDA_TRY(cudaEventRecord(g->copied, stream));
-  const size_t zero = L.off_across - L.off_counters;
+  const size_t zero = L.off_req - L.off_counters;
   if (req->plane.host_tables) JSH_CUDA_TRY(jsh_launch_clear(base + L.off_counters, zero, stream));
   else JSH_CUDA_TRY(cudaMemsetAsync(base + L.off_counters, 0, zero, stream));
   JSH_CUDA_TRY(jsh_launch_plane((const JshRequest*)(base + L.off_req), 1, n_along, stream,
@@ -384,7 +391,7 @@ int jsh_upload_request(JshStage* g, JshRequest* req, const JshRequestLayout& L, 
 // dev_out is NULL the request writes into workspace-owned planes.
 int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_desc* plane, const double* nu_hz,
                    int32_t n_nu, const jsh_params* params, cudaStream_t stream, const jsh_image* dev_out,
-                   JshRequestLayout* L_out, uint64_t* npix_out) {
+                   JshRequestLayout* L_out, uint64_t* npix_out, const JshRequestLayout* layout) {
   if (!nu_hz || !all_finite_positive(nu_hz, n_nu)) {
     jsh_set_error("frequencies must be finite and > 0");
     return JSH_ERR_INVALID;
@@ -394,9 +401,19 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   int st = jsh_prepare_request(ctx, model, plane, params, n_nu, &req, &npix);
   if (st) return st;
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, params->precision, dev_out == nullptr, &L);
-  st = ensure_workspace(ctx, L.total);
-  if (st) return st;
+  if (layout) {
+    L = *layout;
+  } else {
+    // without the segments in FP32 where the budget or the device has no room for them
+    auto lay = [&](bool seg32) {
+      jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, seg32, dev_out == nullptr, &L);
+      return L.total;
+    };
+    const bool mixed = params->precision == JSH_PREC_MIXED;
+    st = mixed && !workspace_fits(ctx, lay(true)) ? JSH_ERR_OOM : ensure_workspace(ctx, lay(mixed));
+    if (st == JSH_ERR_OOM && mixed) st = ensure_workspace(ctx, lay(false));
+    if (st) return st;
+  }
   char* base = (char*)ctx->ws;
   jsh_bind_request(&req, base, L, dev_out == nullptr);
   if (dev_out) {
@@ -426,6 +443,7 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   shape.fused = (req.mix.helical_log && !(params->flags & JSH_FLAG_GENERAL_KERNELS)) ? 1 : 0;
   shape.marks = nullptr;
   shape.mix = &req.mix;
+  if (params->precision == JSH_PREC_MIXED && !req.seg32) shape.single = 1;
   const bool overlap = jsh_overlap_passes(params, shape, npix * (uint64_t)n_nu);
   if (overlap && shape.overlap_key <= 0) shape.overlap_key = JSH_OVERLAP_KEY;
   shape.side = overlap ? ctx->side : nullptr;
@@ -573,7 +591,7 @@ extern "C" int jsh_plane_rays(jsh_ctx* ctx, const jsh_plane_desc* plane, double*
     st = keep_stats(ctx);
     if (st) return st;
     JshRequestLayout L;
-    jsh_request_layout(0, plane->n_along, plane->n_across, 1, JSH_PREC_FP64, false, &L);
+    jsh_request_layout(0, plane->n_along, plane->n_across, 1, false, false, &L);
     const size_t off_o = L.total;
     st = ensure_workspace(ctx, align_up(off_o + sizeof(double) * 3 * npix));
     if (st) return st;
@@ -621,7 +639,7 @@ extern "C" int jsh_trace_plane(jsh_ctx* ctx, const jsh_model_desc* model, const 
   req.npix = npix;
   req.n_nu = 0;  // the hit kernel writes no output planes
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, 1, JSH_PREC_FP64, false, &L);
+  jsh_request_layout(npix, plane->n_along, plane->n_across, 1, false, false, &L);
   st = keep_stats(ctx);
   if (st) return st;
   st = ensure_workspace(ctx, L.total);

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include <atomic>
 #include <mutex>
@@ -45,9 +46,9 @@ struct JshHullSlot {
 
 // Layout of one request's device memory inside an arena allocation.
 struct JshRequestLayout {
-  // [off_req, off_counters) comes from the host, [off_counters, off_across) starts at zero
-  size_t off_req, off_nu, off_fc, off_along_size, off_along_center, off_counters, off_nhit, off_queue, off_buckets,
-      off_iq_count, off_iq_buckets, off_across, off_hits, off_order, off_key, off_iq_items, off_iq_order,
+  // [off_counters, off_req) starts at zero, [off_req, off_across) comes from the host
+  size_t off_counters, off_nhit, off_queue, off_buckets, off_iq_count, off_iq_buckets, off_req, off_nu, off_fc,
+      off_along_size, off_along_center, off_across, off_hits, off_order, off_key, off_iq_items, off_iq_order,
       off_seg32, off_out[7];
   size_t total;
   bool own_outputs;
@@ -82,6 +83,7 @@ struct jsh_ctx {
   std::atomic<uint64_t> used{0};
   void* ws = nullptr;  // workspace of the blocking / device entry points
   size_t ws_cap = 0;
+  size_t ws_refused = SIZE_MAX;  // bytes that the device had no room for
   JshStage stages[JSH_STAGES];               // pinned staging of requests, in turn
   int next_stage = 0;
   unsigned long long* h_counters = nullptr;  // pinned [8]
@@ -132,8 +134,9 @@ class JshWorkspaceUse {
 // Helpers shared by the C-ABI translation units.
 int jsh_prepare_request(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_desc* plane,
                         const jsh_params* params, int32_t n_nu, JshRequest* req, uint64_t* npix);
-// (only mixed requests have the segments in FP32, 128 bytes a pixel)
-void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int32_t n_nu, int precision,
+// seg32: with the segments of the hits in FP32 (mixed precision, 128 bytes a
+// pixel); a request works without them where memory is short.
+void jsh_request_layout(uint64_t npix, uint64_t n_along, uint64_t n_across, int32_t n_nu, bool seg32,
                         bool own_outputs, JshRequestLayout* L);
 void jsh_bind_request(JshRequest* req, char* base, const JshRequestLayout& L, bool own_outputs);
 int jsh_alloc_device(jsh_ctx* ctx, size_t bytes, void** p);
@@ -160,13 +163,16 @@ int jsh_next_stage(jsh_ctx* ctx, const JshRequestLayout& L, JshStage** out);
 // counters, and run ray generation, all on `stream`.
 int jsh_upload_request(JshStage* stage, JshRequest* req, const JshRequestLayout& L, char* base, const double* nu,
                        cudaStream_t stream);
+// Whether the workspace holds `need` bytes or may grow to them within the budget.
+bool workspace_fits(const jsh_ctx* ctx, size_t need);
 // Grow the context workspace to `need` bytes (waits for its previous user).
 int ensure_workspace(jsh_ctx* ctx, size_t need);
 // Enqueue one request on `stream` in the context workspace; dev_out NULL
-// keeps the outputs in workspace-owned planes.  Called with ctx->mu held.
+// keeps the outputs in workspace-owned planes.  `layout`: the request's, in a
+// workspace that holds it (null: chosen here).  Called with ctx->mu held.
 int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_desc* plane, const double* nu_hz,
                    int32_t n_nu, const jsh_params* params, cudaStream_t stream, const jsh_image* dev_out,
-                   JshRequestLayout* L_out, uint64_t* npix_out);
+                   JshRequestLayout* L_out, uint64_t* npix_out, const JshRequestLayout* layout = nullptr);
 // SimulationGeometry: copy the context's view of hull model->hull_id into
 // the compiled model (JSH_ERR_NOT_FOUND for an unknown id); no-op for the
 // analytic geometries.  Called with ctx->mu held.

@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(128) transfer_static_mixed_kernel(const JshReq
   Tally T = tally_new();
   if (w < base[n_req]) {
     Lane L;
-    lane_start(L, reqs, base, n_req, w, false);
+    lane_start<PASS_BOTH>(L, reqs, base, n_req, w, false);
     while (L.phase != PH_IDLE) lane_advance<FULL, PASS_BOTH>(L, reqs, K, T);
   }
   tally_flush(T, reqs);
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? 3 : 1)
       if (b + (unsigned long long)nidle >= total) exhausted = true;
       if (L.phase == PH_IDLE) {
         unsigned long long w = b + (unsigned long long)__popc(idle & lt_mask);
-        if (w < total) lane_start(L, reqs, base, n_req, w, true);
+        if (w < total) lane_start<PASS_BOTH>(L, reqs, base, n_req, w, true);
       }
     }
     unsigned active = __ballot_sync(0xffffffffu, L.phase != PH_IDLE);

@@ -13,6 +13,7 @@
 #pragma once
 
 #include "jsh_model.h"
+#include "jsh_request.h"
 
 namespace jsh {
 
@@ -64,6 +65,27 @@ __device__ __forceinline__ V3 ray_point(V3 o, V3 d, double t) { return vadd(o, v
 struct Seg {
   V3 in, out;
 };
+// The FP32 pair of x (x - hi is exact).
+__device__ __forceinline__ void pair_of(double x, float* p) {
+  p[0] = (float)x;
+  p[1] = (float)sb(x, (double)p[0]);
+}
+// A segment for the mixed path.
+__device__ __forceinline__ JshSeg32 segment32(V3 in, V3 out) {
+  constexpr double inv_pc = 1.0 / JSH_PC;
+  const V3 d = vsub(out, in);
+  JshSeg32 q;
+  pair_of(ml(in.x, inv_pc), q.in);
+  pair_of(ml(in.y, inv_pc), q.in + 2);
+  pair_of(ml(in.z, inv_pc), q.in + 4);
+  pair_of(ml(out.x, inv_pc), q.out);
+  pair_of(ml(out.y, inv_pc), q.out + 2);
+  pair_of(ml(out.z, inv_pc), q.out + 4);
+  q.len_cm = sq(ad(ad(ml(d.x, d.x), ml(d.y, d.y)), ml(d.z, d.z)));
+  pair_of(ml(q.len_cm, inv_pc), q.len);
+  return q;
+}
+
 struct Hits {
   int n;
   uint32_t status;

@@ -65,12 +65,6 @@ __global__ void plane_across_kernel(const JshRequest* __restrict__ reqs) {
 }
 
 // ------------------------------------------------------------------ hit
-// The FP32 pair of x (x - hi is exact).
-__device__ __forceinline__ void pair_of(double x, float* p) {
-  p[0] = (float)x;
-  p[1] = (float)sb(x, (double)p[0]);
-}
-
 __global__ void hit_kernel(const JshRequest* __restrict__ reqs) {
   const JshRequest& R = reqs[blockIdx.y];
   const JshPlane& p = R.plane;
@@ -102,20 +96,7 @@ __global__ void hit_kernel(const JshRequest* __restrict__ reqs) {
     for (int s = 0; s < JSH_MAX_SEG; ++s) {
       if (s >= h.n) break;
       const Seg& S = h.s[s];
-      if (R.P.precision == JSH_PREC_MIXED) {
-        constexpr double inv_pc = 1.0 / JSH_PC;
-        const V3 d = vsub(S.out, S.in);
-        JshSeg32 q;
-        pair_of(ml(S.in.x, inv_pc), q.in);
-        pair_of(ml(S.in.y, inv_pc), q.in + 2);
-        pair_of(ml(S.in.z, inv_pc), q.in + 4);
-        pair_of(ml(S.out.x, inv_pc), q.out);
-        pair_of(ml(S.out.y, inv_pc), q.out + 2);
-        pair_of(ml(S.out.z, inv_pc), q.out + 4);
-        q.len_cm = sq(ad(ad(ml(d.x, d.x), ml(d.y, d.y)), ml(d.z, d.z)));
-        pair_of(ml(q.len_cm, inv_pc), q.len);
-        R.seg32[(uint64_t)slot * JSH_MAX_SEG + s] = q;
-      }
+      if (R.seg32) R.seg32[(uint64_t)slot * JSH_MAX_SEG + s] = segment32(S.in, S.out);
       H.seg[s][0] = S.in.x;
       H.seg[s][1] = S.in.y;
       H.seg[s][2] = S.in.z;

@@ -254,6 +254,22 @@ __device__ __forceinline__ float first_step_divisor(double tau_bg, int n) {
   return ceilf(fmaf(k * l, l, (float)n));
 }
 
+// Segment s of hit h: the hit kernel's record, or (ANY) computed here where the
+// request has no memory for them, with the same rounding, so the same images.
+// Such requests run in the static or the single-kernel form: the code costs the
+// split form's fused IQUV kernel 4 registers and a quarter of its warps.
+static __device__ __noinline__ void segment_of_hit(const JshHit& H, int s, JshSeg32* q) {
+  const double* p = H.seg[s];
+  *q = segment32(mk(p[0], p[1], p[2]), mk(p[3], p[4], p[5]));
+}
+template <bool ANY>
+__device__ __forceinline__ JshSeg32 segment_of(const JshRequest& R, uint32_t h, int s) {
+  if (!ANY || R.seg32) return R.seg32[(uint64_t)h * JSH_MAX_SEG + s];
+  JshSeg32 q;
+  segment_of_hit(R.hits[h], s, &q);
+  return q;
+}
+
 __device__ __forceinline__ void start_segment(Lane& L, DF px, DF py, DF pz, DF len) {
   L.length = len;
   L.t = DF{0.f, 0.f};
@@ -274,8 +290,9 @@ __device__ __forceinline__ double tau_total(const Lane& L) {
   return L.seg == 0 ? df_val(L.tau_seg) : L.tau_bg + df_val(L.tau_seg);
 }
 
+template <int PASS>
 __device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R, const JshMixed& X) {
-  const JshSeg32& S = R.seg32[(uint64_t)L.h * JSH_MAX_SEG + L.seg];
+  const JshSeg32 S = segment_of<PASS == PASS_BOTH>(R, L.h, L.seg);
   start_segment(L, DF{S.in[0], S.in[1]}, DF{S.in[2], S.in[3]}, DF{S.in[4], S.in[5]}, DF{S.len[0], S.len[1]});
   const float len = L.length.hi + L.length.lo;
   if (L.seg == 0) {
@@ -317,6 +334,7 @@ __device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R, 
   }
 }
 
+template <int PASS>
 __device__ __forceinline__ void begin_iquv_segment(Lane& L, const JshRequest& R) {
   const int s = L.seg;
   if (s == L.first_seg) {
@@ -329,7 +347,7 @@ __device__ __forceinline__ void begin_iquv_segment(Lane& L, const JshRequest& R)
     start_segment(L, df_of(ox * INV_PC), df_of(oy * INV_PC), df_of(oz * INV_PC),
                   df_of(seg_len_cm(H, s, ox, oy, oz) * INV_PC));
   } else {
-    const JshSeg32& S = R.seg32[(uint64_t)L.h * JSH_MAX_SEG + s];
+    const JshSeg32 S = segment_of<PASS == PASS_BOTH>(R, L.h, s);
     start_segment(L, DF{S.out[0], S.out[1]}, DF{S.out[2], S.out[3]}, DF{S.out[4], S.out[5]}, DF{S.len[0], S.len[1]});
   }
   L.dt = (L.length.hi + L.length.lo) / L.first_div;
@@ -342,6 +360,7 @@ __device__ __forceinline__ void begin_iquv_segment(Lane& L, const JshRequest& R)
 // Ranked (persistent schedule): all frequencies of a ray together, rays in
 // the heaviest-first order of the ranking kernels; part 1 (the rays after
 // the deep prefix of overlapped passes) starts after the deep prefix.
+template <int PASS>
 __device__ __forceinline__ void lane_start(Lane& L, const JshRequest* __restrict__ reqs,
                                            const unsigned long long* base, int n_req, unsigned long long w,
                                            bool ranked, int part = 0, const JshMixed* one = nullptr) {
@@ -374,7 +393,7 @@ __device__ __forceinline__ void lane_start(Lane& L, const JshRequest* __restrict
   L.ft = 0;
   L.ft_cool = 0;
   L.evals0 = 0;
-  begin_tau_segment(L, R, one ? *one : R.mix);
+  begin_tau_segment<PASS>(L, R, one ? *one : R.mix);
 }
 
 // Per-lane totals of a request's counters (right-hand-side evaluations,
@@ -699,7 +718,7 @@ __device__ __forceinline__ void lane_start_iquv(Lane& L, const JshRequest* __res
     L.x[2] = xe.z;
     L.x[3] = xe.w;
   }
-  begin_iquv_segment(L, R);
+  begin_iquv_segment<PASS_IQUV>(L, R);
 }
 
 // FP32 unit roundoff; the Stokes error norm's noise floor is
@@ -827,7 +846,7 @@ __device__ __forceinline__ void tau_pass_done(Lane& L, const JshRequest* __restr
     L.x[2] = xe.z;
     L.x[3] = xe.w;
   }
-  begin_iquv_segment(L, R);
+  begin_iquv_segment<PASS>(L, R);
 }
 
 // One panel of an active lane's tau pass (or a segment / pass transition).
@@ -1044,7 +1063,7 @@ __device__ __forceinline__ void tau_panel_step(Lane& L, const JshRequest* __rest
 segment_done : {
   if (L.seg + 1 < L.nseg) {
     L.seg++;
-    begin_tau_segment(L, R, X);
+    begin_tau_segment<PASS>(L, R, X);
     return;
   }
   tau_pass_done<PASS, GENERAL>(L, reqs, X, part, T, (grp.sub == 0));
@@ -1203,7 +1222,7 @@ __device__ __forceinline__ void tau_dopri_step(Lane& L, const JshRequest* __rest
 segment_done : {
   if (L.seg + 1 < L.nseg) {
     L.seg++;
-    begin_tau_segment(L, R, X);
+    begin_tau_segment<PASS>(L, R, X);
     return;
   }
   tau_pass_done<PASS, GENERAL>(L, reqs, X, part, T, (grp.sub == 0));
@@ -1634,7 +1653,7 @@ __device__ __forceinline__ void lane_step(Lane& L, const JshRequest* __restrict_
 segment_done : {
   if (L.seg > 0) {
     L.seg--;
-    begin_iquv_segment(L, R);
+    begin_iquv_segment<PASS>(L, R);
     return;
   }
   if (PASS == PASS_IQUV) {

@@ -153,7 +153,8 @@ extern "C" int jsh_observation_run_noalloc(const jsh_model_desc* model, const js
   st = jsh_prepare_request(nullptr, model, plane, params, n_nu, &in.req, &np);
   if (st) return st;
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, params->precision, false, &L);
+  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu,
+                     params->precision == JSH_PREC_MIXED, false, &L);
   const size_t state = L.total - (L.off_out[0] - L.off_seg32);
   if (state > JSH_NOALLOC_STATE_BYTES) {
     jsh_set_error("request needs %zu scratch bytes, more than the %u of the no-alloc array", state,
@@ -176,11 +177,11 @@ extern "C" int jsh_observation_run_noalloc(const jsh_model_desc* model, const js
   memcpy(in.nu, nu_hz, sizeof(double) * n_nu);
   cudaStream_t s = (cudaStream_t)cuda_stream;
   // counters, hit count, work queue and ranking buckets start at zero on
-  // every call (they lie between off_counters and off_across)
+  // every call (they lie between off_counters and off_req)
   noalloc_stage_kernel<<<1, 256, 0, s>>>(in, n_nu, (JshRequest*)(base + L.off_req), (double*)(base + L.off_nu),
                                          (JshFreqConst*)(base + L.off_fc), mixed,
                                          (unsigned long long*)(base + L.off_counters),
-                                         (unsigned)((L.off_across - L.off_counters) / 8));
+                                         (unsigned)((L.off_req - L.off_counters) / 8));
   JSH_CUDA_TRY(cudaGetLastError());
   const JshRequest* d_req = (const JshRequest*)(base + L.off_req);
   JSH_CUDA_TRY(jsh_launch_plane(d_req, 1, plane->n_along, s));

@@ -229,7 +229,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   }
   const bool split = !shape.single;
   const bool overlap = split && shape.overlap_key > 0 && shape.side != nullptr && shape.fork != nullptr;
-  if (max_hits > 0) jsh_launch_rank(d_reqs, n_req, max_hits, overlap ? shape.overlap_key : 0, stream);
+  if (max_hits > 0) jsh_launch_rank(d_reqs, n_req, max_hits, overlap ? shape.overlap_key : 0, split, stream);
   // queue counters: [0] tau (deep prefix or all) / single-kernel form, [1]
   // its IQUV kernel, [2] and [3] the other rays' tau and IQUV kernels
   unsigned long long* q = (unsigned long long*)queue;

@@ -121,7 +121,9 @@ struct JshRequest {
   JshConeRay cone_ray;    // of the plane's rays (jsh_prepare_hit)
   JshParamsDev P;
   JshHit* hits;           // device [npix] (first n_hit valid)
-  JshSeg32* seg32;        // device [npix][JSH_MAX_SEG], mixed precision: the hits' segments
+  // device [npix][JSH_MAX_SEG], mixed precision: the hits' segments; null
+  // where there was no memory for them (static and single-kernel forms only)
+  JshSeg32* seg32;
   // persistent mixed schedule: hit rays ranked by estimated cost, heaviest
   // first (order[rank] = hit index), their cost buckets and the ranking
   // state [JSH_RANK_WORDS] (zeroed with the counters)

@@ -186,11 +186,16 @@ int prepare_request(jsh_server* S, Request* q) {
   int st = jsh_prepare_request(S->ctx, &q->model, &q->plane, &q->params, (int32_t)q->nu.size(), &q->rec, &npix);
   if (st) return st;
   q->npix = npix;
-  jsh_request_layout(npix, q->plane.n_along, q->plane.n_across, (int32_t)q->nu.size(), q->params.precision, true,
-                     &q->L);
   // the record, counters, n_hit, queue, nu and fc live in the slot's control
   // block; the arena block holds the tables, the hit list and the outputs
-  q->arena_bytes = q->L.total - q->L.off_along_size;
+  // (without the segments in FP32 where the arena would not hold them)
+  auto lay = [&](bool seg32) {
+    jsh_request_layout(npix, q->plane.n_along, q->plane.n_across, (int32_t)q->nu.size(), seg32, true, &q->L);
+    q->arena_bytes = q->L.total - q->L.off_along_size;
+  };
+  const bool mixed = q->params.precision == JSH_PREC_MIXED;
+  lay(mixed);
+  if (mixed && q->arena_bytes > S->arena_bytes) lay(false);
   q->fc.resize(q->nu.size());
   if (q->params.precision == JSH_PREC_MIXED) {
     st = jsh_prepare_mixed(&q->rec, q->nu.data(), q->fc.data());
@@ -227,7 +232,7 @@ void bind_empty(Slot& sl, int i) {
 }
 
 // Enqueue (or capture) the launch sequence of slot `sl` for `n_req` records.
-cudaError_t enqueue_slot(jsh_server* S, Slot& sl, int n_req, bool full, bool fused, bool ft) {
+cudaError_t enqueue_slot(jsh_server* S, Slot& sl, int n_req, bool full, bool fused, bool ft, bool single = false) {
   cudaStream_t st = sl.stream;
   const JshRequest* d_recs = (const JshRequest*)sl.dev;
   cudaError_t e = cudaMemcpyAsync(sl.dev, sl.host, sizeof(SlotHost), cudaMemcpyHostToDevice, st);
@@ -241,6 +246,7 @@ cudaError_t enqueue_slot(jsh_server* S, Slot& sl, int n_req, bool full, bool fus
   JshLaunchShape shape = S->ctx->shape;
   shape.fused = fused ? 1 : 0;
   shape.faraday_thick = ft ? 1 : 0;
+  if (single) shape.single = 1;
   unsigned int* queue = (unsigned int*)(sl.dev + sl.counters_off + sl.counters_bytes - 256);
   e = jsh_launch_transfer(d_recs, n_req, S->cfg.precision, JSH_SCHED_PERSISTENT, full,
                           S->cap_pix * (uint64_t)S->cap_nu * (uint64_t)n_req, S->cap_pix, shape, queue,
@@ -286,12 +292,15 @@ int launch_batch(jsh_server* S, Slot& sl) {
   const bool ft = full && S->cfg.precision == JSH_PREC_MIXED &&
                   (sl.batch[0]->params.flags & JSH_FLAG_FARADAY_THICK) != 0;
   cudaError_t e = cudaSuccess;
-  if (S->cfg.use_graphs) {
+  // a request that only fits the arena without its segments in FP32
+  bool single = false;
+  for (int i = 0; i < n; ++i) single = single || (S->cfg.precision == JSH_PREC_MIXED && !sl.host->recs[i].seg32);
+  if (S->cfg.use_graphs && !single) {
     cudaGraphExec_t& gx = sl.graph[full ? 1 : 0][fused ? 1 : 0][ft ? 1 : 0];
     if (!gx) e = build_graph(S, sl, full, fused, ft);  // the mode's graphs: on first use (the slot is idle)
     if (e == cudaSuccess) e = cudaGraphLaunch(gx, sl.stream);
   } else {
-    e = enqueue_slot(S, sl, cap, full, fused, ft);
+    e = enqueue_slot(S, sl, cap, full, fused, ft, single);
   }
   if (e != cudaSuccess) goto fail;
   e = cudaEventRecord(sl.done, sl.stream);

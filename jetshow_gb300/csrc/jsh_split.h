@@ -26,8 +26,9 @@ struct TauLaunch {
 TauLaunch jsh_tau_kernel(bool fused, bool groups, bool one);
 
 // Heaviest-first order of every request's hit rays; deep_key as
-// rank_prefix_kernel.
-void jsh_launch_rank(const JshRequest* d_reqs, int n_req, uint64_t max_hits, int deep_key, cudaStream_t stream);
+// rank_prefix_kernel; seg32: all of them have their segments in FP32.
+void jsh_launch_rank(const JshRequest* d_reqs, int n_req, uint64_t max_hits, int deep_key, bool seg32,
+                     cudaStream_t stream);
 
 // Heaviest-first order of the items the tau kernel handed on (max_items: the
 // batch's bound, the same for each of its requests).

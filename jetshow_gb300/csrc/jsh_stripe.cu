@@ -121,7 +121,7 @@ extern "C" int jsh_observation_run_stripe(jsh_ctx* ctx, const jsh_model_desc* mo
   if (st) return st;
   const uint64_t count = plane->n_along - plane->n_along / 2;
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, 1, JSH_PREC_FP64, false, &L);
+  jsh_request_layout(npix, plane->n_along, plane->n_across, 1, false, false, &L);
   const size_t off_out = (L.total + 255) / 256 * 256;
   st = keep_stats(ctx);
   if (st) return st;

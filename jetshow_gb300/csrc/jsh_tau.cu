@@ -22,6 +22,7 @@ namespace {
 // order; the queue then hands out the heaviest rays first and they run while
 // the bulk fills the GPU, instead of starting late and setting the render's
 // makespan.
+template <bool ANY>
 __global__ void __launch_bounds__(256) rank_cost_kernel(const JshRequest* __restrict__ reqs) {
   __shared__ uint32_t hist[JSH_RANK_BUCKETS];
   const JshRequest& R = reqs[blockIdx.y];
@@ -35,7 +36,7 @@ __global__ void __launch_bounds__(256) rank_cost_kernel(const JshRequest* __rest
     const float wk[4] = {0.173927423f, 0.326072577f, 0.326072577f, 0.173927423f};
     float tau = 0.f;
     for (int s = 0; s < H.nseg && s < 2; ++s) {
-      const JshSeg32& S = R.seg32[(uint64_t)h * JSH_MAX_SEG + s];
+      const JshSeg32 S = segment_of<ANY>(R, h, s);
       const F3 a = f3(S.in[0], S.in[2], S.in[4]), b = f3(S.out[0], S.out[2], S.out[4]);
       const F3 d = b - a;
       float acc = 0.f;
@@ -143,7 +144,7 @@ __global__ void __launch_bounds__(256, 3)
   Tally T = tally_new();
   const unsigned long long total = base[n_req];
   auto start = [&](unsigned long long w) {
-    lane_start(L, reqs, base, n_req, w, true, part, ONE ? &mix : nullptr);
+    lane_start<PASS_TAU>(L, reqs, base, n_req, w, true, part, ONE ? &mix : nullptr);
   };
   if (on_groups(total, kTauGroupsFused)) {
     const LaneGroup grp = lane_group();
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(128, 4)
   float* K = ksh + (GROUPS ? group_slot(grp) : (int)threadIdx.x) * kTauWords;
   run_queue(
       L, queue, base[n_req], refill, grp, GROUPS, false, 0,
-      [&](unsigned long long w) { lane_start(L, reqs, base, n_req, w, true, part); },
+      [&](unsigned long long w) { lane_start<PASS_TAU>(L, reqs, base, n_req, w, true, part); },
       [&] { tau_step<PASS_TAU, true, 0>(L, reqs, reqs[L.r].mix, K, part, T, grp); });
   tally_flush(T, reqs);
 }
@@ -253,9 +254,11 @@ TauLaunch jsh_tau_kernel(bool fused, bool groups, bool one) {
                    sizeof(float) * kTauWords * (groups ? 128 / 32 * kWarpGroups : 128)};
 }
 
-void jsh_launch_rank(const JshRequest* d_reqs, int n_req, uint64_t max_hits, int deep_key, cudaStream_t stream) {
+void jsh_launch_rank(const JshRequest* d_reqs, int n_req, uint64_t max_hits, int deep_key, bool seg32,
+                     cudaStream_t stream) {
   const dim3 g((unsigned)((max_hits + 255) / 256), (unsigned)n_req);
-  rank_cost_kernel<<<g, 256, 0, stream>>>(d_reqs);
+  if (seg32) rank_cost_kernel<false><<<g, 256, 0, stream>>>(d_reqs);
+  else rank_cost_kernel<true><<<g, 256, 0, stream>>>(d_reqs);
   rank_prefix_kernel<<<n_req, 32, 0, stream>>>(d_reqs, deep_key);
   rank_scatter_kernel<<<g, 256, 0, stream>>>(d_reqs);
 }

@@ -85,14 +85,14 @@ __global__ void vis_columns_kernel(const double* __restrict__ along_size, const 
   ycol[j] = along_center[j] * rad_per_cm;
 }
 
-// The rotated (u, v) of each point and its shift factor exp(-2 pi i (u dx + v dy)).
-__global__ void vis_points_kernel(const double* __restrict__ uv, int64_t n, double cr, double sr, double dx, double dy,
-                                  double* __restrict__ uvr, double* __restrict__ shift) {
+// Rotates each (u, v) point in place; and its shift factor exp(-2 pi i (u dx + v dy)).
+__global__ void vis_points_kernel(double* uv, int64_t n, double cr, double sr, double dx, double dy,
+                                  double* __restrict__ shift) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const double u = uv[2 * t], v = uv[2 * t + 1];
-  uvr[2 * t] = u * cr + v * sr;
-  uvr[2 * t + 1] = -u * sr + v * cr;
+  uv[2 * t] = u * cr + v * sr;
+  uv[2 * t + 1] = -u * sr + v * cr;
   double s, c;
   sincos(-2.0 * JSH_PI * (u * dx + v * dy), &s, &c);
   shift[2 * t] = c;
@@ -271,44 +271,48 @@ extern "C" int jsh_observation_visibilities(jsh_ctx* ctx, const jsh_model_desc* 
   const uint64_t npix = plane->n_across * plane->n_along;
   const int n_across = (int)plane->n_across, n_along = (int)plane->n_along;
   const int rows_pad = (n_across + kRows - 1) / kRows * kRows;
+  const unsigned gx = (unsigned)((n_uv + kVisThreads - 1) / kVisThreads);
   // the render's own layout, then the visibility buffers behind it
   JshRequestLayout L;
-  jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, params->precision, true, &L);
-  const size_t o_w = up256(L.total);
-  const size_t o_col = up256(o_w + sizeof(float) * (size_t)n_nu * n_along * rows_pad);
-  const size_t o_y = up256(o_col + sizeof(double) * n_along);
-  const size_t o_uv = up256(o_y + sizeof(double) * n_along);
-  const size_t o_uvr = up256(o_uv + sizeof(double) * 2 * (size_t)n_nu * n_uv);
-  const size_t o_shift = up256(o_uvr + sizeof(double) * 2 * (size_t)n_nu * n_uv);
-  const size_t o_part = up256(o_shift + sizeof(double) * 2 * (size_t)n_nu * n_uv);
-  const unsigned gx = (unsigned)((n_uv + kVisThreads - 1) / kVisThreads);
+  size_t o_w, o_col, o_y, o_uv, o_shift, o_part, o_out;
+  int cols, n_split;
+  auto lay = [&](bool seg32, int ctas_per_sm) {
+    jsh_request_layout(npix, plane->n_along, plane->n_across, n_nu, seg32, true, &L);
+    o_w = up256(L.total);
+    o_col = up256(o_w + sizeof(float) * (size_t)n_nu * n_along * rows_pad);
+    o_y = up256(o_col + sizeof(double) * n_along);
+    o_uv = up256(o_y + sizeof(double) * n_along);
+    o_shift = up256(o_uv + sizeof(double) * 2 * (size_t)n_nu * n_uv);
+    o_part = up256(o_shift + sizeof(double) * 2 * (size_t)n_nu * n_uv);
+    n_split = 1;
+    if (gx > 0) {
+      const int64_t want = (int64_t)ctas_per_sm * ctx->num_sms;
+      n_split = (int)std::min<int64_t>(std::max<int64_t>(1, (want + gx * n_nu - 1) / (gx * (int64_t)n_nu)), n_along);
+    }
+    cols = (n_along + n_split - 1) / n_split;
+    n_split = (n_along + cols - 1) / cols;
+    o_out = up256(o_part + sizeof(double) * 2 * (size_t)n_split * n_nu * n_uv);
+    return up256(o_out + sizeof(double) * 2 * (size_t)n_nu * n_uv);
+  };
   // split the columns so that about 16 CTAs per SM share the work (about 5 are
-  // in flight; the columns differ in their nonzero rows)
-  int n_split = 1;
-  if (gx > 0) {
-    const int64_t want = 16LL * ctx->num_sms;
-    n_split = (int)std::min<int64_t>(std::max<int64_t>(1, (want + gx * n_nu - 1) / (gx * (int64_t)n_nu)), n_along);
-  }
-  const int cols = (n_along + n_split - 1) / n_split;
-  n_split = (n_along + cols - 1) / cols;
-  const size_t o_out = up256(o_part + sizeof(double) * 2 * (size_t)n_split * n_nu * n_uv);
-  const size_t total = up256(o_out + sizeof(double) * 2 * (size_t)n_nu * n_uv);
-  int st = ensure_workspace(ctx, total);
+  // in flight; the columns differ in their nonzero rows); where memory is
+  // short, without the segments in FP32 and with fewer splits' partial sums
+  const bool mixed = params->precision == JSH_PREC_MIXED;
+  int st = workspace_fits(ctx, lay(mixed, 16)) ? ensure_workspace(ctx, lay(mixed, 16)) : JSH_ERR_OOM;
+  if (st == JSH_ERR_OOM) st = ensure_workspace(ctx, lay(false, 4));
   if (st) return st;
   cudaStream_t s = ctx->stream;
   JSH_CUDA_TRY(cudaEventRecord(ctx->ev_start, s));
-  JshRequestLayout L2;
-  uint64_t np2 = 0;
-  st = enqueue_single(ctx, model, plane, nu_hz, n_nu, params, s, nullptr, &L2, &np2);
+  st = enqueue_single(ctx, model, plane, nu_hz, n_nu, params, s, nullptr, nullptr, nullptr, &L);
   if (st) return st;
   JshWorkspaceUse use(ctx, s);
   char* base = (char*)ctx->ws;
   if (n_uv > 0) {
     const int64_t nv = (int64_t)n_nu * n_uv;
     JSH_CUDA_TRY(cudaMemcpyAsync(base + o_uv, uv, sizeof(double) * 2 * nv, cudaMemcpyHostToDevice, s));
-    vis_points_kernel<<<(unsigned)((nv + 127) / 128), 128, 0, s>>>((const double*)(base + o_uv), nv, cos(vis->rot),
+    vis_points_kernel<<<(unsigned)((nv + 127) / 128), 128, 0, s>>>((double*)(base + o_uv), nv, cos(vis->rot),
                                                                    sin(vis->rot), vis->dx, vis->dy,
-                                                                   (double*)(base + o_uvr), (double*)(base + o_shift));
+                                                                   (double*)(base + o_shift));
     JSH_CUDA_TRY(cudaMemsetAsync(base + o_w, 0, sizeof(float) * (size_t)n_nu * n_along * rows_pad, s));
     const double* I = (const double*)(base + L.off_out[2]);
     const double* asz = (const double*)(base + L.off_along_size);
@@ -326,7 +330,7 @@ extern "C" int jsh_observation_visibilities(jsh_ctx* ctx, const jsh_model_desc* 
       JSH_CUDA_TRY(cudaFuncSetAttribute(vis_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileBytes));
     vis_sum_kernel<<<dim3(gx, (unsigned)n_split, (unsigned)n_nu), kVisThreads, smem, s>>>(
         (const float*)(base + o_w), (const double*)(base + o_col), (const double*)(base + o_y),
-        (const double*)(base + o_uvr), n_uv, n_along, rows_pad, 0.5 * (double)(n_across - 1), cols, col_tile,
+        (const double*)(base + o_uv), n_uv, n_along, rows_pad, 0.5 * (double)(n_across - 1), cols, col_tile,
         (double*)(base + o_part));
     vis_reduce_kernel<<<(unsigned)((nv + 255) / 256), 256, 0, s>>>((const double*)(base + o_part),
                                                                    (const double*)(base + o_shift), n_split, n_nu,
