@@ -404,7 +404,10 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
   const int32_t nbx = std::max(1, (int32_t)std::ceil(ex / h)), nby = std::max(1, (int32_t)std::ceil(ey / h));
   const int64_t nbk = (int64_t)nbx * nby;
   const double coord = std::max(std::max(std::fabs(x0), std::fabs(x1)), std::max(std::fabs(y0), std::fabs(y1)));
-  const double margin = 0.01 * h + 16.0 * 5.9604645e-8 * coord;
+  // (the rounding by half a bucket at most: far from the origin, z in [1e5,
+  // 1e5 + 1] pc, it is above the buckets' sides, an FP32 coordinate cannot tell
+  // them apart, and every triangle would be listed in thousands of them)
+  const double margin = 0.01 * h + std::min(16.0 * 5.9604645e-8 * coord, 0.5 * h);
   // visit(t, b) for the buckets of triangle t, in the order of t
   auto for_buckets = [&](auto visit) {
     for (int64_t t = 0; t < n_tri; ++t) {
