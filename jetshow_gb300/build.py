@@ -25,7 +25,7 @@ LIB = os.path.join(OUT, "libjetshow_gb300.so")
 
 CU_SOURCES = ["jsh_persistent.cu", "jsh_persistent_ft.cu", "jsh_forms.cu", "jsh_forms_ft.cu", "jsh_tau.cu", "jsh_fp64.cu",
               "jsh_kernels.cu", "jsh_noalloc.cu", "jsh_stripe.cu", "jsh_visibility.cu"]
-CPP_SOURCES = ["jsh_host.cpp", "jsh_capi.cpp", "jsh_server.cpp", "jsh_autotune.cpp", "jsh_grid.cpp", "jsh_hull.cpp", "jsh_cells.cpp"]
+CPP_SOURCES = ["jsh_host.cpp", "jsh_capi.cpp", "jsh_server.cpp", "jsh_autotune.cpp", "jsh_grid.cpp", "jsh_grid_index.cpp", "jsh_hull.cpp", "jsh_cells.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # Units whose kernels must round identically in every instantiation: the
 # mixed-precision lane machine runs in several kernels (static, single

@@ -25,11 +25,13 @@
 
 #include <algorithm>
 #include <cmath>
+#include <new>
 #include <numeric>
 #include <unordered_map>
 #include <vector>
 
 #include "jsh_context.h"
+#include "jsh_grid_index.h"
 #include "jsh_launch.h"
 
 namespace {
@@ -376,107 +378,18 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
       jsh_set_error("triangle vertex index %d out of range", tri[i]);
       return JSH_ERR_INVALID;
     }
-  double x0 = xy[0], x1 = xy[0], y0 = xy[1], y1 = xy[1];
-  for (int64_t i = 1; i < n; ++i) {
-    x0 = std::min(x0, xy[2 * i]);
-    x1 = std::max(x1, xy[2 * i]);
-    y0 = std::min(y0, xy[2 * i + 1]);
-    y1 = std::max(y1, xy[2 * i + 1]);
+  // 403 278 triangles take 14 ms on 16 Arm cores, 12 of them the index (with a
+  // serial index of two passes over the triangles 85 ms, with lists by bounding
+  // boxes and no records 20 ms)
+  JshGridIndex X;
+  int st = JSH_OK;
+  try {
+    st = jsh_grid_index(xy, n, tri, n_tri, &X);
+  } catch (const std::bad_alloc&) {
+    jsh_set_error("no host memory for the index of %lld triangles", (long long)n_tri);
+    st = JSH_ERR_OOM;
   }
-  if (!std::isfinite(x0) || !std::isfinite(x1) || !std::isfinite(y0) || !std::isfinite(y1)) {
-    jsh_set_error("grid points must be finite");
-    return JSH_ERR_INVALID;
-  }
-  // square buckets, about two per triangle (one for two triangles from 2^26 on);
-  // a triangle is listed in every bucket that it touches, the bucket grown so
-  // that FP32 lookups near an edge still find it: by a hundredth of its side
-  // and by the rounding of the coordinates.  A lookup outside its hint's
-  // triangle is a chain of loads, a bucket and its triangles two at a time:
-  // with half a bucket per triangle, listed by bounding boxes, about 10
-  // triangles a bucket, read one after another through a list, instead of the
-  // 3 to 4 here, a 256^2 render of a 200 000 point grid took 25.2 + 17.3
-  // ms (tau, IQUV kernel), now 19.8 + 15.2; 512^2 76 + 55, now 48 + 44.
-  const double ex = x1 - x0, ey = y1 - y0;
-  const double n_buckets = std::max((double)n_tri / 2.0, std::min(2.0 * (double)n_tri, 67108864.0));
-  double h = std::sqrt(std::max(ex * ey, 1e-300) / std::max(1.0, n_buckets));
-  if (!(h > 0) || !std::isfinite(h)) h = std::max(std::max(ex, ey), 1.0);
-  h = std::max(h, std::max(ex, ey) / 65536.0);  // at most 65536 buckets per side
-  const int32_t nbx = std::max(1, (int32_t)std::ceil(ex / h)), nby = std::max(1, (int32_t)std::ceil(ey / h));
-  const int64_t nbk = (int64_t)nbx * nby;
-  const double coord = std::max(std::max(std::fabs(x0), std::fabs(x1)), std::max(std::fabs(y0), std::fabs(y1)));
-  // (the rounding by half a bucket at most: far from the origin, z in [1e5,
-  // 1e5 + 1] pc, it is above the buckets' sides, an FP32 coordinate cannot tell
-  // them apart, and every triangle would be listed in thousands of them)
-  const double margin = 0.01 * h + std::min(16.0 * 5.9604645e-8 * coord, 0.5 * h);
-  // visit(t, b) for the buckets of triangle t, in the order of t
-  auto for_buckets = [&](auto visit) {
-    for (int64_t t = 0; t < n_tri; ++t) {
-      double px[3], py[3];
-      for (int k = 0; k < 3; ++k) {
-        px[k] = xy[2 * (int64_t)tri[3 * t + k]] - x0;
-        py[k] = xy[2 * (int64_t)tri[3 * t + k] + 1] - y0;
-      }
-      const double bx0 = std::min(px[0], std::min(px[1], px[2])), bx1 = std::max(px[0], std::max(px[1], px[2]));
-      const double by0 = std::min(py[0], std::min(py[1], py[2])), by1 = std::max(py[0], std::max(py[1], py[2]));
-      const int32_t i0 = std::max(0, (int32_t)std::floor((bx0 - margin) / h)),
-                    i1 = std::min(nbx - 1, (int32_t)std::floor((bx1 + margin) / h)),
-                    j0 = std::max(0, (int32_t)std::floor((by0 - margin) / h)),
-                    j1 = std::min(nby - 1, (int32_t)std::floor((by1 + margin) / h));
-      // edge normals, outwards (none for a triangle without area: its box)
-      const double area = (px[1] - px[0]) * (py[2] - py[0]) - (py[1] - py[0]) * (px[2] - px[0]);
-      double nx[3], ny[3], limit[3];
-      for (int k = 0; k < 3; ++k) {
-        const int l = (k + 1) % 3;
-        const double sgn = area > 0 ? 1.0 : area < 0 ? -1.0 : 0.0;
-        nx[k] = sgn * (py[l] - py[k]);
-        ny[k] = sgn * (px[k] - px[l]);
-        // beyond the edge by more than half a bucket (with its margin) either way
-        limit[k] = nx[k] * px[k] + ny[k] * py[k] + (0.5 * h + margin) * (std::fabs(nx[k]) + std::fabs(ny[k]));
-      }
-      for (int32_t j = j0; j <= j1; ++j)
-        for (int32_t i = i0; i <= i1; ++i) {
-          const double cx = (i + 0.5) * h, cy = (j + 0.5) * h;
-          bool apart = false;
-          for (int k = 0; k < 3; ++k) apart = apart || nx[k] * cx + ny[k] * cy > limit[k];
-          // points beyond the last bucket's end are looked up in it
-          if (!apart || i == nbx - 1 || j == nby - 1) visit(t, (int64_t)j * nbx + i);
-        }
-    }
-  };
-  // heads of 7 ids, the longer lists' other ids with a -1 after each list
-  std::vector<int32_t> head((size_t)nbk * 8, -1), count((size_t)nbk, 0);
-  for_buckets([&](int64_t, int64_t b) { ++count[(size_t)b]; });
-  size_t n_more = 0;
-  for (int64_t b = 0; b < nbk; ++b)
-    if (count[(size_t)b] > 7) {
-      if (n_more > (size_t)INT32_MAX - (size_t)count[(size_t)b]) {
-        jsh_set_error("grid too large");
-        return JSH_ERR_INVALID;
-      }
-      head[(size_t)b * 8 + 7] = (int32_t)n_more;
-      n_more += (size_t)count[(size_t)b] - 7 + 1;
-    }
-  std::vector<int32_t> more(n_more, -1);
-  std::fill(count.begin(), count.end(), 0);
-  for_buckets([&](int64_t t, int64_t b) {
-    const int32_t c = count[(size_t)b]++;
-    int32_t* hd = &head[(size_t)b * 8];
-    (c < 7 ? hd[c] : more[(size_t)hd[7] + (size_t)(c - 7)]) = (int32_t)t;
-  });
-  // triangle records: the FP32 operations here round as the device's would
-  std::vector<float> rec((size_t)12 * n_tri);
-  for (int64_t t = 0; t < n_tri; ++t) {
-    float* r = &rec[(size_t)12 * t];
-    for (int k = 0; k < 3; ++k) {
-      r[2 * k] = (float)xy[2 * (int64_t)tri[3 * t + k]];
-      r[2 * k + 1] = (float)xy[2 * (int64_t)tri[3 * t + k] + 1];
-    }
-    r[6] = r[4] - r[0];
-    r[7] = r[5] - r[1];
-    const float area = (r[2] - r[0]) * r[7] - (r[3] - r[1]) * r[6];
-    r[8] = area == 0.f ? NAN : 1.f / area;
-    memcpy(r + 9, tri + 3 * t, 3 * sizeof(int32_t));
-  }
+  if (st) return st;
 
   std::lock_guard<std::mutex> lk(ctx->mu);
   int id = -1;
@@ -489,23 +402,23 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   // a point's fields in whole float4 (the lookups of four fields take one load a vertex)
   const int32_t stride = (n_fields + 3) / 4 * 4;
-  const size_t o_xy = 0, o_rec = o_xy + al(sizeof(double) * 2 * n), o_val = o_rec + al(sizeof(float) * rec.size()),
+  const size_t o_xy = 0, o_rec = o_xy + al(sizeof(double) * 2 * n), o_val = o_rec + al(X.rec.bytes()),
                o_tri = o_val + al(sizeof(float) * (size_t)n * stride), o_bs = o_tri + al(sizeof(int32_t) * 3 * n_tri),
-               o_bi = o_bs + al(sizeof(int32_t) * head.size()), total = o_bi + al(sizeof(int32_t) * more.size());
+               o_bi = o_bs + al(X.head.bytes()), total = o_bi + al(X.more.bytes());
   JSH_CUDA_TRY(cudaSetDevice(ctx->device));
   void* mem = nullptr;
-  int st = jsh_alloc_device(ctx, total, &mem);
+  st = jsh_alloc_device(ctx, total, &mem);
   if (st) return st;
   char* base = (char*)mem;
   cudaError_t e = cudaMemcpy(base + o_xy, xy, sizeof(double) * 2 * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(base + o_rec, rec.data(), sizeof(float) * rec.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(base + o_rec, X.rec.p.get(), X.rec.bytes(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy2D(base + o_val, sizeof(float) * stride, values, sizeof(float) * n_fields, sizeof(float) * n_fields,
                      (size_t)n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(base + o_tri, tri, sizeof(int32_t) * 3 * n_tri, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(base + o_bs, head.data(), sizeof(int32_t) * head.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && !more.empty())
-    e = cudaMemcpy(base + o_bi, more.data(), sizeof(int32_t) * more.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(base + o_bs, X.head.p.get(), X.head.bytes(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && X.more.n)
+    e = cudaMemcpy(base + o_bi, X.more.p.get(), X.more.bytes(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     jsh_free_device(ctx, mem, total);
     jsh_set_error("grid upload failed: %s", cudaGetErrorString(e));
@@ -525,14 +438,14 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
   G.n_tri = n_tri;
   G.n_fields = n_fields;
   G.stride = stride;
-  G.nbx = nbx;
-  G.nby = nby;
-  G.x0 = x0;
-  G.y0 = y0;
-  G.h = h;
-  G.x0f = (float)x0;
-  G.y0f = (float)y0;
-  G.inv_hf = (float)(1.0 / h);
+  G.nbx = X.nbx;
+  G.nby = X.nby;
+  G.x0 = X.x0;
+  G.y0 = X.y0;
+  G.h = X.h;
+  G.x0f = (float)X.x0;
+  G.y0f = (float)X.y0;
+  G.inv_hf = (float)(1.0 / X.h);
   S.used.store(true, std::memory_order_release);
   *grid_id = id;
   return JSH_OK;
