@@ -113,6 +113,32 @@ __device__ inline GridW grid_locate32(const JshGrid& G, float px, float py) {
   if (G.n_tri > 0) grid_search32(G, grid_bucket32(G, px, py), px, py, g);
   return g;
 }
+// A lean grid (where memory is short): the same triangle, its record formed from
+// the vertices with the host's operations.
+__device__ __forceinline__ GridW grid_locate_lean32(const JshGrid& G, float px, float py) {
+  GridW g;
+  g.ok = false;
+  const float fx = (px - G.x0f) * G.inv_hf, fy = (py - G.y0f) * G.inv_hf;
+  if (!(fx >= 0.f && fy >= 0.f)) return g;
+  const int32_t* head = G.bhead + 8 * ((int64_t)min((int)fy, G.nby - 1) * G.nbx + min((int)fx, G.nbx - 1));
+#pragma unroll 1
+  for (int q = 0;; ++q) {
+    if (q == 7 && head[7] < 0) break;
+    const int t = q < 7 ? head[q] : G.bmore[head[7] + (q - 7)];
+    if (t < 0) break;
+    const int32_t* v = G.tri + 3 * (int64_t)t;
+    const double2* xy = reinterpret_cast<const double2*>(G.xy);
+    const double2 a = xy[v[0]], b = xy[v[1]], c = xy[v[2]];
+    GridTri T;
+    T.ab = make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
+    T.ce = make_float4((float)c.x, (float)c.y, (float)c.x - T.ab.x, (float)c.y - T.ab.y);
+    const float area = (T.ab.z - T.ab.x) * T.ce.w - (T.ab.w - T.ab.y) * T.ce.z;
+    if (area == 0.f) continue;
+    T.iv = make_float4(1.f / area, __int_as_float(v[0]), __int_as_float(v[1]), __int_as_float(v[2]));
+    if (grid_tri_in(T, px, py, g)) break;
+  }
+  return g;
+}
 
 // The lanes that run one item together: one, or a group of kGroupLanes.
 struct LaneGroup {
@@ -207,16 +233,18 @@ __device__ __forceinline__ float grid_val32(const JshGrid& G, const GridW& g, in
 // 36.0 + 26.2 ms (tau, IQUV kernel) to 25.0 + 17.5, 512^2 from 114 + 96 to 76
 // + 55 (by later lookups 48 + 44); 415 968 items of a radial field from 1.53 + 1.78 to 1.36 + 1.08.
 static __device__ __noinline__ float sim32(const JshGrid& G, int field, F3 p, float nan_value) {
-  return grid_val32(G, grid_locate32(G, p.z, sqrtf(p.x * p.x + p.y * p.y)), field, nan_value);
+  const float rc = sqrtf(p.x * p.x + p.y * p.y);
+  return grid_val32(G, G.rec ? grid_locate32(G, p.z, rc) : grid_locate_lean32(G, p.z, rc), field, nan_value);
 }
 
 // The simulation workload's four fields from their one grid: Gamma, n, B_p and
-// B_phi at (z, rc) by one point location.
+// B_phi at (z, rc) by one point location (in a lean grid without a hint, and so,
+// point by point, the same on a lane and on a group).
 static __device__ __noinline__ float4 sim_shared32(const JshModel& m, float z, float rc, int* hint, LaneGroup group) {
   const JshGrid& G = m.grids[0];
-  const GridW g = grid_locate32_group(G, z, rc, hint, group);
+  const GridW g = G.rec ? grid_locate32_group(G, z, rc, hint, group) : grid_locate_lean32(G, z, rc);
   const int q = m.f_v >> 2;
-  if (!g.ok || (m.f_n >> 2) != q || (m.fb_p >> 2) != q || (m.fb_phi >> 2) != q)
+  if (!g.ok || !G.rec || (m.f_n >> 2) != q || (m.fb_p >> 2) != q || (m.fb_phi >> 2) != q)
     return make_float4(grid_val32(G, g, m.f_v, 1.0f), grid_val32(G, g, m.f_n, 0.f), grid_val32(G, g, m.fb_p, 0.f),
                        grid_val32(G, g, m.fb_phi, 0.f));
   // all four in one float4 of a point's row: 3 loads for 12, of as many sectors

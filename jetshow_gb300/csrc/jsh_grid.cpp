@@ -381,37 +381,53 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
   // 403 278 triangles take 14 ms on 16 Arm cores, 12 of them the index (with a
   // serial index of two passes over the triangles 85 ms, with lists by bounding
   // boxes and no records 20 ms)
-  JshGridIndex X;
-  int st = JSH_OK;
-  try {
-    st = jsh_grid_index(xy, n, tri, n_tri, &X);
-  } catch (const std::bad_alloc&) {
-    jsh_set_error("no host memory for the index of %lld triangles", (long long)n_tri);
-    st = JSH_ERR_OOM;
-  }
-  if (st) return st;
-
-  std::lock_guard<std::mutex> lk(ctx->mu);
-  int id = -1;
-  for (int g = 0; g < JSH_MAX_GRIDS && id < 0; ++g)
-    if (!ctx->grids[g].used) id = g;
-  if (id < 0) {
-    jsh_set_error("all %d grid slots are in use", JSH_MAX_GRIDS);
-    return JSH_ERR_INVALID;
-  }
+  //
+  // The full index and the fields in whole float4 (the lookups of four fields
+  // take one load a vertex) where they take at most a thirty-second of what the
+  // budget has left; else, or where the device has no room for them, the lean
+  // one, so that a budget that held the grid and its renders still does.
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-  // a point's fields in whole float4 (the lookups of four fields take one load a vertex)
-  const int32_t stride = (n_fields + 3) / 4 * 4;
-  const size_t o_xy = 0, o_rec = o_xy + al(sizeof(double) * 2 * n), o_val = o_rec + al(X.rec.bytes()),
-               o_tri = o_val + al(sizeof(float) * (size_t)n * stride), o_bs = o_tri + al(sizeof(int32_t) * 3 * n_tri),
-               o_bi = o_bs + al(X.head.bytes()), total = o_bi + al(X.more.bytes());
-  JSH_CUDA_TRY(cudaSetDevice(ctx->device));
+  const int32_t padded = (n_fields + 3) / 4 * 4;
+  const uint64_t used = ctx->used.load(), left = ctx->budget > used ? ctx->budget - used : 0;
+  const size_t points = al(sizeof(double) * 2 * n) + al(sizeof(float) * (size_t)n * padded) + al(sizeof(int32_t) * 3 * n_tri);
+  bool lean = points + jsh_grid_full_bytes(n_tri) > left / 32;
+  JshGridIndex X;
+  std::unique_lock<std::mutex> lk(ctx->mu, std::defer_lock);
+  int id = -1, st = JSH_OK;
+  int32_t stride = 0;
+  size_t o_xy = 0, o_rec = 0, o_val = 0, o_tri = 0, o_bs = 0, o_bi = 0, total = 0;
   void* mem = nullptr;
-  st = jsh_alloc_device(ctx, total, &mem);
+  for (;;) {
+    try {
+      st = jsh_grid_index(xy, n, tri, n_tri, lean, &X);
+    } catch (const std::bad_alloc&) {
+      jsh_set_error("no host memory for the index of %lld triangles", (long long)n_tri);
+      st = JSH_ERR_OOM;
+    }
+    if (st) return st;
+    if (!lk.owns_lock()) lk.lock();
+    for (int g = 0; g < JSH_MAX_GRIDS && id < 0; ++g)
+      if (!ctx->grids[g].used) id = g;
+    if (id < 0) {
+      jsh_set_error("all %d grid slots are in use", JSH_MAX_GRIDS);
+      return JSH_ERR_INVALID;
+    }
+    stride = lean ? n_fields : padded;
+    o_rec = o_xy + al(sizeof(double) * 2 * n);
+    o_val = o_rec + al(X.rec.bytes());
+    o_tri = o_val + al(sizeof(float) * (size_t)n * stride);
+    o_bs = o_tri + al(sizeof(int32_t) * 3 * n_tri);
+    o_bi = o_bs + al(X.head.bytes());
+    total = o_bi + al(X.more.bytes());
+    JSH_CUDA_TRY(cudaSetDevice(ctx->device));
+    st = jsh_alloc_device(ctx, total, &mem);
+    if (st != JSH_ERR_OOM || lean) break;
+    lean = true;
+  }
   if (st) return st;
   char* base = (char*)mem;
   cudaError_t e = cudaMemcpy(base + o_xy, xy, sizeof(double) * 2 * n, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(base + o_rec, X.rec.p.get(), X.rec.bytes(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && !lean) e = cudaMemcpy(base + o_rec, X.rec.p.get(), X.rec.bytes(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy2D(base + o_val, sizeof(float) * stride, values, sizeof(float) * n_fields, sizeof(float) * n_fields,
                      (size_t)n, cudaMemcpyHostToDevice);
@@ -429,7 +445,7 @@ extern "C" int jsh_grid_upload(jsh_ctx* ctx, const double* xy, int64_t n, const 
   S.bytes = total;
   JshGrid& G = S.view;
   G.xy = (const double*)(base + o_xy);
-  G.rec = (const float*)(base + o_rec);
+  G.rec = lean ? nullptr : (const float*)(base + o_rec);
   G.val = (const float*)(base + o_val);
   G.tri = (const int32_t*)(base + o_tri);
   G.bhead = (const int32_t*)(base + o_bs);

@@ -1,9 +1,10 @@
 // jsh_grid_index.cpp -- the bucket index and the triangle records of a
 // triangulated grid (the device's lookups: jsh_fields.cuh, jsh_fields32.cuh).
 //
-// Square buckets, about two per triangle (one for two triangles from 2^26
-// buckets on), each with the triangles that it touches, in ascending order, the
-// first seven inline; and a record per triangle.
+// Square buckets, each with the triangles that it touches, in ascending order, the
+// first seven inline.  The full index has about two buckets per triangle (one for
+// two triangles from 2^26 buckets on) and a record per triangle; the lean one,
+// where memory is short, a bucket for two triangles and no records.
 //
 // A mixed-precision lookup outside its hint's triangle is a chain of loads, a
 // bucket and its triangles two at a time: with half a bucket per triangle,
@@ -47,7 +48,13 @@ struct Entry {
 
 }  // namespace
 
-int jsh_grid_index(const double* xy, int64_t n, const int32_t* tri, int64_t n_tri, JshGridIndex* out) {
+size_t jsh_grid_full_bytes(int64_t n_tri) {
+  // heads (two buckets a triangle), records, and the longer lists: few on an
+  // even grid
+  return (size_t)n_tri * (2 * 8 * sizeof(int32_t) + 12 * sizeof(float));
+}
+
+int jsh_grid_index(const double* xy, int64_t n, const int32_t* tri, int64_t n_tri, bool lean, JshGridIndex* out) {
   double x0 = xy[0], x1 = xy[0], y0 = xy[1], y1 = xy[1];
   for (int64_t i = 1; i < n; ++i) {
     x0 = std::min(x0, xy[2 * i]);
@@ -60,7 +67,8 @@ int jsh_grid_index(const double* xy, int64_t n, const int32_t* tri, int64_t n_tr
     return JSH_ERR_INVALID;
   }
   const double ex = x1 - x0, ey = y1 - y0;
-  const double n_buckets = std::max((double)n_tri / 2.0, std::min(2.0 * (double)n_tri, 67108864.0));
+  double n_buckets = (double)n_tri / 2.0;
+  if (!lean) n_buckets = std::max(n_buckets, std::min(2.0 * (double)n_tri, 67108864.0));
   double h = std::sqrt(std::max(ex * ey, 1e-300) / std::max(1.0, n_buckets));
   if (!(h > 0) || !std::isfinite(h)) h = std::max(std::max(ex, ey), 1.0);
   h = std::max(h, std::max(ex, ey) / 65536.0);  // at most 65536 buckets per side
@@ -79,7 +87,7 @@ int jsh_grid_index(const double* xy, int64_t n, const int32_t* tri, int64_t n_tr
   out->h = h;
   out->nbx = nbx;
   out->nby = nby;
-  out->rec.resize((size_t)12 * n_tri);
+  out->rec.resize(lean ? 0 : (size_t)12 * n_tri);
 
   // The triangles in stretches, one a thread: each its records and its (bucket,
   // triangle) entries, once (its time: jsh_grid_upload).
@@ -99,17 +107,18 @@ int jsh_grid_index(const double* xy, int64_t n, const int32_t* tri, int64_t n_tr
           px[k] = xy[2 * (int64_t)tri[3 * t + k]];
           py[k] = xy[2 * (int64_t)tri[3 * t + k] + 1];
         }
-        // the FP32 operations here round as the device's would
-        float* r = &out->rec[(size_t)12 * t];
-        for (int k = 0; k < 3; ++k) {
-          r[2 * k] = (float)px[k];
-          r[2 * k + 1] = (float)py[k];
+        if (!lean) {  // the FP32 operations here round as the device's would
+          float* r = &out->rec[(size_t)12 * t];
+          for (int k = 0; k < 3; ++k) {
+            r[2 * k] = (float)px[k];
+            r[2 * k + 1] = (float)py[k];
+          }
+          r[6] = r[4] - r[0];
+          r[7] = r[5] - r[1];
+          const float area32 = (r[2] - r[0]) * r[7] - (r[3] - r[1]) * r[6];
+          r[8] = area32 == 0.f ? NAN : 1.f / area32;
+          memcpy(r + 9, tri + 3 * t, 3 * sizeof(int32_t));
         }
-        r[6] = r[4] - r[0];
-        r[7] = r[5] - r[1];
-        const float area32 = (r[2] - r[0]) * r[7] - (r[3] - r[1]) * r[6];
-        r[8] = area32 == 0.f ? NAN : 1.f / area32;
-        memcpy(r + 9, tri + 3 * t, 3 * sizeof(int32_t));
         for (int k = 0; k < 3; ++k) {
           px[k] -= x0;
           py[k] -= y0;

@@ -24,11 +24,14 @@ struct JshRaw {
 struct JshGridIndex {
   double x0, y0, h;  // bucket (i, j) covers [x0 + i h, x0 + (i + 1) h) x ...; the last ones what lies beyond
   int32_t nbx, nby;
-  // head [nbx * nby][8], more and rec [n_tri][12] as JshGrid::bhead, bmore and rec
+  // head [nbx * nby][8], more and rec [n_tri][12] (lean: none) as JshGrid::bhead, bmore and rec
   JshRaw<int32_t> head, more;
   JshRaw<float> rec;
 };
 
+// Device bytes of the arrays of a full index: about two buckets a triangle.
+size_t jsh_grid_full_bytes(int64_t n_tri);
+
 // Builds the index of triangles tri [n_tri][3] over points xy [n][2]
 // (vertex ids in range).  A JSH status; throws std::bad_alloc.
-int jsh_grid_index(const double* xy, int64_t n, const int32_t* tri, int64_t n_tri, JshGridIndex* out);
+int jsh_grid_index(const double* xy, int64_t n, const int32_t* tri, int64_t n_tri, bool lean, JshGridIndex* out);

@@ -39,9 +39,9 @@ struct JshGrid {         // device view of an uploaded triangulated (z, r) grid
   const double* xy;      // [n][2] (z, r) in pc
   // [n_tri][12] mixed-precision lookups, a triangle in three float4: FP32
   // vertices a, b, c, the edge c - a, 1 / (twice its area) (NaN for a
-  // degenerate one), and its vertex ids as integer bits
+  // degenerate one), and its vertex ids as integer bits; null in a lean grid
   const float* rec;
-  const float* val;      // [n][stride], stride = n_fields rounded up to float4
+  const float* val;      // [n][stride], stride = n_fields rounded up to float4 (lean: n_fields)
   const int32_t* tri;    // [n_tri][3]
   // [nbx*nby][8] a bucket's triangles in ascending order: the first 7 ids (-1:
   // none) and where the others begin in bmore (-1: none; they end with a -1)

@@ -31,8 +31,11 @@ int main(int argc, char** argv) {
       (int64_t)fread(q.data(), 8, 2 * nq, f) != 2 * nq)
     return 2;
   fclose(f);
-  JshGridIndex X;
-  if (jsh_grid_index(xy.data(), n, tri.data(), nt, &X)) return 3;
+  // argv[2]: the lean index
+  const bool lean = argc > 2;
+  JshGridIndex X, full;
+  if (jsh_grid_index(xy.data(), n, tri.data(), nt, false, &full)) return 3;
+  if (jsh_grid_index(xy.data(), n, tri.data(), nt, lean, &X)) return 3;
   auto id = [&](int64_t b, int k) {
     if (k < 7) return X.head[8 * b + k];
     return X.head[8 * b + 7] < 0 ? -1 : X.more[X.head[8 * b + 7] + (k - 7)];
@@ -54,7 +57,7 @@ int main(int argc, char** argv) {
            orient(a[0], a[1], b[0], b[1], px, py) / area >= 0;
   };
   auto in32 = [&](int64_t t, float px, float py) {
-    const float* r = &X.rec[12 * t];
+    const float* r = &full.rec[12 * t];
     const float w0 = ((r[2] - px) * (r[5] - py) - (r[3] - py) * (r[4] - px)) * r[8];
     const float w1 = ((px - r[0]) * r[7] - (py - r[1]) * r[6]) * r[8];
     return w0 >= -1e-6f && w1 >= -1e-6f && 1.f - w0 - w1 >= -1e-6f;

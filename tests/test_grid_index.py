@@ -1,7 +1,8 @@
 """The bucket index of gridded fields on the CPU (tests/cpp/grid_index_check.cpp):
 against a search of all triangles, in the arithmetic of both lookups, for even
 and strongly graded grids, slivers, rows of buckets, vertices, edge points and
-points at the end of the last bucket; lists longer than the seven inline ids;
+points at the end of the last bucket; lists longer than the seven inline ids, and the
+lean form's lists;
 and its build on several threads: the same index, in the time of a serial one
 or less."""
 import os
@@ -25,14 +26,14 @@ def check(tmp_path_factory):
                     os.path.join(REPO, "tests", "cpp", "grid_index_check.cpp"), os.path.join(CSRC, "jsh_grid_index.cpp"),
                     "-o", exe, "-lpthread"], check=True)
 
-    def run(xy, tri, q):
+    def run(xy, tri, q, lean=False):
         path = str(d / "grid.bin")
         with open(path, "wb") as f:
             f.write(np.array([len(xy), len(tri), len(q)], np.int64).tobytes())
             f.write(np.ascontiguousarray(xy, np.float64).tobytes())
             f.write(np.ascontiguousarray(tri, np.int32).tobytes())
             f.write(np.ascontiguousarray(q, np.float64).tobytes())
-        r = subprocess.run([exe, path], capture_output=True, text=True, timeout=120)
+        r = subprocess.run([exe, path] + ["lean"] * lean, capture_output=True, text=True, timeout=120)
         assert r.returncode == 0, r.stdout + r.stderr
         w = r.stdout.split()
         return dict(buckets=int(w[0]), entries=int(w[2]), longest=int(w[5].rstrip(",")), inside=int(w[6]))
@@ -52,8 +53,9 @@ def grids():
     return {"even": even, "graded": np.vstack([graded, box]), "strip": strip, "fan": fan, "far": far, "box": box}
 
 
+@pytest.mark.parametrize("lean", [False, True])
 @pytest.mark.parametrize("kind", ["even", "graded", "strip", "fan", "far", "box"])
-def test_finds_what_all_triangles_hold(check, kind):
+def test_finds_what_all_triangles_hold(check, kind, lean):
     xy = grids()[kind]
     tri = triangulate(xy)
     rng = np.random.default_rng(11)
@@ -64,7 +66,7 @@ def test_finds_what_all_triangles_hold(check, kind):
     edge = xy[pick[:200, 0]] + rng.random((200, 1)) * (xy[pick[:200, 1]] - xy[pick[:200, 0]])
     q = np.vstack([(w[:, :, None] * xy[pick]).sum(1), edge, xy[:200], lo + (hi - lo) * rng.uniform(-0.05, 1.05, (300, 2)),
                    [hi, [hi[0], lo[1]], [lo[0], hi[1]], lo], np.column_stack([np.full(50, hi[0]), rng.uniform(lo[1], hi[1], 50)])])
-    s = check(xy, tri, q)
+    s = check(xy, tri, q, lean)
     assert s["inside"] > 500
     if kind in ("graded", "fan"):
         assert s["longest"] > 7
@@ -87,7 +89,7 @@ def test_build_time(lib):
 void jsh_set_error(const char*, ...) {}
 extern "C" long long build(const double* xy, long long n, const int* tri, long long m) {
   JshGridIndex X;
-  return jsh_grid_index(xy, n, tri, m, &X) ? -1 : (long long)X.more.n;
+  return jsh_grid_index(xy, n, tri, m, false, &X) ? -1 : (long long)X.more.n;
 }
 """
     import tempfile
