@@ -83,11 +83,12 @@ cudaError_t jsh_launch_plane_rays(const JshPlane& plane, double* d_orig, double*
 cudaError_t jsh_launch_grid_interp(const JshGrid& grid, int field, const double* d_zr, int64_t n,
                                    double nan_value, double* d_out, cudaStream_t stream);
 
-// Largest resident CTAs per SM of the persistent transfer kernel whose launch
-// shape the knobs set (mixed: the IQUV kernel of the split form, or the
-// single-kernel form; compact: its register-capped build; 0 if it cannot run
-// block_size threads).
-int jsh_persistent_occupancy(int precision, bool full, int block_size, bool compact = false, bool single = false);
+// Largest resident CTAs per SM of block_size threads of the persistent transfer
+// kernel that a request of at most `items` work items runs with `shape` (mixed:
+// the IQUV kernel of the split form in the build of its law, its compact and its
+// Faraday-thick build, or the single-kernel form; 0 if it cannot run them).
+int jsh_persistent_occupancy(int precision, bool full, int block_size, const JshLaunchShape& shape, uint64_t items,
+                             int num_sms);
 
 // Nearest cell of n points (cm) of an uploaded cell set (checks), and the
 // random unit directions of n counters (k0, k1, k2) of `seed`.

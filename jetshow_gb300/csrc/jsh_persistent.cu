@@ -15,10 +15,12 @@
 
 #if JSH_FARADAY_THICK_BUILD
 #define JSH_LAUNCH_TRANSFER_MIXED jsh_launch_transfer_mixed_ft
+#define JSH_MIXED_OCCUPANCY jsh_mixed_occupancy_ft
 #define JSH_STATIC_KERNEL jsh_static_kernel_ft
 #define JSH_SINGLE_KERNEL jsh_single_kernel_ft
 #else
 #define JSH_LAUNCH_TRANSFER_MIXED jsh_launch_transfer_mixed
+#define JSH_MIXED_OCCUPANCY jsh_mixed_occupancy
 #define JSH_STATIC_KERNEL jsh_static_kernel
 #define JSH_SINGLE_KERNEL jsh_single_kernel
 #endif
@@ -134,19 +136,6 @@ int occupancy(K kernel, int block, size_t smem) {
   return n;
 }
 
-// Resident CTAs per SM of the IQUV kernel / the single-kernel form.
-int occupancy_mixed(bool split, bool full, int block_size, bool compact) {
-  if (compact && block_size > 128) return 0;
-  const size_t sm = full ? stage_smem<true>(block_size) : stage_smem<false>(block_size);
-  if (!split) return occupancy(JSH_SINGLE_KERNEL(full, compact), block_size, sm);
-  // the general build bounds both (it holds at least the fused one's registers)
-  if (compact)
-    return full ? occupancy(transfer_iquv_general_kernel<true, true, false>, block_size, sm)
-                : occupancy(transfer_iquv_general_kernel<false, true, false>, block_size, sm);
-  return full ? occupancy(transfer_iquv_general_kernel<true, false, false>, block_size, sm)
-              : occupancy(transfer_iquv_general_kernel<false, false, false>, block_size, sm);
-}
-
 }  // namespace
 
 }  // namespace jsh
@@ -188,6 +177,15 @@ cudaError_t launch_prio(void (*kernel)(KArgs...), unsigned grid, unsigned block,
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Work items up to which the kernels for every law put each on a group of
+// lanes, per SM (the host knows the pixels, not the hits: an upper bound).
+// At 29 092 items of a radial field the tau kernel took 287 us on lanes and
+// 217 on groups, the IQUV kernel 686 and 365; 33 640 items of a gridded jet
+// 65.3 and 37.0 ms, 31.7 and 25.2 ms; at 134 556 of them 108 and 134 ms, 95
+// and 90 ms (since then the lookups got faster: 19 + 15 ms at 33 640 items on
+// groups, 48 + 44 ms at 134 556 on lanes), at 415 968 items of a radial field 1.6 and 4.0 ms, 1.6 and 2.7.
+constexpr uint64_t kGroupItemsPerSm = 432;
+
 // IQUV kernel instantiation of a launch.
 IquvKernel iquv_kernel(bool full, bool compact, bool fused, bool groups) {
   if (fused) {
@@ -200,14 +198,19 @@ IquvKernel iquv_kernel(bool full, bool compact, bool fused, bool groups) {
   return full ? transfer_iquv_general_kernel<true, false, false> : transfer_iquv_general_kernel<false, false, false>;
 }
 
-// Work items up to which the kernels for every law put each on a group of
-// lanes, per SM (the host knows the pixels, not the hits: an upper bound).
-// At 29 092 items of a radial field the tau kernel took 287 us on lanes and
-// 217 on groups, the IQUV kernel 686 and 365; 33 640 items of a gridded jet
-// 65.3 and 37.0 ms, 31.7 and 25.2 ms; at 134 556 of them 108 and 134 ms, 95
-// and 90 ms (since then the lookups got faster: 19 + 15 ms at 33 640 items on
-// groups, 48 + 44 ms at 134 556 on lanes), at 415 968 items of a radial field 1.6 and 4.0 ms, 1.6 and 2.7.
-constexpr uint64_t kGroupItemsPerSm = 432;
+// The IQUV kernel of a split launch on at most `items` work items.
+struct IquvLaunch {
+  IquvKernel kernel;
+  bool groups, full, fused;
+  // most threads a CTA of it can have
+  int max_block(bool compact) const { return compact || groups ? 128 : 256; }
+  // the fused build: a lane keeps its five points (full Stokes) or nothing there
+  size_t smem(int block) const { return full ? stage_smem<true>(block, !fused) : stage_smem<false>(block, !fused); }
+};
+IquvLaunch iquv_launch(bool full, const JshLaunchShape& shape, uint64_t items, int num_sms) {
+  const bool fused = shape.fused != 0, groups = !fused && items <= kGroupItemsPerSm * (uint64_t)num_sms;
+  return IquvLaunch{iquv_kernel(full, shape.compact != 0, fused, groups), groups, full, fused};
+}
 
 // CTAs of the deep chain's IQUV kernel per SM (64 threads each) when the
 // passes overlap: room for the deep prefix's longest items from the start,
@@ -237,27 +240,27 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   const int rf = shape.refill_threshold;
   int bs = shape.block_size;
   if (bs > (shape.compact ? 128 : 256)) bs = shape.compact ? 128 : 256;
-  int per_sm = shape.ctas_per_sm > 0 ? shape.ctas_per_sm : occupancy_mixed(split, full, bs, shape.compact);
-  if (per_sm < 1) per_sm = 1;
-  unsigned blocks = (unsigned)(num_sms * per_sm);
-  if ((uint64_t)blocks * bs > need) blocks = (unsigned)((need + bs - 1) / bs);
-  if (blocks == 0) blocks = 1;
-  const size_t smem = full ? stage_smem<true>(bs) : stage_smem<false>(bs);
   if (!split) {
-    const cudaError_t e = allow_storage(JSH_SINGLE_KERNEL(full, shape.compact != 0), smem);
+    const SingleKernel kernel = JSH_SINGLE_KERNEL(full, shape.compact != 0);
+    const size_t smem = full ? stage_smem<true>(bs) : stage_smem<false>(bs);
+    const cudaError_t e = allow_storage(kernel, smem);
     if (e != cudaSuccess) return e;
+    const int per_sm = shape.ctas_per_sm > 0 ? shape.ctas_per_sm : occupancy(kernel, bs, smem);
+    unsigned blocks = (unsigned)(num_sms * std::max(per_sm, 1));
+    if ((uint64_t)blocks * bs > need) blocks = (unsigned)((need + bs - 1) / bs);
+    if (blocks == 0) blocks = 1;
     if (shape.marks) cudaEventRecord(shape.marks[2], stream);
-    JSH_SINGLE_KERNEL(full, shape.compact != 0)<<<blocks, bs, smem, stream>>>(d_reqs, n_req, q, rf);
+    kernel<<<blocks, bs, smem, stream>>>(d_reqs, n_req, q, rf);
     if (shape.marks) cudaEventRecord(shape.marks[3], stream);
     return cudaGetLastError();
   }
   // tau kernel: 256 threads, every CTA it can keep resident (the fused build
   // runs panels only, which keep their sums in registers; the general build
   // keeps Dormand-Prince stages in shared memory)
-  const bool groups = !shape.fused && need <= kGroupItemsPerSm * (uint64_t)num_sms;
+  const IquvLaunch iquv = iquv_launch(full, shape, need, num_sms);
   const bool one = shape.mix != nullptr && n_req == 1;
   const JshMixed mix = one ? *shape.mix : JshMixed{};
-  const TauLaunch tau = jsh_tau_kernel(shape.fused != 0, groups, one);
+  const TauLaunch tau = jsh_tau_kernel(shape.fused != 0, iquv.groups, one);
   const TauKernel tau_k = tau.kernel;
   const int bt = tau.block;
   const size_t smem_t = tau.smem;
@@ -272,17 +275,13 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
     return (unsigned)std::min<uint64_t>(grid, (need + per_cta - 1) / per_cta);
   };
   bl_t = enough(bl_t, bt);
-  const IquvKernel iquv_k = iquv_kernel(full, shape.compact != 0, shape.fused != 0, groups);
-  // the fused build: a lane keeps its five points (full Stokes) or nothing there
-  auto smem_of = [&](int block) {
-    return full ? stage_smem<true>(block, !shape.fused) : stage_smem<false>(block, !shape.fused);
-  };
-  if (groups && bs > 128) bs = 128;
-  const size_t smem_q = smem_of(bs);
+  const IquvKernel iquv_k = iquv.kernel;
+  bs = std::min(bs, iquv.max_block(shape.compact != 0));
+  const size_t smem_q = iquv.smem(bs);
   cudaError_t e = allow_storage(iquv_k, smem_q);
   if (e != cudaSuccess) return e;
   int per_sm_q = shape.ctas_per_sm;
-  if (per_sm_q <= 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_q, iquv_k, bs, smem_q);
+  if (per_sm_q <= 0) per_sm_q = occupancy(iquv_k, bs, smem_q);
   const unsigned blocks_q = enough((unsigned)(num_sms * std::max(per_sm_q, 1)), bs);
   if (!overlap) {
     if (shape.marks) cudaEventRecord(shape.marks[0], stream);
@@ -316,7 +315,7 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   e = cudaEventRecord(shape.fork[0], stream);
   if (e != cudaSuccess) return e;
   e = launch_prio(iquv_k, (unsigned)(num_sms * kDeepIquvPerSm), kDeepIquvBlock,
-                  smem_of(kDeepIquvBlock), stream, prio_hi,
+                  iquv.smem(kDeepIquvBlock), stream, prio_hi,
                   d_reqs, n_req, q + 1, rf, 0);
   if (e != cudaSuccess) return e;
   e = cudaStreamWaitEvent(shape.side, shape.fork[0], 0);
@@ -336,12 +335,28 @@ cudaError_t JSH_LAUNCH_TRANSFER_MIXED(const JshRequest* d_reqs, int n_req, int s
   return cudaGetLastError();
 }
 
+// Resident CTAs per SM of `block` threads of the kernel that a request of at most
+// `items` work items runs with `shape`: the IQUV kernel of the split form, or the
+// single-kernel form; 0 if it cannot run them.
+int JSH_MIXED_OCCUPANCY(bool full, int block, const JshLaunchShape& shape, uint64_t items, int num_sms) {
+  if (shape.single) {
+    if (block > (shape.compact ? 128 : 256)) return 0;
+    return occupancy(JSH_SINGLE_KERNEL(full, shape.compact != 0), block,
+                     full ? stage_smem<true>(block) : stage_smem<false>(block));
+  }
+  const IquvLaunch iquv = iquv_launch(full, shape, (items + 31) / 32 * 32, num_sms);  // as the launch rounds them
+  return block > iquv.max_block(shape.compact != 0) ? 0 : occupancy(iquv.kernel, block, iquv.smem(block));
+}
+
 #if !JSH_FARADAY_THICK_BUILD  // the host functions below are built once
 int jsh_queue64_occupancy(int block_size);
+int jsh_mixed_occupancy_ft(bool full, int block, const JshLaunchShape& shape, uint64_t items, int num_sms);
 
-int jsh_persistent_occupancy(int precision, bool full, int block_size, bool compact, bool single) {
-  if (precision == JSH_PREC_MIXED) return occupancy_mixed(!single, full, block_size, compact);
-  return jsh_queue64_occupancy(block_size);
+int jsh_persistent_occupancy(int precision, bool full, int block_size, const JshLaunchShape& shape, uint64_t items,
+                             int num_sms) {
+  if (precision != JSH_PREC_MIXED) return jsh_queue64_occupancy(block_size);
+  return full && shape.faraday_thick ? jsh_mixed_occupancy_ft(full, block_size, shape, items, num_sms)
+                                     : jsh_mixed_occupancy(full, block_size, shape, items, num_sms);
 }
 
 // ------------------------------------------------------------------ host
