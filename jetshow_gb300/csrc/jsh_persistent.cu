@@ -178,13 +178,19 @@ cudaError_t launch_prio(void (*kernel)(KArgs...), unsigned grid, unsigned block,
 }
 
 // Work items up to which the kernels for every law put each on a group of
-// lanes, per SM (the host knows the pixels, not the hits: an upper bound).
-// At 29 092 items of a radial field the tau kernel took 287 us on lanes and
-// 217 on groups, the IQUV kernel 686 and 365; 33 640 items of a gridded jet
-// 65.3 and 37.0 ms, 31.7 and 25.2 ms; at 134 556 of them 108 and 134 ms, 95
-// and 90 ms (since then the lookups got faster: 19 + 15 ms at 33 640 items on
-// groups, 48 + 44 ms at 134 556 on lanes), at 415 968 items of a radial field 1.6 and 4.0 ms, 1.6 and 2.7.
-constexpr uint64_t kGroupItemsPerSm = 432;
+// lanes, per SM (the host knows the pixels, not the hits: an upper bound; 57 %
+// of these images hit).  Groups against lanes [ms], tau + IQUV kernel of square
+// images at one frequency, 152 SMs:
+//   pixels  items/SM  grid of 200 000 points  sheath flow   radial field
+//   256^2     431     25.2 + 16.8, 36.1 + 16.3  0.52 + 0.53, 1.17 + 0.93  0.27 + 0.20, 0.31 + 0.23
+//   300^2     592     32.5 + 22.5, 36.5 + 23.3  0.66 + 0.67, 1.20 + 0.92  0.34 + 0.27, 0.30 + 0.30
+//   360^2     853     44.5 + 31.6, 37.4 + 27.6  0.83 + 0.87, 1.19 + 1.20  0.48 + 0.39, 0.29 + 0.38
+//   512^2    1725     85.3 + 62.2, 63.7 + 49.9  1.39 + 1.53, 1.48 + 1.39  0.94 + 0.77, 0.53 + 0.59
+// Both kernels change sides between 300^2 and 360^2 on grids, the radial field
+// at 256^2 to 360^2, the sheath at 512^2; Stokes I alone the same or earlier (radial field 0.17
+// against 0.12 ms at 256^2, sheath 0.55 against 0.95 at 300^2).  The line lies
+// between the two sizes at which the grids change.
+constexpr uint64_t kGroupItemsPerSm = 720;
 
 // IQUV kernel instantiation of a launch.
 IquvKernel iquv_kernel(bool full, bool compact, bool fused, bool groups) {

@@ -2,7 +2,7 @@
 parameters take (512, run as 256): every form and build launches, its stage
 storage above the 48 KB of an unasked launch included, and renders bitwise
 what the static schedule does.  The every-law split form runs its lanes here
-(more than 432 items an SM), not its groups."""
+(more items an SM than it puts on groups), not its groups."""
 import math
 
 import numpy as np
@@ -58,7 +58,7 @@ def compare(ctx, jet, plane, blocks, output, flags):
                                        ("sheath", A.FLAG_FARADAY_THICK), ("grid", 0)])
 def test_split_form(ctx, grid_id, output, law, flags):
     # the gridded image is narrow about the jet: few of its rays hit
-    shape, mas = ((128, 520), 6.4 if law != "grid" else 0.02)
+    shape, mas = ((128, 1040), 12.8 if law != "grid" else 0.04)
     st = compare(ctx, model(law, grid_id), square(shape, mas), (64, 128, 256, 512), output, flags)
     assert st["n_work_items"] > 0
 
@@ -77,7 +77,7 @@ def test_shape_tuned_on_another_output(ctx, grid_id):
     full-Stokes requests of every law."""
     from jetshow_gb300.runtime import Context
     c = Context(0)
-    plane = square((128, 520), 6.4)
+    plane = square((128, 1040), 12.8)
     c.autotune(model("fused", grid_id), plane, NU, J.make_params(precision="mixed", schedule="persistent",
                                                                 **W.ACCURATE_I_KW))
     p = J.make_params(precision="mixed", schedule="persistent", **W.ACCURATE_KW)
