@@ -114,7 +114,7 @@ extern "C" int jsh_autotune(jsh_ctx* ctx, const jsh_model_desc* model, const jsh
     st = jsh_prepare_request(ctx, model, plane, &p, n_nu, &req, &npix);
     if (!st) st = jsh_prepare_mixed(&req, nu_hz, fc.data());
     if (st) return st;
-    shape.fused = (req.mix.helical_log && !(p.flags & JSH_FLAG_GENERAL_KERNELS)) ? 1 : 0;
+    shape.fused = jsh_fused_family(req.mix, p.flags) ? 1 : 0;
   }
   auto occupancy = [&](int bs, bool cp) {
     shape.compact = cp ? 1 : 0;

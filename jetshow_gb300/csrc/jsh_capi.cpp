@@ -440,7 +440,7 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   const JshRequest* d_req = (const JshRequest*)(base + L.off_req);
   JSH_CUDA_TRY(jsh_launch_hit(d_req, 1, npix, stream));
   JshLaunchShape shape = jsh_effective_shape(ctx, params);
-  shape.fused = (req.mix.helical_log && !(params->flags & JSH_FLAG_GENERAL_KERNELS)) ? 1 : 0;
+  shape.fused = jsh_fused_family(req.mix, params->flags) ? 1 : 0;
   shape.marks = nullptr;
   shape.mix = &req.mix;
   if (params->precision == JSH_PREC_MIXED && !req.seg32) shape.single = 1;

@@ -553,16 +553,20 @@ __device__ __forceinline__ void coef32_tail(const JshFreqConst& F, const JshMixe
 // force on it.
 enum CoefMode { COEF_KI = 0, COEF_I = 1, COEF_FULL = 2 };
 
-// log2 and exp2 without the scaling that subnormal operands and results need
-// (three instructions each): |p|^2 in pc^2 and |n' x u|^2 are 0 or far above
-// 2^-126 (u and n' have components of order 1, rounded to 2^-24), and so are
-// the densities, fields and coefficients in their units.
+// log2 and exp2; NORMAL: without the scaling that subnormal operands and results
+// need (three instructions each; 512x1024 x 4, tau + IQUV kernel: 0.51 + 1.15
+// ms, with it 0.56 + 1.21), for requests whose densities, fields and powers stay
+// in the normal range (JshMixed::normal_range).
+template <bool NORMAL>
 __device__ __forceinline__ float lg2(float x) {
+  if (!NORMAL) return __log2f(x);
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+template <bool NORMAL>
 __device__ __forceinline__ float ex2(float x) {
+  if (!NORMAL) return exp2f(x);
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
@@ -578,9 +582,10 @@ __device__ __forceinline__ float ex2(float x) {
 // from k_I, eta_I, n', b and w: k_V = -(a_V / a_e) B_par eta_I, eta_V =
 // -(a_eV / a_k) B_par D^2 k_I / w, k_F = a_F n' B_par D, k_C = -a_C c1 n' w^2
 // + (a_C c2 / a_k) k_I, B_par = b (u . n').
+template <bool NORMAL>
 __device__ __forceinline__ void coef32_helical_log(const JshMixed& X, const JshFreqConst& F, F3 p, int mode,
                                                    Coef32& c) {
-  const float l = 0.5f * lg2(fdot(p, p));
+  const float l = 0.5f * lg2<NORMAL>(fdot(p, p));
   const float rc2 = p.x * p.x + p.y * p.y;
   float px = 0.f, py = 0.f;
   if (rc2 > 0.f) {
@@ -596,17 +601,17 @@ __device__ __forceinline__ void coef32_helical_log(const JshMixed& X, const JshF
   const F3 u = f3(st * px, st * py, X.b_sign * X.cos_pitch);
   const F3 nlp = f3(X.nlp[0], X.nlp[1], X.nlp[2]);
   const F3 cr = fcross(nlp, u);
-  const float lw = fmaf(-X.bq[1], l, X.l2_b0D) + 0.5f * lg2(fdot(cr, cr));
+  const float lw = fmaf(-X.bq[1], l, X.l2_b0D) + 0.5f * lg2<NORMAL>(fdot(cr, cr));
   // n' and w^pk as two exp2 of arguments of ~20 each rather than one of ~50:
   // exp2f's relative error is ~ulp(argument), so the split keeps k_I's
   // rounding at the level of the product form
-  const float n_ = ex2(fmaf(-X.nq[1], l, X.l2_n0));
-  c.kI = (F.ak * n_) * ex2(X.pk * lw);
+  const float n_ = ex2<NORMAL>(fmaf(-X.nq[1], l, X.l2_n0));
+  c.kI = (F.ak * n_) * ex2<NORMAL>(X.pk * lw);
   if (mode == COEF_KI) return;
-  c.eI = (F.ae * X.D * n_) * ex2(X.pk_h * lw);
+  c.eI = (F.ae * X.D * n_) * ex2<NORMAL>(X.pk_h * lw);
   if (mode == COEF_I) return;
-  const float bpar = ex2(fmaf(-X.bq[1], l, X.l2_b0)) * fdot(u, nlp);
-  const float w = ex2(lw);
+  const float bpar = ex2<NORMAL>(fmaf(-X.bq[1], l, X.l2_b0)) * fdot(u, nlp);
+  const float w = ex2<NORMAL>(lw);
   const float D = X.D;
   c.kQ = X.kq * c.kI;
   c.eQ = X.eq * c.eI;
@@ -622,7 +627,7 @@ __device__ __forceinline__ void coef32_helical_log(const JshMixed& X, const JshF
 // per-evaluation random direction (JSH_RND_POINTS only); tri_hint: the
 // lane's point-location hint for fields on one shared grid (may be null).
 // GENERAL = false compiles the fused benchmark-family path alone, for
-// kernels launched only on requests whose mix.helical_log is set (the same
+// kernels launched only on requests of jsh_fused_family (the same
 // arithmetic as the general build takes for them).
 template <bool GENERAL = true>
 __device__ __forceinline__ void coef32_rt(const JshRequest& R, const JshMixed& X, const JshFreqConst& F, F3 p, int mode, Coef32& c,
@@ -630,7 +635,7 @@ __device__ __forceinline__ void coef32_rt(const JshRequest& R, const JshMixed& X
                                           int* tri_hint = nullptr, const LaneGroup group = LaneGroup{0u, 0, 0, 1}) {
   const JshModel& m = R.model;
   if (!GENERAL || X.helical_log) {
-    coef32_helical_log(X, F, p, mode, c);
+    coef32_helical_log<!GENERAL>(X, F, p, mode, c);
     return;
   }
   const bool full = mode == COEF_FULL;

@@ -21,7 +21,7 @@ struct JshLaunchShape {
   int compact;           // mixed persistent schedule: the register-capped build (<= 128 threads)
   int single;            // mixed persistent schedule: tau and IQUV passes in one kernel (else split)
   int fused;             // split form: every request of the batch is of the fused benchmark
-                         // family (mix.helical_log): launch the kernels built for it alone
+                         // family (jsh_fused_family): launch the kernels built for it alone
   // mixed persistent schedule, optional: four events recorded on the stream
   // before the tau kernel, after it, after the IQUV ranking and after the
   // IQUV kernel (the single-kernel form records only the last two;

@@ -188,7 +188,7 @@ extern "C" int jsh_observation_run_noalloc(const jsh_model_desc* model, const js
   JSH_CUDA_TRY(jsh_launch_hit(d_req, 1, npix, s));
   JshLaunchShape shape = jsh_params_shape(JshLaunchShape{128, 0, 8, 0}, params);
   shape.mix = &in.req.mix;
-  shape.fused = (in.req.mix.helical_log && !(params->flags & JSH_FLAG_GENERAL_KERNELS)) ? 1 : 0;
+  shape.fused = jsh_fused_family(in.req.mix, params->flags) ? 1 : 0;
   JSH_CUDA_TRY(jsh_launch_transfer(d_req, 1, params->precision, params->schedule, params->output == JSH_OUT_FULL,
                                    npix * (uint64_t)n_nu, npix, shape, (unsigned int*)(base + L.off_queue), sms, s));
   return JSH_OK;

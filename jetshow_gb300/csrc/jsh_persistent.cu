@@ -456,6 +456,10 @@ int jsh_prepare_mixed(JshRequest* req, const double* nu_host, JshFreqConst* fc) 
       X.l2_n0 = (float)log2(n0p);
       X.pk_h = (float)((s + 1.) / 2.);
       X.b_sign = m.bp[0] > 0.0 ? 1.f : -1.f;
+      // the least of each factor between 2^-20 and 2^20 pc
+      const double n_min = X.l2_n0 - 20.0 * fabs(m.np[1]), b_min = X.l2_b0 - 20.0 * fabs(m.bp[1]);
+      const double w_min = std::min(0.0, X.l2_b0D - 20.0 * fabs(m.bp[1]) - 8.0);
+      X.normal_range = (std::min(std::min(n_min, b_min), std::max(1.0, (s + 2.) / 2.) * w_min) > -126.0) ? 1 : 0;
     }
     X.D = (float)D;
     X.gamma = (float)gamma;

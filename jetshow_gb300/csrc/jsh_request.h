@@ -111,8 +111,18 @@ struct JshMixed {
   float tau_min_f;                 // an FP32 depth above this is above tau_min
   float dhi[3], dlo[3];            // ray direction as compensated FP32 pairs
   float tau_max_hi, tau_max_lo;    // tau_max as a compensated FP32 pair
+  // log-domain family: 1 where its factors n', b and w and the powers of w are
+  // normal FP32 numbers from 2^-20 to 2^20 pc and down to |n' x u| = 2^-8 (what
+  // lies beyond adds nothing to an FP32 integral of such a ray)
+  int32_t normal_range;
   const JshFreqConst* fc;  // device [n_nu]
 };
+
+// Whether a request runs the kernels built for the benchmark family alone, whose
+// log2 and exp2 leave out subnormal numbers.
+static inline bool jsh_fused_family(const JshMixed& X, uint32_t flags) {
+  return X.helical_log && X.normal_range && !(flags & JSH_FLAG_GENERAL_KERNELS);
+}
 
 struct JshRequest {
   JshModel model;

@@ -286,7 +286,7 @@ int launch_batch(jsh_server* S, Slot& sl) {
   // the fused kernels serve a batch whose every request is of the benchmark family
   bool fused = S->cfg.precision == JSH_PREC_MIXED;
   for (int i = 0; i < n && fused; ++i)
-    fused = sl.batch[i]->rec.mix.helical_log && !(sl.batch[i]->params.flags & JSH_FLAG_GENERAL_KERNELS);
+    fused = jsh_fused_family(sl.batch[i]->rec.mix, sl.batch[i]->params.flags);
   // a batch holds requests of one kind only: with or without the
   // Faraday-thick mode (full Stokes, mixed precision)
   const bool ft = full && S->cfg.precision == JSH_PREC_MIXED &&
