@@ -91,11 +91,7 @@ struct jsh_ctx {
   JshHullSlot hulls[JSH_MAX_HULLS];
   JshCellSlot cells[JSH_MAX_CELL_SETS];
   bool tuned = false;
-  // 12 idle lanes before a warp fetches items: a start is a divergent stretch
-  // of code that the other lanes wait for (the IQUV kernel of 705 176 items:
-  // 1.58 ms at 1, 1.43 at 8, 1.37 at 12, 1.38 at 16), and a group of lanes is
-  // refilled with a second one
-  JshLaunchShape shape{128, 0, 12, 0};
+  JshLaunchShape shape;
   jsh_stats last{};
   bool last_pending = false;
   size_t last_counters_off = 0, last_nhit_off = 0;

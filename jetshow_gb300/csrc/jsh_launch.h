@@ -14,35 +14,40 @@
 #define JSH_OVERLAP_KEY 43
 #define JSH_OVERLAP_MIN_ITEMS 65536
 
+// The initial values are every entry point's default (a context's may be tuned).
 struct JshLaunchShape {
-  int block_size;        // threads per CTA of the transfer kernel
-  int ctas_per_sm;       // persistent schedule: CTAs per SM (0: occupancy max)
-  int refill_threshold;  // persistent schedule: refill when >= this many lanes idle
-  int compact;           // mixed persistent schedule: the register-capped build (<= 128 threads)
-  int single;            // mixed persistent schedule: tau and IQUV passes in one kernel (else split)
-  int fused;             // split form: every request of the batch is of the fused benchmark
+  int block_size = 128;  // threads per CTA of the transfer kernel
+  int ctas_per_sm = 0;   // persistent schedule: CTAs per SM (0: occupancy max)
+  // persistent schedule: refill when >= this many lanes idle.  A start is a
+  // divergent stretch of code that the other lanes wait for (the IQUV kernel of
+  // 705 176 items: 1.58 ms at 1, 1.43 at 8, 1.37 at 12, 1.38 at 16), and a group
+  // of lanes is refilled with a second one.
+  int refill_threshold = 12;
+  int compact = 0;       // mixed persistent schedule: the register-capped build (<= 128 threads)
+  int single = 0;        // mixed persistent schedule: tau and IQUV passes in one kernel (else split)
+  int fused = 0;         // split form: every request of the batch is of the fused benchmark
                          // family (jsh_fused_family): launch the kernels built for it alone
   // mixed persistent schedule, optional: four events recorded on the stream
   // before the tau kernel, after it, after the IQUV ranking and after the
   // IQUV kernel (the single-kernel form records only the last two;
   // with overlapped passes: before the deep prefix's tau kernel, after the
   // other rays' tau kernel and IQUV ranking, and after both IQUV kernels)
-  cudaEvent_t* marks;
+  cudaEvent_t* marks = nullptr;
   // split form, optional: overlapped passes.  Rays whose rank bucket is at
   // least overlap_key (estimated optical depth >= 2^(overlap_key - 40)) form
   // the deep prefix: its tau pass runs first and its IQUV pass, which holds
   // the render's longest items, runs on `stream` at high priority while the
   // other rays' tau and IQUV passes run on `side` (fork[0] / fork[1]: events
   // of the fork and the join).  0 or no side stream: one serial chain.
-  int overlap_key;
-  cudaStream_t side;
-  cudaEvent_t* fork;
+  int overlap_key = 0;
+  cudaStream_t side = nullptr;
+  cudaEvent_t* fork = nullptr;
   // mixed precision, a launch on one request: its constants on the host (null:
   // the kernels read them from the record)
-  const JshMixed* mix;
+  const JshMixed* mix = nullptr;
   // mixed precision, full Stokes: run the kernels built with the
   // Faraday-thick mode (JSH_FLAG_FARADAY_THICK)
-  int faraday_thick;
+  int faraday_thick = 0;
 };
 
 // Ray generation: along sizes and centres (the sequential recurrences of
