@@ -316,7 +316,11 @@ typedef struct jsh_stats {
   uint64_t n_pixels;
   uint64_t n_hit_pixels;    /* pixels whose ray intersects the geometry  */
   uint64_t n_work_items;    /* hit pixels x frequencies                   */
-  uint64_t rhs_evals;       /* right-hand-side evaluations on the device  */
+  /* right-hand-side evaluations: six a Dormand-Prince step, attempted or
+   * accepted, and one per segment; 15 a panel.  The transfer coefficients of a
+   * step are evaluated at five points, which its last two stages share (six
+   * where every evaluation draws a random direction). */
+  uint64_t rhs_evals;
   uint64_t steps_accepted;
   uint64_t steps_rejected;
   uint32_t status_or;       /* OR of all per-item status bits             */
