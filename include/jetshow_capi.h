@@ -249,6 +249,7 @@ typedef struct jsh_params {
 #define JSH_FLAG_COST_MAP 0x2
 /* Mixed persistent schedule: launch the register-capped build of the
  * transfer kernel (at most 128 threads per CTA; more resident warps per SM).
+ * The benchmark family's IQUV kernel has one build, which holds no more.
  * Results are bitwise those of the default build; jsh_autotune chooses
  * between the two for requests that leave the launch knobs at 0. */
 #define JSH_FLAG_COMPACT_REGS 0x4

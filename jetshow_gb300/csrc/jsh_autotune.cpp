@@ -120,9 +120,10 @@ extern "C" int jsh_autotune(jsh_ctx* ctx, const jsh_model_desc* model, const jsh
     shape.compact = cp ? 1 : 0;
     return jsh_persistent_occupancy(p.precision, full, bs, shape, items, ctx->num_sms);
   };
-  // the register-capped build exists for the mixed kernel only
+  // the register-capped builds: the mixed every-law and single-kernel ones
+  const bool capped = mixed && (!shape.fused || shape.single);
   for (bool cp : {false, true}) {
-    if (cp && !mixed) continue;
+    if (cp && !capped) continue;
     for (int bs : {64, 96, 128, 192, 256}) {
       const int occ = occupancy(bs, cp);
       if (occ < 1) continue;

@@ -605,7 +605,7 @@ extern "C" int jsh_plane_rays(jsh_ctx* ctx, const jsh_plane_desc* plane, double*
     JshWorkspaceUse use(ctx, s);
     st = jsh_upload_request(stage, &req, L, base, nullptr, s);
     if (st) return st;
-    JSH_CUDA_TRY(jsh_launch_plane_rays(req.plane, (double*)(base + off_o), nullptr, s));
+    JSH_CUDA_TRY(jsh_launch_plane_rays(req.plane, (double*)(base + off_o), s));
     JSH_CUDA_TRY(cudaMemcpyAsync(origins, base + off_o, sizeof(double) * 3 * npix, cudaMemcpyDeviceToHost, s));
     JSH_CUDA_TRY(use.end());
     JSH_CUDA_TRY(cudaStreamSynchronize(s));

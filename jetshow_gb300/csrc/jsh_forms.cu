@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(128) transfer_static_mixed_kernel(const JshReq
 // Persistent CTAs: each warp keeps 32 lanes busy, refilling idle lanes from
 // the global queue when at least `refill` of them are idle.  COMPACT builds
 // the kernel for at most 128 threads and 3 resident CTAs per SM, which caps
-// it at 168 registers (166 used, no spills) instead of 184: 12 instead of 10
+// it at 168 registers (no spills) instead of 182: 12 instead of 10
 // resident warps per SM, more latency hiding for the bulk of short rays at
 // the price of issue slots for the long ones; the autotuner picks.
 template <bool FULL, bool COMPACT>

@@ -147,18 +147,14 @@ __global__ void hit_rays_kernel(JshModel m, const double* __restrict__ orig, con
   }
 }
 
-__global__ void plane_rays_kernel(JshPlane p, double* orig, double* sizes) {
+__global__ void plane_rays_kernel(JshPlane p, double* orig) {
   uint64_t pix = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   uint64_t npix = p.n_across * p.n_along;
   if (pix >= npix) return;
-  uint64_t i = pix / p.n_along, j = pix % p.n_along;
-  if (orig) {
-    V3 o = plane_origin(p, i, j);
-    orig[3 * pix] = o.x;
-    orig[3 * pix + 1] = o.y;
-    orig[3 * pix + 2] = o.z;
-  }
-  if (sizes) sizes[pix] = p.along_size[j];
+  V3 o = plane_origin(p, pix / p.n_along, pix % p.n_along);
+  orig[3 * pix] = o.x;
+  orig[3 * pix + 1] = o.y;
+  orig[3 * pix + 2] = o.z;
 }
 
 __global__ void grid_interp_kernel(JshGrid G, int field, const double* zr, int64_t n, double nan_value,
@@ -329,10 +325,10 @@ cudaError_t jsh_launch_hit_rays(const JshModel& model, const double* d_orig, con
   return cudaGetLastError();
 }
 
-cudaError_t jsh_launch_plane_rays(const JshPlane& plane, double* d_orig, double* d_sizes, cudaStream_t stream) {
+cudaError_t jsh_launch_plane_rays(const JshPlane& plane, double* d_orig, cudaStream_t stream) {
   uint64_t npix = plane.n_across * plane.n_along;
   if (npix == 0) return cudaSuccess;
-  plane_rays_kernel<<<(unsigned)((npix + 255) / 256), 256, 0, stream>>>(plane, d_orig, d_sizes);
+  plane_rays_kernel<<<(unsigned)((npix + 255) / 256), 256, 0, stream>>>(plane, d_orig);
   return cudaGetLastError();
 }
 

@@ -80,9 +80,8 @@ cudaError_t jsh_launch_transfer(const JshRequest* d_reqs, int n_req, int precisi
 cudaError_t jsh_launch_hit_rays(const JshModel& model, const double* d_orig, const double* d_dir, int64_t n,
                                 int32_t* d_nseg, double* d_seg, uint32_t* d_status, cudaStream_t stream);
 
-// Plane rays (origins, sizes) of one compiled plane whose along/across tables
-// are filled.
-cudaError_t jsh_launch_plane_rays(const JshPlane& plane, double* d_orig, double* d_sizes, cudaStream_t stream);
+// Ray origins of one compiled plane whose along/across tables are filled.
+cudaError_t jsh_launch_plane_rays(const JshPlane& plane, double* d_orig, cudaStream_t stream);
 
 // Gridded field interpolation at (z, r) points.
 cudaError_t jsh_launch_grid_interp(const JshGrid& grid, int field, const double* d_zr, int64_t n,

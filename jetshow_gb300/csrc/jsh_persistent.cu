@@ -47,8 +47,9 @@ __device__ __forceinline__ void iquv_prefix(const JshRequest* __restrict__ reqs,
 // IQUV kernels: persistent CTAs over the ranked emitted items.
 //
 // The build for the fused benchmark family alone (128 registers, 16 resident
-// warps per SM; with the Faraday-thick mode 142 and 12; COMPACT caps the former
-// for CTAs of at most 128 threads).  With many items they run on a
+// warps per SM; with the Faraday-thick mode 145 and 12; there is no
+// register-capped build of it: capped at the same 16 warps it held 124 and was
+// 1.2 % slower).  With many items they run on a
 // lane each, dealt so that the longest are in different warps, and once the
 // queue is empty a warp's last six are handed to its groups of lanes, which
 // take a step in under half the time: the longest items decide when the launch
@@ -66,8 +67,8 @@ __device__ __forceinline__ void iquv_prefix(const JshRequest* __restrict__ reqs,
 // 6.15 against 6.23; Stokes I alone 2 022 items 43 us on either.
 static_assert(kWarpGroups * kGroupWords <= 32 * kLaneWords, "a warp's groups fit its lanes' storage");
 constexpr int kIquvGroupsFull = kFtm ? 4 : 2, kIquvGroupsI = 1;
-template <bool FULL, bool COMPACT>
-__global__ void __launch_bounds__(COMPACT ? 128 : 256, COMPACT ? (kFtm ? 3 : 4) : 1)
+template <bool FULL>
+__global__ void __launch_bounds__(256, 1)
     transfer_iquv_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
                          int part) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
@@ -194,10 +195,7 @@ constexpr uint64_t kGroupItemsPerSm = 720;
 
 // IQUV kernel instantiation of a launch.
 IquvKernel iquv_kernel(bool full, bool compact, bool fused, bool groups) {
-  if (fused) {
-    if (compact) return full ? transfer_iquv_kernel<true, true> : transfer_iquv_kernel<false, true>;
-    return full ? transfer_iquv_kernel<true, false> : transfer_iquv_kernel<false, false>;
-  }
+  if (fused) return full ? transfer_iquv_kernel<true> : transfer_iquv_kernel<false>;
   if (groups) return full ? transfer_iquv_general_kernel<true, false, true> : transfer_iquv_general_kernel<false, false, true>;
   if (compact)
     return full ? transfer_iquv_general_kernel<true, true, false> : transfer_iquv_general_kernel<false, true, false>;

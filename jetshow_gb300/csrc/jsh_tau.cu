@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256, 3)
 template <bool GROUPS>
 __global__ void __launch_bounds__(128, 4)
     transfer_tau_general_kernel(const JshRequest* __restrict__ reqs, int n_req, unsigned long long* queue, int refill,
-                                int part, const __grid_constant__ JshMixed) {
+                                int part, const __grid_constant__ JshMixed /* the fused build's alone */) {
   __shared__ unsigned long long base[JSH_MAX_BATCH + 1];
   extern __shared__ float ksh[];
   tau_prefix(reqs, n_req, part, base);

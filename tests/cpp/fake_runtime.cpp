@@ -89,7 +89,7 @@ void jsh_prepare_hit(JshRequest*) {}
 cudaError_t jsh_run_peaks(int, double*, double*, double*, cudaStream_t) { return cudaSuccess; }
 cudaError_t jsh_launch_clear(void* p, size_t n, cudaStream_t s) { return cudaMemsetAsync(p, 0, n, s); }
 cudaError_t jsh_launch_plane(const JshRequest*, int, uint64_t, cudaStream_t s, bool) { return op(s), cudaSuccess; }
-cudaError_t jsh_launch_plane_rays(const JshPlane&, double*, double*, cudaStream_t s) { return op(s), cudaSuccess; }
+cudaError_t jsh_launch_plane_rays(const JshPlane&, double*, cudaStream_t s) { return op(s), cudaSuccess; }
 cudaError_t jsh_launch_hit_rays(const JshModel&, const double*, const double*, int64_t, int32_t*, double*, uint32_t*,
                                 cudaStream_t s) {
   return op(s), cudaSuccess;
