@@ -206,7 +206,8 @@ extern "C" int jsh_cells_nearest(jsh_ctx* ctx, int32_t cells_id, const double* p
   }
   JSH_CUDA_TRY(cudaSetDevice(ctx->device));
   const size_t o_p = 0, o_o = up256(sizeof(double) * 3 * n), total = up256(o_o + sizeof(int32_t) * n);
-  int st = ensure_workspace(ctx, total);
+  int st = keep_stats(ctx);
+  if (!st) st = ensure_workspace(ctx, total);
   if (st) return st;
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
   char* b = (char*)ctx->ws;
@@ -228,7 +229,8 @@ extern "C" int jsh_random_directions(jsh_ctx* ctx, uint64_t seed, const uint32_t
   std::lock_guard<std::mutex> lk(ctx->mu);
   JSH_CUDA_TRY(cudaSetDevice(ctx->device));
   const size_t o_k = 0, o_o = up256(sizeof(uint32_t) * 3 * n), total = up256(o_o + sizeof(double) * 3 * n);
-  int st = ensure_workspace(ctx, total);
+  int st = keep_stats(ctx);
+  if (!st) st = ensure_workspace(ctx, total);
   if (st) return st;
   JSH_CUDA_TRY(cudaEventSynchronize(ctx->ws_ready));
   char* b = (char*)ctx->ws;

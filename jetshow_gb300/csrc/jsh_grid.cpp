@@ -487,7 +487,8 @@ extern "C" int jsh_grid_interpolate(jsh_ctx* ctx, int32_t grid_id, int32_t field
   if (n <= 0) return JSH_OK;
   JSH_CUDA_TRY(cudaSetDevice(ctx->device));
   const size_t in_b = (sizeof(double) * 2 * n + 255) / 256 * 256;
-  int st = ensure_workspace(ctx, in_b + sizeof(double) * n);
+  int st = keep_stats(ctx);
+  if (!st) st = ensure_workspace(ctx, in_b + sizeof(double) * n);
   if (st) return st;
   char* base = (char*)ctx->ws;
   JSH_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->ws_ready, 0));
