@@ -337,7 +337,7 @@ int ensure_workspace(jsh_ctx* ctx, size_t need) {
   void* p = nullptr;
   int st = jsh_alloc_device(ctx, cap, &p);
   if (st) {
-    ctx->ws_refused = std::min(ctx->ws_refused, cap);
+    if (ctx->used.load() + cap <= ctx->budget) ctx->ws_refused = std::min(ctx->ws_refused, cap);
     return st;
   }
   ctx->ws = p;

@@ -18,7 +18,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -34,7 +33,7 @@ void in_parallel(int n, F f) {
   for (int k = 1; k < n; ++k) {
     try {
       threads.emplace_back(f, k);
-    } catch (const std::system_error&) {
+    } catch (...) {  // no thread or no memory for one
       f(k);
     }
   }

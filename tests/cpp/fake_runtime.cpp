@@ -17,7 +17,8 @@ using Ops = std::set<int>;
 std::map<void*, Ops> streams, events;
 int n_ops = 0;
 bool fail_transfer = false;
-size_t device_bytes = 0;
+size_t device_bytes = 0, device_limit = (size_t)-1;
+int n_mallocs = 0, last_single = -1;
 std::map<void*, size_t> sizes;
 int failed = 0;
 
@@ -41,6 +42,8 @@ cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { return *f = *t = (size_t)64 << 30, cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) {
+  ++n_mallocs;
+  if (device_bytes + n > device_limit) return cudaErrorMemoryAllocation;
   *p = aligned_alloc(256, (n + 255) / 256 * 256);
   memset(*p, 0xcd, n);
   sizes[*p] = n;
@@ -103,6 +106,7 @@ cudaError_t jsh_launch_transfer(const JshRequest* r, int, int, int, bool, uint64
                                 unsigned*, int, cudaStream_t s) {
   op(s);
   if (h.side) op(h.side);
+  last_single = h.single;
   if (fail_transfer) return cudaErrorInvalidValue;
   if (h.side) {
     cudaEventRecord(h.fork[1], h.side);
@@ -204,12 +208,54 @@ void statistics() {
   jsh_ctx_destroy(c);
 }
 
+// A request goes without its FP32 segments where the budget or the device has no
+// room for them, without another attempt at every call, and has them again when
+// the budget has.
+void short_memory() {
+  const jsh_model_desc m = model();
+  const jsh_plane_desc p = plane(96, 128);
+  const jsh_params P = mixed();
+  const double nu = 1e10;
+  jsh_image img;
+  memset(&img, 0, sizeof(img));
+  const size_t segments = (size_t)96 * 128 * JSH_MAX_SEG * sizeof(JshSeg32);
+  JshRequestLayout L;
+  jsh_request_layout(96 * 128, 128, 96, 1, false, false, &L);
+  for (bool device : {false, true}) {
+    jsh_ctx* c = nullptr;
+    const size_t room = L.total + segments / 2;
+    check(jsh_ctx_create(0, device ? 0 : L.total + segments + 65536, &c) == JSH_OK, "context");
+    if (device) device_limit = device_bytes + room;
+    void* other = nullptr;  // another user of the budget
+    if (!device) {            // so much that the request is refused altogether
+      check(jsh_alloc_device(c, segments + L.total, &other) == JSH_OK, "most memory");
+      check(jsh_observation_run_device(c, &m, &p, &nu, 1, &P, (void*)c->stream, &img) == JSH_ERR_OOM, "refused");
+      jsh_free_device(c, other, segments + L.total);
+    }
+    if (!device) check(jsh_alloc_device(c, segments / 2 + 65536, &other) == JSH_OK, "other memory");
+    for (int k = 0; k < 3; ++k) {
+      check(jsh_observation_run_device(c, &m, &p, &nu, 1, &P, (void*)c->stream, &img) == JSH_OK, "render");
+      check(last_single == 1, "without segments");
+      if (k == 0) n_mallocs = 0;
+    }
+    check(n_mallocs == 0, "no further attempt");
+    if (!device) {
+      jsh_free_device(c, other, segments / 2 + 65536);
+      check(jsh_observation_run_device(c, &m, &p, &nu, 1, &P, (void*)c->stream, &img) == JSH_OK, "render");
+      check(last_single == 0, "with segments");
+    }
+    device_limit = (size_t)-1;
+    jsh_ctx_destroy(c);
+  }
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   if (!strcmp(what, "error")) error_path();
   else if (!strcmp(what, "statistics")) statistics();
+  else if (!strcmp(what, "memory")) short_memory();
   else return 2;
   return failed;
 }

@@ -32,3 +32,7 @@ def test_failed_launch_keeps_the_workspace_in_use(fake):
 
 def test_last_stats_survive_other_calls(fake):
     run(fake, "statistics")
+
+
+def test_segments_by_the_memory_there_is(fake):
+    run(fake, "memory")
