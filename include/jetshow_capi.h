@@ -575,7 +575,7 @@ typedef struct jsh_tuning {
 /* Time the persistent schedule over a grid of kernel builds (default and
  * register-capped), block sizes, CTAs per SM, refill thresholds and serial
  * or overlapped passes on this request and store the fastest in the
- * context; later requests with block_size == 0 use it (the overlap choice
+ * context (its present shape unless another one is faster in turns); later requests with block_size == 0 use it (the overlap choice
  * holds unless a request's flags force one). */
 int jsh_autotune(jsh_ctx* ctx, const jsh_model_desc* model,
                  const jsh_plane_desc* plane, const double* nu_hz,
