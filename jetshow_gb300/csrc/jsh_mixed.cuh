@@ -263,11 +263,16 @@ static __device__ __noinline__ void segment_of_hit(const JshHit& H, int s, JshSe
   *q = segment32(mk(p[0], p[1], p[2]), mk(p[3], p[4], p[5]));
 }
 template <bool ANY>
-__device__ __forceinline__ JshSeg32 segment_of(const JshRequest& R, uint32_t h, int s) {
-  if (!ANY || R.seg32) return R.seg32[(uint64_t)h * JSH_MAX_SEG + s];
-  JshSeg32 q;
-  segment_of_hit(R.hits[h], s, &q);
-  return q;
+__device__ __forceinline__ std::conditional_t<ANY, JshSeg32, const JshSeg32&> segment_of(const JshRequest& R, uint32_t h,
+                                                                                         int s) {
+  if constexpr (ANY) {
+    JshSeg32 q;
+    if (R.seg32) return R.seg32[(uint64_t)h * JSH_MAX_SEG + s];
+    segment_of_hit(R.hits[h], s, &q);
+    return q;
+  } else {
+    return R.seg32[(uint64_t)h * JSH_MAX_SEG + s];
+  }
 }
 
 __device__ __forceinline__ void start_segment(Lane& L, DF px, DF py, DF pz, DF len) {
@@ -292,7 +297,7 @@ __device__ __forceinline__ double tau_total(const Lane& L) {
 
 template <int PASS>
 __device__ __forceinline__ void begin_tau_segment(Lane& L, const JshRequest& R, const JshMixed& X) {
-  const JshSeg32 S = segment_of<PASS == PASS_BOTH>(R, L.h, L.seg);
+  const JshSeg32& S = segment_of<PASS == PASS_BOTH>(R, L.h, L.seg);
   start_segment(L, DF{S.in[0], S.in[1]}, DF{S.in[2], S.in[3]}, DF{S.in[4], S.in[5]}, DF{S.len[0], S.len[1]});
   const float len = L.length.hi + L.length.lo;
   if (L.seg == 0) {
@@ -347,7 +352,7 @@ __device__ __forceinline__ void begin_iquv_segment(Lane& L, const JshRequest& R)
     start_segment(L, df_of(ox * INV_PC), df_of(oy * INV_PC), df_of(oz * INV_PC),
                   df_of(seg_len_cm(H, s, ox, oy, oz) * INV_PC));
   } else {
-    const JshSeg32 S = segment_of<PASS == PASS_BOTH>(R, L.h, s);
+    const JshSeg32& S = segment_of<PASS == PASS_BOTH>(R, L.h, s);
     start_segment(L, DF{S.out[0], S.out[1]}, DF{S.out[2], S.out[3]}, DF{S.out[4], S.out[5]}, DF{S.len[0], S.len[1]});
   }
   L.dt = (L.length.hi + L.length.lo) / L.first_div;

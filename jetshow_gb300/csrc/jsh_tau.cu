@@ -36,7 +36,7 @@ __global__ void __launch_bounds__(256) rank_cost_kernel(const JshRequest* __rest
     const float wk[4] = {0.173927423f, 0.326072577f, 0.326072577f, 0.173927423f};
     float tau = 0.f;
     for (int s = 0; s < H.nseg && s < 2; ++s) {
-      const JshSeg32 S = segment_of<ANY>(R, h, s);
+      const JshSeg32& S = segment_of<ANY>(R, h, s);
       const F3 a = f3(S.in[0], S.in[2], S.in[4]), b = f3(S.out[0], S.out[2], S.out[4]);
       const F3 d = b - a;
       float acc = 0.f;
