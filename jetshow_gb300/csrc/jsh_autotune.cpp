@@ -107,8 +107,8 @@ extern "C" int jsh_autotune(jsh_ctx* ctx, const jsh_model_desc* model, const jsh
 
   // the kernels that this request runs (the render above has checked it)
   const bool full = p.output == JSH_OUT_FULL, mixed = p.precision == JSH_PREC_MIXED;
+  JshRequest req;
   if (mixed) {
-    JshRequest req;
     uint64_t npix = 0;
     std::vector<JshFreqConst> fc((size_t)n_nu);
     st = jsh_prepare_request(ctx, model, plane, &p, n_nu, &req, &npix);
@@ -116,8 +116,9 @@ extern "C" int jsh_autotune(jsh_ctx* ctx, const jsh_model_desc* model, const jsh
     if (st) return st;
     shape.fused = jsh_fused_family(req.mix, p.flags) ? 1 : 0;
   }
+  auto capped_law = [&](int bs) { return mixed && jsh_capped_law(req.mix, shape.single != 0, bs); };
   auto occupancy = [&](int bs, bool cp) {
-    shape.compact = cp ? 1 : 0;
+    shape.compact = cp || capped_law(bs) ? 1 : 0;
     return jsh_persistent_occupancy(p.precision, full, bs, shape, items, ctx->num_sms);
   };
   // the register-capped builds: the mixed every-law and single-kernel ones
@@ -126,7 +127,7 @@ extern "C" int jsh_autotune(jsh_ctx* ctx, const jsh_model_desc* model, const jsh
     if (cp && !capped) continue;
     for (int bs : {64, 96, 128, 192, 256}) {
       const int occ = occupancy(bs, cp);
-      if (occ < 1) continue;
+      if (occ < 1 || (cp && capped_law(bs))) continue;
       std::vector<int> per_sm = {occ};
       if (occ > 1) per_sm.push_back(occ - 1);
       if (occ > 2) per_sm.push_back(1);

@@ -444,6 +444,7 @@ int enqueue_single(jsh_ctx* ctx, const jsh_model_desc* model, const jsh_plane_de
   shape.marks = nullptr;
   shape.mix = &req.mix;
   if (params->precision == JSH_PREC_MIXED && !req.seg32) shape.single = 1;
+  if (params->precision == JSH_PREC_MIXED && jsh_capped_law(req.mix, shape.single != 0, shape.block_size)) shape.compact = 1;
   const bool overlap = jsh_overlap_passes(params, shape, npix * (uint64_t)n_nu);
   if (overlap && shape.overlap_key <= 0) shape.overlap_key = JSH_OVERLAP_KEY;
   shape.side = overlap ? ctx->side : nullptr;

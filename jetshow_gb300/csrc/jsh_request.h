@@ -124,6 +124,15 @@ static inline bool jsh_fused_family(const JshMixed& X, uint32_t flags) {
   return X.helical_log && X.normal_range && !(flags & JSH_FLAG_GENERAL_KERNELS);
 }
 
+// Whether a request runs the register-capped every-law IQUV build unasked: its
+// lookups wait for loads, which 12 warps an SM hide better than 8 to 10 (512^2
+// full Stokes of a 200 000 point grid, 128 threads: 39.6 ms, uncapped 51.1; 64
+// threads 40.0 and 50.8).  The analytic laws gain nothing (a sheath flow at 512^2 3.12
+// and 3.13 ms) or lose (the log-domain family there 1.25 and 1.15).
+static inline bool jsh_capped_law(const JshMixed& X, bool single, int block_size) {
+  return X.sim_shared && !single && block_size <= 128;
+}
+
 struct JshRequest {
   JshModel model;
   JshMixed mix;
