@@ -210,8 +210,9 @@ constexpr int kTauWords = 17;  // the 15 nodes of a panel, odd
 // The I/IQUV kernels' files are compiled twice: as is, and by the _ft.cu files with
 // JSH_FARADAY_THICK_BUILD 1 for requests that ask for the Faraday-thick mode
 // (JSH_FLAG_FARADAY_THICK).  The mode's bookkeeping in the step costs the
-// other requests ~18 % of the IQUV kernel even where it never engages, so
-// the default kernels are built without it.
+// other requests 15 to 33 % of the IQUV kernel even where it never engages
+// (128x128: 75 -> 86 us; 512x1024 x 4: 1.15 -> 1.53 ms), so the default kernels
+// are built without it.
 #ifndef JSH_FARADAY_THICK_BUILD
 #define JSH_FARADAY_THICK_BUILD 0
 #endif

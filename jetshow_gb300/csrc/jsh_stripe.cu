@@ -15,8 +15,9 @@
 // the lanes; their increments are then added in the order of the steps (the
 // sums round as the serial steps do).  A ray that misses keeps tau = 0.  With a thread
 // per pixel the 300 serial evaluations of FP64 set the time: 6.91 ms for the
-// 1 000 pixels of a 2 000-column stripe on 8 CTAs, 0.79 ms with a warp per
-// pixel (0.29 of it the plane's recurrence); 10 000 pixels 8.8 -> 6.6 ms.
+// 1 000 pixels of a 2 000-column stripe on 8 CTAs, 0.39 ms with a warp per
+// pixel (and the plane's recurrence on the host); 10 000 pixels 8.8 -> 5.1 ms,
+// whose 20 000 columns keep the recurrence on the device.
 #include <cuda_runtime.h>
 #include <float.h>
 
